@@ -16,6 +16,7 @@
 #include "../../include/qserve_b200.h"
 #include "common.cuh"
 #include "hybrid_common.cuh"
+#include "hybrid_conv.cuh"
 #include "launch.h"
 
 namespace qs {
@@ -42,6 +43,39 @@ __global__ void embed_pair_kernel(float* __restrict__ out, const int* __restrict
   for (int i = threadIdx.x; i < W; i += blockDim.x) {
     const float v = ldf(e + i) * scale + (b ? ldf(b + i) : 0.f);
     for (int c = 0; c < copies; ++c) out[((size_t)t * copies + c) * W + i] = v;  // every residual stream starts from the embedding
+  }
+}
+// the same four numbers at a time (W a multiple of 4, every base on its 4-element boundary), two words in flight per thread.  6758 rows of 2048: 37.5 ->
+// 19.6 us; 64 rows: 12.7 -> 3 us (a thread's sixteen dependent trips had become one)
+template <typename ST>
+__global__ void __launch_bounds__(256) embed_pair_vec_kernel(float* __restrict__ out, const int* __restrict__ tokens, const int* __restrict__ prev,
+                                                             const ST* __restrict__ table, const ST* __restrict__ pair, int W, int buckets,
+                                                             long long mul_prev, long long mul_cur, float scale, int copies) {
+  const int t = blockIdx.x;
+  const long long tok = tokens[t];
+  const ST* e = table + tok * W;
+  const ST* b = nullptr;
+  if (pair != nullptr) {
+    const long long p = prev[t];
+    const long long row = p < 0 ? buckets : (p * mul_prev + tok * mul_cur) % buckets;
+    b = pair + row * W;
+  }
+  const int step = blockDim.x * 4;
+  for (int i = threadIdx.x * 4; i < W; i += 2 * step) {
+    const bool two = i + step < W;
+    float4 x[2], y[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    x[0] = ld4(e + i);
+    if (b != nullptr) y[0] = ld4(b + i);
+    if (two) {
+      x[1] = ld4(e + i + step);
+      if (b != nullptr) y[1] = ld4(b + i + step);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q == 1 && !two) break;
+      const float4 v = make_float4(x[q].x * scale + y[q].x, x[q].y * scale + y[q].y, x[q].z * scale + y[q].z, x[q].w * scale + y[q].w);
+      for (int c = 0; c < copies; ++c) st4(out + ((size_t)t * copies + c) * W + i + q * step, v);
+    }
   }
 }
 
@@ -192,6 +226,52 @@ __global__ void rope_append_kernel(ST* __restrict__ proj, long long stride, cons
   const ST* vs = row + (size_t)(H + G) * maps * D + (size_t)g * Dv;
   ST* vd = vpool + (cell * G + g) * (size_t)Dv;
   for (int i = threadIdx.x; i < Dv; i += blockDim.x) vd[i] = vs[i];
+}
+
+// bfloat16 rows 16 bytes at a time, one block per token: the token's sines and cosines are formed once (in shared memory) for all its heads and maps.
+// (One block per (token, head) formed them again for every head and moved 2 bytes per access: 6758 tokens of 16 + 4 heads, 2 maps, 88 us; now 21.)
+__global__ void __launch_bounds__(256) rope_append_vec_kernel(__nv_bfloat16* __restrict__ proj, long long stride, const int* __restrict__ tok_slot,
+                                                              const int* __restrict__ tok_pos, const int* __restrict__ block_table, int max_blocks,
+                                                              __nv_bfloat16* __restrict__ kpool, __nv_bfloat16* __restrict__ vpool,
+                                                              const float* __restrict__ inv_freq, float amp, int H, int G, int maps, int D, int Dv,
+                                                              int rot_dims, int page) {
+  extern __shared__ float cs[];  // cos [rot_dims / 2] | sin [rot_dims / 2], times the amplitude
+  const int t = blockIdx.x, pos = tok_pos[t], half = rot_dims >> 1;
+  for (int p = threadIdx.x; p < half; p += blockDim.x) {
+    float s, c;
+    sincosf((float)pos * inv_freq[p], &s, &c);
+    cs[p] = c * amp;
+    cs[half + p] = s * amp;
+  }
+  const int pg = block_table[(size_t)tok_slot[t] * max_blocks + pos / page];
+  const size_t cell = (size_t)pg * page + (pos % page);
+  __nv_bfloat16* row = proj + (size_t)t * stride;
+  auto rotate = [&](uint4 w, int p0) {  // four pairs from pair p0 on
+    uint32_t* x = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float x0 = __uint_as_float(x[q] << 16), x1 = __uint_as_float(x[q] & 0xffff0000u), c = cs[p0 + q], s = cs[half + p0 + q];
+      x[q] = pack_bf16(x0 * c - x1 * s, x1 * c + x0 * s);
+    }
+    return w;
+  };
+  __syncthreads();
+  const int rv = rot_dims >> 3, dv = D >> 3, nq = H * maps * rv, nk = G * maps * dv, nv = G * (Dv >> 3);
+  for (int i = threadIdx.x; i < nq + nk + nv; i += blockDim.x) {
+    if (i < nq) {  // queries: only the rotated entries change
+      const int hm = i / rv, j = i - hm * rv;
+      uint4* a = reinterpret_cast<uint4*>(row + (size_t)hm * D) + j;
+      *a = rotate(*a, j * 4);
+    } else if (i < nq + nk) {
+      const int k = i - nq, gm = k / dv, j = k - gm * dv;
+      uint4 w = reinterpret_cast<const uint4*>(row + (size_t)(H * maps + gm) * D)[j];
+      if (j < rv) w = rotate(w, j * 4);
+      reinterpret_cast<uint4*>(kpool + (cell * G * maps + gm) * D)[j] = w;
+    } else {
+      const int k = i - nq - nk;
+      reinterpret_cast<uint4*>(vpool + cell * G * Dv)[k] = reinterpret_cast<const uint4*>(row + (size_t)(H + G) * maps * D)[k];
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
@@ -551,6 +631,25 @@ __global__ void multimap_combine_kernel(ST* __restrict__ out, long long out_stri
   for (int i = lane; i < Dv; i += 32) stf(dst + i, (maps == 2 ? a[i] - lambda * a[Dv + i] : a[i]) * r);
 }
 
+// ungated heads of 128 numbers, four per lane (6758 tokens x 16 heads x 2 maps: 32 -> 27 us)
+template <typename ST>
+__global__ void __launch_bounds__(128) multimap_combine128_kernel(ST* __restrict__ out, long long out_stride, const float* __restrict__ a_in,
+                                                                  const int* __restrict__ tok_list, int n_list, int H, int maps, float lambda,
+                                                                  float out_scale, float eps, int head_norm) {
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), i = (threadIdx.x & 31) * 4;
+  if (w >= n_list * H) return;
+  const int t = tok_list[w / H], h = w % H;
+  const float* a = a_in + ((size_t)t * H + h) * maps * 128 + i;
+  float4 x = ld4(a);
+  if (maps == 2) {
+    const float4 y = ld4(a + 128);
+    x = make_float4(x.x - lambda * y.x, x.y - lambda * y.y, x.z - lambda * y.z, x.w - lambda * y.w);
+  }
+  float r = out_scale;
+  if (head_norm) r = out_scale / sqrtf(warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w)) / 128.f + eps);
+  st4(out + (size_t)t * out_stride + h * 128 + i, make_float4(x.x * r, x.y * r, x.z * r, x.w * r));
+}
+
 // ---------------------------------------------------------------------------------------------------------------------------------
 // Single tokens on the tensor cores (bfloat16 storage).  The R = H / G query heads that share a key/value head are the rows of one m16n8k16
 // tile, so a key row is loaded once for the group and scored by the tensor cores instead of R warp reductions.  One block = (listed token,
@@ -865,6 +964,51 @@ __global__ void __launch_bounds__(kPrepThreads) delta_prepare_kernel(
   }
 }
 
+// The same for heads of up to 128 channels, four channels per lane: a warp owns one unit and walks a run of neighbouring tokens with the unit's taps
+// and the window of inputs in registers, the unit length is a warp sum, and nothing is loaded twice.  (One block per (token, unit) read every
+// input `taps` times with 2-byte accesses and met in shared memory for every unit: 6758 tokens, 24 units of 128, 253 us; now 56, floor 22.)
+template <typename ST, int TAPS>
+__global__ void __launch_bounds__(128) delta_prepare_walk_kernel(float* __restrict__ prep, const ST* __restrict__ proj, long long stride,
+                                                                 const float* __restrict__ conv_w, float* __restrict__ conv_state,
+                                                                 const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                                                                 const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
+                                                                 const int* __restrict__ entry_start, const int* __restrict__ entry_slot, int T, int H, int G,
+                                                                 int D, int Dv, int taps, float unit_eps, int run) {
+  const int C = 2 * G * D + H * Dv, P = C + 2 * H;
+  const int u = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
+  if (u < 2 * G + H) {
+    const bool qk = u < 2 * G;
+    const int n = qk ? D : Dv, i = lane * 4;
+    const bool in = i < n;
+    const int c = (qk ? u * D : 2 * G * D + (u - 2 * G) * Dv) + (in ? i : 0);  // idle lanes repeat the unit's first channels and store nothing
+    auto walk = conv_walk<ST, 4, TAPS>(conv_w, nullptr, nullptr, taps, c);
+    const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, C, taps};
+    const float q_scale = 1.f / sqrtf((float)D);
+    conv_rows<ST, 4>(walk, proj, stride, nullptr, tab, t0, t1, c, false, [&](int t, float(&y)[4]) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) y[v] = silu_f(y[v]);
+      float r = 1.f;
+      if (qk) {  // warp-uniform
+        const float ss = warp_sum(in ? (y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]) : 0.f);
+        r = 1.f / sqrtf(ss + unit_eps);
+        if (u < G) r *= q_scale;
+      }
+      if (in) st4(prep + (size_t)t * P + c, make_float4(y[0] * r, y[1] * r, y[2] * r, y[3] * r));
+    });
+  }
+  if (blockIdx.y == 0)
+    for (int k = threadIdx.x; k < (t1 - t0) * H; k += 128) {
+      const int t = t0 + k / H, hh = k - k / H * H;
+      const ST* row = proj + (size_t)t * stride + C + H * Dv;
+      const float b = ldf(row + hh), a = ldf(row + H + hh) + dt_bias[hh];
+      const float sp = a > 20.f ? a : log1pf(expf(a));
+      float* o = prep + (size_t)t * P + C + hh;
+      o[0] = 1.f / (1.f + expf(-b));
+      o[H] = expf(-expf(a_log[hh]) * sp);
+    }
+}
+
 // step 1b: the sequence's convolution state after the portion = its last taps-1 inputs (older ones shift out)
 template <typename ST>
 __global__ void delta_conv_state_kernel(float* __restrict__ conv_state, const ST* __restrict__ proj, long long stride,
@@ -1060,6 +1204,19 @@ __global__ void delta_gate_out_kernel(ST* __restrict__ out, long long out_stride
   ST* dst = out + (size_t)t * out_stride + (size_t)h * Dv;
   for (int i = lane; i < Dv; i += 32) stf(dst + i, o[i] * r * norm_w[i] * silu_f(ldf(gate + i)));
 }
+// heads of 128 numbers, four per lane: o, the gate and the gain are in flight together (6758 tokens x 16 heads: 53 us in 2-byte accesses, now 27, floor 17)
+template <typename ST>
+__global__ void __launch_bounds__(128) delta_gate_out128_kernel(ST* __restrict__ out, long long out_stride, const float* __restrict__ o_raw,
+                                                                const ST* __restrict__ gate, long long stride, const float* __restrict__ norm_w, int T, int H,
+                                                                float eps) {
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), i = (threadIdx.x & 31) * 4;
+  if (w >= T * H) return;
+  const int t = w / H, h = w - t * H;
+  const float4 o = ld4(o_raw + (size_t)w * 128 + i), g = ld4(gate + (size_t)t * stride + h * 128 + i), n = ld4(norm_w + i);
+  const float r = 1.f / sqrtf(warp_sum((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w)) / 128.f + eps);
+  st4(out + (size_t)t * out_stride + h * 128 + i, make_float4(o.x * r * n.x * silu_f(g.x), o.y * r * n.y * silu_f(g.y), o.z * r * n.z * silu_f(g.z),
+                                                              o.w * r * n.w * silu_f(g.w)));
+}
 
 inline AttnExtra attn_extra(const qs_attn_extra* e) {
   return e != nullptr ? AttnExtra{e->keep_first, e->slopes, e->gate, (long long)e->gate_stride, e->gate_wide, e->softcap}
@@ -1152,8 +1309,17 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
                  const int* tok_pos, const int* entry_start, const int* entry_len, const int* entry_slot, const int* entry_pos0, int T, int E,
                  int H, int G, int D, int Dv, int taps, float unit_eps, float eps, cudaStream_t s) {
   const int C = 2 * G * D + H * Dv;
-  delta_prepare_kernel<ST><<<dim3(T, 2 * G + H), kPrepThreads, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry,
-                                                                      tok_pos, entry_start, entry_slot, H, G, D, Dv, taps, unit_eps);
+  auto al = [](const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+  if (D % 4 == 0 && D <= 128 && Dv % 4 == 0 && Dv <= 128 && stride % 4 == 0 && (C + 2 * H) % 4 == 0 && al(proj, 4 * sizeof(ST)) && al(prep, 16)) {
+    const int run = conv_run(T);
+    auto walk = taps == 4 ? delta_prepare_walk_kernel<ST, 4> : taps == 3 ? delta_prepare_walk_kernel<ST, 3> : taps == 2 ? delta_prepare_walk_kernel<ST, 2>
+                                                                                                         : delta_prepare_walk_kernel<ST, 0>;
+    walk<<<dim3((T + run - 1) / run, (2 * G + H + 3) / 4), 128, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry, tok_pos,
+                                                                        entry_start, entry_slot, T, H, G, D, Dv, taps, unit_eps, run);
+  } else {
+    delta_prepare_kernel<ST><<<dim3(T, 2 * G + H), kPrepThreads, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry,
+                                                                        tok_pos, entry_start, entry_slot, H, G, D, Dv, taps, unit_eps);
+  }
   if (taps > 1)
     delta_conv_state_kernel<ST><<<dim3((C + 127) / 128, E), 128, 0, s>>>(conv_state, (const ST*)proj, stride, entry_start, entry_len, entry_slot,
                                                                           entry_pos0, C, taps);
@@ -1177,8 +1343,11 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
   else if (D <= 128) { if (Dv >= 64) QS_SCAN(128, 8, 16, 2); else QS_SCAN(128, 4, 16, 1); }
   else QS_SCAN(256, 8, 8, 1);
 #undef QS_SCAN
-  const int warps = T * H;
-  delta_gate_out_kernel<ST><<<(warps + 3) / 4, 128, 0, s>>>((ST*)out, out_stride, o_raw, (const ST*)proj, stride, norm_w, T, H, G, D, Dv, eps);
+  const int warps = T * H, gate_at = 2 * G * D + H * Dv;
+  if (Dv == 128 && stride % 4 == 0 && gate_at % 4 == 0 && out_stride % 4 == 0 && al(proj, 4 * sizeof(ST)) && al(out, 4 * sizeof(ST)) && al(o_raw, 16) && al(norm_w, 16))
+    delta_gate_out128_kernel<ST><<<(warps + 3) / 4, 128, 0, s>>>((ST*)out, out_stride, o_raw, (const ST*)proj + gate_at, stride, norm_w, T, H, eps);
+  else
+    delta_gate_out_kernel<ST><<<(warps + 3) / 4, 128, 0, s>>>((ST*)out, out_stride, o_raw, (const ST*)proj, stride, norm_w, T, H, G, D, Dv, eps);
   return check_cuda(cudaGetLastError(), "hyb_gated_delta");
 }
 
@@ -1202,6 +1371,16 @@ int qs_hyb_embed(float* out, const int32_t* tokens, const int32_t* prev, const v
   QS_REQUIRE(pair_table == nullptr || (prev != nullptr && buckets > 0), "hyb_embed: the pair table needs previous tokens and buckets > 0");
   if (tokens_n == 0) return qs::QS_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  const uintptr_t word = dtype == QS_DTYPE_BF16 ? 7 : 15;  // four elements of the tables
+  if (width % 4 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(pair_table)) & word) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    const int threads = width > 512 ? 256 : 64;
+    QS_DT(dtype,
+          (embed_pair_vec_kernel<__nv_bfloat16><<<tokens_n, threads, 0, s>>>(out, tokens, prev, (const __nv_bfloat16*)table, (const __nv_bfloat16*)pair_table,
+                                                                             width, buckets, mul_prev, mul_cur, scale, copies)),
+          (embed_pair_vec_kernel<float><<<tokens_n, threads, 0, s>>>(out, tokens, prev, (const float*)table, (const float*)pair_table, width, buckets,
+                                                                     mul_prev, mul_cur, scale, copies)));
+    return check_cuda(cudaGetLastError(), "hyb_embed");
+  }
   QS_DT(dtype,
         (embed_pair_kernel<__nv_bfloat16><<<tokens_n, 128, 0, s>>>(out, tokens, prev, (const __nv_bfloat16*)table, (const __nv_bfloat16*)pair_table,
                                                                     width, buckets, mul_prev, mul_cur, scale, copies)),
@@ -1263,6 +1442,13 @@ int qs_hyb_rope_append(void* proj, int64_t stride, const int32_t* tok_slot, cons
   QS_REQUIRE(rot_dims % 2 == 0 && rot_dims <= dim && heads % kv_heads == 0 && page_size > 0, "hyb_rope_append: bad head geometry");
   if (tokens_n == 0) return qs::QS_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (dtype == QS_DTYPE_BF16 && dim % 8 == 0 && vdim % 8 == 0 && rot_dims % 8 == 0 && rot_dims <= 4096 && stride % 8 == 0 && al16(proj) && al16(kpool) && al16(vpool)) {
+    rope_append_vec_kernel<<<tokens_n, 256, rot_dims * sizeof(float), s>>>((__nv_bfloat16*)proj, stride, tok_slot, tok_pos, block_table, max_blocks,
+                                                                           (__nv_bfloat16*)kpool, (__nv_bfloat16*)vpool, inv_freq, amplitude, heads, kv_heads,
+                                                                           maps, dim, vdim, rot_dims, page_size);
+    return check_cuda(cudaGetLastError(), "hyb_rope_append");
+  }
   dim3 grid(tokens_n, heads + kv_heads);
   QS_DT(dtype,
         (rope_append_kernel<__nv_bfloat16><<<grid, 64, 0, s>>>((__nv_bfloat16*)proj, stride, tok_slot, tok_pos, block_table, max_blocks,
@@ -1335,7 +1521,11 @@ int qs_hyb_attention_fast(void* out, int64_t out_stride, const void* q, int64_t 
 #undef QS_TILES
     if (rc) return rc;
     const int warps = n_long * heads;
-    multimap_combine_kernel<__nv_bfloat16><<<(warps + 3) / 4, 128, 0, s>>>((__nv_bfloat16*)out, out_stride, scratch, long_tokens, n_long, heads, maps, vdim,
+    if (vdim == 128 && ex.gate == nullptr && out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0)
+      multimap_combine128_kernel<__nv_bfloat16><<<(warps + 3) / 4, 128, 0, s>>>((__nv_bfloat16*)out, out_stride, scratch, long_tokens, n_long, heads, maps,
+                                                                               lambda, out_scale, eps, head_norm);
+    else
+      multimap_combine_kernel<__nv_bfloat16><<<(warps + 3) / 4, 128, 0, s>>>((__nv_bfloat16*)out, out_stride, scratch, long_tokens, n_long, heads, maps, vdim,
                                                                           lambda, out_scale, eps, head_norm, (const __nv_bfloat16*)ex.gate, ex.gate_stride,
                                                                           ex.gate_wide);
   }

@@ -17,6 +17,7 @@
 #include "../../include/qserve_b200.h"
 #include "common.cuh"
 #include "hybrid_common.cuh"
+#include "hybrid_conv.cuh"
 #include "launch.h"
 
 namespace qs {
@@ -25,119 +26,6 @@ namespace {
 using namespace hyb;
 
 constexpr int kMaxTaps = 17;
-
-// The convolution's inputs of one token, channels c .. c + V - 1: `back` tokens before row t.  Inputs ahead of the portion come from the
-// convolution state, inputs ahead of the sequence are zero; `in_bias` (may be null) belongs to the inputs.
-template <typename ST, int V>
-__device__ __forceinline__ void conv_input(float (&x)[V], const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias,
-                                           const float* st, int t, int local, int pos, int back, int taps, int C, int c) {
-#pragma unroll
-  for (int v = 0; v < V; ++v) x[v] = 0.f;
-  if (pos - back < 0) return;
-  if (local - back >= 0) {
-    const ST* p = in + (size_t)(t - back) * stride + c;
-    if constexpr (V == 4) {
-      const float4 q = ld4(p);
-      x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
-    } else {
-      x[0] = ldf(p);
-    }
-    if (in_bias != nullptr) {
-#pragma unroll
-      for (int v = 0; v < V; ++v) x[v] += in_bias[c + v];
-    }
-  } else {
-    const float* p = st + (size_t)(taps - 1 + local - back) * C + c;
-#pragma unroll
-    for (int v = 0; v < V; ++v) x[v] = p[v];
-  }
-}
-
-// Convolution of row t at channels c .. c + V - 1 (bias included).  In a step of single tokens the thread is the only reader of its channels'
-// state and shifts the token's input in (`shift`); other steps do that in conv_state_kernel afterwards.
-template <typename ST, int V>
-__device__ __forceinline__ void conv_row(float (&y)[V], const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias, float* st,
-                                         const float* __restrict__ w, const float* __restrict__ b, int t, int local, int pos, int taps, int C, int c,
-                                         bool shift) {
-#pragma unroll
-  for (int v = 0; v < V; ++v) y[v] = b != nullptr ? b[c + v] : 0.f;
-  for (int j = 0; j < taps; ++j) {
-    float x[V];
-    conv_input<ST, V>(x, in, stride, in_bias, st, t, local, pos, taps - 1 - j, taps, C, c);
-#pragma unroll
-    for (int v = 0; v < V; ++v) y[v] += w[(size_t)(c + v) * taps + j] * x[v];
-    if (shift && j > 0) {  // input j is slot j - 1 of the next token's state; slot j is read before slot j is written
-#pragma unroll
-      for (int v = 0; v < V; ++v) st[(size_t)(j - 1) * C + c + v] = x[v];
-    }
-  }
-}
-
-// The same for a walk over neighbouring rows, `TAPS` known: the channels' weights and the window of inputs stay in registers.
-template <typename ST, int V, int TAPS>
-struct ConvWalk {
-  float w[V][TAPS], b[V], xb[V], x[TAPS][V];
-  int entry = -1;
-
-  __device__ __forceinline__ ConvWalk(const float* __restrict__ cw, const float* __restrict__ cb, const float* __restrict__ in_bias, int c) {
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      b[v] = cb != nullptr ? cb[c + v] : 0.f;
-      xb[v] = in_bias != nullptr ? in_bias[c + v] : 0.f;
-#pragma unroll
-      for (int j = 0; j < TAPS; ++j) w[v][j] = cw[(size_t)(c + v) * TAPS + j];
-    }
-  }
-  __device__ __forceinline__ void row(float (&y)[V], const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias, float* st, int t, int e,
-                                      int local, int pos, int C, int c, bool shift) {
-    if (e != entry) {
-#pragma unroll
-      for (int j = 0; j < TAPS - 1; ++j) conv_input<ST, V>(x[j], in, stride, in_bias, st, t, local, pos, TAPS - 1 - j, TAPS, C, c);
-      entry = e;
-    } else {
-#pragma unroll
-      for (int j = 0; j < TAPS - 1; ++j)
-#pragma unroll
-        for (int v = 0; v < V; ++v) x[j][v] = x[j + 1][v];
-    }
-    const ST* p = in + (size_t)t * stride + c;
-    if constexpr (V == 4) {
-      const float4 q = ld4(p);
-      x[TAPS - 1][0] = q.x; x[TAPS - 1][1] = q.y; x[TAPS - 1][2] = q.z; x[TAPS - 1][3] = q.w;
-    } else {
-      x[TAPS - 1][0] = ldf(p);
-    }
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      x[TAPS - 1][v] += xb[v];
-      y[v] = b[v];
-#pragma unroll
-      for (int j = 0; j < TAPS; ++j) y[v] += w[v][j] * x[j][v];
-    }
-    if (shift) {
-#pragma unroll
-      for (int j = 1; j < TAPS; ++j)
-#pragma unroll
-        for (int v = 0; v < V; ++v) st[(size_t)(j - 1) * C + c + v] = x[j][v];
-    }
-  }
-};
-// any number of taps
-template <typename ST, int V>
-struct ConvWalk<ST, V, 0> {
-  const float *cw, *cb;
-  int taps;
-  __device__ __forceinline__ ConvWalk(const float* w, const float* b, int n) : cw(w), cb(b), taps(n) {}
-  __device__ __forceinline__ void row(float (&y)[V], const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias, float* st, int t, int,
-                                      int local, int pos, int C, int c, bool shift) {
-    conv_row<ST, V>(y, in, stride, in_bias, st, cw, cb, t, local, pos, taps, C, c, shift);
-  }
-};
-template <typename ST, int V, int TAPS>
-__device__ __forceinline__ ConvWalk<ST, V, TAPS> conv_walk(const float* w, const float* b, const float* in_bias, int taps, int c) {
-  if constexpr (TAPS == 0) return ConvWalk<ST, V, 0>(w, b, taps);
-  else return ConvWalk<ST, V, TAPS>(w, b, in_bias, c);
-}
 
 // silu as the storage type needs it: the special-function unit's exponential and division for bfloat16 results, the exact ones for fp32
 template <typename ST> __device__ __forceinline__ float silu_as(float z) { return sizeof(ST) == 2 ? z * fast_sigmoid(z) : silu_f(z); }
@@ -180,25 +68,25 @@ __global__ void __launch_bounds__(128) ssd_prepare_kernel(float* __restrict__ pr
   const int c = (blockIdx.y * 128 + threadIdx.x) * V;
   const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
   auto walk = conv_walk<ST, V, TAPS>(conv_w, conv_b, nullptr, taps, min(c, C - V));
-  for (int t = t0; t < t1; ++t) {
-    const int e = tok_entry[t];
-    float* o = prep + (size_t)t * P;
-    if (c < C) {
-      float y[V];
-      walk.row(y, proj + inner, stride, nullptr, conv_state + (size_t)entry_slot[e] * (taps - 1) * C, t, e, t - entry_start[e], tok_pos[t], C, c, shift != 0);
+  if (c < C) {
+    const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, C, taps};
+    conv_rows<ST, V>(walk, proj + inner, stride, nullptr, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
+      float* o = prep + (size_t)t * P;
 #pragma unroll
       for (int v = 0; v < V; ++v) y[v] = silu_as<ST>(y[v]);
       if constexpr (V == 4) st4(o + c, make_float4(y[0], y[1], y[2], y[3]));
       else o[c] = y[0];
-    }
-    if (blockIdx.y == 0)
-      for (int h = threadIdx.x; h < H; h += 128) {
-        const float z = ldf(proj + (size_t)t * stride + inner + C + h) + dt_bias[h];
-        const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
-        o[C + h] = dt;
-        o[C + H + h] = expf(-expf(a_log[h]) * dt);
-      }
+    });
   }
+  if (blockIdx.y == gridDim.y - 1)
+    for (int i = threadIdx.x; i < (t1 - t0) * H; i += 128) {
+      const int t = t0 + i / H, h = i - i / H * H;
+      const float z = ldf(proj + (size_t)t * stride + inner + C + h) + dt_bias[h];
+      const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+      float* o = prep + (size_t)t * P + C + h;
+      o[0] = dt;
+      o[H] = expf(-expf(a_log[h]) * dt);
+    }
 }
 
 // state space, step 3: y <- y * silu(z), unit RMS in equal parts of the row, times norm_w and a constant.  One block per (token, part); the part
@@ -254,13 +142,11 @@ __global__ void __launch_bounds__(128) lru_conv_kernel(ST* __restrict__ u, const
   if (c >= W) return;
   const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
   auto walk = conv_walk<ST, V, TAPS>(conv_w, conv_b, x_bias, taps, c);
-  for (int t = t0; t < t1; ++t) {
-    const int e = tok_entry[t];
-    float y[V];
-    walk.row(y, proj + W, stride, x_bias, conv_state + (size_t)entry_slot[e] * (taps - 1) * W, t, e, t - entry_start[e], tok_pos[t], W, c, shift != 0);
+  const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, W, taps};
+  conv_rows<ST, V>(walk, proj + W, stride, x_bias, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
     if constexpr (V == 4) st4(u + (size_t)t * W + c, make_float4(y[0], y[1], y[2], y[3]));
     else stf(u + (size_t)t * W + c, y[0]);
-  }
+  });
 }
 
 // step 2 (between the kernels): gate logits z fp32 [blocks][T][2 W / blocks]: a block's r logits, then its i logits.
@@ -459,9 +345,6 @@ int launch_conv_state(float* conv_state, const ST* in, long long stride, const f
 }
 
 bool aligned(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
-
-// tokens a block of a convolution kernel walks: neighbours find each other's rows in the cache once there are blocks enough
-int conv_run(int T) { return T >= 2048 ? 16 : T >= 512 ? 4 : 1; }
 
 template <typename ST>
 int launch_state_space(void* out, long long out_stride, float* prep, float* o_raw, const void* proj_, long long stride, const float* conv_w,
