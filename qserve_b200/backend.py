@@ -13,6 +13,7 @@ from typing import Optional
 import torch
 
 from ._lib import check, lib
+from . import _bind  # after the library it links against
 
 _HALF = torch.float16
 
@@ -43,33 +44,19 @@ def _cuda(t: torch.Tensor, name: str) -> None:
     _require(t.is_cuda, f"{name} must be on CUDA")  # CHECK_DEVICE, fused_attention.cpp:22
 
 
-_workspaces: dict = {}
-_retired: list = []  # outgrown workspaces, kept alive for graphs captured with them
+def _index(device: torch.device) -> int:
+    return torch.cuda.current_device() if device.index is None else device.index
 
 
 def gemm_workspace(device: torch.device) -> torch.Tensor:
     """Zero-initialised once per device; afterwards owned by the library (self-cleaning split-K counters)."""
-    key = ("gemm", device.index)
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = torch.zeros(lib.qs_gemm_workspace_bytes(), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    return _bind.gemm_workspace(_index(device))
 
 
 def attention_workspace(device: torch.device, batch: int, num_heads: int, head_dim: int) -> torch.Tensor:
-    key = ("attn", device.index)
-    need = lib.qs_attention_workspace_bytes(batch, num_heads, head_dim)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        # a workspace that was handed out is never freed: a captured CUDA graph may still hold its address (the self-cleaning
-        # counters inside must not alias reused memory on replay)
-        if ws is not None:
-            _retired.append(ws)
-        with torch.cuda.device(device):
-            ws = torch.zeros(need, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    """Grown on demand; a work space that was handed out is never freed: a captured CUDA graph may still hold its address (the self-cleaning
+    counters inside must not alias reused memory on replay)."""
+    return _bind.attention_workspace(_index(device), batch, num_heads, head_dim)
 
 
 def set_pdl(enabled: bool) -> bool:
@@ -82,30 +69,12 @@ def set_pdl(enabled: bool) -> bool:
 # --------------------------------------------------------------------------------------------------
 
 
-def _gemm_common(in_feats, kernel, out_feats, k_div: int):
-    _cuda(in_feats, "in_feats"); _cuda(kernel, "kernel"); _cuda(out_feats, "out_feats")
-    _require(in_feats.dtype == torch.int8 and kernel.dtype == torch.int8, "in_feats and kernel must be int8")
-    _require(out_feats.dtype == _HALF, "out_feats must be float16")
-    _require(in_feats.is_contiguous() and kernel.is_contiguous() and out_feats.is_contiguous(), "GEMM operands must be contiguous")
-    M, K = in_feats.size(0), in_feats.size(1)  # gemm_cuda.cu:604-605
-    N = out_feats.size(-1)                     # gemm_cuda.cu:613
-    _require(out_feats.size(-2) == M, "out_feats rows must match in_feats rows")
-    _require(kernel.size(0) == N and kernel.size(1) * k_div == K, f"kernel shape {tuple(kernel.shape)} does not match N={N}, K={K}")
-    return M, N, K
-
-
 def w4a8_per_chn_gemm_forward_cuda(in_feats, kernel, wscales, ascales, w_szs, a_ssums, out_feats, _acc_out=None) -> None:
     """qserve_backend.qgemm_w4a8_per_chn.gemm_forward_cuda (w4a8_per_chn/gemm_cuda.cu:596-652, pybind.cpp:13-16).
 
     out_feats[M,N] (fp16, caller allocated) = (in_feats s8 [M,K] . kernel u4 [N,K/2]) * wscales[n] * ascales[m] - w_szs[n] * a_ssums[m].
     """
-    M, N, K = _gemm_common(in_feats, kernel, out_feats, 2)
-    if M == 0:
-        return
-    ws = gemm_workspace(in_feats.device)
-    _call(in_feats, lib.qs_w4a8_gemm_per_chn, in_feats.data_ptr(), kernel.data_ptr(), wscales.data_ptr(), ascales.data_ptr(), w_szs.data_ptr(),
-                                   a_ssums.data_ptr(), out_feats.data_ptr(), _acc_out.data_ptr() if _acc_out is not None else None,
-                                   M, N, K, ws.data_ptr(), ws.numel())
+    _bind.w4a8_per_chn(in_feats, kernel, wscales, ascales, w_szs, a_ssums, out_feats, _acc_out)
 
 
 def w4a8_per_group_gemm_forward_cuda(in_feats, kernel, zeros, scales_i8, wscales, ascales, out_feats, _acc_out=None) -> None:
@@ -113,26 +82,12 @@ def w4a8_per_group_gemm_forward_cuda(in_feats, kernel, zeros, scales_i8, wscales
 
     Argument order as called by w4a8_linear.py:123-131: (x, qweight, s2_zeros, s2_scales, s1_scales, input_scales, out).
     """
-    M, N, K = _gemm_common(in_feats, kernel, out_feats, 2)
-    _require(zeros.dtype == torch.int8 and scales_i8.dtype == torch.int8, "zeros and scales_i8 must be int8")
-    _require(tuple(zeros.shape) == (K // 128, N) and tuple(scales_i8.shape) == (K // 128, N), "level-2 params must be [K/128, N]")
-    if M == 0:
-        return
-    ws = gemm_workspace(in_feats.device)
-    _call(in_feats, lib.qs_w4a8_gemm_per_group, in_feats.data_ptr(), kernel.data_ptr(), zeros.data_ptr(), scales_i8.data_ptr(), wscales.data_ptr(),
-                                     ascales.data_ptr(), out_feats.data_ptr(), _acc_out.data_ptr() if _acc_out is not None else None,
-                                     M, N, K, ws.data_ptr(), ws.numel())
+    _bind.w4a8_per_group(in_feats, kernel, zeros, scales_i8, wscales, ascales, out_feats, _acc_out)
 
 
 def w8a8_gemm_forward_cuda(in_feats, kernel, wscales, ascales, out_feats, _acc_out=None) -> None:
     """qserve_backend.qgemm_w8a8.w8a8_gemm_forward_cuda (w8a8/w8a8_gemm_cuda.cu:532-577, pybind.cpp:13-17)."""
-    M, N, K = _gemm_common(in_feats, kernel, out_feats, 1)
-    _require(wscales.dtype == _HALF and ascales.dtype == _HALF, "wscales and ascales must be float16 (w8a8_linear.py:99-101 casts them)")
-    if M == 0:
-        return
-    ws = gemm_workspace(in_feats.device)
-    _call(in_feats, lib.qs_w8a8_gemm, in_feats.data_ptr(), kernel.data_ptr(), wscales.data_ptr(), ascales.data_ptr(), out_feats.data_ptr(),
-                           _acc_out.data_ptr() if _acc_out is not None else None, M, N, K, ws.data_ptr(), ws.numel())
+    _bind.w8a8(in_feats, kernel, wscales, ascales, out_feats, _acc_out)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -148,33 +103,8 @@ def single_query_attention(q, k, v, kv_pointers, length_per_sample_: Optional[to
 
     Returns a NEW tensor shaped like q (the reference returns torch::empty_like(q), :205).  Mutates the KV pages.
     """
-    for t, n in ((q, "q"), (k, "k"), (v, "v"), (kv_pointers, "kv_pointers")):
-        _cuda(t, n)
-    _require(q.dtype == _HALF and k.dtype == _HALF and v.dtype == _HALF, "single_query_attention: only float16 is supported (fused_attention.cpp:24-30)")
-    batch = kv_pointers.size(0)
-    nheads, nheads_kv, headdim = q.size(1), k.size(1), k.size(-1)
-    _require(k.stride(2) == 1 and k.stride(1) == headdim, "k must have stride(2) == 1 and stride(1) == head_dim")  # :179
-    _require(v.stride(2) == 1 and v.stride(1) == headdim, "v must have stride(2) == 1 and stride(1) == head_dim")  # :180
-    _require(q.stride(2) == 1 and q.stride(1) == headdim, "q must have stride(2) == 1 and stride(1) == head_dim")
-    _require(kv_pointers.is_contiguous() and kv_pointers.dtype == torch.int64, "kv_pointers must be contiguous int64")  # :182
-    lens_ptr = None
-    if length_per_sample_ is not None:
-        _cuda(length_per_sample_, "length_per_sample")
-        _require(tuple(length_per_sample_.shape) == (batch,), "length_per_sample must have shape (batch_size)")
-        _require(length_per_sample_.is_contiguous(), "length_per_sample must be contiguous")
-        _require(length_per_sample_.dtype == torch.int32, "length_per_sample must be int32")  # :189
-        lens_ptr = length_per_sample_.data_ptr()
-    if alibi_slopes_ is not None:  # accepted, validated and ignored, exactly like the reference (:192-199, :91)
-        _cuda(alibi_slopes_, "alibi_slopes")
-        _require(tuple(alibi_slopes_.shape) == (nheads,) and alibi_slopes_.dtype == torch.float32, "alibi_slopes must be float32 [nheads]")
-    out = torch.empty((q.size(0), nheads, headdim), dtype=q.dtype, device=q.device)
-    ws = attention_workspace(q.device, batch, nheads, headdim)
-    _call(q, lib.qs_single_query_attention, q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), kv_pointers.data_ptr(),
-                                        lens_ptr, out.data_ptr(), batch, nheads, nheads_kv, headdim, kv_pointers.size(-1), int(memory_max_seqlen),
-                                        int(tokens_per_block), int(size_per_token), int(timestep), int(rotary_embedding_dim), float(rotary_base),
-                                        int(bool(neox_rotary_style)), int(bool(int4_kv_cache)), int(bool(kv_cache_with_zeros)), ws.data_ptr(),
-                                        ws.numel())
-    return out
+    return _bind.single_query_attention(q, k, v, kv_pointers, length_per_sample_, alibi_slopes_, memory_max_seqlen, tokens_per_block, size_per_token, timestep,
+                                        rotary_embedding_dim, rotary_base, neox_rotary_style, int4_kv_cache, kv_cache_with_zeros)
 
 
 def apply_bias_rope_update_kv_cache(qkv, seq_lens, padding_offset, kv_pointers: Optional[torch.Tensor], head_num: int, kv_head_num: int,
@@ -265,22 +195,12 @@ def rms_norm(out, input, weight, epsilon: float, use_quant: bool = False) -> Non
 
 def rms_norm_general(out, input, weight, scaling, epsilon: float, use_per_token_quant: bool = False) -> None:
     """layernorm_ops.rms_norm_general (layernorm.cpp:52-54, layernorm_kernels.cu:427-464)."""
-    _cuda(input, "input"); _half_only(input, "rms_norm_general")
-    if _noop(input):
-        return
-    tokens, hidden = _rows(input)
-    _call(input, lib.qs_rms_norm_general, out.data_ptr(), input.data_ptr(), weight.data_ptr(), scaling.data_ptr(), float(epsilon),
-                                  int(bool(use_per_token_quant)), tokens, hidden)
+    _bind.rms_norm_general(out, input, weight, scaling, epsilon, use_per_token_quant)
 
 
 def rms_norm_general_fuse_sum(out, input, weight, input_sum, scaling, epsilon: float, use_per_token_quant: bool = False) -> None:
     """layernorm_ops.rms_norm_general_fuse_sum (layernorm.cpp:56-58, layernorm_kernels.cu:466-508)."""
-    _cuda(input, "input"); _half_only(input, "rms_norm_general_fuse_sum")
-    if _noop(input):
-        return
-    tokens, hidden = _rows(input)
-    _call(input, lib.qs_rms_norm_general_fuse_sum, out.data_ptr(), input.data_ptr(), weight.data_ptr(), input_sum.data_ptr(), scaling.data_ptr(),
-                                           float(epsilon), int(bool(use_per_token_quant)), tokens, hidden)
+    _bind.rms_norm_general_fuse_sum(out, input, weight, input_sum, scaling, epsilon, use_per_token_quant)
 
 
 def invoke_dequant_add_residual_rms_norm_quant(out, input, residual, gamma, scale, epsilon: float) -> None:
@@ -305,30 +225,31 @@ def invoke_dequant_add_residual_rms_norm_quant(out, input, residual, gamma, scal
 
 def invoke_quant(out, input, scale) -> None:
     """fused_kernels.invoke_quant: Tensor scale [tokens] (written) or scalar Half scale (read)  (fused.cpp:52-58)."""
+    if isinstance(scale, torch.Tensor):
+        _bind.invoke_quant(out, input, scale)
+        return
     _cuda(input, "input"); _half_only(input, "invoke_quant")
     _require(input.is_contiguous() and out.is_contiguous(), "invoke_quant: input and out must be contiguous")  # asserts, fused_kernels.cu:202-203
     if _noop(input):
         return
     tokens, hidden = _rows(input)
-    if isinstance(scale, torch.Tensor):
-        _call(input, lib.qs_invoke_quant, out.data_ptr(), input.data_ptr(), scale.data_ptr(), tokens, hidden)
-    else:
-        s = float(torch.tensor(float(scale), dtype=_HALF))
-        _call(input, lib.qs_invoke_quant_scalar, out.data_ptr(), input.data_ptr(), s, tokens, hidden)
+    s = float(torch.tensor(float(scale), dtype=_HALF))
+    _call(input, lib.qs_invoke_quant_scalar, out.data_ptr(), input.data_ptr(), s, tokens, hidden)
 
 
 def invoke_quant_fuse_sum(out, input, input_sum, scale) -> None:
     """fused_kernels.invoke_quant_fuse_sum (fused.cpp:59-69, fused_kernels.cu:234-265)."""
+    if isinstance(scale, torch.Tensor):
+        _bind.invoke_quant_fuse_sum(out, input, input_sum, scale)
+        return
     _cuda(input, "input"); _half_only(input, "invoke_quant_fuse_sum")
     _require(input.is_contiguous() and out.is_contiguous(), "invoke_quant_fuse_sum: input and out must be contiguous")
     if _noop(input):
         return
     tokens, hidden = _rows(input)
-    if isinstance(scale, torch.Tensor):
-        _call(input, lib.qs_invoke_quant_fuse_sum, out.data_ptr(), input.data_ptr(), input_sum.data_ptr(), scale.data_ptr(), tokens, hidden)
-    else:  # scalar overload: static scale, the sum argument is unused by the reference kernel (fused_kernels.cu:131-136)
-        s = float(torch.tensor(float(scale), dtype=_HALF))
-        _call(input, lib.qs_invoke_quant_scalar, out.data_ptr(), input.data_ptr(), s, tokens, hidden)
+    # scalar overload: static scale, the sum argument is unused by the reference kernel (fused_kernels.cu:131-136)
+    s = float(torch.tensor(float(scale), dtype=_HALF))
+    _call(input, lib.qs_invoke_quant_scalar, out.data_ptr(), input.data_ptr(), s, tokens, hidden)
 
 
 def invoke_dequant_add_residual(out, input, residual, scale) -> None:
@@ -361,12 +282,7 @@ def invoke_dequant(out, input, scale) -> None:
 
 def silu_and_mul(out, input) -> None:
     """activation_ops.silu_and_mul (activation.cpp:26, activation_kernels.cu:84-97): out[..., d] = silu(x[..., :d]) * x[..., d:]."""
-    _cuda(input, "input"); _half_only(input, "silu_and_mul")
-    if _noop(input):
-        return
-    d = input.size(-1) // 2
-    tokens = input.numel() // input.size(-1) if input.size(-1) else 0
-    _call(input, lib.qs_silu_and_mul, out.data_ptr(), input.data_ptr(), tokens, d)
+    _bind.silu_and_mul(out, input)
 
 
 def gelu_new(out, input) -> None:
@@ -404,23 +320,12 @@ def invoke_dequant_silu_and_mul_quant(out, input, scale_gate: float, scale_up: f
 
 def add_rms_norm_general(out, hidden_out, x, delta, weight, input_sum: Optional[torch.Tensor], scaling, epsilon: float) -> None:
     """hidden_out = x + delta (fp16, as torch computes `residual + out_buf`), then rms_norm_general[_fuse_sum](out, hidden_out, ...)."""
-    _cuda(x, "x"); _half_only(x, "add_rms_norm_general"); _half_only(delta, "add_rms_norm_general")
-    if _noop(x):
-        return
-    tokens, hidden = _rows(x)
-    _call(x, lib.qs_add_rms_norm_general, out.data_ptr(), hidden_out.data_ptr(), x.data_ptr(), delta.data_ptr(), weight.data_ptr(),
-                                      input_sum.data_ptr() if input_sum is not None else None, scaling.data_ptr(), float(epsilon), tokens, hidden)
+    _bind.add_rms_norm_general(out, hidden_out, x, delta, weight, input_sum, scaling, epsilon)
 
 
 def silu_and_mul_quant(out, input, input_sum: Optional[torch.Tensor], scale) -> None:
     """silu_and_mul(input) followed by invoke_quant[_fuse_sum]; the fp16 activation never leaves the SM."""
-    _cuda(input, "input"); _half_only(input, "silu_and_mul_quant")
-    if _noop(input):
-        return
-    d = input.size(-1) // 2
-    tokens = input.numel() // input.size(-1)
-    _call(input, lib.qs_silu_and_mul_quant, out.data_ptr(), input.data_ptr(), input_sum.data_ptr() if input_sum is not None else None, scale.data_ptr(),
-                                    tokens, d)
+    _bind.silu_and_mul_quant(out, input, input_sum, scale)
 
 
 def single_query_attention_quant(q, k, v, kv_pointers, length_per_sample, memory_max_seqlen: int, tokens_per_block: int, size_per_token: int,
@@ -428,20 +333,8 @@ def single_query_attention_quant(q, k, v, kv_pointers, length_per_sample, memory
                                  out_q, out_scale, out_sum: Optional[torch.Tensor]) -> None:
     """single_query_attention + invoke_quant[_fuse_sum] in one launch: out_q int8 [B, Hq*D], out_scale / out_sum fp16 [B].
     Bit-identical to the two reference ops run back to back (llama_w4a8_unpad.py:265-283)."""
-    batch = kv_pointers.size(0)
-    if batch == 0:
-        return
-    nheads, nheads_kv, headdim = q.size(1), k.size(1), k.size(-1)
-    _require(q.dtype == _HALF and q.stride(2) == 1 and q.stride(1) == headdim, "q must be float16 with stride(1) == head_dim")
-    _require(k.stride(1) == headdim and v.stride(1) == headdim and kv_pointers.is_contiguous(), "k, v, kv_pointers layout")
-    _require(out_q.dtype == torch.int8 and out_q.is_contiguous() and out_q.numel() == batch * nheads * headdim, "out_q must be int8 [B, Hq*D]")
-    ws = attention_workspace(q.device, batch, nheads, headdim)
-    _call(q, lib.qs_single_query_attention_quant, q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), kv_pointers.data_ptr(),
-                                              length_per_sample.data_ptr(), out_q.data_ptr(), out_scale.data_ptr(),
-                                              out_sum.data_ptr() if out_sum is not None else None, batch, nheads, nheads_kv, headdim,
-                                              kv_pointers.size(-1), int(memory_max_seqlen), int(tokens_per_block), int(size_per_token), int(timestep),
-                                              int(rotary_embedding_dim), float(rotary_base), int(bool(int4_kv_cache)), int(bool(kv_cache_with_zeros)),
-                                              ws.data_ptr(), ws.numel())
+    _bind.single_query_attention_quant(q, k, v, kv_pointers, length_per_sample, memory_max_seqlen, tokens_per_block, size_per_token, timestep,
+                                       rotary_embedding_dim, rotary_base, int4_kv_cache, kv_cache_with_zeros, out_q, out_scale, out_sum)
 
 
 class PeerContext:

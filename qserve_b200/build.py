@@ -1,4 +1,4 @@
-"""Build libqserve_b200.so (sm_100a only) in-tree with nvcc.
+"""Build libqserve_b200.so (sm_100a only) in-tree with nvcc, and the CPython binding of its hot operators with g++.
 
 The shared library is the product: a C-ABI (include/qserve_b200.h) with no torch or Python dependency.
 `python -m qserve_b200.build` rebuilds it; `ensure_built()` is what `__graft_entry__.build()` calls.
@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libqserve_b200.so")
+BIND = os.path.join(HERE, "_bind.so")  # CPython binding of the hot operators (bind.cpp): the one part that is built against torch
 SOURCES = ["capi.cu", "gemm.cu", "attention.cu", "prefill_attention.cu", "elementwise.cu", "hybrid.cu", "hybrid_blocks.cu", "hybrid_linear.cu", "hybrid_latent.cu",
            "hybrid_recurrent.cu"]
 HEADERS = ["common.cuh", "hybrid_common.cuh", "hybrid_conv.cuh", "launch.h", os.path.join("..", "..", "include", "qserve_b200.h")]
@@ -62,6 +63,31 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
+def _build_bind() -> str:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    path = os.path.join(CSRC, "bind.cpp")
+    flags = ["-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    want = " ".join([_digest([path, os.path.join(CSRC, "..", "..", "include", "qserve_b200.h")]), torch.__version__, sys.version, *flags])
+    stamp = os.path.join(BUILD, "bind.stamp")
+    if os.path.exists(BIND) and os.path.exists(stamp) and open(stamp).read() == want:
+        return BIND
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = [f"-isystem{p}" for p in include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]]
+    cmd = ["g++", path, "-o", BIND] + flags + inc + [f"-L{p}" for p in library_paths()] + [f"-L{HERE}", "-l:libqserve_b200.so", "-lc10", "-lc10_cuda",
+           "-ltorch", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed for bind.cpp")
+    with open(stamp, "w") as f:
+        f.write(want)
+    return BIND
+
+
 def ensure_built(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     if force:
@@ -77,6 +103,7 @@ def ensure_built(verbose: bool = False, force: bool = False) -> str:
         subprocess.check_call(cmd)
         with open(stamp, "w") as f:
             f.write(want)
+    _build_bind()
     return LIB
 
 
