@@ -161,6 +161,19 @@ __device__ __forceinline__ void cap_scores(float (&s)[N][4], float in, float out
 
 }  // namespace hyb
 
+// hybrid_tile.cu: prompt portions as 64-row tiles; normalised per-map outputs to a_out [token][head][map][128]
+struct UmmaTiles {
+  float* a_out;
+  const void *q, *kpool, *vpool;
+  long long q_stride;
+  const int *tile_entry, *tile_row0, *entry_start, *entry_len, *entry_slot, *entry_pos0, *block_table;
+  int n_tiles, max_blocks, H, G, maps, page, chunk, window, keep;
+  const float *sinks, *slopes;
+  float scale_log2, cap_in, cap_out;
+};
+bool umma_tiles_supported(const UmmaTiles& p, int D, int Dv, float scale);
+int umma_tiles(const UmmaTiles& p, int tokens, cudaStream_t s);
+
 // hybrid_linear.cu: S <- a S + B (dt x)^T, o = S^T C + skip_h x over prepared rows (ssd_row_floats); state fp32 [slots][H][N][Dv]
 int ssd_scan(float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
              const int* entry_pos0, int T, int E, int H, int G, int N, int Dv, cudaStream_t s);

@@ -1,0 +1,87 @@
+"""Prompt tiles of the hybrid decoders' attention on tcgen05 (heads of 128 numbers, an even number of query heads per key / value head, pages of whole
+64-key blocks) against the plain CUDA-core kernel over the same cache, which works one token at a time in fp32: every mask and option, portions that
+begin inside a tile, a page or a window, tiles with few rows, and cells past a portion's end that hold NaN."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _run(dev, H, G, maps, lens, pos0, page, D=128, chunk=0, window=0, keep=0, sinks=False, slopes=False, softcap=0.0, gate=None, scale=None, seed=0, spoil=True):
+    from qserve_b200._lib import AttnExtra, check, lib
+    from qserve_b200.hybrid import StepBatch
+
+    g = torch.Generator(device=dev).manual_seed(seed + sum(lens))
+    r = lambda *s: torch.randn(*s, device=dev, generator=g)
+    E, T = len(lens), sum(lens)
+    blocks = [-(-(p + n) // page) for n, p in zip(lens, pos0)]
+    table = torch.zeros(E, max(blocks), dtype=torch.int32, device=dev)
+    ids = torch.randperm(sum(blocks), device=dev, generator=g).to(torch.int32)
+    at = 0
+    for e, n in enumerate(blocks):
+        table[e, :n] = ids[at:at + n]
+        at += n
+    k, v = r(sum(blocks), page, G, maps * D).to(BF), r(sum(blocks), page, G, D).to(BF)
+    if spoil:  # whatever lies behind a sequence's last position
+        for e, (n, p) in enumerate(zip(lens, pos0)):
+            end = (p + n) % page
+            if end:
+                k[table[e, blocks[e] - 1].long(), end:] = float("nan")
+                v[table[e, blocks[e] - 1].long(), end:] = float("nan")
+    W = H * maps * D
+    q = r(T, W + (H * D if gate else 0)).to(BF)
+    b = StepBatch.build([(e, p, -1, [1] * n) for e, (n, p) in enumerate(zip(lens, pos0))], table, dev)
+    sk = r(H) if sinks else None
+    sl = 2.0 ** (-8.0 * torch.arange(1, H + 1, device=dev) / H) if slopes else None
+    gp = q.data_ptr() + W * 2 if gate else None
+    ex = ctypes.byref(AttnExtra(keep, sl.data_ptr() if slopes else None, gp, q.stride(0), 1 if gate == "wide" else 0, softcap))
+    scale = scale if scale is not None else D ** -0.5
+    scratch = torch.full((int(lib.qs_hyb_attention_scratch_floats(T, H, G, maps, D)),), float("nan"), device=dev)
+    p = lambda t: None if t is None else t.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for fast in (True, False):
+        out = torch.zeros(T, H * D, dtype=BF, device=dev)
+        if fast:
+            check(lib.qs_hyb_attention_fast(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), p(b.tok_slot), p(b.tok_pos),
+                                            table.data_ptr(), table.shape[1], p(b.tile_entry), p(b.tile_row0), b.n_tiles, p(b.long_tokens), b.n_long,
+                                            p(b.short_tokens), b.n_short, p(b.entry_start), p(b.entry_len), p(b.entry_slot), p(b.entry_pos0),
+                                            scratch.data_ptr(), H, G, maps, D, D, scale, 0.35, 0.8, 1e-5, 1 if maps == 2 else 0, page, chunk, window, p(sk), ex, 0, s))
+        else:
+            check(lib.qs_hyb_attention(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), p(b.tok_slot), p(b.tok_pos),
+                                       table.data_ptr(), table.shape[1], T, H, G, maps, D, D, scale, 0.35, 0.8, 1e-5, 1 if maps == 2 else 0, page, chunk,
+                                       window, p(sk), ex, 0, s))
+        outs.append(out.float())
+    assert torch.isfinite(outs[1]).all() and torch.isfinite(outs[0]).all()
+    # both kernels are fp32 up to the output's rounding: one bfloat16 unit, plus fp32 noise next to zero
+    assert ((outs[0] - outs[1]).abs() <= 2 ** -7 * outs[1].abs() + 3e-4).all(), (outs[0] - outs[1]).abs().max()
+    assert ((outs[0] - outs[1]).norm() / outs[1].norm()) < 2e-3
+
+
+@pytest.mark.parametrize("H,G,maps,lens,pos0,page", [
+    (4, 2, 2, [64], [0], 64),                     # one whole tile
+    (2, 1, 1, [16, 17, 63, 65, 128, 129], [0] * 6, 64),
+    (8, 2, 2, [200, 90], [0, 37], 64),            # a portion that begins inside a page
+    (4, 1, 1, [40, 3, 100], [1000, 64, 191], 128),  # beside a short portion (single-token kernel)
+    (16, 4, 2, [300], [5], 192),
+    (6, 1, 1, [70], [0], 64),                     # six heads of one group
+])
+def test_causal(dev, H, G, maps, lens, pos0, page):
+    _run(dev, H, G, maps, lens, pos0, page)
+
+
+@pytest.mark.parametrize("kw", [dict(chunk=100), dict(window=70), dict(window=1), dict(window=64, keep=5), dict(window=90, keep=130), dict(sinks=True),
+                                dict(slopes=True), dict(softcap=5.0), dict(softcap=50.0, slopes=True, window=150), dict(sinks=True, chunk=64), dict(gate="head"),
+                                dict(gate="wide", window=33, keep=64, slopes=True), dict(scale=2.5)], ids=str)
+def test_options(dev, kw):
+    _run(dev, 4, 2, 1, [150, 66, 400], [0, 129, 31], 64, **kw)
+    if not set(kw) & {"gate"}:
+        _run(dev, 4, 2, 2, [90], [200], 128, **kw)
+
+
+@pytest.mark.parametrize("H,G,page,D,scale", [(3, 3, 64, 128, None), (4, 2, 48, 128, None), (4, 2, 64, 64, None), (4, 2, 64, 128, -0.1)])
+def test_shapes_that_stay_on_the_general_tiles(dev, H, G, page, D, scale):
+    _run(dev, H, G, 1, [130], [7], page, D=D, scale=scale)
