@@ -1,4 +1,4 @@
-"""Long runs of a retention or state space layer in chunks of 64 tokens on tcgen05 against the recurrence in 64 bits over the same prepared rows: runs at
+"""Long runs of a retention, state space or gated delta layer in chunks of 64 tokens on tcgen05 against the recurrence in 64 bits over the same prepared rows: runs at
 the edges of a chunk and of the rule that takes them (32 tokens, 256 in the batch), short runs in the same batch, continued runs, sequences with states of their own in a
 shuffled order, states of fewer than 128 rows, decays of exactly zero, and 32-bit storage, which keeps the token-by-token scan."""
 import pytest
@@ -92,4 +92,46 @@ def test_retention(lens, pos0, H, D, Dv, dtype):
     q, k, v = prep[:, :H * D].view(T, H, D), prep[:, H * D:2 * H * D].view(T, H, D), prep[:, 2 * H * D:].view(T, H, Dv)
     one = torch.ones(T, H, device=dev)
     _check(o.view(T, H, Dv), state, q, k, v, one, decay * one, torch.zeros(H, dtype=torch.float64, device=dev), S0, lens, pos0, start, slots)
+    assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("lens,pos0", RUNS)
+@pytest.mark.parametrize("H,G,D,Dv,dtype", [(8, 2, 128, 128, BF), (4, 4, 72, 128, BF), (12, 2, 128, 128, BF), (4, 1, 104, 128, BF), (2, 1, 128, 128, BF), (4, 2, 128, 64, BF), (4, 2, 128, 128, torch.float32)])
+def test_gated_delta(lens, pos0, H, G, D, Dv, dtype):
+    from qserve_b200._lib import check, lib
+
+    dev, taps = "cuda", 4
+    gen = torch.Generator(device=dev).manual_seed(sum(lens) + D + H)
+    r = lambda *s: torch.randn(*s, device=dev, generator=gen)
+    T, E, C = sum(lens), len(lens), 2 * G * D + H * Dv
+    W = (C + H * Dv + 2 * H + 7) // 8 * 8
+    proj, cw, cs = r(T, W).to(dtype), r(C, taps) * 0.5, r(E, taps - 1, C)
+    a_log, dt_bias, nw = r(H) * 0.5, r(H) * 0.5, torch.ones(Dv, device=dev)
+    a_log[0], a_log[1] = 60.0, -30.0  # decays of 0 and of 1
+    S0 = r(E, H, D, Dv) * 0.3
+    state = S0.clone()
+    tab, start, slots = _tables(lens, pos0, dev)
+    prep, o, out = torch.full((T, C + 2 * H), float("nan"), device=dev), torch.full((T, H * Dv), float("nan"), device=dev), torch.zeros(T, H * Dv, dtype=dtype, device=dev)
+    p = lambda t: t.data_ptr()
+    check(lib.qs_hyb_gated_delta(p(out), H * Dv, p(prep), p(o), p(proj), W, p(cw), p(cs), p(state), p(a_log), p(dt_bias), p(nw), *map(p, tab), T, E, H, G, D, Dv,
+                                 taps, 1e-6, 1e-5, 0 if dtype is BF else 1, torch.cuda.current_stream().cuda_stream))
+    q, k = (prep[:, i * G * D:(i + 1) * G * D].view(T, G, D).repeat_interleave(H // G, 1).double() for i in (0, 1))
+    v, b, a = prep[:, 2 * G * D:C].view(T, H, Dv).double(), prep[:, C:C + H].double(), prep[:, C + H:C + 2 * H].double()
+    for e, n in enumerate(lens):
+        S = S0[slots[e]].double() if pos0[e] else torch.zeros_like(S0[0], dtype=torch.float64)
+        O = []
+        for t in range(start[e], start[e] + n):
+            S = a[t][:, None, None] * S
+            u = b[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][..., None] * u[:, None]
+            O.append(torch.einsum("hdv,hd->hv", S, q[t]))
+        # keys are unit vectors and write strengths below one, so a step does not enlarge an error: what a chunk's sums add (a few units of fp32 of the
+        # state's size, as for the other recurrences) meets at most sqrt(chunks) of its kind
+        eps = 2.0 ** -20 * max(1.0, (n / 64) ** 0.5)
+        O, got = torch.stack(O), o.view(T, H, Dv)[start[e]:start[e] + n].double()
+        scale = max(O.norm() / O.numel() ** 0.5, S.norm() / S.numel() ** 0.5)
+        assert (got - O).norm() <= eps * scale * O.numel() ** 0.5, (e, ((got - O).norm() / O.norm()).item())
+        assert (state[slots[e]].double() - S).norm() <= eps * S.norm(), (e, ((state[slots[e]].double() - S).norm() / S.norm()).item())
+        for h in range(H):  # each head by itself: the largest error of a number against the head's own size
+            assert (got[:, h] - O[:, h]).abs().max() <= 16 * eps * max(O[:, h].abs().max(), S[h].abs().max()), (e, h)
     assert torch.isfinite(out).all()
