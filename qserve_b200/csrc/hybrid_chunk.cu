@@ -45,7 +45,6 @@ constexpr int kSub = kChunk * 128;           // bytes of a swizzled sub-tile: 64
 constexpr int kPlane = 2 * kSub;             // one term of a [64][128] operand
 constexpr int kThreads = 512;                // warps 0 .. 7 rows (two per tensor memory quarter), 8 .. 14 operands, 15 issuer
 constexpr int kLongRun = kLongRunTokens;     // shorter runs of a batch stay with the token-by-token scans
-constexpr int kLongBatch = 256;
 
 // tensor memory columns: S^T fp32; the three terms of S^T (64 columns each), later the chunk's addition to S^T; S q; the products with P per head.  The
 // values' three terms (32 columns each) lie behind the addition, the third over the columns of S q that have been read.
@@ -763,16 +762,23 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(const LongScan
 
 }  // namespace
 
-// Two heads of 64 values share their q and g; a row's pieces begin on 32-byte words.  Batches of 32 tokens an entry on average and 256 altogether: below
-// that the token-by-token scans' many small blocks are as fast (64 state space heads of 128 x 64, whole call, token by token / chunks: one run of 32 31 / 49
-// us, of 64 41 / 54, of 128 64 / 64, of 2048 702 / 315; 32 runs of 32 196 / 176, of 64 338 / 208; 60 single tokens and a run of 2000 1105 / 400; 4 runs of
-// about 1500 1343 / 474; 16 delta heads of 128 x 128: 32 runs of 32 149 / 128, of 64 275 / 159, 60 single tokens and a run of 2000 1195 / 437, 4 runs of
-// about 1500 1279 / 495).
+// Two heads of 64 values share their q and g; a row's pieces begin on 32-byte words.  Which is faster: token by token a run costs 0.4 us a token, and 5 ns
+// a token for every 128 value rows of the batch when those fill the machine; chunks cost 50 us for the second kernel and the wait for the longest chain, and
+// 8 us a chunk for every 148 of them.  The host knows the runs' average only.  Measured (whole call, us, token by token / chunks): 16 delta heads of 128 x 128
+//   1 x 256 121 / 101, 2 x 128 74 / 83, 4 x 64 59 / 75, 8 x 32 54 / 70, 32 x 32 149 / 128, 32 x 64 275 / 159, 60 single tokens and 2000 1195 / 437,
+//   1 x 2048 846 / 363, 4 x about 1500 1279 / 495
+// 64 state space heads of 128 x 64
+//   1 x 32 31 / 49, 1 x 64 41 / 54, 1 x 128 64 / 64, 32 x 32 197 / 176, 32 x 64 338 / 208, 60 single tokens and 2000 1131 / 400, 1 x 2048 702 / 315,
+//   4 x about 1500 1343 / 474
 bool long_chunks_supported(const LongScan& p, int T, int E, bool delta) {
   auto al32 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 31) == 0; };
   const bool heads = p.Dv == 128 || (!delta && p.Dv == 64 && p.head_div % 2 == 0);
-  return T >= kLongRun * E && T >= kLongBatch && p.D > 64 && p.D <= kState && p.D % 8 == 0 && heads && p.P % 8 == 0 && p.q_at % 8 == 0 && p.g_at % 8 == 0 && p.v_at % 8 == 0 &&
-         al32(p.prep) && al32(p.o_raw) && p.H <= 65535;
+  if (!(heads && p.D > 64 && p.D <= kState && p.D % 8 == 0 && p.P % 8 == 0 && p.q_at % 8 == 0 && p.g_at % 8 == 0 && p.v_at % 8 == 0 && al32(p.prep) &&
+        al32(p.o_raw) && p.H <= 65535 && E > 0 && T / E >= kLongRun))
+    return false;
+  const long long run = T / E, blocks = static_cast<long long>(E) * p.H * p.Dv / 128;
+  const long long tokens_ns = run * std::max(400ll, 5 * blocks), chunks_ns = 50000 + 8000 * ((run + kChunk - 1) / kChunk) * ((blocks + 147) / 148);
+  return chunks_ns < tokens_ns;
 }
 
 int long_chunks(const LongScan& p, int T, int E, bool delta, cudaStream_t s) {

@@ -126,12 +126,12 @@ __host__ __device__ __forceinline__ int scan_row_floats(int mode, int H, int G, 
   return (mode == kScanChannelDecay ? 3 : 2) * H * D + H * Dv;
 }
 
-template <int DP, int PARTS, int CH, int CPT, int MODE, bool VEC>  // VEC: 16-byte staging (D, Dv, the prepared row and its base allow it)
+template <int DP, int PARTS, int CH, int CPT, int MODE, bool VEC, bool SHORT = false>  // VEC: 16-byte staging (D, Dv, the prepared row and its base allow it)
 __global__ void __launch_bounds__(128) linear_scan_kernel(float* __restrict__ o_raw, const float* __restrict__ prep, float* __restrict__ state,
                                                           const float* __restrict__ head_decay, const int* __restrict__ entry_start,
                                                           const int* __restrict__ entry_len, const int* __restrict__ entry_slot,
-                                                          const int* __restrict__ entry_pos0, int H, int G, int D, int Dv, int longest) {
-  // runs of more than `longest` tokens are another kernel's
+                                                          const int* __restrict__ entry_pos0, int H, int G, int D, int Dv) {
+  // SHORT: runs of kLongRunTokens and more are another kernel's (a bound read from a parameter in every launch made the scan itself slower)
   // head_decay [H]: kScanHeadDecay the decay, kScanTokenDecay the skip factor
   extern __shared__ __align__(16) float sm[];  // [2][CH][ROW]
   constexpr bool TOKEN = MODE == kScanTokenDecay;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(128) linear_scan_kernel(float* __restrict__ o_
   auto vec_at = [&](int which) { return TOKEN ? H * Dv + (1 - which) * GD + gh * D : which * GD + h * D; };
   const int val_at = (TOKEN ? 0 : NVEC * GD) + h * Dv, num_at = H * Dv + 2 * GD + h;
   const int n = entry_len[e], s0 = entry_start[e];
-  if (n > longest) return;
+  if (SHORT && n >= kLongRunTokens) return;
   const bool fresh = entry_pos0[e] == 0;
   float decay = MODE == kScanHeadDecay ? head_decay[h] : 0.f;
   const float skip = TOKEN ? head_decay[h] : 0.f;
@@ -305,16 +305,16 @@ int launch_scan(bool chunks, float* o_raw, const float* prep, float* state, cons
   constexpr int NVEC = MODE == kScanChannelDecay ? 3 : 2;
   const int P = scan_row_floats(MODE, H, G, D, Dv);
   const bool vec = D % 4 == 0 && Dv % 4 == 0 && P % 4 == 0 && (reinterpret_cast<uintptr_t>(prep) & 15) == 0;
-  int longest = 0x7fffffff;
-  if constexpr (MODE == kScanHeadDecay || MODE == kScanTokenDecay) {  // one decay per token and head: long runs go in chunks on the tensor cores (16-bit storage)
+  constexpr bool LONG = MODE == kScanHeadDecay || MODE == kScanTokenDecay;
+  bool in_chunks = false;
+  if constexpr (LONG) {  // one decay per token and head: long runs go in chunks on the tensor cores (16-bit storage)
     constexpr bool TOKEN = MODE == kScanTokenDecay;
     const int HDv = H * Dv, GD = G * D;
     const LongScan ls{o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, D, Dv, P, H / G, TOKEN ? HDv + GD : 0,
                       TOKEN ? HDv : GD, TOKEN ? 0 : 2 * GD, TOKEN ? HDv + 2 * GD : -1, TOKEN ? HDv + 2 * GD + H : -1, TOKEN ? 1 : 0};
-    if (chunks && long_chunks_supported(ls, T, E, false)) {
+    in_chunks = chunks && long_chunks_supported(ls, T, E, false);
+    if (in_chunks)
       if (int rc = long_chunks(ls, T, E, false, s)) return rc;
-      longest = kLongRunTokens - 1;
-    }
   }
 #define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
   do {                                                                                                                                        \
@@ -322,8 +322,10 @@ int launch_scan(bool chunks, float* o_raw, const float* prep, float* state, cons
     const size_t smb = (size_t)2 * CH * (NVEC * PARTS * (DP / PARTS + 4) + cols + (MODE == kScanTokenDecay ? 4 : 0)) * sizeof(float);            \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
     auto kern = vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>;                 \
+    if constexpr (LONG && DP == 128)                                                                                                          \
+      if (in_chunks) kern = linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true, true>;                                                         \
     if (smb > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);                                   \
-    kern<<<grid, 128, smb, s>>>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv, longest);        \
+    kern<<<grid, 128, smb, s>>>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                 \
   } while (0)
   // rows of a column per thread: all of them up to 32, 32 or 16 above (the parts of a column meet through shuffles).  Long runs of tokens
   // (prompt portions) take two adjacent columns per thread where the head has the columns for it: a q / g word read from shared memory then

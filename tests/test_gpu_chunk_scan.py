@@ -1,5 +1,5 @@
 """Long runs of a retention, state space or gated delta layer in chunks of 64 tokens on tcgen05 against the recurrence in 64 bits over the same prepared rows: runs at
-the edges of a chunk and of the rule that takes them (32 tokens, 256 in the batch), short runs in the same batch, continued runs, sequences with states of their own in a
+the edges of a chunk and of the rule that takes them (32 tokens), a batch below the rule, short runs in the same batch, continued runs, sequences with states of their own in a
 shuffled order, states of fewer than 128 rows, decays of exactly zero, and 32-bit storage, which keeps the token-by-token scan."""
 import pytest
 import torch
@@ -39,7 +39,7 @@ def _check(o, state, q, g, v, b, a, skip, S0, lens, pos0, start, slots):
             assert (x - ref).norm() <= 2.0 ** -20 * ref.norm(), (lens, e, ((x - ref).norm() / ref.norm()).item())
 
 
-RUNS = [([31, 32, 33, 200], [0, 0, 9, 0]), ([63, 193], [0, 7]), ([64, 65, 127], [7, 0, 0]), ([128, 1, 129, 40], [0, 12, 3, 0]), ([300], [0]), ([255], [5])]
+RUNS = [([31, 32, 33, 800], [0, 0, 9, 0]), ([63, 449], [0, 7]), ([64, 65, 640], [7, 0, 0]), ([128, 1, 129, 766], [0, 12, 3, 0]), ([300], [0]), ([255], [5]), ([128], [3])]
 
 
 @pytest.mark.parametrize("lens,pos0", RUNS)
