@@ -145,12 +145,12 @@ __device__ __forceinline__ void conv_rows(Walk& walk, const ST* __restrict__ in,
     int e[N], pos[N];
     float own[N][V];
 #pragma unroll
-    for (int q = 0; q < N; ++q) {
-      const int tt = min(t + q, t1 - 1);
-      e[q] = tab.tok_entry[tt];
-      pos[q] = tab.tok_pos[tt];
-      walk.fetch(own[q], in, stride, tt, c);
-    }
+    for (int q = 0; q < N; ++q)  // (the last row again instead of nothing: 21 us where a walk of one row takes 18, 256 rows of 6144 channels)
+      if (q == 0 || t + q < t1) {
+        e[q] = tab.tok_entry[t + q];
+        pos[q] = tab.tok_pos[t + q];
+        walk.fetch(own[q], in, stride, t + q, c);
+      }
 #pragma unroll
     for (int q = 0; q < N; ++q)
       if (t + q < t1) {
