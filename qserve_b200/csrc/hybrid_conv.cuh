@@ -135,17 +135,17 @@ __device__ __forceinline__ ConvWalk<ST, V, TAPS> conv_walk(const float* w, const
   else return ConvWalk<ST, V, TAPS>(w, b, in_bias, c);
 }
 
-// Rows t0 .. t1 - 1 at channels c .. c + V - 1 in order, `use(t, y)` takes each.  The inputs and tables of four rows are fetched together: one at a
-// time, every row waited for its own load.
-template <typename ST, int V, typename Walk, typename Use>
+// Rows t0 .. t1 - 1 at channels c .. c + V - 1 in order, `use(t, y)` takes each.  The inputs and tables of N rows are fetched together: one at a time,
+// every row waited for its own load.  A walk of one row (conv_run) takes N = 1: the other rows' code costs registers (256 rows of 6144 channels: 21 us
+// with N = 4, 19 with 1; single tokens of 64 sequences 6.9).
+template <typename ST, int V, int N = 4, typename Walk, typename Use>
 __device__ __forceinline__ void conv_rows(Walk& walk, const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias, const ConvTables& tab,
                                           int t0, int t1, int c, bool shift, Use use) {
-  constexpr int N = 4;
   for (int t = t0; t < t1; t += N) {
     int e[N], pos[N];
     float own[N][V];
 #pragma unroll
-    for (int q = 0; q < N; ++q)  // (the last row again instead of nothing: 21 us where a walk of one row takes 18, 256 rows of 6144 channels)
+    for (int q = 0; q < N; ++q)
       if (q == 0 || t + q < t1) {
         e[q] = tab.tok_entry[t + q];
         pos[q] = tab.tok_pos[t + q];

@@ -13,6 +13,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/qserve_b200.h"
 #include "common.cuh"
@@ -57,7 +58,7 @@ __global__ void conv_state_kernel(float* __restrict__ conv_state, const ST* __re
 //   a = exp(-exp(A_log) dt)
 // grid (runs of `run` tokens, blocks of 128 V channels)
 // ---------------------------------------------------------------------------------------------------------------------------------
-template <typename ST, int V, int TAPS>
+template <typename ST, int V, int TAPS, int ROWS>
 __global__ void __launch_bounds__(128) ssd_prepare_kernel(float* __restrict__ prep, const ST* __restrict__ proj, long long stride,
                                                           const float* __restrict__ conv_w, const float* __restrict__ conv_b, float* conv_state,
                                                           const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(128) ssd_prepare_kernel(float* __restrict__ pr
   auto walk = conv_walk<ST, V, TAPS>(conv_w, conv_b, nullptr, taps, min(c, C - V));
   if (c < C) {
     const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, C, taps};
-    conv_rows<ST, V>(walk, proj + inner, stride, nullptr, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
+    conv_rows<ST, V, ROWS>(walk, proj + inner, stride, nullptr, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
       float* o = prep + (size_t)t * P;
 #pragma unroll
       for (int v = 0; v < V; ++v) y[v] = silu_as<ST>(y[v]);
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(256) ssd_out_kernel(ST* __restrict__ out, long
 // gated linear unit.  projection row: [W y | W x] (biases not yet added)
 // step 1: u = convolution of x + x_bias, in the storage type [T][W]
 // ---------------------------------------------------------------------------------------------------------------------------------
-template <typename ST, int V, int TAPS>
+template <typename ST, int V, int TAPS, int ROWS>
 __global__ void __launch_bounds__(128) lru_conv_kernel(ST* __restrict__ u, const ST* __restrict__ proj, long long stride, const float* __restrict__ x_bias,
                                                        const float* __restrict__ conv_w, const float* __restrict__ conv_b, float* conv_state,
                                                        const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(128) lru_conv_kernel(ST* __restrict__ u, const
   const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
   auto walk = conv_walk<ST, V, TAPS>(conv_w, conv_b, x_bias, taps, c);
   const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, W, taps};
-  conv_rows<ST, V>(walk, proj + W, stride, x_bias, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
+  conv_rows<ST, V, ROWS>(walk, proj + W, stride, x_bias, tab, t0, t1, c, shift != 0, [&](int t, float(&y)[V]) {
     if constexpr (V == 4) st4(u + (size_t)t * W + c, make_float4(y[0], y[1], y[2], y[3]));
     else stf(u + (size_t)t * W + c, y[0]);
   });
@@ -356,8 +357,12 @@ int launch_state_space(void* out, long long out_stride, float* prep, float* o_ra
   const int inner = H * Dv, C = inner + 2 * G * N, run = conv_run(T), shift = T == E && taps > 1;
   const bool v4 = C % 4 == 0 && inner % 4 == 0 && stride % 4 == 0 && aligned(proj, 4 * sizeof(ST)) && aligned(prep, 16);
   dim3 grid((T + run - 1) / run, (C + (v4 ? 512 : 128) - 1) / (v4 ? 512 : 128));
-  auto prepare = !v4 ? ssd_prepare_kernel<ST, 1, 0> : taps == 4 ? ssd_prepare_kernel<ST, 4, 4> : taps == 3 ? ssd_prepare_kernel<ST, 4, 3>
-                 : taps == 2 ? ssd_prepare_kernel<ST, 4, 2> : ssd_prepare_kernel<ST, 4, 0>;
+  auto pick = [&](auto rows) {
+    constexpr int R = decltype(rows)::value;
+    return !v4 ? ssd_prepare_kernel<ST, 1, 0, R> : taps == 4 ? ssd_prepare_kernel<ST, 4, 4, R> : taps == 3 ? ssd_prepare_kernel<ST, 4, 3, R>
+           : taps == 2 ? ssd_prepare_kernel<ST, 4, 2, R> : ssd_prepare_kernel<ST, 4, 0, R>;
+  };
+  auto prepare = run == 1 ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 4>{});
   prepare<<<grid, 128, 0, s>>>(prep, proj, stride, conv_w, conv_b, conv_state, a_log, dt_bias, tok_entry, tok_pos, entry_start, entry_slot, T, H, G, N, Dv,
                                taps, run, shift);
   if (!shift)
@@ -380,8 +385,12 @@ int launch_lru_conv(void* u, const void* proj_, long long stride, const float* x
   const int run = conv_run(T), shift = T == E && taps > 1;
   const bool v4 = W % 4 == 0 && stride % 4 == 0 && aligned(proj, 4 * sizeof(ST)) && aligned(u, 4 * sizeof(ST));
   dim3 grid((T + run - 1) / run, (W + (v4 ? 512 : 128) - 1) / (v4 ? 512 : 128));
-  auto conv = !v4 ? lru_conv_kernel<ST, 1, 0> : taps == 4 ? lru_conv_kernel<ST, 4, 4> : taps == 3 ? lru_conv_kernel<ST, 4, 3>
-              : taps == 2 ? lru_conv_kernel<ST, 4, 2> : lru_conv_kernel<ST, 4, 0>;
+  auto pick = [&](auto rows) {
+    constexpr int R = decltype(rows)::value;
+    return !v4 ? lru_conv_kernel<ST, 1, 0, R> : taps == 4 ? lru_conv_kernel<ST, 4, 4, R> : taps == 3 ? lru_conv_kernel<ST, 4, 3, R>
+           : taps == 2 ? lru_conv_kernel<ST, 4, 2, R> : lru_conv_kernel<ST, 4, 0, R>;
+  };
+  auto conv = run == 1 ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 4>{});
   conv<<<grid, 128, 0, s>>>((ST*)u, proj, stride, x_bias, conv_w, conv_b, conv_state, tok_entry, tok_pos, entry_start, entry_slot, T, W, taps, run, shift);
   if (!shift) return launch_conv_state<ST>(conv_state, proj + W, stride, x_bias, entry_start, entry_len, entry_slot, entry_pos0, E, W, taps, s);
   return check_cuda(cudaGetLastError(), "hyb_lru_conv");
