@@ -156,10 +156,9 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   __shared__ uint32_t s_last;
 
   // Every warp initialises the barriers of ITS OWN ring (lane 0, the lane that later arms them and issues the copies), so no block-wide
-  // barrier is needed between initialisation and first use.  Round 1 let thread 0 initialise all rings without a barrier: harmless while every
-  // CTA of a single-wave launch sat in griddepcontrol.wait long enough, but a late CTA of a multi-wave launch (64 kv heads x 64 sequences =
-  // 4096 CTAs at Qwen1.5-72B) could arm a ring before thread 0 had initialised it -- the initialisation then wiped the pending transaction
-  // count and that warp waited forever (found in round 2: one hung warp per ~10^8 slices, profiles/r02_notes.md).
+  // barrier is needed between initialisation and first use.  With thread 0 initialising all rings and no barrier, a late CTA
+  // of a multi-wave launch (64 kv heads x 64 sequences = 4096 CTAs at Qwen1.5-72B), which does not sit in griddepcontrol.wait, could arm a ring ahead
+  // of its initialisation, which then wiped the pending transaction count: that warp waited forever (one in ~10^8 slices).
   if (lane == 0) {
     for (int i = 0; i < R; ++i) mbar_init(&s_full[warp][i], 1);
     fence_barrier_init();

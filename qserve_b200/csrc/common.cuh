@@ -238,8 +238,7 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
 // named barrier over `threads` threads (a multiple of 32) of the CTA; id 0 is __syncthreads
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // arrive on the mbarrier at the same CTA-relative offset in CTA `rank` of the cluster.  Default semantics (release at CTA scope) on purpose:
-// `.release.cluster` compiles to MEMBAR.ALL.GPU + ERRBAR in front of the arrive (and `try_wait.acquire.cluster` to a CCTL.IVALL behind the wait),
-// ~1 us per pipeline stage.  The data these barriers guard is tensor memory / TMA-written shared memory, ordered by tcgen05.wait::st +
+// `.release.cluster` (with `try_wait.acquire.cluster` behind the wait) costs ~1 us per pipeline stage.  The data these barriers guard is tensor memory / TMA-written shared memory, ordered by tcgen05.wait::st +
 // tcgen05.fence::before_thread_sync on the producer side and tcgen05.fence::after_thread_sync on the consumer side, not by generic-proxy fences;
 // the consumer waits with the ordinary mbar_wait.
 __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank) {

@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(kThreads) argmax_rows_kernel(long long* __rest
 // Register-resident fast path of N1 and of its fused forms (per-token quantisation, H <= 8 * kThreads * CH, CH <= 2: every model of the
 // benchmark).  ONE body serves rms_norm_general[_fuse_sum], add_rms_norm_general and its peer (fused all-reduce) form, so the fused and the
 // unfused ops are bit-identical by construction.  Against the shared-memory kernels above it keeps the row in registers (no re-reads) and needs
-// 4 block barriers instead of 9: a decode-size row op is a pure latency chain (profiles/r02_notes.md), every barrier and round trip counts.
+// 4 block barriers instead of 9: a decode-size row op is a pure latency chain, every barrier and round trip counts.
 // Arithmetic and reduction trees are those of layernorm_quant_kernel (same thread -> element map, same shuffle order).
 // ------------------------------------------------------------------------------------------------
 template <typename Op>

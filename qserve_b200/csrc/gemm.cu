@@ -52,7 +52,7 @@ constexpr bool kPairCvt = QS_PAIR_CVT != 0;
 #ifndef QS_DECODE_CVT
 #define QS_DECODE_CVT 1
 #endif
-constexpr bool kDecodeCvt = QS_DECODE_CVT != 0;  // the same choice for the epilogue of gemm_kernel (A/B: profiles/r02_notes.md 4b)
+constexpr bool kDecodeCvt = QS_DECODE_CVT != 0;  // the same choice for the epilogue of gemm_kernel
 constexpr int kPairThreads = 384;  // gemm_pair_kernel: the 8 warps of gemm_kernel + 4 more epilogue warps
 // warp roles: 0 weight producer | 1 TMEM owner + MMA issuer (even stages) | 2..5 unpack + TMEM epilogue | 6 activation producer |
 // 7 MMA issuer (odd stages).
@@ -141,10 +141,9 @@ __device__ __forceinline__ void st_dsmem_u32(uint32_t addr, uint32_t v) {
 }
 
 // INT32 -> FP32, round to nearest even, without the conversion instruction:  v = hi * 65536 + lo, both halves are converted exactly by the
-// 1.5 * 2^23 magic-number add, and the single rounding of the fused multiply-add equals cvt.rn.f32.s32(v).  Round 1 used it in every epilogue
-// on the assumption that I2F is a quarter-rate XU instruction; the pipe micro-benchmark (profiles/r01_ubench_pipes.txt: 2.5 cycles per warp
-// instruction, against 5 x ~2 for this sequence) and the A/B of round 2 say otherwise (decode step 2.797 -> 2.771 ms, prefill tiles +2 %), so the
-// kernels now convert with the instruction; this stays as the -DQS_DECODE_CVT=0 / -DQS_PAIR_CVT=0 variant.
+// 1.5 * 2^23 magic-number add, and the single rounding of the fused multiply-add equals cvt.rn.f32.s32(v).  The conversion instruction
+// is faster (2.5 cycles per warp instruction measured, against 5 x ~2 for this sequence; decode step 2.797 -> 2.771 ms, prefill tiles +2 %), so the
+// kernels convert with it; this stays as the -DQS_DECODE_CVT=0 / -DQS_PAIR_CVT=0 variant.
 __device__ __forceinline__ float int2float_rn_noxu(int32_t v) {
   const int32_t hi = v >> 16, lo = v & 0xFFFF;
   const float fhi = __fsub_rn(__int_as_float(0x4B400000 + hi), 12582912.f);
@@ -183,7 +182,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
   // its iteration, which the (in-order) unpack warps can only fill after the OTHER issuer's commit for the iteration three back -- and that issuer
   // had waited for the very activation / weight phase in question.  W8A8 has no such guard (operands come straight from TMA-completed barriers,
   // which may complete out of order): its rings must have even depth, so that every barrier belongs to one issuer and is observed phase by phase.
-  // (Round 2: a 3-deep W8A8 weight ring produced a launch failure in the first test that used it.)
+  // (A 3-deep W8A8 weight ring produced a launch failure in the first test that used it.)
   static_assert(MODE != kModeW8 || (WS % 2 == 0 && AS % 2 == 0), "W8A8: ring depths must be even (two alternating MMA issuers)");
   extern __shared__ __align__(1024) uint8_t smem[];  // no static shared memory in this kernel: the window starts 1024-aligned
   if (threadIdx.x == 0 && (smem_u32(smem) & 1023u) != 0) __trap();
@@ -538,7 +537,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 // at 52 %.  In a CTA pair each SM unpacks its own 128 channels into its own tensor memory (A operand) but stages only HALF of the 256 tokens of
 // the activation tile (B operand); the 2-CTA MMA reads the other half from the peer SM.  L2 -> SM traffic halves (2.7 GB for the shape above).
 // The first version of this kernel (one tile per launch-time CTA pair, 1 pair per TPC because of its 512 TMEM columns) lost all of that again to
-// un-overlapped per-tile fill / drain (24 us per tile for 8.3 us of MMA work; profiles/r02_notes.md), hence the persistent form: operand rings run
+// un-overlapped per-tile fill / drain (24 us per tile for 8.3 us of MMA work), hence the persistent form: operand rings run
 // across tile boundaries, the only exposed per-tile cost is the accumulator drain (TMEM -> registers -> global, no shared-memory staging).
 //
 // Roles per CTA (384 threads): warp 0 weight producer | warp 1 TMEM allocator, leader: MMA issuer (even stages) | warps 2..5 unpack + epilogue |
@@ -1086,7 +1085,7 @@ int dispatch_gemm(const GemmArgs& a) {
     static const bool no_pair = getenv("QS_GEMM_NO_PAIR") != nullptr;  // A/B hooks
     static const int pair_min_m = getenv("QS_GEMM_PAIR_MIN_M") ? atoi(getenv("QS_GEMM_PAIR_MIN_M")) : 512;
     // Below 512 tokens the pair kernel pays only if its 256-token tiles are as well filled as the 128-token ones (an even number of 128-token
-    // tiles: M in (128, 256] or (384, 512)) and there is at least one pair tile per TPC (measured, profiles/r02_notes.md 4b: gate_up at M = 256
+    // tiles: M in (128, 256] or (384, 512)) and there is at least one pair tile per TPC (measured: gate_up at M = 256
     // 30.4 vs 35.5 us, at M = 320 58.1 vs 50.5; o_proj (16 pair tiles) at M = 256 16.6 vs 12.0)
     const int t128 = (a.M + 127) / 128;
     const bool small_ok = a.M > 128 && t128 % 2 == 0 && (a.N / kBM / 2) * ((a.M + 255) / 256) >= num_sms() / 2;
@@ -1095,7 +1094,7 @@ int dispatch_gemm(const GemmArgs& a) {
   int nt = a.force_nt > 0 ? a.force_nt : 0;
   if (nt == 0) {
     // prefill-sized M: 128-token tiles with TWO co-resident CTAs per SM beat the 256-token tile (one CTA per SM) by 14-15 % (M = 1024: 2071 vs
-    // 1796 TOP/s, M = 4096: 2388 vs 2100, profiles/r02_notes.md): a tile's setup, pipeline fill and epilogue hide behind the sibling's main loop
+    // 1796 TOP/s, M = 4096: 2388 vs 2100): a tile's setup, pipeline fill and epilogue hide behind the sibling's main loop
     nt = a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
   }
   if (nt == 32) return launch_gemm<MODE, 32, (w8 ? 2 : grp ? 4 : 5), 4>(a);
