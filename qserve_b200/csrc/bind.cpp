@@ -2,8 +2,9 @@
 //
 // Each function checks its tensors, takes the current stream of their device and calls the C ABI (include/qserve_b200.h).  The checks, the argument
 // conversion and the current-stream lookup cost 5 us per linear layer and 20 us per attention call as Python over ctypes -- more than most of these
-// kernels run; here they cost well under 1 us.  What is called, and what is refused with which error, is unchanged; the Python functions of
-// backend.py keep the names, argument orders and defaults and pass everything on by position.
+// kernels run; here a call takes about 3 us with its launch.  What is called, what is taken (whatever int(), float() and bool() take) and what is refused is
+// as it was there: an argument that is no tensor raises TypeError, everything else what torch's own functions raise.  The Python functions of backend.py
+// keep the names, argument orders and defaults and pass everything on by position.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
@@ -12,6 +13,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <stdexcept>
@@ -22,43 +24,38 @@
 
 namespace {
 
-struct PyError {};  // a Python error is set
-
 struct Args {
   PyObject* const* a;
   Py_ssize_t n;
   const at::Tensor& tensor(int i) const {
     if (!THPVariable_Check(a[i])) {
       PyErr_Format(PyExc_TypeError, "argument %d must be a tensor, not %s", i + 1, Py_TYPE(a[i])->tp_name);
-      throw PyError();
+      throw python_error();
     }
     return THPVariable_Unpack(a[i]);
   }
   bool none(int i) const { return a[i] == Py_None; }
-  void* ptr(int i) const { return none(i) ? nullptr : tensor(i).data_ptr(); }
-  long long integer(int i) const {
-    PyObject* o = a[i];
-    if (PyLong_Check(o)) {
-      const long long v = PyLong_AsLongLong(o);
-      if (v == -1 && PyErr_Occurred()) throw PyError();
-      return v;
-    }
-    PyObject* n = PyNumber_Long(o);  // whatever int() takes
-    if (n == nullptr) throw PyError();
-    const long long v = PyLong_AsLongLong(n);
+  void* ptr(int i) const { return tensor(i).data_ptr(); }
+  void* ptr_or_none(int i) const { return none(i) ? nullptr : ptr(i); }
+  int small(int i) const {  // whatever int() takes, in the low bits of a C int
+    if (PyLong_Check(a[i])) return static_cast<int>(PyLong_AsUnsignedLongLongMask(a[i]));
+    PyObject* n = PyNumber_Long(a[i]);
+    if (n == nullptr) throw python_error();
+    const int v = static_cast<int>(PyLong_AsUnsignedLongLongMask(n));
     Py_DECREF(n);
-    if (v == -1 && PyErr_Occurred()) throw PyError();
     return v;
   }
-  int small(int i) const { return static_cast<int>(integer(i)); }
-  float real(int i) const {
-    const double v = PyFloat_AsDouble(a[i]);
-    if (v == -1.0 && PyErr_Occurred()) throw PyError();
-    return static_cast<float>(v);
+  float real(int i) const {  // whatever float() takes
+    if (PyFloat_Check(a[i])) return static_cast<float>(PyFloat_AS_DOUBLE(a[i]));
+    PyObject* n = PyNumber_Float(a[i]);
+    if (n == nullptr) throw python_error();
+    const float v = static_cast<float>(PyFloat_AS_DOUBLE(n));
+    Py_DECREF(n);
+    return v;
   }
   int truth(int i) const {
     const int v = PyObject_IsTrue(a[i]);
-    if (v < 0) throw PyError();
+    if (v < 0) throw python_error();
     return v;
   }
 };
@@ -92,12 +89,14 @@ Workspaces& workspaces() {
   return *w;
 }
 at::Tensor& grown(std::vector<at::Tensor>& v, int dev, size_t need) {
+  require(dev >= 0 && dev < c10::cuda::device_count(), "no such CUDA device");
   if (static_cast<int>(v.size()) <= dev) v.resize(dev + 1);
   at::Tensor& ws = v[dev];
   if (!ws.defined() || static_cast<size_t>(ws.numel()) < need) {
-    if (ws.defined()) workspaces().retired.push_back(ws);
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
-    ws = at::zeros({static_cast<int64_t>(need)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+    at::Tensor next = at::zeros({static_cast<int64_t>(need)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+    if (ws.defined()) workspaces().retired.push_back(ws);
+    ws = std::move(next);
   }
   return ws;
 }
@@ -122,9 +121,11 @@ Gemm gemm_common(const at::Tensor& x, const at::Tensor& w, const at::Tensor& out
   require(x.is_contiguous() && w.is_contiguous() && out.is_contiguous(), "GEMM operands must be contiguous");
   const int64_t M = x.size(0), K = x.size(1), N = out.size(-1);
   require(out.size(-2) == M, "out_feats rows must match in_feats rows");
-  if (w.size(0) != N || w.size(1) * k_div != K)
-    throw std::runtime_error("kernel shape (" + std::to_string(w.size(0)) + ", " + std::to_string(w.size(1)) + ") does not match N=" + std::to_string(N) +
-                             ", K=" + std::to_string(K));
+  if (w.size(0) != N || w.size(1) * k_div != K) {
+    std::string shape;
+    for (const int64_t n : w.sizes()) shape += (shape.empty() ? "" : ", ") + std::to_string(n);
+    throw std::runtime_error("kernel shape (" + shape + ") does not match N=" + std::to_string(N) + ", K=" + std::to_string(K));
+  }
   return {static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)};
 }
 int8_t* s8(void* p) { return static_cast<int8_t*>(p); }
@@ -134,7 +135,8 @@ PyObject* w4a8_per_chn(const Args& a) {  // in_feats, kernel, wscales, ascales, 
   const Gemm g = gemm_common(x, w, out, 2);
   if (g.M == 0) return none();
   void *p[8];
-  for (int i = 0; i < 8; ++i) p[i] = a.ptr(i);
+  for (int i = 0; i < 7; ++i) p[i] = a.ptr(i);
+  p[7] = a.ptr_or_none(7);
   at::Tensor& ws = gemm_ws(x.get_device());
   void* wp = ws.data_ptr();
   const size_t wn = ws.numel();
@@ -149,7 +151,8 @@ PyObject* w4a8_per_group(const Args& a) {  // in_feats, kernel, zeros, scales_i8
   require(fits(z) && fits(s2), "level-2 params must be [K/128, N]");
   if (g.M == 0) return none();
   void *p[8];
-  for (int i = 0; i < 8; ++i) p[i] = a.ptr(i);
+  for (int i = 0; i < 7; ++i) p[i] = a.ptr(i);
+  p[7] = a.ptr_or_none(7);
   at::Tensor& ws = gemm_ws(x.get_device());
   void* wp = ws.data_ptr();
   const size_t wn = ws.numel();
@@ -162,7 +165,8 @@ PyObject* w8a8(const Args& a) {  // in_feats, kernel, wscales, ascales, out_feat
   require(a.tensor(2).scalar_type() == at::kHalf && a.tensor(3).scalar_type() == at::kHalf, "wscales and ascales must be float16 (w8a8_linear.py:99-101 casts them)");
   if (g.M == 0) return none();
   void *p[6];
-  for (int i = 0; i < 6; ++i) p[i] = a.ptr(i);
+  for (int i = 0; i < 5; ++i) p[i] = a.ptr(i);
+  p[5] = a.ptr_or_none(5);
   at::Tensor& ws = gemm_ws(x.get_device());
   void* wp = ws.data_ptr();
   const size_t wn = ws.numel();
@@ -228,7 +232,7 @@ PyObject* single_query_attention_quant(const Args& a) {  // the 16 arguments of 
   require_cuda(q, "q");
   at::Tensor& ws = attention_ws(q.get_device(), static_cast<int>(batch), static_cast<int>(heads), static_cast<int>(dim));
   void *qp = q.data_ptr(), *kp = k.data_ptr(), *vp = v.data_ptr(), *tp = kvp.data_ptr(), *lens = a.tensor(4).data_ptr(), *op = oq.data_ptr(), *sp = a.tensor(14).data_ptr(),
-       *up = a.ptr(15), *wp = ws.data_ptr();
+       *up = a.ptr_or_none(15), *wp = ws.data_ptr();
   const int64_t qs = q.stride(0), ks = k.stride(0), vs = v.stride(0), blocks = kvp.size(-1);
   const size_t wn = ws.numel();
   launch(q, [&](void* s) {
@@ -282,7 +286,7 @@ PyObject* quant(const at::Tensor& o, const at::Tensor& x, const at::Tensor* sum,
   if (x.numel() == 0) return none();
   const Rows r = rows_of(x);
   void *op_ = o.data_ptr(), *xp = x.data_ptr(), *sc = scale.data_ptr(), *su = sum != nullptr ? sum->data_ptr() : nullptr;
-  launch(x, [&](void* s) { return su != nullptr ? qs_invoke_quant_fuse_sum(s8(op_), xp, su, sc, r.tokens, r.width, s) : qs_invoke_quant(s8(op_), xp, sc, r.tokens, r.width, s); });
+  launch(x, [&](void* s) { return sum != nullptr ? qs_invoke_quant_fuse_sum(s8(op_), xp, su, sc, r.tokens, r.width, s) : qs_invoke_quant(s8(op_), xp, sc, r.tokens, r.width, s); });
   return none();
 }
 PyObject* invoke_quant(const Args& a) {  // out, input, scale tensor
@@ -307,7 +311,7 @@ PyObject* silu_and_mul_quant(const Args& a) {  // out, input, input_sum or None,
   half_only(x, "silu_and_mul_quant");
   if (x.numel() == 0) return none();
   const Rows r = rows_of(x);
-  void *o = a.tensor(0).data_ptr(), *xp = x.data_ptr(), *su = a.ptr(2), *sc = a.tensor(3).data_ptr();
+  void *o = a.tensor(0).data_ptr(), *xp = x.data_ptr(), *su = a.ptr_or_none(2), *sc = a.tensor(3).data_ptr();
   launch(x, [&](void* s) { return qs_silu_and_mul_quant(s8(o), xp, su, sc, r.tokens, r.width / 2, s); });
   return none();
 }
@@ -318,7 +322,7 @@ PyObject* add_rms_norm_general(const Args& a) {  // out, hidden_out, x, delta, w
   half_only(a.tensor(3), "add_rms_norm_general");
   if (x.numel() == 0) return none();
   const Rows r = rows_of(x);
-  void *o = a.tensor(0).data_ptr(), *h = a.tensor(1).data_ptr(), *xp = x.data_ptr(), *d = a.tensor(3).data_ptr(), *w = a.tensor(4).data_ptr(), *su = a.ptr(5),
+  void *o = a.tensor(0).data_ptr(), *h = a.tensor(1).data_ptr(), *xp = x.data_ptr(), *d = a.tensor(3).data_ptr(), *w = a.tensor(4).data_ptr(), *su = a.ptr_or_none(5),
        *sc = a.tensor(6).data_ptr();
   const float eps = a.real(7);
   launch(x, [&](void* s) { return qs_add_rms_norm_general(s8(o), h, xp, d, w, su, sc, eps, r.tokens, r.width, s); });
@@ -337,12 +341,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   try {
     return Fn(Args{args, n});
-  } catch (const PyError&) {
-    return nullptr;
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {  // as torch's own functions raise them: IndexError for a missing dimension, OutOfMemoryError, RuntimeError for the rest
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }
