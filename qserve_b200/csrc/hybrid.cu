@@ -1042,9 +1042,7 @@ __device__ __forceinline__ float part_sum(float v) {
   return v;
 }
 
-// VEC: rows of `prep`, D and Dv are multiples of 4 floats: stage with 16-byte copies.  SHORT: runs of kLongRunTokens and more are another kernel's (a bound
-// read from a parameter in every launch made the scan itself slower: 2 runs of 128, 16 heads: 50 -> 61 us)
-template <int DP, int PARTS, int CH, int CPT, bool VEC, bool SHORT = false>
+template <int DP, int PARTS, int CH, int CPT, bool VEC>  // VEC: rows of `prep`, D and Dv are multiples of 4 floats: stage with 16-byte copies
 __global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o_raw, const float* __restrict__ prep, float* __restrict__ state,
                                                          const int* __restrict__ entry_start, const int* __restrict__ entry_len,
                                                          const int* __restrict__ entry_slot, const int* __restrict__ entry_pos0, int H, int G, int D,
@@ -1056,7 +1054,6 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o_r
   const int tid = threadIdx.x, part = tid % PARTS, cl = tid / PARTS, col0 = cg * COLS + cl * CPT;  // CPT adjacent columns per thread
   const int C = 2 * G * D + H * Dv, P = C + 2 * H;
   const int n = entry_len[e], s0 = entry_start[e];
-  if (SHORT && n >= kLongRunTokens) return;
   const bool fresh = entry_pos0[e] == 0;
   float* Sg = state + ((size_t)entry_slot[e] * H + h) * (size_t)D * Dv;
   float S[CPT][Q];
@@ -1328,13 +1325,6 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
                                                                           entry_pos0, C, taps);
   // 16-byte staging needs every q / k / v run of a prepared row on a 16-byte boundary
   const bool vec = D % 4 == 0 && Dv % 4 == 0 && (C + 2 * H) % 4 == 0 && (reinterpret_cast<uintptr_t>(prep) & 15) == 0;
-  bool chunks = false;
-  if (sizeof(ST) == 2) {  // 16-bit storage: long runs go in chunks on the tensor cores
-    const LongScan ls{o_raw, prep, state, nullptr, entry_start, entry_len, entry_slot, entry_pos0, H, D, Dv, C + 2 * H, H / G, 0, G * D, 2 * G * D, C, C + H, 0};
-    chunks = long_chunks_supported(ls, T, E, true);
-    if (chunks)
-      if (int rc = long_chunks(ls, T, E, true, s)) return rc;
-  }
   // rows of a column per thread: all of them up to 64 (a warp then reads q / k as broadcasts), 64 above
 #define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
   do {                                                                                                                                        \
@@ -1342,8 +1332,6 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
     const size_t sm = (size_t)2 * CH * (2 * PARTS * (DP / PARTS + 4) + cols + 4) * sizeof(float);                                             \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
     auto kern = vec ? delta_scan_kernel<DP, PARTS, CH, CPT, true> : delta_scan_kernel<DP, PARTS, CH, CPT, false>;                             \
-    if constexpr (DP == 128 && PARTS == 8)                                                                                                    \
-      if (chunks) kern = delta_scan_kernel<DP, PARTS, CH, CPT, true, true>;                                                                   \
     if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);                                     \
     kern<<<grid, 128, sm, s>>>(o_raw, prep, state, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                              \
   } while (0)

@@ -161,21 +161,6 @@ __device__ __forceinline__ void cap_scores(float (&s)[N][4], float in, float out
 
 }  // namespace hyb
 
-// hybrid_chunk.cu: recurrences over long runs of tokens.  A prepared row has P floats; q / g of head h start at q_at / g_at + (h / head_div) D, its
-// values at v_at + h Dv, its write strength at b_at + h (negative: 1) and its decay at a_at + h (negative: the fixed decay head_num[h]).
-// skip: o += head_num[h] v.  Runs of fewer than kLongRunTokens tokens are left to the caller's token-by-token scan.
-struct LongScan {
-  float* o_raw;
-  const float* prep;
-  float* state;
-  const float* head_num;
-  const int *entry_start, *entry_len, *entry_slot, *entry_pos0;
-  int H, D, Dv, P, head_div, q_at, g_at, v_at, b_at, a_at, skip;
-};
-constexpr int kLongRunTokens = 32;
-bool long_chunks_supported(const LongScan& p, int T, int E, bool delta);
-int long_chunks(const LongScan& p, int T, int E, bool delta, cudaStream_t s);
-
 // hybrid_tile.cu: prompt portions as 64-row tiles; normalised per-map outputs to a_out [token][head][map][128]
 struct UmmaTiles {
   float* a_out;
@@ -189,9 +174,8 @@ struct UmmaTiles {
 bool umma_tiles_supported(const UmmaTiles& p, int D, int Dv, float scale);
 int umma_tiles(const UmmaTiles& p, int tokens, cudaStream_t s);
 
-// hybrid_linear.cu: S <- a S + B (dt x)^T, o = S^T C + skip_h x over prepared rows (ssd_row_floats); state fp32 [slots][H][N][Dv]; chunks: long runs may
-// go in chunks on the tensor cores
-int ssd_scan(bool chunks, float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
+// hybrid_linear.cu: S <- a S + B (dt x)^T, o = S^T C + skip_h x over prepared rows (ssd_row_floats); state fp32 [slots][H][N][Dv]
+int ssd_scan(float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
              const int* entry_pos0, int T, int E, int H, int G, int N, int Dv, cudaStream_t s);
 
 }  // namespace qs

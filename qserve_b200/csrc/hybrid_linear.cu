@@ -126,12 +126,11 @@ __host__ __device__ __forceinline__ int scan_row_floats(int mode, int H, int G, 
   return (mode == kScanChannelDecay ? 3 : 2) * H * D + H * Dv;
 }
 
-template <int DP, int PARTS, int CH, int CPT, int MODE, bool VEC, bool SHORT = false>  // VEC: 16-byte staging (D, Dv, the prepared row and its base allow it)
+template <int DP, int PARTS, int CH, int CPT, int MODE, bool VEC>  // VEC: 16-byte staging (D, Dv, the prepared row and its base allow it)
 __global__ void __launch_bounds__(128) linear_scan_kernel(float* __restrict__ o_raw, const float* __restrict__ prep, float* __restrict__ state,
                                                           const float* __restrict__ head_decay, const int* __restrict__ entry_start,
                                                           const int* __restrict__ entry_len, const int* __restrict__ entry_slot,
                                                           const int* __restrict__ entry_pos0, int H, int G, int D, int Dv) {
-  // SHORT: runs of kLongRunTokens and more are another kernel's (a bound read from a parameter in every launch made the scan itself slower)
   // head_decay [H]: kScanHeadDecay the decay, kScanTokenDecay the skip factor
   extern __shared__ __align__(16) float sm[];  // [2][CH][ROW]
   constexpr bool TOKEN = MODE == kScanTokenDecay;
@@ -146,7 +145,6 @@ __global__ void __launch_bounds__(128) linear_scan_kernel(float* __restrict__ o_
   auto vec_at = [&](int which) { return TOKEN ? H * Dv + (1 - which) * GD + gh * D : which * GD + h * D; };
   const int val_at = (TOKEN ? 0 : NVEC * GD) + h * Dv, num_at = H * Dv + 2 * GD + h;
   const int n = entry_len[e], s0 = entry_start[e];
-  if (SHORT && n >= kLongRunTokens) return;
   const bool fresh = entry_pos0[e] == 0;
   float decay = MODE == kScanHeadDecay ? head_decay[h] : 0.f;
   const float skip = TOKEN ? head_decay[h] : 0.f;
@@ -300,30 +298,17 @@ __global__ void linear_out_kernel(ST* __restrict__ out, long long out_stride, co
 }
 
 template <int MODE>
-int launch_scan(bool chunks, float* o_raw, const float* prep, float* state, const float* head_decay, const int* entry_start, const int* entry_len,
+int launch_scan(float* o_raw, const float* prep, float* state, const float* head_decay, const int* entry_start, const int* entry_len,
                 const int* entry_slot, const int* entry_pos0, int T, int E, int H, int G, int D, int Dv, cudaStream_t s) {
   constexpr int NVEC = MODE == kScanChannelDecay ? 3 : 2;
   const int P = scan_row_floats(MODE, H, G, D, Dv);
   const bool vec = D % 4 == 0 && Dv % 4 == 0 && P % 4 == 0 && (reinterpret_cast<uintptr_t>(prep) & 15) == 0;
-  constexpr bool LONG = MODE == kScanHeadDecay || MODE == kScanTokenDecay;
-  bool in_chunks = false;
-  if constexpr (LONG) {  // one decay per token and head: long runs go in chunks on the tensor cores (16-bit storage)
-    constexpr bool TOKEN = MODE == kScanTokenDecay;
-    const int HDv = H * Dv, GD = G * D;
-    const LongScan ls{o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, D, Dv, P, H / G, TOKEN ? HDv + GD : 0,
-                      TOKEN ? HDv : GD, TOKEN ? 0 : 2 * GD, TOKEN ? HDv + 2 * GD : -1, TOKEN ? HDv + 2 * GD + H : -1, TOKEN ? 1 : 0};
-    in_chunks = chunks && long_chunks_supported(ls, T, E, false);
-    if (in_chunks)
-      if (int rc = long_chunks(ls, T, E, false, s)) return rc;
-  }
 #define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
   do {                                                                                                                                        \
     constexpr int cols = 128 / PARTS * CPT;                                                                                                   \
     const size_t smb = (size_t)2 * CH * (NVEC * PARTS * (DP / PARTS + 4) + cols + (MODE == kScanTokenDecay ? 4 : 0)) * sizeof(float);            \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
     auto kern = vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>;                 \
-    if constexpr (LONG && DP == 128)                                                                                                          \
-      if (in_chunks) kern = linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true, true>;                                                         \
     if (smb > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);                                   \
     kern<<<grid, 128, smb, s>>>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                 \
   } while (0)
@@ -347,9 +332,9 @@ int launch_scan(bool chunks, float* o_raw, const float* prep, float* state, cons
 
 }  // namespace
 
-int ssd_scan(bool chunks, float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
+int ssd_scan(float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
              const int* entry_pos0, int T, int E, int H, int G, int N, int Dv, cudaStream_t s) {
-  return launch_scan<kScanTokenDecay>(chunks, o_raw, prep, state, skip, entry_start, entry_len, entry_slot, entry_pos0, T, E, H, G, N, Dv, s);
+  return launch_scan<kScanTokenDecay>(o_raw, prep, state, skip, entry_start, entry_len, entry_slot, entry_pos0, T, E, H, G, N, Dv, s);
 }
 
 }  // namespace qs
@@ -377,7 +362,7 @@ int qs_hyb_gate_recurrence(void* out, int64_t out_stride, float* prep, float* o_
   const int HD = heads * dim, HDv = heads * vdim;
   QS_DT(dtype, (gate_prepare_kernel<__nv_bfloat16><<<tokens_n, 256, 0, s>>>(prep, (const __nv_bfloat16*)proj, stride, f_bias, lower, HD, HDv)),
         (gate_prepare_kernel<float><<<tokens_n, 256, 0, s>>>(prep, (const float*)proj, stride, f_bias, lower, HD, HDv)));
-  if (int rc = launch_scan<kScanChannelGate>(false, o_raw, prep, state, nullptr, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
+  if (int rc = launch_scan<kScanChannelGate>(o_raw, prep, state, nullptr, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
   const int warps = tokens_n * heads;
   QS_DT(dtype,
         (linear_out_kernel<__nv_bfloat16><<<(warps + 3) / 4, 128, 0, s>>>((__nv_bfloat16*)out, out_stride, o_raw, norm_w, nullptr, 0, tokens_n, heads,
@@ -401,7 +386,7 @@ int qs_hyb_retention(void* out, int64_t out_stride, float* prep, float* o_raw, c
                                                                            heads, dim, vdim)),
         (retention_prepare_kernel<float><<<tokens_n, 256, rot_dims * sizeof(float), s>>>(prep, (const float*)proj, stride, tok_pos, inv_freq, rot_dims, k_scale, heads, dim,
                                                                   vdim)));
-  if (int rc = launch_scan<kScanHeadDecay>(dtype == QS_DTYPE_BF16, o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
+  if (int rc = launch_scan<kScanHeadDecay>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
   const int warps = tokens_n * heads;
   const size_t gate_off = (size_t)2 * heads * dim + (size_t)heads * vdim;  // the output gate follows q | k | v in the projection row
   QS_DT(dtype,
@@ -426,7 +411,7 @@ int qs_hyb_gated_linear(void* out, int64_t out_stride, float* prep, float* o_raw
   QS_DT(dtype,
         (gated_linear_prepare_kernel<__nv_bfloat16><<<tokens_n, 256, 0, s>>>(prep, (const __nv_bfloat16*)proj, stride, z, z_bias, inv_tau, q_scale, HD, HDv)),
         (gated_linear_prepare_kernel<float><<<tokens_n, 256, 0, s>>>(prep, (const float*)proj, stride, z, z_bias, inv_tau, q_scale, HD, HDv)));
-  if (int rc = launch_scan<kScanChannelDecay>(false, o_raw, prep, state, nullptr, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
+  if (int rc = launch_scan<kScanChannelDecay>(o_raw, prep, state, nullptr, entry_start, entry_len, entry_slot, entry_pos0, tokens_n, entries, heads, heads, dim, vdim, s)) return rc;
   const int warps = tokens_n * heads;
   const size_t gate_off = (size_t)2 * HD + (size_t)HDv;  // the output gate follows q | k | v in the projection row
   QS_DT(dtype,

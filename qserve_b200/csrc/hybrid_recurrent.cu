@@ -367,7 +367,7 @@ int launch_state_space(void* out, long long out_stride, float* prep, float* o_ra
                                taps, run, shift);
   if (!shift)
     if (int rc = launch_conv_state<ST>(conv_state, proj + inner, stride, nullptr, entry_start, entry_len, entry_slot, entry_pos0, E, C, taps, s)) return rc;
-  if (int rc = ssd_scan(sizeof(ST) == 2, o_raw, prep, state, skip, entry_start, entry_len, entry_slot, entry_pos0, T, E, H, G, N, Dv, s)) return rc;
+  if (int rc = ssd_scan(o_raw, prep, state, skip, entry_start, entry_len, entry_slot, entry_pos0, T, E, H, G, N, Dv, s)) return rc;
   const int part = inner / norm_groups, threads = part >= 1024 ? 256 : 128;
   const size_t smb = (size_t)part * sizeof(float);
   const int vec = part % 4 == 0 && stride % 4 == 0 && out_stride % 4 == 0 && aligned(proj, 4 * sizeof(ST)) && aligned(out, 4 * sizeof(ST)) &&
