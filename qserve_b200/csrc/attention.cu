@@ -176,7 +176,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   const long long* kptrs = kv_pointers + (static_cast<size_t>(b) * 2 + 0) * max_blocks;
   const long long* vptrs = kv_pointers + (static_cast<size_t>(b) * 2 + 1) * max_blocks;
   const int n_pages = (tlen + kPageTokens - 1) / kPageTokens;
-  const int pps = nsplit > 1 ? ((n_pages + nsplit - 1) / nsplit + 1) & ~1 : n_pages;  // even: the two warp pairs of a split get the same number of pages
+  const int pps = (n_pages + nsplit - 1) / nsplit;
   const int p_begin = split * pps, p_end = min(n_pages, p_begin + pps);
   const int last_blk = tlen / pg.tokens_per_block;  // page receiving the new token
 
@@ -642,7 +642,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     if (s_last) {
       // One warp per head, lane = split for the weights (nsplit <= 32), lane = 4 dims for the sum: the maxima and sums of all splits arrive in one
       // round trip to L2 and the partial rows of several splits are in flight together.  (Walking the splits one dependent load after the other
-      // kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits.)
+      // kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits.)  The sums run over the splits in order.
       __threadfence();
       for (int r = warp; r < Gc; r += kWarps) {
         const float* pr = ws_part + (static_cast<size_t>(b) * num_heads + h0 + r) * nsplit * (kD + 2);
@@ -652,15 +652,13 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
 #pragma unroll
         for (int m = 16; m >= 1; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
         const float e = (ms == -CUDART_INF_F) ? 0.f : exp2f(ms - M);
-        float L = ls * e;
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) L += __shfl_xor_sync(0xffffffffu, L, m);
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
         for (int sp = 0; sp < nsplit; ++sp) {
           const float2* row = reinterpret_cast<const float2*>(pr + sp * (kD + 2));  // 130 floats per split: 8-byte aligned
           const float2 x = __ldcg(row + lane), y = __ldcg(row + 32 + lane);
           const float w = __shfl_sync(0xffffffffu, e, sp);
+          L = fmaf(__shfl_sync(0xffffffffu, ls, sp), w, L);
           acc[0] = fmaf(x.x, w, acc[0]); acc[1] = fmaf(x.y, w, acc[1]);
           acc[2] = fmaf(y.x, w, acc[2]); acc[3] = fmaf(y.y, w, acc[3]);
         }
@@ -911,13 +909,12 @@ int decode_attention(const DecodeAttnArgs& a) {
   const int G = a.num_heads / a.num_kv_heads;
   const int gparts = (G + kMaxG - 1) / kMaxG;
   const int gx = a.num_kv_heads * gparts;
-  // context splits: as many CTAs as the machine holds at a time and no more (a last wave of a few CTAs costs a whole CTA's time), never more than one
-  // split per 256 tokens.  Resident CTAs per SM: 4 (128 registers), with INT8 pages 3 (67 KB of page slices each).
+  // context splits: enough CTAs to fill the machine (4 resident CTAs per SM), never more than one split per 256 tokens
   int nsplit = 1;
   const int ctas = gx * a.batch;
-  const int slots = num_sms() * (a.int4_kv ? 4 : 3);
+  const int slots = num_sms() * 4;
   if (2 * ctas <= slots && a.timestep > 512) {
-    nsplit = slots / ctas;
+    nsplit = (slots + ctas - 1) / ctas;
     const int cap = (a.timestep + 255) / 256;
     if (nsplit > cap) nsplit = cap;
     if (nsplit > 32) nsplit = 32;
