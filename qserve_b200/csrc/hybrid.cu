@@ -1514,7 +1514,7 @@ int qs_hyb_attention_fast(void* out, int64_t out_stride, const void* q, int64_t 
     const UmmaTiles ut{scratch, q, kpool, vpool, q_stride, tile_entry, tile_row0, entry_start, entry_len, entry_slot, entry_pos0, block_table, n_tiles,
                        max_blocks, heads, kv_heads, maps, page_size, chunk, window, ex.keep_first, sinks, ex.slopes, scale * 1.4426950408889634f,
                        cap_in(ex, scale), cap_out(ex)};
-    if (umma_tiles_supported(ut, dim, vdim, scale)) rc = umma_tiles(ut, n_long + n_short, s);
+    if (umma_tiles_supported(ut, dim, vdim, scale)) rc = umma_tiles(ut, s);
     else switch (vdim / 16) {
       case 2: QS_TILES(2, kTileKeysPrompt); break;
       case 4: QS_TILES(4, kTileKeysPrompt); break;

@@ -172,7 +172,7 @@ struct UmmaTiles {
   float scale_log2, cap_in, cap_out;
 };
 bool umma_tiles_supported(const UmmaTiles& p, int D, int Dv, float scale);
-int umma_tiles(const UmmaTiles& p, int tokens, cudaStream_t s);
+int umma_tiles(const UmmaTiles& p, cudaStream_t s);
 
 // hybrid_linear.cu: S <- a S + B (dt x)^T, o = S^T C + skip_h x over prepared rows (ssd_row_floats); state fp32 [slots][H][N][Dv]
 int ssd_scan(float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,

@@ -70,8 +70,8 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
 }
 
 template <bool EXTRA>  // EXTRA: a score cap and / or a distance bias
-__global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                                                               const __grid_constant__ CUtensorMap map_v, const UmmaTiles p) {
+__global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                                                               const UmmaTiles p) {
   extern __shared__ __align__(1024) uint8_t sm[];
   // the last tiles of an entry are the longest: they go first, all heads of a tile together
   const int tile = p.n_tiles - 1 - static_cast<int>(blockIdx.y), pairs = p.H >> 1;
@@ -88,10 +88,9 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 12);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
-    for (int i = 0; i < 12; ++i) mbar_init(&bar[i], i == 2 ? 4 : 1);
+    for (int i = 0; i < 12; ++i) mbar_init(&bar[i], i == 0 || i == 2 ? 4 : 1);
     fence_barrier_init();
   }
   if (warp == 5) tmem_alloc<kTmemCols>(s_tmem);
@@ -102,9 +101,6 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
 
   if (warp == 4) {
     if (lane == 0) {
-      mbar_expect_tx(bar_q, 2 * kSubQ);
-      for (int hh = 0; hh < 2; ++hh)
-        for (int c = 0; c < 2; ++c) tma_load_2d(sm + c * kSubQ + hh * kRows * 128, &map_q, ((h0 + hh) * p.maps + m) * kD + c * 64, tok0, bar_q);
       const int* bt = p.block_table + static_cast<size_t>(p.entry_slot[e]) * p.max_blocks;
       auto cell = [&](int i) {
         const int pos = block_at(i) * kKeys;
@@ -153,6 +149,21 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
       }
     }
   } else {
+    {
+      // the queries, into the layout TMA gives the keys.  Not by TMA: a tensor map would have to end at the last token's row, which only the entries' tables
+      // on the device tell
+      const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + static_cast<long long>(tok0) * p.q_stride + (h0 * p.maps + m) * kD;
+#pragma unroll 8
+      for (int j = 0; j < 16; ++j) {
+        const int r = (threadIdx.x >> 4) + j * 8, w = threadIdx.x & 15, qr = r & (kRows - 1);
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (qr < n_rows) x = *reinterpret_cast<const uint4*>(q + qr * p.q_stride + (r >> 6) * p.maps * kD + w * 8);
+        *reinterpret_cast<uint4*>(sm + (w >> 3) * kSubQ + r * 128 + (((w & 7) ^ (r & 7)) << 4)) = x;
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_q);
+    }
     const int row = (warp & 1) * 32 + lane, h = h0 + (warp >> 1);
     const uint32_t t_s = tmem + (static_cast<uint32_t>(warp * 32) << 16), t_o = t_s + kColO;
     const int qpos = qpos0 + row, fk = first_key(qpos, p.chunk, p.window);
@@ -300,19 +311,18 @@ int tensor_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, ui
 }  // namespace
 
 // Heads of 128 and 128 numbers (one swizzled pair of sub-tiles each), an even number of query heads per key / value head (they share the MMA's rows), pages
-// of whole key blocks, a positive scale (the maximum is taken ahead of it), 16-byte rows for TMA.
+// of whole key blocks, a positive scale (the maximum is taken ahead of it), 16-byte rows.
 bool umma_tiles_supported(const UmmaTiles& p, int D, int Dv, float scale) {
   auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
   return D == kD && Dv == kD && p.G > 0 && p.H % (2 * p.G) == 0 && p.page % kKeys == 0 && scale > 0.f && p.q_stride % 8 == 0 && al16(p.q) && al16(p.kpool) &&
          al16(p.vpool) && al16(p.a_out) && p.n_tiles <= 65535;
 }
 
-int umma_tiles(const UmmaTiles& p, int tokens, cudaStream_t s) {
-  CUtensorMap q, k, v;
-  // the pools' extent is not known here: every row that is addressed comes from the block table
+int umma_tiles(const UmmaTiles& p, cudaStream_t s) {
+  CUtensorMap k, v;
+  // the pools' extent is not known here: every row that is addressed lies in a page of the block table
   const uint64_t cells = 0x7fffffff;
-  int rc = tensor_map(&q, p.q, tokens, static_cast<uint64_t>(p.H) * p.maps * kD, p.q_stride);
-  if (!rc) rc = tensor_map(&k, p.kpool, cells, static_cast<uint64_t>(p.G) * p.maps * kD, static_cast<uint64_t>(p.G) * p.maps * kD);
+  int rc = tensor_map(&k, p.kpool, cells, static_cast<uint64_t>(p.G) * p.maps * kD, static_cast<uint64_t>(p.G) * p.maps * kD);
   if (!rc) rc = tensor_map(&v, p.vpool, cells, static_cast<uint64_t>(p.G) * kD, static_cast<uint64_t>(p.G) * kD);
   if (rc) return rc;
   const bool extra = p.cap_in > 0.f || p.slopes != nullptr;
@@ -322,7 +332,7 @@ int umma_tiles(const UmmaTiles& p, int tokens, cudaStream_t s) {
     if (int r = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem), "hyb tile attention smem")) return r;
     done[extra][device_ordinal()] = true;
   }
-  kern<<<dim3(p.H / 2 * p.maps, p.n_tiles), kThreads, kSmem, s>>>(q, k, v, p);
+  kern<<<dim3(p.H / 2 * p.maps, p.n_tiles), kThreads, kSmem, s>>>(k, v, p);
   return check_cuda(cudaGetLastError(), "hyb_attention tiles");
 }
 

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 
-def _run(dev, H, G, maps, lens, pos0, page, D=128, chunk=0, window=0, keep=0, sinks=False, slopes=False, softcap=0.0, gate=None, scale=None, seed=0, spoil=True):
+def _run(dev, H, G, maps, lens, pos0, page, D=128, chunk=0, window=0, keep=0, sinks=False, slopes=False, softcap=0.0, gate=None, scale=None, seed=0, spoil=True, tiles_only=False):
     from qserve_b200._lib import AttnExtra, check, lib
     from qserve_b200.hybrid import StepBatch
 
@@ -48,13 +48,16 @@ def _run(dev, H, G, maps, lens, pos0, page, D=128, chunk=0, window=0, keep=0, si
         if fast:
             check(lib.qs_hyb_attention_fast(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), p(b.tok_slot), p(b.tok_pos),
                                             table.data_ptr(), table.shape[1], p(b.tile_entry), p(b.tile_row0), b.n_tiles, p(b.long_tokens), b.n_long,
-                                            p(b.short_tokens), b.n_short, p(b.entry_start), p(b.entry_len), p(b.entry_slot), p(b.entry_pos0),
+                                            None if tiles_only else p(b.short_tokens), 0 if tiles_only else b.n_short, p(b.entry_start), p(b.entry_len), p(b.entry_slot), p(b.entry_pos0),
                                             scratch.data_ptr(), H, G, maps, D, D, scale, 0.35, 0.8, 1e-5, 1 if maps == 2 else 0, page, chunk, window, p(sk), ex, 0, s))
         else:
             check(lib.qs_hyb_attention(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), p(b.tok_slot), p(b.tok_pos),
                                        table.data_ptr(), table.shape[1], T, H, G, maps, D, D, scale, 0.35, 0.8, 1e-5, 1 if maps == 2 else 0, page, chunk,
                                        window, p(sk), ex, 0, s))
         outs.append(out.float())
+    if tiles_only:
+        assert 0 < b.n_long < T
+        outs = [o[b.long_tokens.long()] for o in outs]
     assert torch.isfinite(outs[1]).all() and torch.isfinite(outs[0]).all()
     # both kernels are fp32 up to the output's rounding: one bfloat16 unit, plus fp32 noise next to zero
     assert ((outs[0] - outs[1]).abs() <= 2 ** -7 * outs[1].abs() + 3e-4).all(), (outs[0] - outs[1]).abs().max()
@@ -85,3 +88,8 @@ def test_options(dev, kw):
 @pytest.mark.parametrize("H,G,page,D,scale", [(3, 3, 64, 128, None), (4, 2, 48, 128, None), (4, 2, 64, 64, None), (4, 2, 64, 128, -0.1)])
 def test_shapes_that_stay_on_the_general_tiles(dev, H, G, page, D, scale):
     _run(dev, H, G, 1, [130], [7], page, D=D, scale=scale)
+
+
+def test_tiles_without_the_short_portions(dev):
+    """A call that lists the tiles of a mixed step alone: its token rows go past the number of rows it lists."""
+    _run(dev, 4, 2, 2, [3, 9, 130, 1, 70], [0, 70, 5, 640, 0], 64, tiles_only=True)
