@@ -128,8 +128,10 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
         const int st = i & 1;
         const uint32_t ph = (static_cast<uint32_t>(i) >> 1) & 1u;
         mbar_wait(&k_full[st], ph);
+        // S goes over the columns of the previous block's P, and products of different shapes and accumulators have no order of their own: the products
+        // with P must have retired
+        if (i > 0) mbar_wait(bar_o, static_cast<uint32_t>(i - 1) & 1u);
         tc_fence_after();
-        // S goes over the columns of the previous block's P: the tensor pipe runs products in issue order
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks)
           mma_ss(tmem, umma_desc_sw128(smem_u32(sm + (ks >> 2) * kSubQ)) + (ks & 3) * 2,
