@@ -177,9 +177,10 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       for (int j = 0; j < n_kb; ++j) {
         const uint32_t ph = static_cast<uint32_t>(j) & 1u;
         mbar_wait(bar_kfull, ph);
+        // S = Q K^T.  The S columns also hold the previous block's P, and MMAs of different shapes and accumulators have no order of their own: the previous
+        // O += P V must have retired.
+        if (j > 0) mbar_wait(bar_o, ph ^ 1u);
         tc_fence_after();
-        // S = Q K^T.  The S columns also hold the previous block's P: the tensor pipe executes MMAs in issue order, so this overwrite follows
-        // the previous O += P V.
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks) {
           const uint32_t off = (ks >> 2) * kSubBytes;
