@@ -2,7 +2,7 @@
 //
 // One CTA = one 64-row tile of an entry x TWO query heads that share a key / value head (the 128 rows of the MMA: rows 0 .. 63 the first head's, 64 .. 127
 // the second's) x one score map.  Keys are walked in blocks of 64 (a block lies in one page: page sizes are multiples of 64):
-//     S = Q K^T      8 x tcgen05.mma 128 x 64 x 16, operands as TMA delivers them (128-byte swizzle), fp32 accumulators in tensor memory
+//     S = Q K^T      8 x tcgen05.mma 128 x 64 x 16, K as TMA delivers it (128-byte swizzle) and Q laid out alike, fp32 accumulators in tensor memory
 //     softmax        4 warps, thread = row: mask, optional cap and distance bias, running maximum and sum in the base-2 domain, fp32
 //     O += P V       the fp32 weights enter as three bfloat16 terms (p = hi + mid + lo, 24 mantissa bits), written over S and beside it in tensor
 //                    memory; 3 x 4 x tcgen05.mma 128 x 128 x 16, B = the V block as TMA delivers it ([key][dim]: MN-major)
