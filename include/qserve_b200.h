@@ -116,7 +116,7 @@ QS_API int qs_apply_bias_rope_update_kv_cache(void* qkv, const int32_t* seq_lens
                                        int int4_kv_cache, int kv_cache_with_zeros, void* stream);
 
 /* Prompt-phase attention: replaces the third-party call flash_attn.flash_attn_varlen_func(q, k, v, cu_seqlens, cu_seqlens, max_seqlen,
- *   max_seqlen, dropout_p=0.0, causal=True) at qserve/modeling/models/llama_w4a8_unpad.py:232-242 (SURVEY.md section 8, row f-3).
+ *   max_seqlen, dropout_p=0.0, causal=True) at qserve/modeling/models/llama_w4a8_unpad.py:232-242.
  *   q [T,Hq,128], k / v [T,Hkv,128] fp16: strided views of the qkv buffer apply_bias_rope_update_kv_cache has rotated in place (row strides in
  *   halfs, multiples of 8); cu_seqlens int32 [batch+1] shared by queries and keys; out fp16 [T,Hq,128].  Causal, no dropout, GQA by
  *   Hq / Hkv.  fp32 softmax, P rounded to fp16 before the second MMA (as flash-attn does); tcgen05 kind::f16, sm_100a only.
@@ -150,13 +150,13 @@ QS_API int qs_invoke_quant(int8_t* out, const void* input, void* scale /* fp16 [
 QS_API int qs_invoke_quant_scalar(int8_t* out, const void* input, float scale, int tokens, int hidden, void* stream);
 QS_API int qs_invoke_quant_fuse_sum(int8_t* out, const void* input, void* input_sum, void* scale, int tokens, int hidden, void* stream);
 /* Tensor-parallel extension (no reference counterpart: the reference has tp_size = 1 hard-coded, llama_w4a8_unpad.py:115).
- * SURVEY.md 8e parity rule: all ranks quantise their K shard of a token with the same scale.  qs_row_absmax writes the local
+ * Parity rule: all ranks quantise their K shard of a token with the same scale.  qs_row_absmax writes the local
  * per-token max |x| (fp32 [tokens]); the caller max-all-reduces it; qs_invoke_quant_given_amax then does the arithmetic of
  * invoke_quant[_fuse_sum] with that amax (input_sum, may be null, is the LOCAL shard's row sum). */
-/* Tensor-parallel extension: the sum-all-reduce of a row-parallel GEMM output fused into its consumer ("fused into
- * the GEMM epilogue ... over NVLink").  delta_ptrs[r] = address, valid in THIS process, of rank r's fp16 partial [tokens, hidden] of this
+/* Tensor-parallel extension: the sum-all-reduce of a row-parallel GEMM output fused into its consumer over NVLink.
+ * delta_ptrs[r] = address, valid in THIS process, of rank r's fp16 partial [tokens, hidden] of this
  * phase (peer-mapped symmetric memory); flag_ptrs[r] = rank r's flag pad (16 x u32, zero-initialised, peer-mapped); state = 4 x u32 of
- * local device memory, zero-initialised, owned by the library afterwards.  phase 0 / 1 = o_proj / down_proj (two buffers: see DESIGN.md 6).
+ * local device memory, zero-initialised, owned by the library afterwards.  phase 0 / 1 = o_proj / down_proj (two buffers).
  * Semantics: delta = fp16(sum over ranks, fp32, rank order) ; then exactly qs_add_rms_norm_general(out, hidden_out, x, delta, ...).
  * All ranks must issue the same sequence of peer calls. */
 QS_API int qs_add_rms_norm_general_peer(int8_t* out, void* hidden_out, const void* x, const void* const* delta_ptrs, void* const* flag_ptrs, void* state,
@@ -181,7 +181,7 @@ QS_API int qs_dequant_silu_and_mul_quant(int8_t* out, const int32_t* input, floa
 
 /* ---------------------------------------------------------------------------------------------------------
  * Fused extensions (NOT part of the reference surface; bit-identical to the op sequences they replace).
- * Used by qserve_b200/decode.py to cut the launch count of the decode step (SURVEY.md section 8f-2).
+ * Used by qserve_b200/decode.py to cut the launch count of the decode step.
  * --------------------------------------------------------------------------------------------------------- */
 /* hidden_out = half(x + delta)   [the torch `residual + out_buf` of llama_w4a8_unpad.py:348,360]
  * followed by rms_norm_general[_fuse_sum](out, hidden_out, weight, input_sum | NULL, scaling, epsilon, per_token=1)      */

@@ -1,4 +1,4 @@
-"""QServe checkpoints: produce and consume the reference's real-quantised state dict (SURVEY.md section 8f-1).
+"""QServe checkpoints: produce and consume the reference's real-quantised state dict.
 
 * `quantize_w4a8` / `quantize_w8a8` -- the arithmetic of `W4A8OF16LinearDynamicInputScale.from_linear`
   (qserve/modeling/layers/quantized_linear/w4a8_linear.py:136-332) and `W8A8OF16LinearDynamicInputScale.from_linear`
@@ -33,7 +33,7 @@ def pack_int4(q: torch.Tensor) -> torch.Tensor:
 
     A 32x32 tile is 512 contiguous bytes = 32 lanes x 16 B; lane t = c*4 + e, byte j = d*8 + b*4 + f holds
     q[32 n32 + 8 b + c, 32 k32 + 16 d + 4 e + f] in its low and the same element of row +16 in its high nibble
-    (SURVEY.md appendix A1; the consumer side is gemm_cuda.cu:286-298)."""
+    (the consumer side is gemm_cuda.cu:286-298)."""
     N, K = q.shape
     if N % 32 or K % 32:
         raise ValueError(f"pack_int4: N={N} and K={K} must be multiples of 32")

@@ -5,7 +5,7 @@
 //           kernels/csrc/fused_attention/applyBiasRopeUpdateKVCache.h:94-455 (prefill append),
 //           kernels/csrc/fused_attention/input_metadata_helper.cu:11-45.
 //
-// B200 design (DESIGN.md 3.2): the reference launches one CTA per *query* head and therefore streams every KV head
+// B200 design: the reference launches one CTA per *query* head and therefore streams every KV head
 // Hq/Hkv times; here one CTA (4 warps) owns a (sequence, KV head, context split) and serves all query heads of the GQA
 // group from a single pass over the pages, so HBM traffic is the algorithmic minimum.  Every warp streams its own 32-token
 // slices of the pages with cp.async.bulk into a private shared-memory ring; the (<= 8 heads) x 32-token QK^T and PV

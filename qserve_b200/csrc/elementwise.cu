@@ -192,7 +192,7 @@ constexpr int kGammaPre = 4;  // gamma chunks (8 halves each) a thread keeps in 
 //      rounds once to fp16 -- the value an fp16 all-reduce would have delivered, without its per-hop roundings -- and continues as
 //      add_rms_norm_general.  No NCCL call, no extra kernel boundary, the NVLink transfer overlaps the other rows' norm arithmetic.
 // Two phases (o_proj / down_proj) use two buffers, so a rank that runs ahead can never overwrite a partial a slower peer still reads:
-// buffer p is rewritten only after a kernel that waited for the peers' NEXT-phase flags (see DESIGN.md 6).
+// buffer p is rewritten only after a kernel that waited for the peers' NEXT-phase flags.
 struct PeerArgs {
   const __half* delta[8];   // partial-output buffer of this phase on every rank (peer-mapped addresses), indexed by rank
   uint32_t* flags[8];       // flag pad of every rank (peer-mapped): 16 x u32, [phase * 8 + source rank]
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kThreads) quant_per_token_kernel(int8_t* __res
   }
 }
 
-// Tensor-parallel parity rule (SURVEY.md 8e): a row-parallel GEMM keeps INT32 partial sums that add up to the single-GPU
+// Tensor-parallel parity rule: a row-parallel GEMM keeps INT32 partial sums that add up to the single-GPU
 // accumulators only if every rank quantises its K shard of a token with the SAME per-token scale.  row_absmax -> [M] fp32
 // max-allreduce -> quant_given_amax does exactly the arithmetic of quant_per_token_kernel with the global amax; the row sum
 // (per-channel W4A8 zero-point term) stays the LOCAL shard's sum.

@@ -4,7 +4,7 @@
 //           kernels/csrc/qgemm/w4a8_per_group/gemm_cuda.cu:328-702,
 //           kernels/csrc/qgemm/w8a8/w8a8_gemm_cuda.cu:267-577        (reference: mma.sync + ldmatrix + cp.async)
 //
-// B200 design (see DESIGN.md "GEMM"):
+// B200 design:
 //   * swap-AB: the 128 output channels of a tile are the UMMA M dimension, the tokens are UMMA N (<= 256),
 //     so decode-sized batches (M = 64 tokens) still use full-height 128-row tensor-core instructions.
 //   * the packed INT4 weights are consumed in the checkpoint's own "compute-aware reordered" layout

@@ -11,8 +11,8 @@
 //
 // Why: mma.sync with register fragments left the tensor pipe 51 % busy at 260 TFLOP/s of executed work (keys loaded once per head, 4 warps x 168
 // registers).  Both heads of the pair read one copy of K and V here, and the three terms cost issue slots only once, on the way to tensor memory.
-// Measured: 4 prompts of 1297 .. 2048 tokens, 16 heads, 4 key / value heads, 2 maps: 732 -> 243 us (795 TFLOP/s of executed work, 0.48 of the measured bf16
-// peak); what bounds it is the chain S -> softmax -> P -> O of a block with two CTAs to interleave.
+// Measured: 4 prompts of 1297 .. 2048 tokens, 16 heads, 4 key / value heads, 2 maps: 732 -> 259 us (746 TFLOP/s of executed work, 0.45 of the measured bf16
+// peak); what bounds it is the chain S -> softmax -> P -> O of a block with two CTAs to interleave.  The next block's S waits for O (without: 243).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math_constants.h>

@@ -2,7 +2,7 @@
 //
 // Replaces the third-party call on the reference's prompt path: flash_attn_varlen_func(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen,
 // dropout_p=0, causal=True) in qserve/modeling/models/llama_w4a8_unpad.py:232-242, where q / k / v are strided views of the post-RoPE fp16 qkv
-// buffer that fused_attention.apply_bias_rope_update_kv_cache has just rotated in place (SURVEY.md section 8 row f-3).
+// buffer that fused_attention.apply_bias_rope_update_kv_cache has just rotated in place.
 //
 // One CTA = one (sequence, query head, block of 128 query rows).  Per block of 128 keys:
 //     S = Q K^T      8 x tcgen05.mma 128x128x16, both operands K-major in shared memory (TMA, 128-byte swizzle), fp32 accumulators in TMEM

@@ -1,16 +1,16 @@
 """Decode-step runner: the reference's per-layer op sequence over the drop-in `qserve_backend` API, with persistent
 activation buffers and whole-step CUDA-graph capture.
 
-This is the measurement harness for BASELINE.json's metric (tokens/s, Llama-3-8B W4A8KV4 decode) and the
-"step-level CUDA-graph runner under the unchanged model code" of SURVEY.md section 8f-2.  It issues exactly the calls
+This is the measurement harness for the headline metric (tokens/s, Llama-3-8B W4A8KV4 decode) and the
+step-level CUDA-graph runner under the unchanged model code.  It issues exactly the calls
 `LlamaDecoderLayer.forward` issues (qserve/modeling/models/llama_w4a8_unpad.py:330-361, 69-93, 186-291; W8A8:
 llama_w8a8_unpad.py) with the same argument marshalling, on synthetic weights of the named architecture
 (random INT4/INT8 codes, scales chosen so that activations stay O(1); there is no network for checkpoints).
 
-Tensor parallelism (SURVEY.md section 8e) is Megatron style: qkv / gate_up column parallel, o_proj / down_proj row parallel
+Tensor parallelism is Megatron style: qkv / gate_up column parallel, o_proj / down_proj row parallel
 (split along K in multiples of 128), KV heads sharded, one NCCL sum-allreduce of [M, hidden] fp16 after each row-parallel
 GEMM.  Two quantisation modes for the inputs of the row-parallel GEMMs:
-  * `tp_exact=True` -- SURVEY.md 8e parity rule: the per-token amax is max-all-reduced ([M] fp32) so every rank uses the SAME
+  * `tp_exact=True` -- parity rule: the per-token amax is max-all-reduced ([M] fp32) so every rank uses the SAME
     scale, the activation sum stays the local K shard's: the INT32 partial sums of the ranks add up to the single-GPU
     accumulators bit for bit (tests/test_gpu_tp.py); costs one extra tiny collective per row-parallel GEMM;
   * `tp_exact=False` (throughput mode) -- every rank quantises its shard with its own per-token scale inside the fused
@@ -196,7 +196,7 @@ class DecodeRunner:
     def _quant(self, out_q, x):
         """Per-token quantisation of the input of a ROW-parallel GEMM (o_proj, down_proj)."""
         if self.tp_size > 1 and self.tp_exact:
-            # SURVEY.md 8e: same per-token scale on all ranks (global amax), local-K-shard activation sum
+            # same per-token scale on all ranks (global amax), local-K-shard activation sum
             _ext.row_absmax(self.q_amax, x)
             if not self.no_comm:
                 torch.distributed.all_reduce(self.q_amax, op=torch.distributed.ReduceOp.MAX, group=self.pg)
@@ -409,7 +409,7 @@ class DecodeRunner:
         return sum(l.weight_bytes() for ly in self.layers for l in (ly["qkv"], ly["o"], ly["gate_up"], ly["down"]))
 
     def kv_bytes_per_step(self) -> int:
-        """Algorithmic KV traffic (SURVEY.md 8d): codes + scale/zero of K and V for ctx tokens, + q in / o out."""
+        """Algorithmic KV traffic: codes + scale/zero of K and V for ctx tokens, + q in / o out."""
         B, D = self.batch, self.cfg.head_dim
         per_layer = B * self.Hkv * self.ctx * D * self.kv_bits // 8 * 2 + B * self.Hkv * self.ctx * 8 + 4 * B * self.Hq * D
         return per_layer * self.L

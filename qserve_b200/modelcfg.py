@@ -1,5 +1,5 @@
 """Architecture table of the benchmark models (pure Python: importing it does NOT load libqserve_b200.so, so the CPU
-baseline arm of bench.py can use it without touching the product library).  Dimensions: SURVEY.md section 8."""
+baseline arm of bench.py can use it without touching the product library)."""
 from __future__ import annotations
 
 from dataclasses import dataclass

@@ -1,7 +1,6 @@
 """Run the reference's UNMODIFIED Python model code (`qserve/modeling/**`) over this repo's `qserve_backend`.
 
-north_star: "... keeps the qserve_backend torch-extension op signatures so qserve/modeling and the in-flight-batching engine
-drop in unchanged".  This module is the proof harness for that sentence: it imports the reference's
+The operator signatures of `qserve_backend` are kept so that qserve/modeling drops in unchanged; this module shows it: it imports the reference's
 `LlamaForCausalLM` (qserve/modeling/models/llama_w4a8_unpad.py:417-477) -- which in turn imports the reference's own
 `W4A8OF16LinearDynamicInputScale`, `RMSNormGeneral`, `SiluAndMulQuant`, `InputMetadata` / `ActivationBuffer` -- with
 `qserve_backend` resolving to THIS repo, fills its buffers with the same synthetic weights / KV pages a `DecodeRunner` owns

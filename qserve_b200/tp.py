@@ -1,4 +1,4 @@
-"""Tensor-parallel sharding of QServe checkpoints (host-side logic, SURVEY.md section 8e).
+"""Tensor-parallel sharding of QServe checkpoints (host-side logic).
 
 The packed INT4 layout (w4a8_linear.py:292-322) stores one 32x32 tile per 512 contiguous bytes, tiles K-major inside
 a 32-channel band, so
