@@ -18,7 +18,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libqserve_b200.so")
 BIND = os.path.join(HERE, "_bind.so")  # CPython binding of the hot operators (bind.cpp): the one part that is built against torch
 SOURCES = ["capi.cu", "gemm.cu", "attention.cu", "prefill_attention.cu", "elementwise.cu", "hybrid.cu", "hybrid_blocks.cu", "hybrid_linear.cu", "hybrid_latent.cu",
-           "hybrid_recurrent.cu", "hybrid_tile.cu"]
+           "hybrid_recurrent.cu", "hybrid_scan.cu", "hybrid_tile.cu"]
 HEADERS = ["common.cuh", "hybrid_common.cuh", "hybrid_conv.cuh", "launch.h", os.path.join("..", "..", "include", "qserve_b200.h")]
 
 NVCC_FLAGS = [

@@ -174,6 +174,21 @@ struct UmmaTiles {
 bool umma_tiles_supported(const UmmaTiles& p, int D, int Dv, float scale);
 int umma_tiles(const UmmaTiles& p, cudaStream_t s);
 
+// hybrid_scan.cu: a recurrence over prepared rows (what the modes compute stands there).  A row has `row` floats; vectors q, g, a of head h start at
+// p.q + (h / heads_per_vec) * D and so on, its values at v + h * Dv, its two numbers of the token (kScanTokenDecay: dt, a; kScanDelta: beta, decay) at n0 + h
+// and n1 + h.
+constexpr int kScanHeadDecay = 0, kScanChannelGate = 1, kScanChannelDecay = 2, kScanTokenDecay = 3, kScanDelta = 4;
+struct ScanArgs {
+  float* o_raw;              // [tokens][H][Dv]
+  const float* prep;
+  float* state;              // [slots][H][D][Dv]
+  const float* head_number;  // [H] or null
+  const int *entry_start, *entry_len, *entry_slot, *entry_pos0;
+  int row, q, g, a, v, n0, n1, heads_per_vec, E, H, D, Dv;
+};
+bool column_scan_takes(const ScanArgs& p);
+int column_scan(const ScanArgs& p, int mode, cudaStream_t s);
+
 // hybrid_linear.cu: S <- a S + B (dt x)^T, o = S^T C + skip_h x over prepared rows (ssd_row_floats); state fp32 [slots][H][N][Dv]
 int ssd_scan(float* o_raw, const float* prep, float* state, const float* skip, const int* entry_start, const int* entry_len, const int* entry_slot,
              const int* entry_pos0, int T, int E, int H, int G, int N, int Dv, cudaStream_t s);

@@ -118,8 +118,6 @@ __device__ __forceinline__ float part_sum(float v) {
   return v;
 }
 
-constexpr int kScanHeadDecay = 0, kScanChannelGate = 1, kScanChannelDecay = 2, kScanTokenDecay = 3;
-
 // floats of a prepared row; G: heads that have a q / g of their own
 __host__ __device__ __forceinline__ int scan_row_floats(int mode, int H, int G, int D, int Dv) {
   if (mode == kScanTokenDecay) return ssd_row_floats(H, G, D, Dv);
@@ -303,30 +301,39 @@ int launch_scan(float* o_raw, const float* prep, float* state, const float* head
   constexpr int NVEC = MODE == kScanChannelDecay ? 3 : 2;
   const int P = scan_row_floats(MODE, H, G, D, Dv);
   const bool vec = D % 4 == 0 && Dv % 4 == 0 && P % 4 == 0 && (reinterpret_cast<uintptr_t>(prep) & 15) == 0;
-#define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
+  // Long runs of tokens (prompt portions) on 65 to 128 rows: hybrid_scan.cu, bit for bit the kernel below with 8 parts and 2 columns.  Steps of mostly single
+  // tokens are bound by reading and writing the state and keep one column per thread of four parts
+  const bool long_runs = T >= 32 * E;
+  if (long_runs && D > 64 && D <= 128 && Dv >= 64) {
+    ScanArgs a{o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, P, 0, G * D, 2 * G * D, NVEC * G * D, 0, 0, H / G, E, H, D, Dv};
+    if (MODE == kScanTokenDecay) a.q = H * Dv + G * D, a.g = H * Dv, a.a = a.v = 0, a.n0 = H * Dv + 2 * G * D, a.n1 = a.n0 + H;
+    if (column_scan_takes(a)) return column_scan(a, MODE, s);
+  }
+#define QS_SCAN_AS(DP, PARTS, CH, CPT, KERNEL)                                                                                                           \
   do {                                                                                                                                        \
     constexpr int cols = 128 / PARTS * CPT;                                                                                                   \
     const size_t smb = (size_t)2 * CH * (NVEC * PARTS * (DP / PARTS + 4) + cols + (MODE == kScanTokenDecay ? 4 : 0)) * sizeof(float);            \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
-    auto kern = vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>;                 \
+    auto kern = KERNEL;                 \
     if (smb > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);                                   \
     kern<<<grid, 128, smb, s>>>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                 \
   } while (0)
+#define QS_SCAN(DP, PARTS, CH, CPT) QS_SCAN_AS(DP, PARTS, CH, CPT, (vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>))
   // rows of a column per thread: all of them up to 32, 32 or 16 above (the parts of a column meet through shuffles).  Long runs of tokens
   // (prompt portions) take two adjacent columns per thread where the head has the columns for it: a q / g word read from shared memory then
   // feeds two columns; steps of mostly single tokens are bound by reading and writing the state and keep one column per thread
-  const bool long_runs = T >= 32 * E;
   if (D <= 16) QS_SCAN(16, 1, 16, 1);
   else if (D <= 32) QS_SCAN(32, 1, 16, 1);
   else if (D <= 64) { if (Dv >= 128 && long_runs) QS_SCAN(64, 2, 16, 2); else QS_SCAN(64, 2, 16, 1); }
   // (three row vectors per token: chunks of 8 tokens keep a block's staging near 32 KB, so that as many blocks share an SM as with two)
-  else if (D <= 128) {
-    if (Dv >= 64 && long_runs) { if (NVEC == 3) QS_SCAN(128, 8, 8, 2); else QS_SCAN(128, 8, 16, 2); }
+  else if (D <= 128) {  // (long runs of rows, values and state in 16-byte words do not come here)
+    if (Dv >= 64 && long_runs) { if (NVEC == 3) QS_SCAN_AS(128, 8, 8, 2, (linear_scan_kernel<128, 8, 8, 2, MODE, false>)); else QS_SCAN_AS(128, 8, 16, 2, (linear_scan_kernel<128, 8, 16, 2, MODE, false>)); }
     else QS_SCAN(128, 4, 16, 1);
   }
   else if (D <= 256) QS_SCAN(256, 8, 8, 1);
   else QS_SCAN(512, 16, 4, 1);
 #undef QS_SCAN
+#undef QS_SCAN_AS
   return check_cuda(cudaGetLastError(), "hyb linear scan");
 }
 

@@ -1,0 +1,73 @@
+"""The recurrences over heads of 65 to 128 state rows (hybrid_scan.cu) against the general kernels, which take the same rows when the state does not lie on a
+16-byte boundary: the same sums in the same order, so the same bits, for every recurrence, every number of columns per thread (which follows the number of
+(sequence, head, column) units), heads that fill neither the rows nor the column blocks, odd and even runs, runs of one token, and more sequences than a
+warp has lanes."""
+import pytest
+import torch
+
+from .test_gpu_long_runs import F32, DEV, GatedDelta, Retention, StateSpace, _Layer, _tables
+
+pytestmark = pytest.mark.gpu
+
+
+class _OwnVectors(_Layer):
+    """Rows with a q, a g [and a decay] of every head."""
+
+    def __init__(self, seed, dtype, slots, H, G, D, Dv):
+        super().__init__(seed, dtype, slots)
+        self.H, self.D, self.Dv, r = H, D, Dv, self.rand
+        self.bias, self.low, self.norm_w = r(H * D), torch.rand(H * D, device=DEV, generator=self.gen) * 0.9, torch.ones(Dv, device=DEV)
+        self.state = r(slots, H, D, Dv) * 0.3
+
+
+class GateRecurrence(_OwnVectors):
+    W = property(lambda self: 2 * self.H * self.D + self.H * self.Dv)
+
+    def step(self, proj, lens, pos0, slots):
+        from qserve_b200._lib import check, lib
+
+        tab, _ = _tables(lens, pos0, slots)
+        T, p = sum(lens), lambda t: t.data_ptr()
+        prep, o, out = self.buffers(T, self.W, self.H * self.Dv)
+        check(lib.qs_hyb_gate_recurrence(p(out), self.H * self.Dv, p(prep), p(o), p(proj), proj.stride(0), p(self.bias), p(self.low), p(self.norm_w), p(self.state),
+                                         *map(p, tab[2:]), T, len(lens), self.H, self.D, self.Dv, 1e-5, self.dt, self.stream()))
+        return prep, o, out
+
+
+class GatedLinear(_OwnVectors):
+    W = property(lambda self: 2 * self.H * (self.D + self.Dv))
+
+    def step(self, proj, lens, pos0, slots):
+        from qserve_b200._lib import check, lib
+
+        tab, _ = _tables(lens, pos0, slots)
+        T, p = sum(lens), lambda t: t.data_ptr()
+        prep, o, out = self.buffers(T, 3 * self.H * self.D + self.H * self.Dv, self.H * self.Dv)
+        z = proj.float().sum(1, keepdim=True) * 0.1 + self.bias
+        check(lib.qs_hyb_gated_linear(p(out), self.H * self.Dv, p(prep), p(o), p(proj), proj.stride(0), p(z), p(self.bias), 16.0, p(self.norm_w), p(self.state),
+                                      *map(p, tab[2:]), T, len(lens), self.H, self.D, self.Dv, 1e-5, self.dt, self.stream()))
+        return prep, o, out
+
+
+RUNS = {"1 column": ([35, 64, 37], [0, 5, 0], 2), "2 columns": ([33, 1, 100, 45, 36], [0, 3, 8, 0, 1], 8), "4 columns": ([32, 77, 1, 95, 40, 34], [0, 5, 4, 0, 0, 9], 24),
+        "40 sequences": ([32 + i % 5 for i in range(40)], [i % 3 for i in range(40)], 4)}
+
+
+@pytest.mark.parametrize("runs", RUNS)
+@pytest.mark.parametrize("D,Dv", [(128, 128), (128, 64), (68, 100), (100, 132)])
+@pytest.mark.parametrize("kind", [StateSpace, Retention, GatedDelta, GateRecurrence, GatedLinear])
+def test_bits_of_the_general_kernel(kind, D, Dv, runs):
+    lens, pos0, H = RUNS[runs]
+    got = []
+    for aligned in (True, False):
+        layer = kind(7, F32, len(lens), H, 1 if kind in (StateSpace, GatedDelta) else H, D, Dv)
+        if kind is Retention:
+            layer.decay, layer.skip = torch.rand(H, device=DEV, generator=layer.gen), torch.zeros(H, device=DEV)
+        if not aligned:
+            shifted = torch.empty(layer.state.numel() + 1, device=DEV)[1:].view_as(layer.state)
+            layer.state = shifted.copy_(layer.state)
+        proj = layer.rand(sum(lens), layer.W)
+        _, o, _ = layer.step(proj, lens, pos0, list(range(len(lens)))[::-1])
+        assert torch.isfinite(o).all()
+        got.append((o, layer.state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
