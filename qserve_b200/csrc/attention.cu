@@ -88,24 +88,24 @@ constexpr int kAttnThreadsV2 = kAttnConsumers;  // no dedicated producer warp: e
 constexpr int kPageTokens = 64;
 constexpr int kOStride = kD + 4;  // floats per (warp, head) row of the merge buffer
 
-// One stage = the 32-token slice of one 64-token page of one kv head that a warp consumes in one iteration:
-// K codes | V codes | K scales | K zeros | V scales | V zeros.  Each warp owns a private ring of kStages such slices, filled by
-// its lane 0 with six cp.async.bulk copies and guarded by one "full" mbarrier per slot (the refill of a slot is issued by the
-// same warp right after it has consumed it, so no "empty" barrier and no producer warp are needed).
+// A warp consumes 32-token slices of the 64-token pages of one kv head.  Each warp owns a private ring of kSlots slots, filled by its lane 0 with
+// cp.async.bulk copies and guarded by one "full" mbarrier per slot (the refill of a slot is issued by the same warp right after it has consumed it, so no
+// "empty" barrier and no producer warp are needed).  INT4: a slot holds a whole slice, K codes | V codes | K scales | K zeros | V scales | V zeros, and the
+// ring two.  INT8: a slot holds one half of a slice, first K, then V (codes | scales | zeros), and the ring three: 135 KB are on their way per SM where two
+// whole slices take so much that only three CTAs fit, and 64 sequences x 8 heads need a second wave (45 us, now 34; INT4 with slots of halves: 3 % slower,
+// its CTAs fit either way and a wait more per slice is what remains).
 constexpr int kSliceTokens = 32;
 template <int BITS>
 struct StageLayout {
   static constexpr int kCodes = kPageTokens * kD * BITS / 8;       // bytes of K (or V) codes of one head-page
   static constexpr int kSliceCodes = kSliceTokens * kD * BITS / 8;  // ... of one 32-token slice
-  static constexpr int kOffK = 0;
-  static constexpr int kOffV = kSliceCodes;
-  static constexpr int kOffKs = 2 * kSliceCodes;   // fp16 [32]
-  static constexpr int kOffKz = kOffKs + 64;
-  static constexpr int kOffVs = kOffKz + 64;
-  static constexpr int kOffVz = kOffVs + 64;
-  static constexpr int kBytes = kOffVz + 64;
-  static constexpr int kStages = 2;
-  static constexpr int kWarpBytes = kStages * kBytes;  // private ring of one warp (also holds its partial O^T at the end)
+  static constexpr int kPerSlice = BITS == 4 ? 1 : 2;               // slots of a slice
+  static constexpr int kSlots = BITS == 4 ? 2 : 3;
+  static constexpr int kOffV = kPerSlice == 1 ? kSliceCodes : 0;    // V codes in their slot
+  static constexpr int kOffKm = kPerSlice == 1 ? 2 * kSliceCodes : kSliceCodes;  // fp16 K scales [32] | zeros [32]
+  static constexpr int kOffVm = kPerSlice == 1 ? kOffKm + 128 : kOffKm;
+  static constexpr int kBytes = kOffVm + 128;
+  static constexpr int kWarpBytes = kSlots * kBytes;  // private ring of one warp (also holds its partial O^T at the end)
   static_assert(kWarpBytes >= kMaxG * kOStride * 4, "the per-warp ring must hold the warp's partial output");
 };
 
@@ -132,7 +132,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
                         int timestep, int nsplit, float* __restrict__ ws_part, uint32_t* __restrict__ ws_cnt, uint32_t* __restrict__ tok_cnt, int8_t* __restrict__ q_out,
                         __half* __restrict__ q_scale, __half* __restrict__ q_sum, unsigned long long* __restrict__ prof) {
   using SL = StageLayout<BITS>;
-  constexpr int R = SL::kStages;
+  constexpr int R = SL::kSlots;
   const int G = num_heads / num_kv_heads;
   const int gparts = (G + kMaxG - 1) / kMaxG;
   const int hk = blockIdx.x / gparts;
@@ -145,7 +145,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   const int g = lane >> 2, q4 = lane & 3;
 
   extern __shared__ __align__(128) uint8_t smem_attn[];
-  uint8_t* s_ring = smem_attn;                                           // kWarps private rings of R slices
+  uint8_t* s_ring = smem_attn;                                           // kWarps private rings of R slots
   __shared__ __align__(16) __half s_q[kMaxG * kD];
   __shared__ __align__(16) __half s_k[kD];
   __shared__ __align__(16) __half s_v[kD];
@@ -177,6 +177,17 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   const long long* vptrs = kv_pointers + (static_cast<size_t>(b) * 2 + 1) * max_blocks;
   const int n_pages = (tlen + kPageTokens - 1) / kPageTokens;
   const int pps = nsplit > 1 ? (n_pages + nsplit - 1) / nsplit : n_pages;  // no division ahead of the first copy where there are no splits
+  // splits that hold pages: a CTA beyond them leaves empty partial rows behind and takes no part in the merge (with a prologue and a place in the merge of
+  // its own it was the last to finish where it did not fit the first wave)
+  const int used = nsplit > 1 ? max(1, (n_pages + pps - 1) / max(pps, 1)) : 1;
+  if (split >= used) {
+    pdl_wait();
+    for (int i = threadIdx.x; i < Gc * (kD + 2); i += kAttnThreadsV2) {
+      const int r = i / (kD + 2), d = i - r * (kD + 2);
+      ws_part[((static_cast<size_t>(b) * num_heads + h0 + r) * nsplit + split) * (kD + 2) + d] = d == kD ? -CUDART_INF_F : 0.f;
+    }
+    return;
+  }
   const int p_begin = split * pps, p_end = min(n_pages, p_begin + pps);
   const int last_blk = tlen / pg.tokens_per_block;  // page receiving the new token
 
@@ -187,41 +198,62 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   uint8_t* my_ring = s_ring + warp * SL::kWarpBytes;
   uint64_t* my_full = &s_full[warp][0];
   const int zoff = pg.num_kv_heads * pg.tokens_per_block * 2;  // bytes from a scale row to the zero row
-  long long kp_l = 0, vp_l = 0;  // lane l: page pointers of this warp's page (batch * 32 + l)
-  auto load_ptr_batch = [&](int j0) {
+  long long kp_l = 0, vp_l = 0;  // lane l: page pointers of this warp's pages (batch * 32 + l); K runs ahead of V
+  auto load_ptrs = [&](long long& ptr, const long long* table, int j0) {
     const int pidx = my_first + 2 * (j0 + lane);
-    kp_l = (pidx < p_end) ? kptrs[pidx] : 0;
-    vp_l = (pidx < p_end) ? vptrs[pidx] : 0;
+    ptr = (pidx < p_end) ? table[pidx] : 0;
   };
-  auto issue = [&](int j, int slot) {  // all lanes call; lane 0 issues the six copies of this warp's j-th slice into `slot`
-    const long long kp_j = __shfl_sync(0xffffffffu, kp_l, j & 31), vp_j = __shfl_sync(0xffffffffu, vp_l, j & 31);
-    if (lane == 0) {
-      const uint8_t* kpage = reinterpret_cast<const uint8_t*>(kp_j);
-      const uint8_t* vpage = reinterpret_cast<const uint8_t*>(vp_j);
+  // all lanes call; lane 0 issues the copies of this warp's u-th slot contents into slot `slot`: slice u, or half u & 1 of slice u >> 1
+  const int units = SL::kPerSlice * n_my;
+  auto issue = [&](int u, int slot) {
+    const int j = u / SL::kPerSlice;
+    auto copy = [&](const uint8_t* page, int codes_at, int meta_at) {
       uint8_t* dst = my_ring + slot * SL::kBytes;
-      fence_proxy_async();  // the slot was last read through the generic proxy
-      mbar_expect_tx(&my_full[slot], SL::kBytes);
-      bulk_copy_g2s(dst + SL::kOffK, kpage + static_cast<size_t>(hk) * SL::kCodes + hslice * SL::kSliceCodes, SL::kSliceCodes, &my_full[slot]);
-      bulk_copy_g2s(dst + SL::kOffV, vpage + static_cast<size_t>(hk) * SL::kCodes + hslice * SL::kSliceCodes, SL::kSliceCodes, &my_full[slot]);
-      const uint8_t* kmeta = kpage + pg.code_bytes + hk * 128 + hslice * 64;
-      const uint8_t* vmeta = vpage + pg.code_bytes + hk * 128 + hslice * 64;
-      bulk_copy_g2s(dst + SL::kOffKs, kmeta, 64, &my_full[slot]);
-      bulk_copy_g2s(dst + SL::kOffKz, kmeta + zoff, 64, &my_full[slot]);
-      bulk_copy_g2s(dst + SL::kOffVs, vmeta, 64, &my_full[slot]);
-      bulk_copy_g2s(dst + SL::kOffVz, vmeta + zoff, 64, &my_full[slot]);
+      bulk_copy_g2s(dst + codes_at, page + static_cast<size_t>(hk) * SL::kCodes + hslice * SL::kSliceCodes, SL::kSliceCodes, &my_full[slot]);
+      const uint8_t* meta = page + pg.code_bytes + hk * 128 + hslice * 64;
+      bulk_copy_g2s(dst + meta_at, meta, 64, &my_full[slot]);
+      bulk_copy_g2s(dst + meta_at + 64, meta + zoff, 64, &my_full[slot]);
+    };
+    if constexpr (SL::kPerSlice == 1) {
+      const long long kp = __shfl_sync(0xffffffffu, kp_l, j & 31), vp = __shfl_sync(0xffffffffu, vp_l, j & 31);
+      if (lane == 0) {
+        fence_proxy_async();  // the slot was last read through the generic proxy
+        mbar_expect_tx(&my_full[slot], SL::kBytes);
+        copy(reinterpret_cast<const uint8_t*>(kp), 0, SL::kOffKm);
+        copy(reinterpret_cast<const uint8_t*>(vp), SL::kOffV, SL::kOffVm);
+      }
+    } else {
+      const long long ptr = __shfl_sync(0xffffffffu, (u & 1) ? vp_l : kp_l, j & 31);
+      if (lane == 0) {
+        fence_proxy_async();
+        mbar_expect_tx(&my_full[slot], SL::kBytes);
+        copy(reinterpret_cast<const uint8_t*>(ptr), 0, SL::kOffKm);
+      }
     }
   };
-  load_ptr_batch(0);
+  // what follows u into its slot, once every lane is done with u
+  auto refill = [&](int u, int slot) {
+    __syncwarp();
+    const int next = u + R, j = next / SL::kPerSlice;
+    if (next < units) {
+      if ((j & 31) == 0) {
+        if (SL::kPerSlice == 1 || !(next & 1)) load_ptrs(kp_l, kptrs, j);
+        if (SL::kPerSlice == 1 || (next & 1)) load_ptrs(vp_l, vptrs, j);
+      }
+      issue(next, slot);
+    }
+  };
+  load_ptrs(kp_l, kptrs, 0);
+  load_ptrs(vp_l, vptrs, 0);
   pdl_wait();
   qs_trace(QS_K_ATTN, 1);
   if (threadIdx.x == 0) ATTN_PROF(1);
-  for (int j = 0; j < R && j < n_my; ++j) issue(j, j);  // the cache stream starts before the new-token work below
-  if (threadIdx.x == 0) ATTN_PROF(3);
   {
     // ================================ consumer warps ================================
     // ---- new token: RoPE (NeoX, position tlen) of q and k; stage q, k, v in shared memory.
-    //      Thread t rotates the pair (i, i + 64), i = t % 64, of rows t / 64, t / 64 + 2, ... (row Gc is k): the global loads
-    //      go out first, the cos / sin of its own pair is computed while they are in flight (no table, no extra barrier) ----
+    //      Thread t rotates the pair (i, i + 64), i = t % 64, of rows t / 64, t / 64 + 2, ... (row Gc is k): the global loads go out first, ahead of the
+    //      first copies, which wait for the page pointers; the cos / sin of its own pair is computed while they are in flight (no table, no extra
+    //      barrier) ----
     const int half_rot = rotary_dim / 2;  // == 64 (checked on the host)
     const int ri = threadIdx.x & 63, r0 = threadIdx.x >> 6;
     const __half* kg = k_in + static_cast<size_t>(b) * k_stride + static_cast<size_t>(hk) * kD;
@@ -238,10 +270,12 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       }
     }
     const __half vnew = vg[threadIdx.x];
+    for (int u = 0; u < R && u < units; ++u) issue(u, u);  // the cache stream starts before the new-token work below
+    if (threadIdx.x == 0) ATTN_PROF(3);
     float sn, cs;
     {
-      const float inv_freq = __fdiv_rn(static_cast<float>(tlen), powf(rotary_base, __fdiv_rn(static_cast<float>(2 * ri), static_cast<float>(rotary_dim))));
-      sincosf(inv_freq, &sn, &cs);
+      const float angle = __fdiv_rn(static_cast<float>(tlen), powf(rotary_base, __fdiv_rn(static_cast<float>(2 * ri), static_cast<float>(rotary_dim))));
+      sincosf(angle, &sn, &cs);
     }
 #pragma unroll
     for (int e = 0; e < kRowsPerThread; ++e) {
@@ -358,8 +392,9 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     // warp w consumes tokens [32 (w & 1), +32) of the pages whose index has parity (w >> 1): two 16-token MMA chunks per
     // iteration share one barrier wait, one max reduction and one set of address computations
     const int hbase = hslice * kSliceTokens;
-    int s = 0;
+    int s = 0;  // the slot at hand
     uint32_t ph = 0;
+    auto advance = [&]() { if (++s == R) { s = 0; ph ^= 1; } };
     if (threadIdx.x == 0) ATTN_PROF(4);
     for (int j = 0; j < n_my; ++j) {
       const int pidx = my_first + 2 * j;
@@ -367,37 +402,35 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       if (threadIdx.x == 0 && j == 0) ATTN_PROF(5);
       const uint8_t* st = my_ring + s * SL::kBytes;
       const int t0 = pidx * kPageTokens + hbase;  // first token of this warp's 32-token slice
-      if (t0 < tlen) {
-        // per-token (scale, c = -scale * zero) pairs of the 32 K and 32 V tokens, converted to fp32 ONCE per token here
-        // (fp16 -> fp32 conversions run on the slow XU pipe: the logit code below must not repeat them per thread)
-        {
-          const __half* kp = reinterpret_cast<const __half*>(st + SL::kOffKs) + lane;
-          const __half* vp = reinterpret_cast<const __half*>(st + SL::kOffVs) + lane;
-          const __half ksc = kp[0], kzp = kp[32], vsc = vp[0], vzp = vp[32];
-          float2 fk, fv;
-          if constexpr (BITS == 4) {
-            // c = half(-s * z): the fp16 product of two fp16 values, rounded once
-            fk = __half22float2(__halves2half2(ksc, __hmul(__hneg(ksc), kzp)));
-            fv = __half22float2(__halves2half2(vsc, __hmul(__hneg(vsc), vzp)));
-          } else {
-            fk = __half22float2(__halves2half2(ksc, kzp));
-            fv = __half22float2(__halves2half2(vsc, vzp));
-            fk.y = -fk.x * fk.y;  // aux holds the zero point: c = -s * z in fp32
-            fv.y = -fv.x * fv.y;
-          }
-          fk.x *= sm_scale;
-          fk.y *= sm_scale;
-          if (t0 + lane >= tlen) fk = fv = make_float2(0.f, 0.f);  // unwritten slots: force finite zeros (their logits are masked below)
-          s_meta[warp][0][lane] = fk;
-          s_meta[warp][1][lane] = fv;
+      const bool live = t0 < tlen;
+      // per-token (scale, c = -scale * zero) pairs of the 32 tokens of a half, converted to fp32 ONCE per token here
+      // (fp16 -> fp32 conversions run on the slow XU pipe: the logit code below must not repeat them per thread)
+      auto pairs = [&](int which) {
+        const __half* mp = reinterpret_cast<const __half*>(st + (which ? SL::kOffVm : SL::kOffKm)) + lane;
+        const __half scale = mp[0], zero = mp[32];
+        float2 f;
+        if constexpr (BITS == 4) {
+          f = __half22float2(__halves2half2(scale, __hmul(__hneg(scale), zero)));  // c = half(-s * z): the fp16 product of two fp16 values, rounded once
+        } else {
+          f = __half22float2(__halves2half2(scale, zero));
+          f.y = -f.x * f.y;  // aux holds the zero point: c = -s * z in fp32
         }
+        if (which == 0) {
+          f.x *= sm_scale;
+          f.y *= sm_scale;
+        }
+        if (t0 + lane >= tlen) f = make_float2(0.f, 0.f);  // unwritten slots: force finite zeros (their logits are masked below)
+        s_meta[warp][which][lane] = f;
+      };
+      float sc[2][4] = {};
+      if (live) {
+        pairs(0);
+        if (SL::kPerSlice == 1) pairs(1);
         __syncwarp();
         // ---- S^T (2 x 16 tokens x 8 heads) on biased codes: 16 MMAs ----
-        float sc[2][4];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          sc[c][0] = sc[c][1] = sc[c][2] = sc[c][3] = 0.f;
-          const uint8_t* krow = st + SL::kOffK + (c * kChunk + tokA) * kRow;
+          const uint8_t* krow = st + (c * kChunk + tokA) * kRow;
           if constexpr (BITS == 4) {
             const uint4 ka = *reinterpret_cast<const uint4*>(krow + q4 * 16);
             const uint4 kb = *reinterpret_cast<const uint4*>(krow + 8 * kRow + q4 * 16);
@@ -422,6 +455,18 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
                        __byte_perm(wa[w], kMagic, 0x7352), __byte_perm(wb[w], kMagic, 0x7352), qb0[w], qb1[w]);
             }
           }
+        }
+      }
+      if constexpr (SL::kPerSlice == 2) {
+        refill(2 * j, s);
+        advance();
+        mbar_wait(&my_full[s], ph);
+        st = my_ring + s * SL::kBytes;
+      }
+      if (live) {
+        if (SL::kPerSlice == 2) {
+          pairs(1);
+          __syncwarp();
         }
         // ---- logits (log2 units) of tokens A = tokA, B = 8 + tokA of both chunks for heads 2q4, 2q4+1 ----
         float tl[2][4], vs[2][2], vc[2][2];
@@ -522,13 +567,8 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
           }
         }
       }
-      __syncwarp();
-      // refill the slot just consumed with the slice R iterations ahead
-      if (j + R < n_my) {
-        if (((j + R) & 31) == 0) load_ptr_batch(j + R);
-        issue(j + R, s);
-      }
-      if (++s == R) { s = 0; ph ^= 1; }
+      refill(SL::kPerSlice * (j + 1) - 1, s);
+      advance();
     }
 
     if (threadIdx.x == 0) ATTN_PROF(6);
@@ -633,7 +673,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     uint32_t* cnt = ws_cnt + static_cast<size_t>(b) * gridDim.x + blockIdx.x;
     if (threadIdx.x == 0) {
       const uint32_t old = atomicAdd(cnt, 1u);
-      const bool last = (old == static_cast<uint32_t>(nsplit - 1));
+      const bool last = (old == static_cast<uint32_t>(used - 1));
       if (last) *cnt = 0;
       s_last = last ? 1u : 0u;
     }
@@ -646,15 +686,15 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       __threadfence();
       for (int r = warp; r < Gc; r += kWarps) {
         const float* pr = ws_part + (static_cast<size_t>(b) * num_heads + h0 + r) * nsplit * (kD + 2);
-        const float ms = (lane < nsplit) ? __ldcg(pr + lane * (kD + 2) + kD) : -CUDART_INF_F;
-        const float ls = (lane < nsplit) ? __ldcg(pr + lane * (kD + 2) + kD + 1) : 0.f;
+        const float ms = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD) : -CUDART_INF_F;
+        const float ls = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD + 1) : 0.f;
         float M = ms;
 #pragma unroll
         for (int m = 16; m >= 1; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
         const float e = (ms == -CUDART_INF_F) ? 0.f : exp2f(ms - M);
         float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
-        for (int sp = 0; sp < nsplit; ++sp) {
+        for (int sp = 0; sp < used; ++sp) {
           const float2* row = reinterpret_cast<const float2*>(pr + sp * (kD + 2));  // 130 floats per split: 8-byte aligned
           const float2 x = __ldcg(row + lane), y = __ldcg(row + 32 + lane);
           const float w = __shfl_sync(0xffffffffu, e, sp);
@@ -909,9 +949,10 @@ int decode_attention(const DecodeAttnArgs& a) {
   const int G = a.num_heads / a.num_kv_heads;
   const int gparts = (G + kMaxG - 1) / kMaxG;
   const int gx = a.num_kv_heads * gparts;
-  // context splits: enough CTAs to fill the machine (4 resident CTAs per SM), never more than one split per 256 tokens.  One resident wave (fewer and longer
-  // splits) is faster -- 4 sequences x 8000 tokens x 8 heads, INT8: 24 us where this rule takes 32 -- but a longer walk loses more bits of the V product's
-  // biased accumulator: error against 64 bits 4.6e-4 -> 5.3e-4 there, 9 x 5000 x 32 heads 9.9e-4 -> 3.1e-3 (INT8) and 8.2e-3 -> 1.3e-2 (INT4).
+  // context splits: enough CTAs to fill the machine (4 resident CTAs per SM), never more than one split per 256 tokens.  Fewer and longer splits are no
+  // way to save prologues: a longer walk loses more bits of the V product's biased accumulator (one wave of three CTAs per SM: error against 64 bits
+  // 4.6e-4 -> 5.3e-4 at 4 sequences x 8000 tokens x 8 heads, 9 x 5000 x 32 heads 9.9e-4 -> 3.1e-3 (INT8) and 8.2e-3 -> 1.3e-2 (INT4)).  The count is
+  // rounded up, so a few CTAs may miss the first wave: those without pages leave at once (4 x 8000, INT8: 32 us with three CTAs per SM, now 22).
   int nsplit = 1;
   const int ctas = gx * a.batch;
   const int slots = num_sms() * 4;
