@@ -799,96 +799,140 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
 }
 
 // ------------------------------------------------------------------------------------------------
-// K2: prefill RoPE + KV quantise + page append: one warp per (token, KV head): it rotates the G query heads of the group and the key head with
-//     ONE evaluation of the position's sines / cosines (the first version, one warp per query head, spent its time in 32 redundant
-//     powf / sincosf per token: 365 us per layer for the 8 x 1024-token prompt batch), then quantises and appends K and V.
-//     applyBiasRopeUpdateKVCache.h:94-455 (STORE_QKV = true, no bias, NeoX)
+// K2: prefill RoPE + KV quantise + page append.   applyBiasRopeUpdateKVCache.h:94-455 (STORE_QKV = true, no bias, NeoX)
+//     One block per token, one evaluation of the position's 64 sines / cosines for all its heads, through shared memory: with a warp per (token, KV head)
+//     the sines of a token were evaluated eight times over, which was most of the instructions (6108 tokens, 32 + 8 + 8 heads, INT4 pages: 57 us, now 31; the bytes take 22).
+//     Half a warp takes a head row: lane l of 16 the elements 4 l .. and 64 + 4 l .., eight bytes each (WIDE; a row that does not start on an 8-byte boundary
+//     goes in halves), and the rows of a batch are on their way together.
 // ------------------------------------------------------------------------------------------------
-template <int BITS>
+constexpr int kAppendRows = 6;  // head rows of a half-warp on their way together
+template <int BITS, bool WIDE>
 __global__ void __launch_bounds__(128) prefill_append_kernel(__half* __restrict__ qkv, const int* __restrict__ seq_lens,
                                                              const int* __restrict__ padding_offset, const long long* __restrict__ kv_pointers,
-                                                             int num_tokens, int max_blocks, int num_heads, int num_kv_heads, int seq_len,
+                                                             int max_blocks, int num_heads, int num_kv_heads, int seq_len,
                                                              PageGeom pg, float rotary_base, int rotary_dim, int max_positions) {
+  __shared__ __align__(16) float s_cos[kD / 2], s_sin[kD / 2];
   if (threadIdx.x == 0) pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int G = num_heads / num_kv_heads;
-  const int warps_per_cta = blockDim.x >> 5;
-  const long long n_work = static_cast<long long>(num_tokens) * num_kv_heads;
-  const int n = (num_heads + 2 * num_kv_heads) * kD;
-  const int half_rot = rotary_dim / 2;
-  for (long long wi = static_cast<long long>(blockIdx.x) * warps_per_cta + (threadIdx.x >> 5); wi < n_work;
-       wi += static_cast<long long>(gridDim.x) * warps_per_cta) {
-    const int token = static_cast<int>(wi / num_kv_heads), kvh = static_cast<int>(wi - static_cast<long long>(token) * num_kv_heads);
-    const int gtok = token + (padding_offset ? padding_offset[token] : 0);
-    const int bidx = gtok / seq_len, pos = gtok - bidx * seq_len;
-    const int len = seq_lens[bidx];
-    if (pos >= len) continue;  // padded slot (cannot happen with un-padded inputs)
-    __half* trow = qkv + static_cast<size_t>(token) * n;
-    // lane handles rotary pairs i = 2*lane, 2*lane+1  (i in [0, 64)) -> dims i and i + half_rot: one half2 at each end
-    float cs[2], sn[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int i = 2 * lane + e;
-      const float inv_freq = __fdiv_rn(static_cast<float>(pos), powf(rotary_base, __fdiv_rn(static_cast<float>(2 * i), static_cast<float>(rotary_dim))));
-      sincosf(inv_freq, &sn[e], &cs[e]);
+  const int token = blockIdx.x;
+  const int gtok = token + (padding_offset ? padding_offset[token] : 0);
+  const int bidx = gtok / seq_len, pos = gtok - bidx * seq_len;
+  const int len = seq_lens[bidx];
+  if (pos >= len) return;  // padded slot (cannot happen with un-padded inputs)
+  const int rows = num_heads + 2 * num_kv_heads, n = rows * kD;
+  const int sub = threadIdx.x >> 4, l = threadIdx.x & 15;  // half-warp, lane of it
+  constexpr int kSubs = 8;
+  __half* trow = qkv + static_cast<size_t>(token) * n + 4 * l;
+  auto load4 = [&](const __half* p) {
+    if constexpr (WIDE) return *reinterpret_cast<const uint2*>(p);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
+    return make_uint2(q[0], q[1]);
+  };
+  auto store4 = [&](__half* p, uint2 v) {
+    if constexpr (WIDE) {
+      *reinterpret_cast<uint2*>(p) = v;
+    } else {
+      uint32_t* q = reinterpret_cast<uint32_t*>(p);
+      q[0] = v.x;
+      q[1] = v.y;
     }
-    auto rotate = [&](__half* row, float (&lo)[2], float (&hi)[2]) {  // in place; returns the rotated values (rounded to fp16) as floats
-      __half2* p0 = reinterpret_cast<__half2*>(row + 2 * lane);
-      __half2* p1 = reinterpret_cast<__half2*>(row + half_rot + 2 * lane);
-      const float2 a = __half22float2(*p0), b = __half22float2(*p1);
-      const float x0[2] = {a.x, a.y}, x1[2] = {b.x, b.y};
-      __half r0[2], r1[2];
+  };
+  uint2 lo[kAppendRows], hi[kAppendRows];
+  auto fetch = [&](int r0) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        r0[e] = __float2half_rn(__fsub_rn(__fmul_rn(cs[e], x0[e]), __fmul_rn(sn[e], x1[e])));
-        r1[e] = __float2half_rn(__fadd_rn(__fmul_rn(cs[e], x1[e]), __fmul_rn(sn[e], x0[e])));
-        lo[e] = __half2float(r0[e]);
-        hi[e] = __half2float(r1[e]);
+    for (int e = 0; e < kAppendRows; ++e) {
+      const int r = r0 + sub + kSubs * e;
+      if (r < rows) {
+        lo[e] = load4(trow + static_cast<size_t>(r) * kD);
+        hi[e] = load4(trow + static_cast<size_t>(r) * kD + kD / 2);
       }
-      *p0 = __halves2half2(r0[0], r0[1]);
-      *p1 = __halves2half2(r1[0], r1[1]);
-    };
-    float t0[2], t1[2];
-    for (int g = 0; g < G; ++g) rotate(trow + static_cast<size_t>(kvh * G + g) * kD, t0, t1);
-    float kx[4], vx[4];  // dims 2l, 2l+1, 64+2l, 65+2l
-    rotate(trow + static_cast<size_t>(num_heads + kvh) * kD, t0, t1);
-    kx[0] = t0[0]; kx[1] = t0[1]; kx[2] = t1[0]; kx[3] = t1[1];
-    {
-      const __half* vrow = trow + static_cast<size_t>(num_heads + num_kv_heads + kvh) * kD;
-      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(vrow + 2 * lane));
-      const float2 b = __half22float2(*reinterpret_cast<const __half2*>(vrow + half_rot + 2 * lane));
-      vx[0] = a.x; vx[1] = a.y; vx[2] = b.x; vx[3] = b.y;
     }
-    if (kv_pointers == nullptr) continue;
-    if (pos < max(len - max_positions, 0)) continue;  // outside the cyclic window (:268-271)
-    const int blk = pos / pg.tokens_per_block, slot = pos - blk * pg.tokens_per_block;
-    const float L = (BITS == 4) ? 15.f : 255.f;
+  };
+  fetch(0);
+  if (threadIdx.x < kD / 2) {
+    const int i = threadIdx.x;
+    const float angle = __fdiv_rn(static_cast<float>(pos), powf(rotary_base, __fdiv_rn(static_cast<float>(2 * i), static_cast<float>(rotary_dim))));
+    sincosf(angle, &s_sin[i], &s_cos[i]);
+  }
+  __syncthreads();
+  const float4 cs = *reinterpret_cast<const float4*>(s_cos + 4 * l), sn = *reinterpret_cast<const float4*>(s_sin + 4 * l);
+  const bool append = kv_pointers != nullptr && pos >= max(len - max_positions, 0);  // otherwise outside the cyclic window (:268-271)
+  const int blk = pos / pg.tokens_per_block, slot = pos - blk * pg.tokens_per_block;
+  for (int r0 = 0; r0 < rows; r0 += kSubs * kAppendRows) {
+    if (r0 > 0) fetch(r0);
 #pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      const float* x = which ? vx : kx;
-      float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), mn = fminf(fminf(x[0], x[1]), fminf(x[2], x[3]));
+    for (int e = 0; e < kAppendRows; ++e) {
+      const int r = r0 + sub + kSubs * e;
+      if (r0 + (threadIdx.x >> 5) * 2 + kSubs * e >= rows) continue;  // warp-uniform
+      const bool live = r < rows, rotated = r < num_heads + num_kv_heads;
+      const __half2* ph = reinterpret_cast<const __half2*>(&lo[e]);
+      const __half2* qh = reinterpret_cast<const __half2*>(&hi[e]);
+      float x[8];
+      {
+        const float2 a = __half22float2(ph[0]), b = __half22float2(ph[1]), c = __half22float2(qh[0]), d = __half22float2(qh[1]);
+        x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+        x[4] = c.x; x[5] = c.y; x[6] = d.x; x[7] = d.y;
+      }
+      if (live && rotated) {
+        const float c4[4] = {cs.x, cs.y, cs.z, cs.w}, s4[4] = {sn.x, sn.y, sn.z, sn.w};
+        __half2 o[4];
 #pragma unroll
-      for (int m = 16; m >= 1; m >>= 1) {
+        for (int j = 0; j < 4; ++j) {
+          const float f0 = x[j], f1 = x[4 + j];
+          x[j] = __fsub_rn(__fmul_rn(c4[j], f0), __fmul_rn(s4[j], f1));
+          x[4 + j] = __fadd_rn(__fmul_rn(c4[j], f1), __fmul_rn(s4[j], f0));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          o[j] = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
+          const float2 f = __half22float2(o[j]);  // what follows sees the rotated values as they are stored
+          x[2 * j] = f.x;
+          x[2 * j + 1] = f.y;
+        }
+        store4(trow + static_cast<size_t>(r) * kD, make_uint2(*reinterpret_cast<uint32_t*>(&o[0]), *reinterpret_cast<uint32_t*>(&o[1])));
+        store4(trow + static_cast<size_t>(r) * kD + kD / 2, make_uint2(*reinterpret_cast<uint32_t*>(&o[2]), *reinterpret_cast<uint32_t*>(&o[3])));
+      }
+      const bool mine = append && live && r >= num_heads;
+      if (!__any_sync(0xffffffffu, mine)) continue;
+      float mx = x[0], mn = x[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) {
+        mx = fmaxf(mx, x[j]);
+        mn = fminf(mn, x[j]);
+      }
+#pragma unroll
+      for (int m = 8; m >= 1; m >>= 1) {
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
         mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, m));
       }
+      if (!mine) continue;
+      const int which = r >= num_heads + num_kv_heads, kvh = r - num_heads - which * num_kv_heads;
       __half sc, zp;
-      kv_quant_params(mx, mn, L, sc, zp);
+      kv_quant_params(mx, mn, (BITS == 4) ? 15.f : 255.f, sc, zp);
       const float inv_s = __fdiv_rn(1.0f, __half2float(sc)), zf = __half2float(zp);
       uint8_t* page = reinterpret_cast<uint8_t*>(kv_pointers[(static_cast<size_t>(bidx) * 2 + which) * max_blocks + blk]);
-      const uint32_t c0 = kv_quant_code(x[0], inv_s, zf), c1 = kv_quant_code(x[1], inv_s, zf);
-      const uint32_t c2 = kv_quant_code(x[2], inv_s, zf), c3 = kv_quant_code(x[3], inv_s, zf);
+      uint32_t c[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) c[j] = kv_quant_code(x[j], inv_s, zf);
       if constexpr (BITS == 4) {
-        uint8_t* row = page + static_cast<size_t>(kvh * pg.tokens_per_block + slot) * (kD / 2);
-        row[lane] = static_cast<uint8_t>((c0 & 0xF) | ((c1 & 0xF) << 4));        // dims 2l, 2l+1
-        row[32 + lane] = static_cast<uint8_t>((c2 & 0xF) | ((c3 & 0xF) << 4));   // dims 64+2l, 65+2l
+        // dims 4 l .. 4 l + 3 are bytes 2 l, 2 l + 1 of the row, dims 64 + 4 l .. bytes 32 + 2 l ..
+        uint16_t* row = reinterpret_cast<uint16_t*>(page + static_cast<size_t>(kvh * pg.tokens_per_block + slot) * (kD / 2));
+        row[l] = static_cast<uint16_t>((c[0] & 0xF) | ((c[1] & 0xF) << 4) | ((c[2] & 0xF) << 8) | ((c[3] & 0xF) << 12));
+        row[16 + l] = static_cast<uint16_t>((c[4] & 0xF) | ((c[5] & 0xF) << 4) | ((c[6] & 0xF) << 8) | ((c[7] & 0xF) << 12));
       } else {
         uint8_t* row = page + static_cast<size_t>(kvh * pg.tokens_per_block + slot) * kD;
-        reinterpret_cast<uint16_t*>(row)[lane] = static_cast<uint16_t>(c0 | (c1 << 8));
-        reinterpret_cast<uint16_t*>(row + 64)[lane] = static_cast<uint16_t>(c2 | (c3 << 8));
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t lo2 = c[4 * k] | (c[4 * k + 1] << 8), hi2 = c[4 * k + 2] | (c[4 * k + 3] << 8);
+          if ((reinterpret_cast<uintptr_t>(page) & 3) == 0) {
+            reinterpret_cast<uint32_t*>(row + 64 * k)[l] = lo2 | (hi2 << 16);
+          } else {  // scales and zeros are fp16, so a page lies on a 2-byte boundary at least
+            reinterpret_cast<uint16_t*>(row + 64 * k)[2 * l] = static_cast<uint16_t>(lo2);
+            reinterpret_cast<uint16_t*>(row + 64 * k)[2 * l + 1] = static_cast<uint16_t>(hi2);
+          }
+        }
       }
-      if (lane == 0) {
+      if (l == 0) {
         __half* meta = reinterpret_cast<__half*>(page + pg.code_bytes);
         meta[kvh * pg.tokens_per_block + slot] = sc;
         meta[pg.num_kv_heads * pg.tokens_per_block + kvh * pg.tokens_per_block + slot] = zp;
@@ -1028,15 +1072,13 @@ int prefill_rope_append(const PrefillAppendArgs& a) {
   const int bits = a.int4_kv ? 4 : 8;
   QS_REQUIRE(a.size_per_token == a.num_kv_heads * kD * bits / 8, "apply_bias_rope_update_kv_cache: size_per_token=%d does not match", a.size_per_token);
   PageGeom pg{a.tokens_per_block, a.tokens_per_block * a.size_per_token, a.num_kv_heads};
-  const long long work = static_cast<long long>(a.num_tokens) * a.num_kv_heads;  // one warp per (token, KV head)
-  long long blocks = (work + 3) / 4;
-  if (blocks > static_cast<long long>(num_sms()) * 16) blocks = static_cast<long long>(num_sms()) * 16;
   auto run = [&](auto kern) {
-    return launch_pdl(kern, dim3(static_cast<unsigned>(blocks)), dim3(128), 0, a.stream, "apply_bias_rope_update_kv_cache", static_cast<__half*>(a.qkv),
-                      a.seq_lens, a.padding_offset, a.kv_pointers, a.num_tokens, a.max_blocks, a.num_heads, a.num_kv_heads, a.seq_len, pg,
-                      a.rotary_base, a.rotary_dim, a.max_positions);
+    return launch_pdl(kern, dim3(a.num_tokens), dim3(128), 0, a.stream, "apply_bias_rope_update_kv_cache", static_cast<__half*>(a.qkv), a.seq_lens,
+                      a.padding_offset, a.kv_pointers, a.max_blocks, a.num_heads, a.num_kv_heads, a.seq_len, pg, a.rotary_base, a.rotary_dim, a.max_positions);
   };
-  return a.int4_kv ? run(prefill_append_kernel<4>) : run(prefill_append_kernel<8>);
+  const bool wide = (reinterpret_cast<uintptr_t>(a.qkv) & 7) == 0;
+  if (a.int4_kv) return wide ? run(prefill_append_kernel<4, true>) : run(prefill_append_kernel<4, false>);
+  return wide ? run(prefill_append_kernel<8, true>) : run(prefill_append_kernel<8, false>);
 }
 
 int padding_offsets(int* out, const int* cu_seqlens, int batch, int max_seqlen, void* stream) {

@@ -761,42 +761,51 @@ __global__ void __launch_bounds__(kThreads) rms_norm_kernel(void* __restrict__ o
 // ------------------------------------------------------------------------------------------------
 // A0: silu_and_mul   activation_kernels.cu:10-30
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ __half silu_h(__half x) {
-  const float f = __half2float(x);
-  return __float2half_rn(__fdiv_rn(f, __fadd_rn(1.0f, expf(-f))));
-}
 // Grid-stride over 16-byte vectors of the [tokens, d] output with two vectors per thread in flight: at prompt sizes (8192 x 14336) the first version
-// -- one CTA per 1024 outputs, 114688 short-lived CTAs -- left a third of the HBM bandwidth unused; now 705 MB in 143 us = 4.9 TB/s.
-__global__ void __launch_bounds__(256) silu_and_mul_kernel(__half* __restrict__ out, const __half* __restrict__ in, int d, long long n_vec) {
+// -- one CTA per 1024 outputs, 114688 short-lived CTAs -- left a third of the HBM bandwidth unused.  All CTAs are resident at once (kSiluCtas per SM: with
+// eight launched where registers let six run, the last two per SM ran by themselves); the results go to fp16 in pairs (the scalar conversion runs at half
+// the rate, on the unit that expf and the division need), and a vector's row and column follow from the last one's without a 64-bit division.
+// 5000 rows of 2 x 14336 (430 MB): 92 us, now 84.
+constexpr int kSiluCtas = 6;
+__global__ void __launch_bounds__(256, kSiluCtas) silu_and_mul_kernel(__half* __restrict__ out, const __half* __restrict__ in, int d, long long n_vec) {
   qs_trace(QS_K_SILU, 0);
   if (threadIdx.x == 0) pdl_launch_dependents();  // dependents may become resident (and prefetch static data) right away
   pdl_wait();
   qs_trace(QS_K_SILU, 1);
-  const int vpr = d / 8;  // vectors per output row
-  auto one = [&](long long v, uint4& x, uint4& y) {
-    const long long row = v / vpr;
-    const int c = static_cast<int>(v - row * vpr);
-    const uint4* gx = reinterpret_cast<const uint4*>(in + row * 2 * d);
-    x = __ldg(gx + c);
-    y = __ldg(gx + vpr + c);
+  const unsigned vpr = d / 8;  // vectors per output row
+  const unsigned stride = gridDim.x * blockDim.x;
+  const unsigned row_step = stride / vpr, col_step = stride - row_step * vpr;
+  const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned row = first / vpr, col = first - row * vpr;
+  auto one = [&](uint4& x, uint4& y) {  // the vector at (row, col), then on to the thread's next one
+    const uint4* gx = reinterpret_cast<const uint4*>(in) + static_cast<size_t>(row) * 2 * vpr + col;
+    x = __ldg(gx);
+    y = __ldg(gx + vpr);
+    row += row_step;
+    col += col_step;
+    if (col >= vpr) {
+      col -= vpr;
+      ++row;
+    }
   };
   auto act = [&](const uint4& x, const uint4& y) {
-    const __half* xh = reinterpret_cast<const __half*>(&x);
-    const __half* yh = reinterpret_cast<const __half*>(&y);
+    const __half2* xh = reinterpret_cast<const __half2*>(&x);
+    const __half2* yh = reinterpret_cast<const __half2*>(&y);
     uint4 o;
-    __half* oh = reinterpret_cast<__half*>(&o);
+    __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
-#pragma unroll
-    for (int j = 0; j < 8; ++j) oh[j] = __hmul(silu_h(xh[j]), yh[j]);
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(xh[j]);
+      oh[j] = __hmul2(__floats2half2_rn(__fdiv_rn(f.x, __fadd_rn(1.0f, expf(-f.x))), __fdiv_rn(f.y, __fadd_rn(1.0f, expf(-f.y)))), yh[j]);
+    }
     return o;
   };
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   uint4* go = reinterpret_cast<uint4*>(out);
-  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < n_vec; v += 2 * stride) {
+  for (long long v = first; v < n_vec; v += 2ll * stride) {
     uint4 x0, y0, x1 = make_uint4(0, 0, 0, 0), y1 = x1;
     const bool two = v + stride < n_vec;
-    one(v, x0, y0);
-    if (two) one(v + stride, x1, y1);
+    one(x0, y0);
+    if (two) one(x1, y1);
     go[v] = act(x0, y0);
     if (two) go[v + stride] = act(x1, y1);
   }
@@ -1154,6 +1163,172 @@ __global__ void __launch_bounds__(kThreads) norm_quant_fast_kernel(int8_t* __res
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Prompts: the row operations of up to 4096 columns with 128 threads (norm) or a warp (quantisation) per row.  With 512 threads per row four rows are in
+// work per SM, each a chain of a load and three to five block barriers with 16 bytes per thread on their way; with these 16 rows are.
+// 5000 rows of 4096: norm 34.6 -> 24.1 us (61 MB), with the sum 46 -> 29, 6108 rows quantised with the sum 28.3 -> 19.7.  Below the limits a row per 512
+// threads is level or better: 592 rows are in work at once there.  (A warp per row for the norm as well: 18 us where 512 rows take 10, 5000 take 33.)
+// ------------------------------------------------------------------------------------------------
+constexpr int kRowVecs = 16;  // 16-byte vectors of a lane: a warp holds the row
+constexpr int kNormRowMin = 592, kQuantRowMin = 1184;
+
+// Same bits as norm_quant_fast_kernel<false, false, 1>: thread (warp k, lane l) holds what threads 32 (4 k + i) + l, i = 0 .. 3, hold there, and the sums go
+// through the same tree (the lanes of each of the 16 warps, then the warps).
+constexpr int kNormRowThreads = 128;
+__global__ void __launch_bounds__(kNormRowThreads) norm_quant_rows_kernel(int8_t* __restrict__ out, const __half* __restrict__ x, const __half* __restrict__ gamma,
+                                                                          __half* __restrict__ input_sum, __half* __restrict__ scaling, float eps, int H,
+                                                                          int ref_block) {
+  extern __shared__ __align__(16) uint8_t sm[];  // half(y) row, only for the fused sum
+  __shared__ float red[2][16], red_max[4];
+  __shared__ long long red_ll[4];
+  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = H / 8;
+  qs_trace(QS_K_NORM, 0);
+  if (threadIdx.x == 0) pdl_launch_dependents();
+  auto at = [&](int i) { return (warp * 4 + i) * 32 + lane; };
+  uint4 g[4], xv[4];  // gamma is a static weight: fetched before waiting for the producer of x
+#pragma unroll
+  for (int i = 0; i < 4; ++i) g[i] = at(i) < nvec ? __ldg(reinterpret_cast<const uint4*>(gamma) + at(i)) : make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait();
+  qs_trace(QS_K_NORM, 1);
+  const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) xv[i] = at(i) < nvec ? __ldg(src + at(i)) : make_uint4(0u, 0u, 0u, 0u);
+  auto sum = [&](float (&v)[4], float* buf) {  // v[i]: thread 32 (4 warp + i) + lane's; a level leaves each lane half of its values while there are several
+    const bool u4 = lane & 16, u3 = lane & 8;
+    const float a0 = u4 ? v[2] : v[0], a1 = u4 ? v[3] : v[1], b0 = u4 ? v[0] : v[2], b1 = u4 ? v[1] : v[3];
+    const float c0 = a0 + __shfl_xor_sync(0xffffffffu, b0, 16), c1 = a1 + __shfl_xor_sync(0xffffffffu, b1, 16);
+    float r = (u3 ? c1 : c0) + __shfl_xor_sync(0xffffffffu, u3 ? c0 : c1, 8);
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) r += __shfl_xor_sync(0xffffffffu, r, m);
+    if ((lane & 7) == 0) buf[warp * 4 + (lane >> 4) * 2 + ((lane >> 3) & 1)] = r;
+    __syncthreads();
+    return warp_reduce(lane < 16 ? buf[lane] : 0.f, OpSum());
+  };
+  float p[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2* h = reinterpret_cast<const __half2*>(&xv[i]);
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h[j]);
+      s += f.x + f.y;
+    }
+    p[i] = s;
+  }
+  const float mean = __fdiv_rn(sum(p, red[0]), static_cast<float>(H));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2* h = reinterpret_cast<const __half2*>(&xv[i]);
+    float vs = 0.f;
+    if (at(i) < nvec) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(h[j]);
+        const float a = f.x - mean, b = f.y - mean;
+        vs += a * a + b * b;
+      }
+    }
+    p[i] = vs;
+  }
+  const float rstd = __frsqrt_rn(__fadd_rn(__fdiv_rn(sum(p, red[1]), static_cast<float>(H)), eps));
+  float amax = __half2float(__float2half_rn(1e-6f));
+  float y[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (at(i) >= nvec) continue;
+    const __half* h = reinterpret_cast<const __half*>(&xv[i]);
+    const __half* gh = reinterpret_cast<const __half*>(&g[i]);
+    uint4 yv;
+    __half* yh = reinterpret_cast<__half*>(&yv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      y[i][j] = __fmul_rn(__fmul_rn(__fsub_rn(__half2float(h[j]), mean), rstd), __half2float(gh[j]));
+      yh[j] = __float2half_rn(y[i][j]);
+      amax = fmaxf(amax, fabsf(__half2float(yh[j])));
+    }
+    if (input_sum) reinterpret_cast<uint4*>(sm)[at(i)] = yv;
+  }
+  amax = warp_reduce(amax, OpMax());
+  if (lane == 0) red_max[warp] = amax;
+  __syncthreads();  // publishes the row of half(y) as well
+  amax = fmaxf(fmaxf(red_max[0], red_max[1]), fmaxf(red_max[2], red_max[3]));
+  if (input_sum) {
+    // reference thread t (of ref_block threads) accumulates y_h[t], y_h[t + ref_block], ... sequentially IN FP16 (layernorm_kernels.cu:275,286); eight
+    // neighbouring threads at a time, their sums added exactly
+    long long part = 0;
+    for (int c = threadIdx.x; c < ref_block / 8; c += kNormRowThreads) {
+      __half2 acc[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] = __float2half2_rn(0.f);
+      for (int k = c; k < nvec; k += ref_block / 8) {
+        const uint4 v = reinterpret_cast<const uint4*>(sm)[k];
+        const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = __hadd2(acc[j], h[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(acc[j]);
+        part += fx_of_half(f.x) + fx_of_half(f.y);
+      }
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
+    if (lane == 0) red_ll[warp] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) input_sum[row] = __float2half_rn(fx_to_float((red_ll[0] + red_ll[1]) + (red_ll[2] + red_ll[3])));
+  }
+  if (threadIdx.x == 0) scaling[row] = __float2half_rn(__fdiv_rn(amax, 127.f));
+  const float qs_ = __fdiv_rn(127.f, amax);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (at(i) < nvec) store_q8(out + static_cast<size_t>(row) * H, at(i), y[i], qs_);
+}
+
+__global__ void __launch_bounds__(128, 4) quant_rows_kernel(int8_t* __restrict__ out, const __half* __restrict__ in, __half* __restrict__ input_sum,
+                                                            __half* __restrict__ scale, int H, int tokens) {
+  qs_trace(QS_K_QUANT, 0);
+  if (threadIdx.x == 0) pdl_launch_dependents();
+  pdl_wait();
+  qs_trace(QS_K_QUANT, 1);
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, nvec = H / 8;
+  if (row >= tokens) return;
+  const uint4* src = reinterpret_cast<const uint4*>(in + static_cast<size_t>(row) * H);
+  uint4 xv[kRowVecs];
+#pragma unroll
+  for (int w = 0; w < kRowVecs; ++w) xv[w] = w * 32 + lane < nvec ? __ldg(src + w * 32 + lane) : make_uint4(0u, 0u, 0u, 0u);
+  float amax = 0.f;
+  long long s = 0;
+#pragma unroll
+  for (int w = 0; w < kRowVecs; ++w) {
+    const __half2* h = reinterpret_cast<const __half2*>(&xv[w]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h[j]);
+      if (input_sum) s += fx_of_half(f.x) + fx_of_half(f.y);
+      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+  }
+  amax = warp_reduce(amax, OpMax());
+  if (input_sum) {
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (lane == 0) input_sum[row] = __float2half_rn(fx_to_float(s));
+  }
+  if (lane == 0) scale[row] = __float2half_rn(__fdiv_rn(amax, 127.f));
+  const float qs_ = __fdiv_rn(127.f, amax);
+#pragma unroll
+  for (int w = 0; w < kRowVecs; ++w)
+    if (w * 32 + lane < nvec) {
+      const __half* h = reinterpret_cast<const __half*>(&xv[w]);
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __half2float(h[j]);
+      store_q8(out + static_cast<size_t>(row) * H, w * 32 + lane, v, qs_);
+    }
+}
+
 template <typename Kern, typename... Args>
 int launch(Kern kern, dim3 grid, dim3 block, size_t smem, void* stream, const char* what, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -1185,6 +1360,10 @@ int launch_norm_fast(void* out_q, void* hidden_out, const void* x, const void* d
   int ref_block = hidden < 1024 ? hidden : 1024;
   ref_block = 32 * ((ref_block + 31) / 32);  // layernorm_kernels.cu:433-436
   const size_t smem = input_sum ? static_cast<size_t>(hidden) * 2 : 0;
+  if constexpr (!ADD && !PEER)
+    if (nvec <= 4 * kNormRowThreads && tokens >= kNormRowMin)
+      return launch(norm_quant_rows_kernel, dim3(tokens), dim3(kNormRowThreads), smem, stream, what, static_cast<int8_t*>(out_q), static_cast<const __half*>(x),
+                    static_cast<const __half*>(gamma), static_cast<__half*>(input_sum), static_cast<__half*>(scaling), eps, hidden, ref_block);
   auto go = [&](auto kern) {
     return launch(kern, dim3(tokens), dim3(kThreads), smem, stream, what, static_cast<int8_t*>(out_q), static_cast<__half*>(hidden_out),
                   static_cast<const __half*>(x), static_cast<const __half*>(delta), static_cast<const __half*>(gamma), static_cast<__half*>(input_sum),
@@ -1235,6 +1414,9 @@ int quant_per_token(void* out_q, const void* in, void* input_sum, void* scale, i
       return launch(kern, dim3(tokens), dim3(kThreads), 0, stream, "invoke_quant", static_cast<int8_t*>(out_q), static_cast<const __half*>(in),
                     static_cast<__half*>(input_sum), static_cast<__half*>(scale), hidden);
     };
+    if (nvec <= 32 * kRowVecs && tokens >= kQuantRowMin)
+      return launch(quant_rows_kernel, dim3((tokens + 3) / 4), dim3(128), 0, stream, "invoke_quant", static_cast<int8_t*>(out_q), static_cast<const __half*>(in),
+                    static_cast<__half*>(input_sum), static_cast<__half*>(scale), hidden, tokens);
     if (nvec <= kThreads) return go(quant_per_token_fast_kernel<1>);
     if (nvec <= 2 * kThreads) return go(quant_per_token_fast_kernel<2>);
     if (nvec <= 4 * kThreads) return go(quant_per_token_fast_kernel<4>);
@@ -1271,8 +1453,8 @@ int silu_and_mul(void* out, const void* in, int tokens, int d, void* stream) {
   if (tokens == 0) return QS_OK;
   QS_REQUIRE(d > 0 && d % 8 == 0, "silu_and_mul: d=%d must be a positive multiple of 8", d);
   const long long n_vec = static_cast<long long>(tokens) * (d / 8);
-  const long long want = (n_vec + 255) / 256;  // one vector per thread up to 8 CTAs per SM (decode sizes), then two per thread and loop iteration
-  const long long cap = static_cast<long long>(num_sms()) * 8;
+  const long long want = (n_vec + 255) / 256;  // one vector per thread while the CTAs are resident at once (decode sizes), then two per thread and loop iteration
+  const long long cap = static_cast<long long>(num_sms()) * kSiluCtas;
   return launch(silu_and_mul_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0, stream, "silu_and_mul", static_cast<__half*>(out),
                 static_cast<const __half*>(in), d, n_vec);
 }
