@@ -4,15 +4,17 @@
 // the second's) x one score map.  Keys are walked in blocks of 64 (a block lies in one page: page sizes are multiples of 64):
 //     S = Q K^T      8 x tcgen05.mma 128 x 64 x 16, K as TMA delivers it (128-byte swizzle) and Q laid out alike, fp32 accumulators in tensor memory
 //     softmax        4 warps, thread = row: mask, optional cap and distance bias, running maximum and sum in the base-2 domain, fp32
-//     O += P V       the fp32 weights enter as three bfloat16 terms (p = hi + mid + lo, 24 mantissa bits), written over S and beside it in tensor
-//                    memory; 3 x 4 x tcgen05.mma 128 x 128 x 16, B = the V block as TMA delivers it ([key][dim]: MN-major)
-// O is rescaled only when a row's maximum has grown by more than 2^8 (numerator and denominator share the stale maximum).  256 tensor memory columns and
-// 96 KB of shared memory per CTA: two CTAs per SM, one's softmax under the other's products.  Two key / value blocks are in flight per CTA.
+//     O += P V       the fp32 weights enter as three bfloat16 terms (p = hi + mid + lo, 24 mantissa bits), the first two in tensor memory, the last in
+//                    shared memory laid out like Q; 3 x 4 x tcgen05.mma 128 x 128 x 16, B = the V block as TMA delivers it ([key][dim]: MN-major)
+// S, the two terms and O fill the 256 tensor memory columns of a CTA without sharing any, so the next block's S is computed while this block's softmax goes
+// on, and P V while the next softmax does.  O is rescaled only when a row's maximum has grown by more than 2^8 (numerator and denominator share the stale
+// maximum).  112 KB of shared memory per CTA: two CTAs per SM.  Two key / value blocks are in flight per CTA.
 //
 // Why: mma.sync with register fragments left the tensor pipe 51 % busy at 260 TFLOP/s of executed work (keys loaded once per head, 4 warps x 168
-// registers).  Both heads of the pair read one copy of K and V here, and the three terms cost issue slots only once, on the way to tensor memory.
-// Measured: 4 prompts of 1297 .. 2048 tokens, 16 heads, 4 key / value heads, 2 maps: 732 -> 259 us (746 TFLOP/s of executed work, 0.45 of the measured bf16
-// peak); what bounds it is the chain S -> softmax -> P -> O of a block with two CTAs to interleave.  The next block's S waits for O (without: 243).
+// registers).  Both heads of the pair read one copy of K and V here, and the three terms cost issue slots only once.
+// Measured: 4 prompts of 1297 .. 2048 tokens, 16 heads, 4 key / value heads, 2 maps: mma.sync 732 us; with all three terms in tensor memory, two of them
+// over S, so that the next S waited for P V, 275; now 210 (tensor pipe 61 % busy).  What bounds it is a warp's softmax of 64 keys a row, 870 instructions
+// with two warps per scheduler to interleave.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math_constants.h>
@@ -33,9 +35,9 @@ constexpr int kD = 128, kRows = 64, kKeys = 64;
 constexpr int kThreads = 192;                    // warps 0 .. 3 softmax / epilogue, warp 4 TMA, warp 5 tensor memory + MMA issuer
 constexpr int kSubQ = 128 * 128, kSubK = kKeys * 128;  // bytes of a swizzled sub-tile: rows of 64 numbers
 constexpr int kBlock = 2 * kSubK;                // a K or V block
-constexpr int kOffK = 2 * kSubQ, kOffV = kOffK + 2 * kBlock, kOffBar = kOffV + 2 * kBlock;
+constexpr int kOffK = 2 * kSubQ, kOffV = kOffK + 2 * kBlock, kOffLo = kOffV + 2 * kBlock, kOffBar = kOffLo + kSubQ;
 constexpr int kSmem = kOffBar + 128;
-constexpr uint32_t kTmemCols = 256, kColLo = 64, kColO = 128;  // S [0, 64), then P hi [0, 32), mid [32, 64), lo [64, 96); O [128, 256)
+constexpr uint32_t kTmemCols = 256, kColHi = 64, kColMid = 96, kColO = 128;  // S [0, 64) | P hi [64, 96) | P mid [96, 128) | O [128, 256)
 constexpr float kGrow = 8.f;                     // base-2 units
 
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32_t b_mn_major) {
@@ -85,12 +87,13 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
 
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kOffBar);
   uint64_t *bar_q = bar, *bar_s = bar + 1, *bar_p = bar + 2, *bar_o = bar + 3, *k_full = bar + 4, *k_free = bar + 6, *v_full = bar + 8, *v_free = bar + 10;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 12);
+  uint64_t* bar_read = bar + 12;  // S has been read
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 13);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
-    for (int i = 0; i < 12; ++i) mbar_init(&bar[i], i == 0 || i == 2 ? 4 : 1);
+    for (int i = 0; i < 13; ++i) mbar_init(&bar[i], i == 0 || i == 2 || i == 12 ? 4 : 1);
     fence_barrier_init();
   }
   if (warp == 5) tmem_alloc<kTmemCols>(s_tmem);
@@ -123,14 +126,10 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
   } else if (warp == 5) {
     if (lane == 0) {
       constexpr uint32_t qk = idesc_bf16(128, kKeys, 0u), pv = idesc_bf16(128, kD, 1u);
-      mbar_wait(bar_q, 0);
-      for (int i = 0; i < n_walk; ++i) {
+      auto scores = [&](int i) {  // S of block i
         const int st = i & 1;
-        const uint32_t ph = (static_cast<uint32_t>(i) >> 1) & 1u;
-        mbar_wait(&k_full[st], ph);
-        // S goes over the columns of the previous block's P, and products of different shapes and accumulators have no order of their own: the products
-        // with P must have retired
-        if (i > 0) mbar_wait(bar_o, static_cast<uint32_t>(i - 1) & 1u);
+        mbar_wait(&k_full[st], (static_cast<uint32_t>(i) >> 1) & 1u);
+        if (i > 0) mbar_wait(bar_read, static_cast<uint32_t>(i - 1) & 1u);
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks)
@@ -138,14 +137,24 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
                  umma_desc_sw128(smem_u32(sm + kOffK + st * kBlock + (ks >> 2) * kSubK)) + (ks & 3) * 2, qk, ks > 0 ? 1u : 0u);
         umma_commit(bar_s);
         umma_commit(&k_free[st]);
+      };
+      mbar_wait(bar_q, 0);
+      scores(0);
+      for (int i = 0; i < n_walk; ++i) {
+        if (i + 1 < n_walk) scores(i + 1);  // S and P share no columns: while the softmax of block i goes on
+        const int st = i & 1;
         mbar_wait(bar_p, static_cast<uint32_t>(i) & 1u);
-        mbar_wait(&v_full[st], ph);
+        mbar_wait(&v_full[st], (static_cast<uint32_t>(i) >> 1) & 1u);
         tc_fence_after();
+        auto values = [&](int kk) { return desc_mn(smem_u32(sm + kOffV + st * kBlock + kk * 2048), kSubK); };
+        // the small terms first
 #pragma unroll
-        for (int t = 2; t >= 0; --t)  // the small terms first
+        for (int kk = 0; kk < kKeys / 16; ++kk)
+          mma_ss(tmem + kColO, umma_desc_sw128(smem_u32(sm + kOffLo)) + kk * 2, values(kk), pv, (i > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
-          for (int kk = 0; kk < kKeys / 16; ++kk)
-            mma_ts(tmem + kColO, tmem + t * 32 + kk * 8, desc_mn(smem_u32(sm + kOffV + st * kBlock + kk * 2048), kSubK), pv, (i > 0 || t < 2 || kk > 0) ? 1u : 0u);
+        for (int t = 1; t >= 0; --t)
+#pragma unroll
+          for (int kk = 0; kk < kKeys / 16; ++kk) mma_ts(tmem + kColO, tmem + (t ? kColMid : kColHi) + kk * 8, values(kk), pv, 1u);
         umma_commit(&v_free[st]);
         umma_commit(bar_o);
       }
@@ -193,6 +202,9 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
           s[8 + (k >> 2)][k & 3] = __uint_as_float(q[k]);
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_read);  // the next block's S may follow
       if (EXTRA) {
         if (p.cap_in > 0.f) cap_scores(s, p.cap_in, p.cap_out);
         if (slope2 != 0.f) {
@@ -212,11 +224,14 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
       for (int k = 0; k < kKeys; ++k) top[k & 3] = fmaxf(top[k & 3], s[k >> 2][k & 3]);
       const float m_blk = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * sc;  // the scale is positive
       const bool grow = (m_blk - m_used) > kGrow;
-      if (i > 0) {
-        mbar_wait(bar_o, ph ^ 1u);  // the previous O += P V has retired
-        tc_fence_after();
-      }
+      auto retired = [&]() {  // the previous O += P V: O may be rescaled, P overwritten
+        if (i > 0) {
+          mbar_wait(bar_o, ph ^ 1u);
+          tc_fence_after();
+        }
+      };
       if (__any_sync(0xffffffffu, grow)) {
+        retired();
         const float m_new = grow ? m_blk : m_used;
         const float alpha = !grow ? 1.f : m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m_new);
         if (i > 0) {
@@ -246,9 +261,16 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
         lo[k] = pack_bf16(a, b);
       }
       l += sum[0] + sum[1];
-      tmem_st32(t_s, hi);
-      tmem_st32(t_s + 32, mid);
-      tmem_st32(t_s + kColLo, lo);
+      retired();
+      tmem_st32(t_s + kColHi, hi);
+      tmem_st32(t_s + kColMid, mid);
+      {
+        const int r = threadIdx.x;  // of 128, laid out like the queries
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+          *reinterpret_cast<uint4*>(sm + kOffLo + r * 128 + ((w ^ (r & 7)) << 4)) = make_uint4(lo[4 * w], lo[4 * w + 1], lo[4 * w + 2], lo[4 * w + 3]);
+        fence_proxy_async();
+      }
       const int valid = last_qpos - key0 + 1;
       if (valid < kKeys) {  // the walk's last block: cells past the portion's end may hold anything, and 0 x NaN would enter O
         uint8_t* vb = sm + kOffV + (i & 1) * kBlock;
