@@ -4,16 +4,18 @@
 // dropout_p=0, causal=True) in qserve/modeling/models/llama_w4a8_unpad.py:232-242, where q / k / v are strided views of the post-RoPE fp16 qkv
 // buffer that fused_attention.apply_bias_rope_update_kv_cache has just rotated in place.
 //
-// One CTA = one (sequence, query head, block of 128 query rows).  Per block of 128 keys:
-//     S = Q K^T      8 x tcgen05.mma 128x128x16, both operands K-major in shared memory (TMA, 128-byte swizzle), fp32 accumulators in TMEM
+// One CTA = one (sequence, query head, block of 128 query rows).  Per block of 64 keys:
+//     S = Q K^T      8 x tcgen05.mma 128x64x16, both operands K-major in shared memory (TMA, 128-byte swizzle), fp32 accumulators in TMEM
 //     softmax        4 warps, thread = query row (TMEM lane): running max / sum in the log2 domain, P = exp2(..) rounded to fp16 and written
-//                    back into tensor memory OVER the S columns it came from (P is the A operand of the next MMA)
-//     O += P V       8 x tcgen05.mma 128x128x16, A from tensor memory, B = the V tile exactly as TMA delivers it ([key][dim] rows: an MN-major
-//                    operand), accumulating in a second TMEM region
+//                    into tensor memory (P is the A operand of the next MMA)
+//     O += P V       4 x tcgen05.mma 128x128x16, A from tensor memory, B = the V tile exactly as TMA delivers it ([key][dim] rows: an MN-major
+//                    operand), accumulating in a third TMEM region
+// S, P and O share no TMEM columns (64 + 32 + 128 of the CTA's 256), so the next block's S is computed while this block's softmax goes on, and P V while
+// the next softmax does.  Blocks of 128 keys left room for P only over S, so the next S waited for P V: 8 prompts of 539 .. 1024 tokens x 32 heads 103 us, now
+// 89; 2 x 4096 tokens 374 -> 305 us (0.73 -> 0.90 PFLOP/s), 8192 tokens 674 -> 557.
 // The O accumulator is rescaled only when a row's maximum has grown by more than 2^8 since the last rescale (the sum uses the same stale
 // maximum, so the quotient is exact up to rounding); the decision is taken per warp because tcgen05.ld/st are warp-collective.
-// 256 TMEM columns and 96 KB of shared memory per CTA: two CTAs per SM, one's softmax overlaps the other's MMAs.
-// K and V are single-buffered, each re-filled as soon as the MMA that read it has retired (tcgen05.commit -> mbarrier -> TMA warp).
+// 256 TMEM columns and 96 KB of shared memory per CTA: two CTAs per SM, one's softmax overlaps the other's MMAs.  K and V are double-buffered.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -29,13 +31,15 @@ namespace {
 
 constexpr int kD = 128;         // head dim
 constexpr int kBQ = 128;        // query rows per CTA (UMMA M)
-constexpr int kBKV = 128;       // keys per block (UMMA N of S, K extent of PV)
+constexpr int kBKV = 64;        // keys per block (UMMA N of S, K extent of PV)
 constexpr int kThreads = 192;   // warps 0..3 softmax / epilogue, warp 4 TMA producer, warp 5 TMEM allocator + MMA issuer
 constexpr int kTileBytes = kBQ * kD * 2;      // 32 KB: two swizzled [128 rows x 64 halfs] sub-tiles
 constexpr int kSubBytes = kTileBytes / 2;     // 16 KB
-constexpr int kOffQ = 0, kOffK = kTileBytes, kOffV = 2 * kTileBytes, kOffBar = 3 * kTileBytes;
+constexpr int kKvBytes = kBKV * kD * 2;       // 16 KB: a K or V block, two sub-tiles of 64 rows
+constexpr int kKvSub = kKvBytes / 2;
+constexpr int kOffQ = 0, kOffK = kTileBytes, kOffV = kOffK + 2 * kKvBytes, kOffBar = kOffV + 2 * kKvBytes;
 constexpr int kSmemBytes = kOffBar + 128;
-constexpr uint32_t kTmemCols = 256;           // S / P: columns [0, 128), O: columns [128, 256)
+constexpr uint32_t kTmemCols = 256, kColP = 64, kColO = 128;  // S: columns [0, 64), P: [64, 96), O: [128, 256)
 constexpr float kRescaleThreshold = 8.f;      // log2 units
 
 // kind::f16 instruction descriptor: D = f32, A = B = f16, A K-major; B K-major (S = Q K^T) or MN-major (O = P V)
@@ -115,28 +119,28 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   if (qb < 0) return;                                      // uniform per CTA: nothing has been allocated yet
   if (threadIdx.x == 0 && (smem_u32(smem) & 1023u) != 0) __trap();
   const int hkv = h / (p.num_heads / p.num_kv_heads);
-  const int n_kb = qb + 1;  // causal, q and k positions coincide: key blocks 0 .. qb
+  // causal, q and k positions coincide: the key blocks up to the query block's last row, as far as the sequence goes
+  const int n_kb = (min((qb + 1) * kBQ, seq_len) + kBKV - 1) / kBKV;
 
   uint8_t* s_q = smem + kOffQ;
-  uint8_t* s_k = smem + kOffK;
-  uint8_t* s_v = smem + kOffV;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kOffBar);
   uint64_t* bar_q = bar + 0;       // Q tile landed
-  uint64_t* bar_kfull = bar + 1;   // K block landed
-  uint64_t* bar_kfree = bar + 2;   // S = Q K^T retired: the K buffer may be refilled
-  uint64_t* bar_vfull = bar + 3;
-  uint64_t* bar_vfree = bar + 4;   // O += P V retired: the V buffer may be refilled
-  uint64_t* bar_s = bar + 5;       // S complete in tensor memory
-  uint64_t* bar_p = bar + 6;       // P written by the four softmax warps (4 arrivals)
-  uint64_t* bar_o = bar + 7;       // O += P V retired: O may be rescaled / read
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 8);
+  uint64_t* bar_s = bar + 1;       // S complete in tensor memory
+  uint64_t* bar_read = bar + 2;    // S read by the four softmax warps (4 arrivals): the next one may follow
+  uint64_t* bar_p = bar + 3;       // P written by the four softmax warps (4 arrivals)
+  uint64_t* bar_o = bar + 4;       // O += P V retired: O may be rescaled / read, P overwritten
+  uint64_t* bar_kfull = bar + 5;   // [2] K block landed
+  uint64_t* bar_kfree = bar + 7;   // [2] S = Q K^T retired: the K buffer may be refilled
+  uint64_t* bar_vfull = bar + 9;   // [2]
+  uint64_t* bar_vfree = bar + 11;  // [2] O += P V retired: the V buffer may be refilled
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 13);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    for (int i = 0; i < 8; ++i) mbar_init(&bar[i], i == 6 ? 4 : 1);
+    for (int i = 0; i < 13; ++i) mbar_init(&bar[i], i == 2 || i == 3 ? 4 : 1);
     fence_barrier_init();
   }
   if (warp == 5) tmem_alloc<kTmemCols>(s_tmem);
@@ -144,7 +148,6 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_s = *s_tmem;
-  const uint32_t tmem_o = tmem_s + kBKV;
   if (threadIdx.x == 0) pdl_launch_dependents();
 
   if (warp == 4) {
@@ -156,16 +159,17 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       tma_load_2d(s_q, &tmap_q, h * kD, q_row, bar_q);
       tma_load_2d(s_q + kSubBytes, &tmap_q, h * kD + 64, q_row, bar_q);
       for (int j = 0; j < n_kb; ++j) {
-        const int k_row = seq_start + j * kBKV;
-        const uint32_t ph = static_cast<uint32_t>(j) & 1u;
-        mbar_wait(bar_kfree, ph ^ 1u);  // a fresh barrier passes the wait on the "previous" phase
-        mbar_expect_tx(bar_kfull, kTileBytes);
-        tma_load_2d(s_k, &tmap_k, hkv * kD, k_row, bar_kfull);
-        tma_load_2d(s_k + kSubBytes, &tmap_k, hkv * kD + 64, k_row, bar_kfull);
-        mbar_wait(bar_vfree, ph ^ 1u);
-        mbar_expect_tx(bar_vfull, kTileBytes);
-        tma_load_2d(s_v, &tmap_v, hkv * kD, k_row, bar_vfull);
-        tma_load_2d(s_v + kSubBytes, &tmap_v, hkv * kD + 64, k_row, bar_vfull);
+        const int k_row = seq_start + j * kBKV, st = j & 1;
+        const uint32_t ph = (static_cast<uint32_t>(j) >> 1) & 1u;
+        uint8_t *kb = smem + kOffK + st * kKvBytes, *vb = smem + kOffV + st * kKvBytes;
+        mbar_wait(&bar_kfree[st], ph ^ 1u);  // a fresh barrier passes the wait on the "previous" phase
+        mbar_expect_tx(&bar_kfull[st], kKvBytes);
+        tma_load_2d(kb, &tmap_k, hkv * kD, k_row, &bar_kfull[st]);
+        tma_load_2d(kb + kKvSub, &tmap_k, hkv * kD + 64, k_row, &bar_kfull[st]);
+        mbar_wait(&bar_vfree[st], ph ^ 1u);
+        mbar_expect_tx(&bar_vfull[st], kKvBytes);
+        tma_load_2d(vb, &tmap_v, hkv * kD, k_row, &bar_vfull[st]);
+        tma_load_2d(vb + kKvSub, &tmap_v, hkv * kD + 64, k_row, &bar_vfull[st]);
       }
     }
   } else if (warp == 5) {
@@ -173,77 +177,102 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     if (lane == 0) {
       constexpr uint32_t idesc_qk = umma_idesc_f16(kBQ, kBKV, 0u);
       constexpr uint32_t idesc_pv = umma_idesc_f16(kBQ, kD, 1u);
-      mbar_wait(bar_q, 0);
-      for (int j = 0; j < n_kb; ++j) {
-        const uint32_t ph = static_cast<uint32_t>(j) & 1u;
-        mbar_wait(bar_kfull, ph);
-        // S = Q K^T.  The S columns also hold the previous block's P, and MMAs of different shapes and accumulators have no order of their own: the previous
-        // O += P V must have retired.
-        if (j > 0) mbar_wait(bar_o, ph ^ 1u);
+      auto products = [&](int j, uint32_t at) {  // Q K^T of block j
+        const int st = j & 1;
+        mbar_wait(&bar_kfull[st], (static_cast<uint32_t>(j) >> 1) & 1u);
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks) {
-          const uint32_t off = (ks >> 2) * kSubBytes;
-          const uint64_t adesc = umma_desc_sw128(smem_u32(s_q + off)) + (ks & 3) * 2;
-          const uint64_t bdesc = umma_desc_sw128(smem_u32(s_k + off)) + (ks & 3) * 2;
-          umma_f16_ss(tmem_s, adesc, bdesc, idesc_qk, ks > 0 ? 1u : 0u);
+          const uint64_t adesc = umma_desc_sw128(smem_u32(s_q + (ks >> 2) * kSubBytes)) + (ks & 3) * 2;
+          const uint64_t bdesc = umma_desc_sw128(smem_u32(smem + kOffK + st * kKvBytes + (ks >> 2) * kKvSub)) + (ks & 3) * 2;
+          umma_f16_ss(at, adesc, bdesc, idesc_qk, ks > 0 ? 1u : 0u);
         }
+      };
+      auto scores = [&](int j) {  // S of block j
+        if (j > 0) mbar_wait(bar_read, static_cast<uint32_t>(j - 1) & 1u);
+        products(j, tmem_s);
+        // the first maximum is that of two blocks: the second one's scores, into the columns where O will be, for their maximum alone
+        if (j == 0 && n_kb > 1) products(1, tmem_s + kColO);
         umma_commit(bar_s);
-        umma_commit(bar_kfree);
-        mbar_wait(bar_p, ph);
-        mbar_wait(bar_vfull, ph);
+        umma_commit(&bar_kfree[j & 1]);
+      };
+      mbar_wait(bar_q, 0);
+      scores(0);
+      for (int j = 0; j < n_kb; ++j) {
+        if (j + 1 < n_kb) scores(j + 1);  // while the softmax of block j goes on
+        const int st = j & 1;
+        mbar_wait(bar_p, static_cast<uint32_t>(j) & 1u);
+        mbar_wait(&bar_vfull[st], (static_cast<uint32_t>(j) >> 1) & 1u);
         tc_fence_after();
         // O += P V: A = P (fp16 pairs, 8 TMEM columns per 16 keys), B = V rows [key][dim] = MN-major, 16 keys (2 KB) per instruction
 #pragma unroll
         for (int kk = 0; kk < kBKV / 16; ++kk) {
-          const uint64_t bdesc = umma_desc_sw128_mn(smem_u32(s_v + kk * 2048), kSubBytes);
-          umma_f16_ts(tmem_o, tmem_s + kk * 8, bdesc, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          const uint64_t bdesc = umma_desc_sw128_mn(smem_u32(smem + kOffV + st * kKvBytes + kk * 2048), kKvSub);
+          umma_f16_ts(tmem_s + kColO, tmem_s + kColP + kk * 8, bdesc, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
         }
-        umma_commit(bar_vfree);
+        umma_commit(&bar_vfree[st]);
         umma_commit(bar_o);
       }
     }
   } else {
     // ===================================== softmax + epilogue: thread = query row =====================================
     const int row = warp * 32 + lane;
-    const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
-    const uint32_t t_s = tmem_s + lane_off, t_o = tmem_o + lane_off;
+    const uint32_t t_s = tmem_s + (static_cast<uint32_t>(warp * 32) << 16), t_o = t_s + kColO;
     const int q_pos = qb * kBQ + row;  // position inside the sequence
     float m_used = -CUDART_INF_F;      // the maximum the accumulated O and l are expressed against (log2 domain, scaled)
     float l = 0.f;
+    // A row's largest weight against the maximum that is used is exactly 1 and rounds to fp16 without an error; the first 128 keys hold it more often than
+    // the first 64 (error against 64 bits 0.6 % larger with the first block's own maximum), so the second block's scores have a say in the first maximum
+    float second = -CUDART_INF_F;
+    if (n_kb > 1) {
+      mbar_wait(bar_s, 0);
+      tc_fence_after();
+      uint32_t r[2][32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_o + c * 32, r[c]);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (kBKV + c * 32 + i <= q_pos) second = fmaxf(second, __uint_as_float(r[c][i]));
+    }
     for (int j = 0; j < n_kb; ++j) {
       const uint32_t ph = static_cast<uint32_t>(j) & 1u;
-      const bool diag = (j == qb);
       mbar_wait(bar_s, ph);
       tc_fence_after();
-      // ---- the whole S row (128 fp32) comes into registers with ONE TMEM round trip ----
+      // ---- the whole S row (64 fp32) comes into registers with ONE TMEM round trip ----
       uint32_t r[kBKV / 32][32];
 #pragma unroll
       for (int c = 0; c < kBKV / 32; ++c) tmem_ld_32x32b_x32(t_s + c * 32, r[c]);
       tmem_wait_ld();
-      float m_blk = -CUDART_INF_F;
-      if (diag) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_read);
+      if (j * kBKV + kBKV - 1 > qb * kBQ + warp * 32) {  // warp-uniform: the block reaches past the warp's first row
 #pragma unroll
         for (int c = 0; c < kBKV / 32; ++c)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 32; ++i)
             if (j * kBKV + c * 32 + i > q_pos) r[c][i] = 0xff800000u;  // -inf: exp2 turns it into an exact 0
-            m_blk = fmaxf(m_blk, __uint_as_float(r[c][i]));
-          }
-      } else {
-#pragma unroll
-        for (int c = 0; c < kBKV / 32; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i) m_blk = fmaxf(m_blk, __uint_as_float(r[c][i]));
       }
-      m_blk *= p.scale_log2;
+      float top[4] = {second, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+      second = -CUDART_INF_F;
+#pragma unroll
+      for (int c = 0; c < kBKV / 32; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], __uint_as_float(r[c][i]));
+      const float m_blk = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * p.scale_log2;
       // ---- lazy rescale of O and l (warp-uniform decision) ----
-      const bool grow = (m_blk - m_used) > kRescaleThreshold;  // true on the first block (m_used = -inf)
-      if (j > 0) {
-        mbar_wait(bar_o, ph ^ 1u);  // the previous O += P V has retired (also: P of the previous block is no longer needed)
-        tc_fence_after();
-      }
+      const bool grow = (m_blk - m_used) > kRescaleThreshold;  // true on the first block (m_used = -inf; every row sees its first key there)
+      auto retired = [&]() {  // the previous O += P V
+        if (j > 0) {
+          mbar_wait(bar_o, ph ^ 1u);
+          tc_fence_after();
+        }
+      };
       if (__any_sync(0xffffffffu, grow)) {
+        retired();
         const float m_new = grow ? m_blk : m_used;
         const float alpha = (m_used == -CUDART_INF_F) ? 0.f : ex2_approx(m_used - m_new);  // 1 for rows that keep their maximum
         if (j > 0) {
@@ -260,22 +289,20 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         l *= alpha;
         m_used = m_new;
       }
-      // ---- P = exp2(s * scale - m_used), rounded to fp16, written over the S columns (all of S is in registers by now) ----
+      // ---- P = exp2(s * scale - m_used), rounded to fp16 ----
+      uint32_t pk[32];
 #pragma unroll
-      for (int hc = 0; hc < 2; ++hc) {
-        uint32_t pk[32];
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float p0 = ex2_approx(fmaf(__uint_as_float(r[hc * 2 + (i >> 5)][i & 31]), p.scale_log2, -m_used));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(r[hc * 2 + (i >> 5)][(i & 31) + 1]), p.scale_log2, -m_used));
-          const __half2 h2 = __floats2half2_rn(p0, p1);
-          // the row sum is taken over the ROUNDED probabilities: numerator (the MMA sees fp16 P) and denominator then agree
-          const float2 f = __half22float2(h2);
-          l += f.x + f.y;
-          pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
-        }
-        tmem_st_32x32b_x32(t_s + hc * 32, pk);
+      for (int i = 0; i < 64; i += 2) {
+        const float p0 = ex2_approx(fmaf(__uint_as_float(r[i >> 5][i & 31]), p.scale_log2, -m_used));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(r[i >> 5][(i & 31) + 1]), p.scale_log2, -m_used));
+        const __half2 h2 = __floats2half2_rn(p0, p1);
+        // the row sum is taken over the ROUNDED probabilities: numerator (the MMA sees fp16 P) and denominator then agree
+        const float2 f = __half22float2(h2);
+        l += f.x + f.y;
+        pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
       }
+      retired();
+      tmem_st_32x32b_x32(t_s + kColP, pk);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -329,13 +356,13 @@ PFN_encodeTiled get_encode() {
   return fn;
 }
 
-// fp16 [rows, cols] with a row pitch of `stride` elements; box = 64 columns (128 B, swizzled) x 128 rows
-int make_tmap_f16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t stride) {
+// fp16 [rows, cols] with a row pitch of `stride` elements; box = 64 columns (128 B, swizzled) x box_rows rows
+int make_tmap_f16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t stride, uint32_t box_rows) {
   PFN_encodeTiled enc = get_encode();
   if (!enc) return set_error(QS_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {stride * 2};
-  cuuint32_t box[2] = {64, 128};
+  cuuint32_t box[2] = {64, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -360,11 +387,11 @@ int prefill_attention(const PrefillAttnArgs& a) {
   QS_REQUIRE(a.q_stride >= a.num_heads * kD && a.k_stride >= a.num_kv_heads * kD && a.v_stride >= a.num_kv_heads * kD && a.out_stride >= a.num_heads * kD,
              "prefill_attention: row stride smaller than the row");
   CUtensorMap tq, tk, tv;
-  int rc = make_tmap_f16(&tq, a.q, a.num_tokens, static_cast<uint64_t>(a.num_heads) * kD, a.q_stride);
+  int rc = make_tmap_f16(&tq, a.q, a.num_tokens, static_cast<uint64_t>(a.num_heads) * kD, a.q_stride, kBQ);
   if (rc) return rc;
-  rc = make_tmap_f16(&tk, a.k, a.num_tokens, static_cast<uint64_t>(a.num_kv_heads) * kD, a.k_stride);
+  rc = make_tmap_f16(&tk, a.k, a.num_tokens, static_cast<uint64_t>(a.num_kv_heads) * kD, a.k_stride, kBKV);
   if (rc) return rc;
-  rc = make_tmap_f16(&tv, a.v, a.num_tokens, static_cast<uint64_t>(a.num_kv_heads) * kD, a.v_stride);
+  rc = make_tmap_f16(&tv, a.v, a.num_tokens, static_cast<uint64_t>(a.num_kv_heads) * kD, a.v_stride, kBKV);
   if (rc) return rc;
   static bool attr_set[kMaxDevices] = {};
   bool& done = attr_set[device_ordinal()];
