@@ -219,6 +219,16 @@ __device__ __forceinline__ void umma_i8_ts_2cta(uint32_t d_tmem, uint32_t a_tmem
       : "memory");
 }
 // arrive (once all previously issued MMAs of this thread have completed) on the mbarrier at this CTA-relative offset in BOTH CTAs of the pair
+// the same with A (this CTA's half of its rows, the peer's at the same place) from shared memory
+__device__ __forceinline__ void umma_i8_ss_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      :
+      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit_2cta(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                "h"(static_cast<uint16_t>(3))

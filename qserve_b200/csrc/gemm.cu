@@ -32,6 +32,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -43,7 +44,7 @@ namespace {
 
 constexpr int kBM = 128;  // output channels per tile (UMMA M)
 constexpr int kBK = 128;  // K sub-block (= one g128 group, one 128-byte swizzled activation row)
-constexpr int kSub = 2;    // sub-blocks per pipeline stage: per-stage barrier latencies are amortised over 256 K
+constexpr int kSub = 2;    // W4A8: sub-blocks per pipeline stage: per-stage barrier latencies are amortised over 256 K
 constexpr int kNumThreads = 256;
 #ifndef QS_PAIR_CVT
 #define QS_PAIR_CVT 1
@@ -59,6 +60,11 @@ constexpr int kPairThreads = 384;  // gemm_pair_kernel: the 8 warps of gemm_kern
 // All eight warps take part in the final reduce / scale / store phase.
 
 enum { kModeW4Chn = 0, kModeW4Grp = 1, kModeW8 = 2 };
+
+// W8A8 stages are bytes rather than latencies (its weights are twice as large and nothing unpacks them): 128 K, so that twice as many stages are on their way
+// in the same shared memory, and 128-token tiles fit two CTAs per SM (28672 x 4096 at 128 tokens: 45 us, now 41)
+template <int MODE>
+constexpr int kSubOf = MODE == kModeW8 ? 1 : kSub;
 
 struct GemmParams {
   const uint8_t* s2_scales;  // per-group: [K/128, N] (shuffled per 32 columns, as stored in the checkpoint)
@@ -79,6 +85,7 @@ struct GemmParams {
 // is already on chip when the preceding activation kernel finishes.
 template <int MODE, int NT, int WS, int AS>
 struct Cfg {
+  static constexpr int kSub = kSubOf<MODE>;
   static constexpr int kActStages = AS;  // activation ring (L2-resident operand): deep enough to cover the TMA round trip
   static constexpr int kActSub = NT * kBK;                                       // one swizzled [NT x 128 B] activation sub-tile
   static constexpr int kWSub = (MODE == kModeW8) ? kBM * kBK : kBM * kBK / 2;   // int8 rows or packed int4 tiles of one sub-block
@@ -253,7 +260,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
       const int w_row = (MODE == kModeW8) ? n_tile * kBM : n_tile * 4;  // W8: row of [N,K]; W4: band index
       const uint8_t* s2s = p.s2_scales + static_cast<size_t>(n_tile) * kBM;
       const uint8_t* s2z = p.s2_zeros + static_cast<size_t>(n_tile) * kBM;
-      // one stage = kSub sub-blocks of 128 K.  A sub-block past the end of K (K % 256 == 128) is zero-filled by the
+      // one stage = C::kSub sub-blocks of 128 K.  A sub-block past the end of K (K % 256 == 128) is zero-filled by the
       // tensor maps (weights and activations), so it contributes nothing; its g128 params are re-read from the last group.
       int s = 0;
       uint32_t ph = 0;  // parity of the (it / WS - 1)-th completion of wempty[s]
@@ -261,8 +268,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
         if (it >= WS) mbar_wait(&bar_wempty[s], ph);
         mbar_expect_tx(&bar_wfull[s], C::kWStageTx);
 #pragma unroll
-        for (int u = 0; u < kSub; ++u) {
-          const int kb = (kb_begin + it) * kSub + u;
+        for (int u = 0; u < C::kSub; ++u) {
+          const int kb = (kb_begin + it) * C::kSub + u;
           // W4: u64 elements, 256 per 128-K block of one band (4 tiles x 512 B); W8: bytes
           tma_load_2d(s_w + s * C::kWBytes + u * C::kWSub, &tmap_w, (MODE == kModeW8) ? kb * kBK : kb * 256, w_row, &bar_wfull[s]);
           if constexpr (MODE == kModeW4Grp) {
@@ -288,8 +295,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
         if (it >= kActStages) mbar_wait(&bar_xempty[s], ph);
         mbar_expect_tx(&bar_xfull[s], C::kActBytes);
 #pragma unroll
-        for (int u = 0; u < kSub; ++u)
-          tma_load_2d(s_act + s * C::kActBytes + u * C::kActSub, &tmap_act, ((kb_begin + it) * kSub + u) * kBK, a_row, &bar_xfull[s]);
+        for (int u = 0; u < C::kSub; ++u)
+          tma_load_2d(s_act + s * C::kActBytes + u * C::kActSub, &tmap_act, ((kb_begin + it) * C::kSub + u) * kBK, a_row, &bar_xfull[s]);
         if (++s == kActStages) { s = 0; if (it >= kActStages) ph ^= 1; }
       }
     }
@@ -314,7 +321,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
         if (it == 0) QS_PROF(4);
         tc_fence_after();
 #pragma unroll
-        for (int u = 0; u < kSub; ++u) {
+        for (int u = 0; u < C::kSub; ++u) {
           const uint64_t bdesc = umma_desc_sw128(smem_u32(s_act + sx * C::kActBytes + u * C::kActSub));
 #pragma unroll
           for (int t = 0; t < kBK / 32; ++t) {
@@ -361,7 +368,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
           tc_fence_after();
         }
 #pragma unroll
-        for (int u = 0; u < kSub; ++u) {
+        for (int u = 0; u < C::kSub; ++u) {
           const uint8_t* wsrc = s_w + s * C::kWBytes + u * C::kWSub + quad * 2048 + lane * 16;
           const uint32_t tdst = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + NT + ta * C::kAStageCols + u * (kBK / 4);
           uint32_t sc4 = 0, zp4 = 0;
@@ -572,6 +579,51 @@ struct PairCfg {
   static constexpr int kSmemBytes = kOffMisc + 16;
   static_assert(kSmemBytes <= 226 * 1024, "shared memory overflow");
 };
+
+// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and the NT / 2 tokens from column col0 on, 32 at a time; a
+// warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum: the tokens'
+template <int MODE, int NT, bool ACC>
+__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int m0, int n, float ws, float wz, const float* s_asc, const float* s_asum) {
+  const int tok_end = min(NT, p.M - m0);
+#pragma unroll 1
+  for (int c = 0; c < NT / 64; ++c) {
+    const int tok0 = col0 + c * 32;
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(trow + tok0, r);
+    tmem_wait_ld();
+    __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
+    if (tok0 + 32 <= tok_end) {
+      // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
+      float as[32], am[32];
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
+        as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
+        if constexpr (MODE == kModeW4Chn) {
+          const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
+          am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
+        } else {
+          am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
+        out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
+        if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
+        if (tok0 + i < tok_end) {
+          const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
+          out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
+          if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+        }
+      }
+    }
+  }
+}
 
 template <int MODE, bool ACC>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -792,7 +844,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         if (epi_tid == 0 && lt == 0) QS_PROF(8);
       }
       // ------------------------------ epilogue: this CTA's 128 channels x 256 tokens, TMEM -> registers -> global ------------------------------
-      // thread = one channel (TMEM lane) x 128 tokens; a warp's store covers 32 consecutive channels of one token = 64 B (two full sectors)
       pdl_wait();
       const int m0 = m_tile * NT;
       float* s_asc = s_row + (lt & 1) * 2 * NT;  // double-buffered by tile parity: a fast warp may already fill the next tile's values
@@ -811,45 +862,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       mbar_wait(bar_dfull, lt & 1);  // every MMA of the tile has retired
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(9);
       tc_fence_after();
-      const int tok_end = min(NT, p.M - m0);
-#pragma unroll 1
-      for (int c = 0; c < NT / 64; ++c) {
-        const int tok0 = col0 + c * 32;
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(trow + tok0, r);
-        tmem_wait_ld();
-        __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
-        if (tok0 + 32 <= tok_end) {
-          // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
-          float as[32], am[32];
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
-            as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
-            if constexpr (MODE == kModeW4Chn) {
-              const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
-              am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
-            } else {
-              am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
-            out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
-            if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
-            if (tok0 + i < tok_end) {
-              const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
-              out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
-              if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-            }
-          }
-        }
-      }
+      pair_drain<MODE, NT, ACC>(p, trow, col0, m0, n, ws, wz, s_asc, s_asum);
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(10);
       if (lt + 1 < my_tiles) zero_fill();  // hands the accumulator back to the MMA issuers
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(11);
@@ -864,6 +877,155 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
   qs_trace(QS_K_GEMM, 2);
   if (threadIdx.x == 0) QS_PROF(12);
   if (warp == 1) tmem_dealloc_2cta<C::kTmemCols>(tmem_base);
+}
+
+// =============================================================================================
+// The same for W8A8: nothing to unpack, so both operands come from shared memory as TMA delivers them (A: each CTA its 128 channels, B: each CTA half of the
+// 256 tokens), tensor memory holds two accumulators, and a tile's epilogue runs under the next tile's products.
+// Roles per CTA: warp 0 weight producer (never waits for the previous kernel) | warp 6 activation producer | leader's warps 1 and 7: MMA issuers (even / odd
+// stages) | warps 2..5 and 8..11 epilogue.  One ring of 128-K stages for both operands; both CTAs' copies signal the leader's "full" barrier.
+// 4096 tokens, 28672 x 4096: 595 us with 128-token tiles, now 266 (3.6 POP/s); 4096 x 14336: 286 -> 152.
+// =============================================================================================
+struct PairW8Cfg {
+  static constexpr int NT = 256, NH = NT / 2;
+  static constexpr int kStages = 6;             // even: a barrier belongs to one issuer
+  static constexpr int kOperand = kBM * kBK;    // 16 KB: 128 swizzled rows of 128 bytes, channels or tokens
+  static constexpr int kOffAct = kStages * kOperand;
+  static constexpr int kOffRow = 2 * kStages * kOperand;  // float ascales[2][NT] (by tile parity)
+  static constexpr int kOffBar = kOffRow + 2 * NT * 4;
+  static constexpr int kOffMisc = kOffBar + (2 * kStages + 4) * 8;
+  static constexpr int kSmemBytes = kOffMisc + 16;
+  static_assert(kSmemBytes <= 226 * 1024 && kBM == PairW8Cfg::NH, "shared memory overflow");
+};
+
+template <bool ACC>
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) {
+  using C = PairW8Cfg;
+  constexpr int NT = C::NT, ST = C::kStages;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (threadIdx.x == 0 && (smem_u32(smem) & 1023u) != 0) __trap();
+  uint8_t *s_w = smem, *s_act = smem + C::kOffAct;
+  float* s_row = reinterpret_cast<float*>(smem + C::kOffRow);
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(smem + C::kOffBar);  // leader only: both operands of both CTAs have landed
+  uint64_t* bar_empty = bar_full + ST;   // MMA commit (multicast) -> this CTA's producers
+  uint64_t* bar_dfull = bar_empty + ST;  // [2] both issuers' last commits of a tile (multicast): its accumulator is complete
+  uint64_t* bar_zero = bar_dfull + 2;    // [2] leader only: accumulator drained and zero-filled in both CTAs (16 arrivals)
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + C::kOffMisc);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = (rank == 0);
+  const int n_pairs = static_cast<int>(gridDim.x) >> 1, pair = static_cast<int>(blockIdx.x) >> 1;
+  const int total = p.m_tiles * ((p.N / kBM) >> 1);
+  const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;  // >= 1: the host launches at most `total` pairs
+  const int n_kb = p.kb_per_tile;
+  qs_trace(QS_K_GEMM, 0);
+  if (threadIdx.x == 0) QS_PROF(0);
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmap_act);
+    tma_prefetch_desc(&tmap_w);
+    for (int i = 0; i < ST; ++i) { mbar_init(&bar_full[i], 1); mbar_init(&bar_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bar_dfull[i], 2); mbar_init(&bar_zero[i], 16); }
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc_2cta<512>(s_tmem);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them remotely
+  tc_fence_after();
+  const uint32_t tmem_base = *s_tmem;
+  if (threadIdx.x == 0) { pdl_launch_dependents(); QS_PROF(1); }
+  auto tile_m = [&](int lt) { return (pair + lt * n_pairs) % p.m_tiles; };
+  auto tile_n = [&](int lt) { return 2 * ((pair + lt * n_pairs) / p.m_tiles) + static_cast<int>(rank); };
+
+  if (warp == 0 || warp == 6) {
+    if (lane == 0) {
+      const bool weights = warp == 0;
+      if (!weights) pdl_wait();
+      uint8_t* ring = weights ? s_w : s_act;
+      int s = 0;
+      uint32_t ph = 0;
+      for (int lt = 0; lt < my_tiles; ++lt) {
+        const int row = weights ? tile_n(lt) * kBM : tile_m(lt) * NT + static_cast<int>(rank) * C::NH;
+        for (int it = 0; it < n_kb; ++it) {
+          mbar_wait(&bar_empty[s], ph ^ 1);  // a fresh barrier passes the wait on the "previous" phase
+          if (weights && leader) mbar_expect_tx(&bar_full[s], 4 * C::kOperand);
+          if (weights) tma_load_2d_pair(ring + s * C::kOperand, &tmap_w, it * kBK, row, &bar_full[s]);
+          else tma_load_2d_pair(ring + s * C::kOperand, &tmap_act, it * kBK, row, &bar_full[s]);
+          if (++s == ST) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (leader && (warp == 1 || warp == 7)) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = umma_idesc_i8(2 * kBM, NT, 1u, 1u);
+      const int g_end = my_tiles * n_kb;
+      int it = (warp == 1) ? 0 : 1, s = it, lt = 0;
+      uint32_t ph = 0;
+      bool fresh = true;
+      for (int g = it; g < g_end; g += 2) {
+        if (fresh) {
+          mbar_wait(&bar_zero[lt & 1], (static_cast<uint32_t>(lt) >> 1) & 1u);
+          fresh = false;
+        }
+        mbar_wait(&bar_full[s], ph);
+        tc_fence_after();
+        const uint64_t adesc = umma_desc_sw128(smem_u32(s_w + s * C::kOperand)), bdesc = umma_desc_sw128(smem_u32(s_act + s * C::kOperand));
+#pragma unroll
+        for (int t = 0; t < kBK / 32; ++t) umma_i8_ss_2cta(tmem_base + (lt & 1) * NT, adesc + t * 2, bdesc + t * 2, idesc, 1u);
+        umma_commit_2cta(&bar_empty[s]);
+        s += 2;
+        if (s >= ST) { s -= ST; ph ^= 1; }
+        it += 2;
+        if (it >= n_kb) {  // that was this issuer's last stage of the tile (n_kb >= 2: both own at least one)
+          umma_commit_2cta(&bar_dfull[lt & 1]);
+          it -= n_kb;
+          ++lt;
+          fresh = true;
+        }
+      }
+    }
+  } else if ((warp >= 2 && warp <= 5) || warp >= 8) {
+    // a warp reaches the TMEM lanes 32 * (warp % 4) ..: the two warps of a quadrant take half of the token columns each
+    const int quad = warp & 3, col0 = warp < 8 ? 0 : NT / 2, epi_tid = quad * 32 + lane;
+    const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    auto zero_fill = [&](int buf) {
+#pragma unroll
+      for (int c = 0; c < NT / 2; c += 8) {
+        tmem_st_16x128b_x2(trow + buf * NT + col0 + c, 0u, 0u, 0u, 0u);
+        tmem_st_16x128b_x2(trow + buf * NT + col0 + c + (16u << 16), 0u, 0u, 0u, 0u);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(&bar_zero[buf], 0);
+    };
+    zero_fill(0);
+    zero_fill(1);
+    pdl_wait();
+    for (int lt = 0; lt < my_tiles; ++lt) {
+      const int m0 = tile_m(lt) * NT, n = tile_n(lt) * kBM + epi_tid, buf = lt & 1;
+      float* s_asc = s_row + buf * NT;  // a fast warp may already fill the next tile's values
+      const int j = col0 + epi_tid;     // the eight warps fetch one token's scale each
+      s_asc[j] = (m0 + j) < p.M ? __half2float(p.ascales[m0 + j]) : 0.f;
+      const float ws = __half2float(__ldg(p.wscales + n));
+      named_bar_sync(1, 256);
+      mbar_wait(&bar_dfull[buf], (static_cast<uint32_t>(lt) >> 1) & 1u);
+      tc_fence_after();
+      pair_drain<kModeW8, NT, ACC>(p, trow + buf * NT, col0, m0, n, ws, 0.f, s_asc, s_asc);
+      if (lt + 2 < my_tiles) zero_fill(buf);
+    }
+  } else {
+    pdl_wait();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer may still read this CTA's operands / arrive on its barriers until its own last MMA has retired
+  qs_trace(QS_K_GEMM, 2);
+  if (threadIdx.x == 0) QS_PROF(12);
+  if (warp == 1) tmem_dealloc_2cta<512>(tmem_base);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -984,7 +1146,7 @@ int launch_gemm(const GemmArgs& a) {
   p.M = a.M; p.N = a.N; p.K = a.K;
   const int n_tiles = a.N / kBM;
   p.m_tiles = (a.M + NT - 1) / NT;
-  p.kb_per_tile = (a.K + kSub * kBK - 1) / (kSub * kBK);  // pipeline stages of 256 K (the last one may be half zero-filled)
+  p.kb_per_tile = (a.K + C::kSub * kBK - 1) / (C::kSub * kBK);  // pipeline stages (W4A8: of 256 K, the last one may be half zero-filled)
   const int tiles = n_tiles * p.m_tiles;
   p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.force_split) : 1;  // NT = 256: no room for the receive buffer
 
@@ -1023,7 +1185,9 @@ int launch_gemm(const GemmArgs& a) {
 // prefill: CTA pairs (cta_group::2), 256 channels x 256 tokens per pair
 template <int MODE>
 int launch_gemm_pair(const GemmArgs& a) {
-  using C = PairCfg<MODE>;
+  constexpr bool w8 = MODE == kModeW8;
+  using C = std::conditional_t<w8, PairW8Cfg, PairCfg<MODE>>;
+  constexpr int stage_k = kSubOf<MODE> * kBK;
   GemmParams p{};
   p.s2_scales = static_cast<const uint8_t*>(a.s2_scales);
   p.s2_zeros = static_cast<const uint8_t*>(a.s2_zeros);
@@ -1036,15 +1200,18 @@ int launch_gemm_pair(const GemmArgs& a) {
   p.M = a.M; p.N = a.N; p.K = a.K;
   const int n_tiles = a.N / kBM;
   p.m_tiles = (a.M + C::NT - 1) / C::NT;
-  p.kb_per_tile = (a.K + kSub * kBK - 1) / (kSub * kBK);
+  p.kb_per_tile = (a.K + stage_k - 1) / stage_k;
   p.split = 1;
   p.prof = static_cast<unsigned long long*>(a.prof);
   CUtensorMap tm_act, tm_w;
   int rc = make_tmap_u8(&tm_act, a.act, a.M, a.K, C::NH);
   if (rc) return rc;
-  rc = make_tmap_w4(&tm_w, a.weight, a.N, a.K);
+  rc = w8 ? make_tmap_u8(&tm_w, a.weight, a.N, a.K, kBM) : make_tmap_w4(&tm_w, a.weight, a.N, a.K);
   if (rc) return rc;
-  auto kern = a.acc_out ? gemm_pair_kernel<MODE, true> : gemm_pair_kernel<MODE, false>;
+  auto kern = [&] {
+    if constexpr (w8) return a.acc_out ? gemm_pair_w8_kernel<true> : gemm_pair_w8_kernel<false>;
+    else return a.acc_out ? gemm_pair_kernel<MODE, true> : gemm_pair_kernel<MODE, false>;
+  }();
   static bool attr_set[2][kMaxDevices] = {};
   bool& done = attr_set[a.acc_out ? 1 : 0][device_ordinal()];
   if (!done) {
@@ -1081,14 +1248,15 @@ int dispatch_gemm(const GemmArgs& a) {
   // weight-ring depths (256-K stages) chosen so that NT <= 128 fits two CTAs per SM (<= 113 KB smem, <= 256 TMEM columns)
   constexpr bool w8 = (MODE == kModeW8), grp = (MODE == kModeW4Grp);
   QS_REQUIRE(a.force_nt == 0 || a.force_nt == 32 || a.force_nt == 64 || a.force_nt == 128, "gemm: tile tokens must be 32, 64 or 128");
-  if constexpr (MODE != kModeW8) {
+  {
     static const bool no_pair = getenv("QS_GEMM_NO_PAIR") != nullptr;  // A/B hooks
     static const int pair_min_m = getenv("QS_GEMM_PAIR_MIN_M") ? atoi(getenv("QS_GEMM_PAIR_MIN_M")) : 512;
     // Below 512 tokens the pair kernel pays only if its 256-token tiles are as well filled as the 128-token ones (an even number of 128-token
     // tiles: M in (128, 256] or (384, 512)) and there is at least one pair tile per TPC (measured: gate_up at M = 256
-    // 30.4 vs 35.5 us, at M = 320 58.1 vs 50.5; o_proj (16 pair tiles) at M = 256 16.6 vs 12.0)
+    // 30.4 vs 35.5 us, at M = 320 58.1 vs 50.5; o_proj (16 pair tiles) at M = 256 16.6 vs 12.0).  W8A8: wherever the 128-token tiles are more than the SMs
+    // (28672 x 4096, M = 200 43 vs 65 us, 300 59 vs 72; 6144 x 4096, M = 400 25 vs 31, but M = 300, 144 tiles, 24.5 vs 22.5; 4096 x 4096, M = 400 22.5 vs 20.5)
     const int t128 = (a.M + 127) / 128;
-    const bool small_ok = a.M > 128 && t128 % 2 == 0 && (a.N / kBM / 2) * ((a.M + 255) / 256) >= num_sms() / 2;
+    const bool small_ok = a.M > 128 && (w8 ? (a.N / kBM) * t128 > num_sms() : t128 % 2 == 0 && (a.N / kBM / 2) * ((a.M + 255) / 256) >= num_sms() / 2);
     if (!no_pair && a.force_nt == 0 && a.force_split == 0 && (a.M >= pair_min_m || small_ok) && (a.N / kBM) % 2 == 0 && a.K >= 512) return launch_gemm_pair<MODE>(a);
   }
   int nt = a.force_nt > 0 ? a.force_nt : 0;
@@ -1097,13 +1265,14 @@ int dispatch_gemm(const GemmArgs& a) {
     // 1796 TOP/s, M = 4096: 2388 vs 2100): a tile's setup, pipeline fill and epilogue hide behind the sibling's main loop
     nt = a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
   }
-  if (nt == 32) return launch_gemm<MODE, 32, (w8 ? 2 : grp ? 4 : 5), 4>(a);
-  if (nt == 64) return launch_gemm<MODE, 64, (w8 ? 2 : grp ? 3 : 4), (w8 ? 2 : 3)>(a);
+  if (nt == 32) return launch_gemm<MODE, 32, (grp || w8 ? 4 : 5), 4>(a);
+  if (nt == 64) return launch_gemm<MODE, 64, (w8 ? 4 : grp ? 3 : 4), (w8 ? 4 : 3)>(a);
   if constexpr (w8) {
-    // W8A8 at 65..128 tokens: the 4-deep weight ring (4 x 32 KB) leaves no room for the split-K receive buffer, so the narrow layers of a batch-128
-    // step ran on 32-48 CTAs (down_proj 35 us = 0.25 of the HBM peak).  Layers that want a split take a 2-deep ring (even depth: see the kernel).
+    // W8A8 at 65..128 tokens: layers that want a split run one CTA per SM beside the receive buffer and take a deeper activation ring
     const int tiles = (a.N / kBM) * ((a.M + 127) / 128);
-    if (a.force_split != 1 && tiles * 2 <= num_sms()) return launch_gemm<MODE, 128, 2, 2>(a);
+    if (a.force_split != 1 && tiles * 2 <= num_sms()) return launch_gemm<MODE, 128, 4, 4>(a);
+    // one CTA per SM at most: it may as well have all of the shared memory
+    if (tiles <= num_sms()) return launch_gemm<MODE, 128, 8, 4>(a);
   }
   return launch_gemm<MODE, 128, (w8 ? 4 : 2), 2>(a);
 }
