@@ -13,8 +13,9 @@
 // Why: mma.sync with register fragments left the tensor pipe 51 % busy at 260 TFLOP/s of executed work (keys loaded once per head, 4 warps x 168
 // registers).  Both heads of the pair read one copy of K and V here, and the three terms cost issue slots only once.
 // Measured: 4 prompts of 1297 .. 2048 tokens, 16 heads, 4 key / value heads, 2 maps: mma.sync 732 us; with all three terms in tensor memory, two of them
-// over S, so that the next S waited for P V, 275; now 210 (tensor pipe 61 % busy).  What bounds it is a warp's softmax of 64 keys a row, 870 instructions
-// with two warps per scheduler to interleave.
+// over S, so that the next S waited for P V, 275; with columns of their own 210; with the tiles of all entries in order of length, the queries fetched ahead
+// of the set-up and whole rows stored 192.  A step of 64 keys takes a CTA 1.56 us, two CTAs per SM: 0.85 of the tensor pipe's time for its products (S is 64
+// wide); a tile's set-up (2.6 us: tables, queries, first keys) and end (2.5) come on top, for 13.6 steps on average.  Eight softmax warps per CTA: 239.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math_constants.h>
@@ -75,7 +76,7 @@ template <bool EXTRA>  // EXTRA: a score cap and / or a distance bias
 __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                                                const UmmaTiles p) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  // the last tiles of an entry are the longest: they go first, all heads of a tile together
+  // the last tiles of the list are the longest (of an entry always, of the list where the caller has sorted it): they go first, all heads of a tile together
   const int tile = p.n_tiles - 1 - static_cast<int>(blockIdx.y), pairs = p.H >> 1;
   const int hp = blockIdx.x % pairs, m = blockIdx.x / pairs, h0 = hp * 2, g = h0 / (p.H / p.G);
   const int e = p.tile_entry[tile], r0 = p.tile_row0[tile];
@@ -97,6 +98,16 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
     fence_barrier_init();
   }
   if (warp == 5) tmem_alloc<kTmemCols>(s_tmem);
+  uint4 queries[16];  // on their way while the first keys are asked for
+  if (warp < 4) {
+    const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + static_cast<long long>(tok0) * p.q_stride + (h0 * p.maps + m) * kD;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int r = (threadIdx.x >> 4) + j * 8, w = threadIdx.x & 15, qr = r & (kRows - 1);
+      queries[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (qr < n_rows) queries[j] = *reinterpret_cast<const uint4*>(q + qr * p.q_stride + (r >> 6) * p.maps * kD + w * 8);
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -160,21 +171,16 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
       }
     }
   } else {
-    {
-      // the queries, into the layout TMA gives the keys.  Not by TMA: a tensor map would have to end at the last token's row, which only the entries' tables
-      // on the device tell
-      const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + static_cast<long long>(tok0) * p.q_stride + (h0 * p.maps + m) * kD;
-#pragma unroll 8
-      for (int j = 0; j < 16; ++j) {
-        const int r = (threadIdx.x >> 4) + j * 8, w = threadIdx.x & 15, qr = r & (kRows - 1);
-        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-        if (qr < n_rows) x = *reinterpret_cast<const uint4*>(q + qr * p.q_stride + (r >> 6) * p.maps * kD + w * 8);
-        *reinterpret_cast<uint4*>(sm + (w >> 3) * kSubQ + r * 128 + (((w & 7) ^ (r & 7)) << 4)) = x;
-      }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_q);
+    // the queries, into the layout TMA gives the keys.  Not by TMA: a tensor map would have to end at the last token's row, which only the entries' tables
+    // on the device tell
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int r = (threadIdx.x >> 4) + j * 8, w = threadIdx.x & 15;
+      *reinterpret_cast<uint4*>(sm + (w >> 3) * kSubQ + r * 128 + (((w & 7) ^ (r & 7)) << 4)) = queries[j];
     }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_q);
     const int row = (warp & 1) * 32 + lane, h = h0 + (warp >> 1);
     const uint32_t t_s = tmem + (static_cast<uint32_t>(warp * 32) << 16), t_o = t_s + kColO;
     const int qpos = qpos0 + row, fk = first_key(qpos, p.chunk, p.window);
@@ -287,19 +293,31 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
     mbar_wait(bar_o, static_cast<uint32_t>(n_walk - 1) & 1u);
     tc_fence_after();
     const float inv = 1.f / l;
-    float* dst = p.a_out + ((static_cast<size_t>(tok0 + row) * p.H + h) * p.maps + m) * kD;
+    // Through shared memory (every product has retired: the buffers are free), so that a warp stores whole rows; a lane per row touched 32 lines with every
+    // store
+    constexpr int kPitch = kD * 4 + 16;
+    uint8_t* mine = sm + kOffK + warp * 32 * kPitch;
+    static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the key, value and weight buffers");
 #pragma unroll 1
-    for (int c = 0; c < kD / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(t_o + c * 32, r);
+    for (int c = 0; c < kD / 32; c += 2) {
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
+      tmem_ld_32x32b_x32(t_o + c * 32 + 32, r[1]);
       tmem_wait_ld();
-      if (row < n_rows) {
 #pragma unroll
-        for (int v = 0; v < 8; ++v)
-          *reinterpret_cast<float4*>(dst + c * 32 + v * 4) = make_float4(__uint_as_float(r[v * 4]) * inv, __uint_as_float(r[v * 4 + 1]) * inv,
-                                                                         __uint_as_float(r[v * 4 + 2]) * inv, __uint_as_float(r[v * 4 + 3]) * inv);
+      for (int v = 0; v < 16; ++v) {
+        const uint32_t* x = &r[v >> 3][(v & 7) * 4];
+        *reinterpret_cast<float4*>(mine + lane * kPitch + c * 128 + v * 16) =
+            make_float4(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv, __uint_as_float(x[2]) * inv, __uint_as_float(x[3]) * inv);
       }
     }
+    __syncwarp();
+    const int row0 = (warp & 1) * 32;
+    float* dst = p.a_out + ((static_cast<size_t>(tok0 + row0) * p.H + h) * p.maps + m) * kD + lane * 4;
+    const size_t step = static_cast<size_t>(p.H) * p.maps * kD;
+#pragma unroll 16
+    for (int r = 0; r < 32; ++r)
+      if (row0 + r < n_rows) *reinterpret_cast<float4*>(dst + r * step) = *reinterpret_cast<const float4*>(mine + r * kPitch + lane * 16);
   }
   tc_fence_before();
   __syncthreads();

@@ -11,8 +11,9 @@
 //     O += P V       4 x tcgen05.mma 128x128x16, A from tensor memory, B = the V tile exactly as TMA delivers it ([key][dim] rows: an MN-major
 //                    operand), accumulating in a third TMEM region
 // S, P and O share no TMEM columns (64 + 32 + 128 of the CTA's 256), so the next block's S is computed while this block's softmax goes on, and P V while
-// the next softmax does.  Blocks of 128 keys left room for P only over S, so the next S waited for P V: 8 prompts of 539 .. 1024 tokens x 32 heads 103 us, now
-// 89; 2 x 4096 tokens 374 -> 305 us (0.73 -> 0.90 PFLOP/s), 8192 tokens 674 -> 557.
+// the next softmax does.  Blocks of 128 keys left room for P only over S, so the next S waited for P V: 8 prompts of 539 .. 1024 tokens x 32 heads 103 us,
+// then 89; with the longest query blocks of all sequences first and whole rows stored 86.  2 x 4096 tokens 374 -> 271 us (0.73 -> 1.01 PFLOP/s), 8192 tokens
+// 674 -> 489.
 // The O accumulator is rescaled only when a row's maximum has grown by more than 2^8 since the last rescale (the sum uses the same stale
 // maximum, so the quotient is exact up to rounding); the decision is taken per warp because tcgen05.ld/st are warp-collective.
 // 256 TMEM columns and 96 KB of shared memory per CTA: two CTAs per SM, one's softmax overlaps the other's MMAs.  K and V are double-buffered.
@@ -105,18 +106,19 @@ struct PrefillAttnParams {
   long long out_stride;
   int num_heads, num_kv_heads;
   float scale_log2;       // softmax scale * log2(e)
+  int q_blocks;           // query blocks of the longest sequence, as far as this launch goes
 };
 
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const PrefillAttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int b = blockIdx.z, h = blockIdx.y;
+  const int b = blockIdx.y, h = blockIdx.x;
   const int seq_start = __ldg(p.cu_seqlens + b);
   const int seq_len = __ldg(p.cu_seqlens + b + 1) - seq_start;
   const int n_qb = (seq_len + kBQ - 1) / kBQ;
-  const int qb = n_qb - 1 - static_cast<int>(blockIdx.x);  // the longest (last) query blocks of a sequence are scheduled first
-  if (qb < 0) return;                                      // uniform per CTA: nothing has been allocated yet
+  const int qb = p.q_blocks - 1 - static_cast<int>(blockIdx.z);  // the last query blocks see most keys: they are scheduled first
+  if (qb >= n_qb) return;                                                        // uniform per CTA: nothing has been allocated yet
   if (threadIdx.x == 0 && (smem_u32(smem) & 1023u) != 0) __trap();
   const int hkv = h / (p.num_heads / p.num_kv_heads);
   // causal, q and k positions coincide: the key blocks up to the query block's last row, as far as the sequence goes
@@ -312,27 +314,37 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     mbar_wait(bar_o, static_cast<uint32_t>(n_kb - 1) & 1u);
     tc_fence_after();
     const float inv = 1.f / l;
-    const bool valid = q_pos < seq_len;
-    __half* dst = p.out + static_cast<long long>(seq_start + q_pos) * p.out_stride + h * kD;
+    // through shared memory (every product has retired: the K and V buffers are free), so that half a warp stores a whole row; a lane per row touched 32
+    // lines with every store
+    constexpr int kPitch = kD * 2 + 16;
+    uint8_t* mine = smem + kOffK + warp * 32 * kPitch;
+    static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the K and V buffers");
 #pragma unroll 1
-    for (int c = 0; c < kD / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(t_o + c * 32, r);
+    for (int c = 0; c < kD / 32; c += 2) {
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
+      tmem_ld_32x32b_x32(t_o + c * 32 + 32, r[1]);
       tmem_wait_ld();
-      if (valid) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          uint4 o;
-          uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+      for (int v = 0; v < 8; ++v) {
+        uint4 o;
+        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const __half2 h2 = __floats2half2_rn(__uint_as_float(r[v * 8 + 2 * e]) * inv, __uint_as_float(r[v * 8 + 2 * e + 1]) * inv);
-            ow[e] = *reinterpret_cast<const uint32_t*>(&h2);
-          }
-          *reinterpret_cast<uint4*>(dst + c * 32 + v * 8) = o;
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t* x = &r[v >> 2][(v & 3) * 8 + 2 * e];
+          const __half2 h2 = __floats2half2_rn(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv);
+          ow[e] = *reinterpret_cast<const uint32_t*>(&h2);
         }
+        *reinterpret_cast<uint4*>(mine + lane * kPitch + c * 64 + v * 16) = o;
       }
     }
+    __syncwarp();
+    const int pos0 = qb * kBQ + warp * 32 + (lane >> 4);
+    __half* dst = p.out + static_cast<long long>(seq_start + pos0) * p.out_stride + h * kD + (lane & 15) * 8;
+#pragma unroll 8
+    for (int r = 0; r < 32; r += 2)
+      if (pos0 + r < seq_len)
+        *reinterpret_cast<uint4*>(dst + static_cast<long long>(r) * p.out_stride) = *reinterpret_cast<const uint4*>(mine + (r + (lane >> 4)) * kPitch + (lane & 15) * 16);
   }
   tc_fence_before();
   __syncthreads();
@@ -408,7 +420,6 @@ int prefill_attention(const PrefillAttnArgs& a) {
   p.num_kv_heads = a.num_kv_heads;
   p.scale_log2 = a.softmax_scale * 1.4426950408889634f;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((a.max_seqlen + kBQ - 1) / kBQ, a.num_heads, a.batch);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(a.stream);
@@ -417,7 +428,14 @@ int prefill_attention(const PrefillAttnArgs& a) {
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, prefill_attention_kernel, tq, tk, tv, p), "prefill attention launch");
+  constexpr int kMaxZ = 65535;  // (8.4 M tokens)
+  for (int left = (a.max_seqlen + kBQ - 1) / kBQ; left > 0; left -= kMaxZ) {
+    p.q_blocks = left;
+    cfg.gridDim = dim3(a.num_heads, a.batch, left < kMaxZ ? left : kMaxZ);
+    rc = check_cuda(cudaLaunchKernelEx(&cfg, prefill_attention_kernel, tq, tk, tv, p), "prefill attention launch");
+    if (rc) return rc;
+  }
+  return QS_OK;
 }
 
 }  // namespace qs

@@ -106,6 +106,8 @@ class StepBatch:
     tile_row0: Optional[torch.Tensor] = None     # int32 [n_tiles] first row of the tile within its entry
     long_tokens: Optional[torch.Tensor] = None   # int32 [n_long] rows covered by tiles
     short_tokens: Optional[torch.Tensor] = None  # int32 [n_short] all other rows
+    seen_entry: Optional[torch.Tensor] = None    # the tiles again, those that see most positions last
+    seen_row0: Optional[torch.Tensor] = None
 
     # when `build` is told the page size: (slot, first position, tokens) of the entries of at least TILE_MIN tokens, for `context`
     page_size: int = 0
@@ -123,7 +125,7 @@ class StepBatch:
         E = len(entries)
         tiles = [(i, r0) for i, e in enumerate(entries) if len(e[3]) >= StepBatch.TILE_MIN for r0 in range(0, len(e[3]), StepBatch.TILE_ROWS)]
         nt = len(tiles)
-        host = torch.empty(6 * T + 4 * E + 2 * nt, dtype=torch.int32)
+        host = torch.empty(6 * T + 4 * E + 4 * nt, dtype=torch.int32)
         tok, prev, slot, pos, ent, lists = (host[i * T:(i + 1) * T] for i in range(6))
         es, el, eslot, ep0 = (host[6 * T + i * E: 6 * T + (i + 1) * E] for i in range(4))
         r, longs, shorts = 0, [], []
@@ -143,7 +145,9 @@ class StepBatch:
             r += n
         lists[:] = torch.tensor(longs + shorts, dtype=torch.int32)
         if nt:
-            host[6 * T + 4 * E:] = torch.tensor([t[0] for t in tiles] + [t[1] for t in tiles], dtype=torch.int32)
+            # once in the entries' order, once by how many positions their rows see: the attention kernels start with the last
+            seen = sorted(tiles, key=lambda t: entries[t[0]][1] + t[1])
+            host[6 * T + 4 * E:] = torch.tensor([x[k] for x2 in (tiles, seen) for k in (0, 1) for x in x2], dtype=torch.int32)
         return host, (T, E, nt, len(longs), len(shorts))
 
     @staticmethod
@@ -152,7 +156,8 @@ class StepBatch:
         T, E, nt, n_long, n_short = sizes
         v = [d[i * T:(i + 1) * T] for i in range(5)] + [d[6 * T + i * E: 6 * T + (i + 1) * E] for i in range(4)]
         o = 6 * T + 4 * E
-        return StepBatch(T, E, *v, block_table, nt, n_long, n_short, d[o:o + nt], d[o + nt:o + 2 * nt], d[5 * T:5 * T + n_long], d[5 * T + n_long:6 * T])
+        t = [d[o + i * nt:o + (i + 1) * nt] for i in range(4)]
+        return StepBatch(T, E, *v, block_table, nt, n_long, n_short, t[0], t[1], d[5 * T:5 * T + n_long], d[5 * T + n_long:6 * T], t[2], t[3])
 
     @staticmethod
     def build(entries: Sequence[tuple], block_table: torch.Tensor, device: torch.device, page_size: int = 0) -> "StepBatch":
@@ -313,7 +318,7 @@ class MultiMapAttentionMixer(_Mixer):
             # prompt portions as 64-row tiles on the tensor cores, single tokens and short portions with a head group as the tile's rows
             check(lib.qs_hyb_attention_fast(out.data_ptr(), out.stride(0), proj.data_ptr(), proj.stride(0), run_cache["k"].data_ptr(),
                                             run_cache["v"].data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
-                                            _p(b.tile_entry), _p(b.tile_row0), b.n_tiles, _p(b.long_tokens), b.n_long, _p(b.short_tokens), b.n_short,
+                                            _p(b.seen_entry), _p(b.seen_row0), b.n_tiles, _p(b.long_tokens), b.n_long, _p(b.short_tokens), b.n_short,
                                             _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), scratch.data_ptr(), m.heads,
                                             m.kv_heads, m.maps, m.dim, m.vdim, m.scale, self.lam, self.out_scale, self.eps,
                                             1 if m.head_norm else 0, page_size, m.chunk, m.window, _p(self.sinks), extra, dt, stream))
@@ -547,7 +552,7 @@ class LatentAttentionMixer(_Mixer):
             direct = not latent and not m.gate
             otok = out if direct else torch.empty((T, H * Dv), dtype=proj.dtype, device=dev)
             check(lib.qs_hyb_attention_fast(otok.data_ptr(), otok.stride(0), q.data_ptr(), q.stride(0), keys.data_ptr(), values.data_ptr(), _p(b.tok_slot),
-                                            _p(b.tok_pos), ctx_table.data_ptr(), ctx_table.shape[1], _p(b.tile_entry), _p(b.tile_row0), b.n_tiles,
+                                            _p(b.tok_pos), ctx_table.data_ptr(), ctx_table.shape[1], _p(b.seen_entry), _p(b.seen_row0), b.n_tiles,
                                             _p(b.long_tokens), b.n_long, None, 0, _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0),
                                             scratch.data_ptr(), H, H, 1, D + R, Dv, m.scale, 0.0, 1.0, self.eps, 0, page_size, m.chunk, m.window,
                                             _p(self.sinks), None, dt, stream))
