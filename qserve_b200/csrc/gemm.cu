@@ -77,6 +77,7 @@ struct GemmParams {
   int32_t* acc_out;          // optional: raw INT32 accumulators [M, N] (parity tests)
   int M, N, K;
   int m_tiles, kb_per_tile, split;
+  int nt;                    // pair kernels: tokens of a tile, a multiple of 32 up to 256
   unsigned long long* prof;  // optional: 16 globaltimer stamps per CTA (tools/gemm_timeline.py)
 };
 
@@ -536,7 +537,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 }
 
 // =============================================================================================
-// Prefill tiles (M >= 512, W4A8): a PAIR of CTAs on the two SMs of a TPC computes 256-channel x 256-token tiles with cta_group::2 UMMAs,
+// Prefill tiles (M >= 512, W4A8): a PAIR of CTAs on the two SMs of a TPC computes tiles of 256 channels x 128 to 256 tokens
+// (pair_tokens, below; the figures here are those of 256) with cta_group::2 UMMAs,
 // persistently (one pair per TPC walks the tile list).
 //
 // Why: with 128-token tiles every CTA pulls its whole 128 x K weight band AND its whole 128 x K activation band out of L2: M = 4096 x N = 28672 x
@@ -556,8 +558,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 // =============================================================================================
 template <int MODE>
 struct PairCfg {
-  static constexpr int NT = 256;                       // tokens per pair tile (UMMA N)
-  static constexpr int NH = NT / 2;                    // tokens staged per CTA
+  static constexpr int NT = 256;                       // most tokens of a pair tile (UMMA N); the buffers are laid out for these
+  static constexpr int NH = NT / 2;                    // most tokens staged per CTA
   static constexpr int WS = 4, AS = 4, TA = 4;         // powers of two (stage = iteration & (depth - 1))
   static constexpr int kActSub = NH * kBK;             // 16 KB: one swizzled [128 x 128 B] activation sub-tile (this CTA's half)
   static constexpr int kActBytes = kSub * kActSub;     // 32 KB per stage
@@ -580,49 +582,76 @@ struct PairCfg {
   static_assert(kSmemBytes <= 226 * 1024, "shared memory overflow");
 };
 
-// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and the NT / 2 tokens from column col0 on, 32 at a time; a
-// warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum: the tokens'
-template <int MODE, int NT, bool ACC>
-__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int m0, int n, float ws, float wz, const float* s_asc, const float* s_asum) {
-  const int tok_end = min(NT, p.M - m0);
-#pragma unroll 1
-  for (int c = 0; c < NT / 64; ++c) {
-    const int tok0 = col0 + c * 32;
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(trow + tok0, r);
-    tmem_wait_ld();
-    __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
-    if (tok0 + 32 <= tok_end) {
-      // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
-      float as[32], am[32];
+// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and `cols` tokens from column col0 on, 32 (at last 16) at a
+// time; a warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum:
+// the tokens', m0: the tile's first token
+template <int MODE, bool ACC, int CH>
+__device__ __forceinline__ void pair_drain_chunk(const GemmParams& p, uint32_t trow, int tok0, int m0, int n, float ws, float wz, const float* s_asc,
+                                                 const float* s_asum) {
+  uint32_t r[CH];
+  if constexpr (CH == 32) tmem_ld_32x32b_x32(trow + tok0, r);
+  else tmem_ld_32x32b_x16(trow + tok0, r);
+  tmem_wait_ld();
+  const int tok_end = p.M - m0;
+  __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
+  if (tok0 + CH <= tok_end) {
+    // whole chunk inside M: no per-token branches, the scales come in as vectors, CH independent chains
+    float as[CH], am[CH];
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
-        as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
-        if constexpr (MODE == kModeW4Chn) {
-          const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
-          am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
-        } else {
-          am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
-        }
+    for (int i = 0; i < CH; i += 4) {
+      const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
+      as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
+      if constexpr (MODE == kModeW4Chn) {
+        const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
+        am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
+      } else {
+        am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
       }
+    }
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
+    for (int i = 0; i < CH; ++i) {
+      const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
+      out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
+      if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
+      if (tok0 + i < tok_end) {
+        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
         out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
         if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
-        if (tok0 + i < tok_end) {
-          const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
-          out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
-          if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-        }
-      }
     }
   }
+}
+template <int MODE, bool ACC>
+__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int cols, int m0, int n, float ws, float wz, const float* s_asc,
+                                           const float* s_asum) {
+  int c = 0;
+#pragma unroll 1
+  for (; c + 16 < cols; c += 32) pair_drain_chunk<MODE, ACC, 32>(p, trow, col0 + c, m0, n, ws, wz, s_asc, s_asum);
+  if (c < cols) pair_drain_chunk<MODE, ACC, 16>(p, trow, col0 + c, m0, n, ws, wz, s_asc, s_asum);
+}
+// zero-fills an accumulator's columns [col0, col0 + cols) of the warp's 32 lanes
+__device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols) {
+  auto eight = [&](int c) {
+    tmem_st_16x128b_x2(trow + col0 + c, 0u, 0u, 0u, 0u);
+    tmem_st_16x128b_x2(trow + col0 + c + (16u << 16), 0u, 0u, 0u, 0u);
+  };
+  if (cols == 128) {  // (a loop takes 1 % of a tile of 4096 K longer)
+#pragma unroll
+    for (int c = 0; c < 128; c += 8) eight(c);
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+      eight(c);
+      eight(c + 8);
+    }
+  }
+  tmem_wait_st();
+  tc_fence_before();
+  __syncwarp();
 }
 
 template <int MODE, bool ACC>
@@ -654,7 +683,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int total = p.m_tiles * ((p.N / kBM) >> 1);
   const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;  // >= 1: the host launches at most `total` pairs
-  const int n_kb = p.kb_per_tile;
+  const int n_kb = p.kb_per_tile, nt = p.nt, nh = nt >> 1;
   qs_trace(QS_K_GEMM, 0);
   if (threadIdx.x == 0) QS_PROF(0);
 
@@ -715,10 +744,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       int s = 0;
       uint32_t ph = 0;
       for (int lt = 0; lt < my_tiles; ++lt) {
-        const int a_row = tile_m(lt) * NT + static_cast<int>(rank) * C::NH;
+        const int a_row = tile_m(lt) * nt + static_cast<int>(rank) * nh;
         for (int it = 0; it < n_kb; ++it) {
           mbar_wait(&bar_xempty[s], ph ^ 1);
-          if (leader) mbar_expect_tx(&bar_xfull[s], 2 * C::kActBytes);  // my half + the peer's half
+          if (leader) mbar_expect_tx(&bar_xfull[s], 2 * kSub * nh * kBK);  // my half + the peer's half
 #pragma unroll
           for (int u = 0; u < kSub; ++u)
             tma_load_2d_pair(s_act + s * C::kActBytes + u * C::kActSub, &tmap_act, (it * kSub + u) * kBK, a_row, &bar_xfull[s]);
@@ -727,9 +756,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       }
     }
   } else if (leader && (warp == 1 || warp == 7)) {
-    // ===================================== leader: two MMA issuers (even / odd iterations), 256 x 256 x 32 INT8 UMMAs over both SMs ==========
+    // ===================================== leader: two MMA issuers (even / odd iterations), 256 x nt x 32 INT8 UMMAs over both SMs ==========
     if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_i8(2 * kBM, NT, 1u, 1u);
+      const uint32_t idesc = umma_idesc_i8(2 * kBM, nt, 1u, 1u);
       const int g_end = my_tiles * n_kb;
       int it = (warp == 1) ? 0 : 1;  // iteration inside the current tile
       int lt = 0;
@@ -775,18 +804,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
     const bool unpacker = warp < 8;           // first / second warp of its lane quadrant
     const int quad = warp & 3;
     const int usel = unpacker ? 0 : 1;        // the 128-K sub-block of a stage this warp unpacks
-    const int col0 = unpacker ? 0 : NT / 2;   // first accumulator column (token) of this warp's half
+    const int col0 = unpacker ? 0 : nh;   // first accumulator column (token) of this warp's half
     const int epi_tid = quad * 32 + lane;     // channel inside the tile
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     auto zero_fill = [&]() {
-#pragma unroll
-      for (int c = 0; c < NT / 2; c += 8) {
-        tmem_st_16x128b_x2(trow + col0 + c, 0u, 0u, 0u, 0u);
-        tmem_st_16x128b_x2(trow + col0 + c + (16u << 16), 0u, 0u, 0u, 0u);
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
+      pair_zero(trow, col0, nh);
       if (lane == 0) mbar_arrive_cluster(bar_zero, 0);
     };
     zero_fill();
@@ -843,9 +865,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         }
         if (epi_tid == 0 && lt == 0) QS_PROF(8);
       }
-      // ------------------------------ epilogue: this CTA's 128 channels x 256 tokens, TMEM -> registers -> global ------------------------------
+      // ------------------------------ epilogue: this CTA's 128 channels x nt tokens, TMEM -> registers -> global ------------------------------
       pdl_wait();
-      const int m0 = m_tile * NT;
+      const int m0 = m_tile * nt;
       float* s_asc = s_row + (lt & 1) * 2 * NT;  // double-buffered by tile parity: a fast warp may already fill the next tile's values
       float* s_asum = s_asc + NT;
       {
@@ -862,7 +884,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       mbar_wait(bar_dfull, lt & 1);  // every MMA of the tile has retired
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(9);
       tc_fence_after();
-      pair_drain<MODE, NT, ACC>(p, trow, col0, m0, n, ws, wz, s_asc, s_asum);
+      pair_drain<MODE, ACC>(p, trow, col0, nh, m0, n, ws, wz, s_asc, s_asum);
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(10);
       if (lt + 1 < my_tiles) zero_fill();  // hands the accumulator back to the MMA issuers
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(11);
@@ -881,7 +903,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
 
 // =============================================================================================
 // The same for W8A8: nothing to unpack, so both operands come from shared memory as TMA delivers them (A: each CTA its 128 channels, B: each CTA half of the
-// 256 tokens), tensor memory holds two accumulators, and a tile's epilogue runs under the next tile's products.
+// the tile's tokens), tensor memory holds two accumulators, and a tile's epilogue runs under the next tile's products.
 // Roles per CTA: warp 0 weight producer (never waits for the previous kernel) | warp 6 activation producer | leader's warps 1 and 7: MMA issuers (even / odd
 // stages) | warps 2..5 and 8..11 epilogue.  One ring of 128-K stages for both operands; both CTAs' copies signal the leader's "full" barrier.
 // 4096 tokens, 28672 x 4096: 595 us with 128-token tiles, now 266 (3.6 POP/s); 4096 x 14336: 286 -> 152.
@@ -919,7 +941,7 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
   const int n_pairs = static_cast<int>(gridDim.x) >> 1, pair = static_cast<int>(blockIdx.x) >> 1;
   const int total = p.m_tiles * ((p.N / kBM) >> 1);
   const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;  // >= 1: the host launches at most `total` pairs
-  const int n_kb = p.kb_per_tile;
+  const int n_kb = p.kb_per_tile, nt = p.nt, nh = nt >> 1;
   qs_trace(QS_K_GEMM, 0);
   if (threadIdx.x == 0) QS_PROF(0);
   if (warp == 0 && lane == 0) {
@@ -947,10 +969,10 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
       int s = 0;
       uint32_t ph = 0;
       for (int lt = 0; lt < my_tiles; ++lt) {
-        const int row = weights ? tile_n(lt) * kBM : tile_m(lt) * NT + static_cast<int>(rank) * C::NH;
+        const int row = weights ? tile_n(lt) * kBM : tile_m(lt) * nt + static_cast<int>(rank) * nh;
         for (int it = 0; it < n_kb; ++it) {
           mbar_wait(&bar_empty[s], ph ^ 1);  // a fresh barrier passes the wait on the "previous" phase
-          if (weights && leader) mbar_expect_tx(&bar_full[s], 4 * C::kOperand);
+          if (weights && leader) mbar_expect_tx(&bar_full[s], 2 * (kBM + nh) * kBK);
           if (weights) tma_load_2d_pair(ring + s * C::kOperand, &tmap_w, it * kBK, row, &bar_full[s]);
           else tma_load_2d_pair(ring + s * C::kOperand, &tmap_act, it * kBK, row, &bar_full[s]);
           if (++s == ST) { s = 0; ph ^= 1; }
@@ -959,7 +981,7 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
     }
   } else if (leader && (warp == 1 || warp == 7)) {
     if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_i8(2 * kBM, NT, 1u, 1u);
+      const uint32_t idesc = umma_idesc_i8(2 * kBM, nt, 1u, 1u);
       const int g_end = my_tiles * n_kb;
       int it = (warp == 1) ? 0 : 1, s = it, lt = 0;
       uint32_t ph = 0;
@@ -988,24 +1010,17 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
     }
   } else if ((warp >= 2 && warp <= 5) || warp >= 8) {
     // a warp reaches the TMEM lanes 32 * (warp % 4) ..: the two warps of a quadrant take half of the token columns each
-    const int quad = warp & 3, col0 = warp < 8 ? 0 : NT / 2, epi_tid = quad * 32 + lane;
+    const int quad = warp & 3, col0 = warp < 8 ? 0 : nh, epi_tid = quad * 32 + lane;
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     auto zero_fill = [&](int buf) {
-#pragma unroll
-      for (int c = 0; c < NT / 2; c += 8) {
-        tmem_st_16x128b_x2(trow + buf * NT + col0 + c, 0u, 0u, 0u, 0u);
-        tmem_st_16x128b_x2(trow + buf * NT + col0 + c + (16u << 16), 0u, 0u, 0u, 0u);
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
+      pair_zero(trow + buf * NT, col0, nh);
       if (lane == 0) mbar_arrive_cluster(&bar_zero[buf], 0);
     };
     zero_fill(0);
     zero_fill(1);
     pdl_wait();
     for (int lt = 0; lt < my_tiles; ++lt) {
-      const int m0 = tile_m(lt) * NT, n = tile_n(lt) * kBM + epi_tid, buf = lt & 1;
+      const int m0 = tile_m(lt) * nt, n = tile_n(lt) * kBM + epi_tid, buf = lt & 1;
       float* s_asc = s_row + buf * NT;  // a fast warp may already fill the next tile's values
       const int j = col0 + epi_tid;     // the eight warps fetch one token's scale each
       s_asc[j] = (m0 + j) < p.M ? __half2float(p.ascales[m0 + j]) : 0.f;
@@ -1013,7 +1028,7 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
       named_bar_sync(1, 256);
       mbar_wait(&bar_dfull[buf], (static_cast<uint32_t>(lt) >> 1) & 1u);
       tc_fence_after();
-      pair_drain<kModeW8, NT, ACC>(p, trow + buf * NT, col0, m0, n, ws, 0.f, s_asc, s_asc);
+      pair_drain<kModeW8, ACC>(p, trow + buf * NT, col0, nh, m0, n, ws, 0.f, s_asc, s_asc);
       if (lt + 2 < my_tiles) zero_fill(buf);
     }
   } else {
@@ -1182,7 +1197,26 @@ int launch_gemm(const GemmArgs& a) {
   return check_cuda(cudaLaunchKernelEx(&cfg, kern, tm_act, tm_w, p), "gemm launch");
 }
 
-// prefill: CTA pairs (cta_group::2), 256 channels x 256 tokens per pair
+// Tokens of a pair tile.  All pairs take a tile at a time, so the rounds count, and a round takes a share of its time whatever the tile's tokens: the group
+// scales' unpacking 0.71 of that of 256 tokens, per-channel weights 0.25, W8A8 0.57 (its operands' way out of L2), measured at 4736 tokens with 128 to 256 per
+// tile, 4096 x 4096.  4096 x 14336 at 512 tokens: 45 us with 256 per tile, 35 with 128; 4096 x 4096 at 4736: 76 with 256 (4.1 rounds), 70 with 224 (4.8).
+int pair_tokens(int M, int N, int mode) {
+  const float fixed = mode == kModeW4Grp ? 0.71f : mode == kModeW4Chn ? 0.25f : 0.57f;
+  const int pairs = num_sms() / 2;
+  int best = 256;
+  float best_cost = 0.f;
+  for (int nt = 256; nt >= 128; nt -= 32) {
+    const long long tiles = static_cast<long long>((M + nt - 1) / nt) * (N / kBM / 2);
+    const float cost = static_cast<float>((tiles + pairs - 1) / pairs) * (fixed + (1.f - fixed) * static_cast<float>(nt) / 256.f);
+    if (nt == 256 || cost < 0.98f * best_cost) {
+      best = nt;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// prefill: CTA pairs (cta_group::2), 256 channels x 128 to 256 tokens per pair
 template <int MODE>
 int launch_gemm_pair(const GemmArgs& a) {
   constexpr bool w8 = MODE == kModeW8;
@@ -1199,12 +1233,13 @@ int launch_gemm_pair(const GemmArgs& a) {
   p.acc_out = static_cast<int32_t*>(a.acc_out);
   p.M = a.M; p.N = a.N; p.K = a.K;
   const int n_tiles = a.N / kBM;
-  p.m_tiles = (a.M + C::NT - 1) / C::NT;
+  p.nt = pair_tokens(a.M, a.N, MODE);
+  p.m_tiles = (a.M + p.nt - 1) / p.nt;
   p.kb_per_tile = (a.K + stage_k - 1) / stage_k;
   p.split = 1;
   p.prof = static_cast<unsigned long long*>(a.prof);
   CUtensorMap tm_act, tm_w;
-  int rc = make_tmap_u8(&tm_act, a.act, a.M, a.K, C::NH);
+  int rc = make_tmap_u8(&tm_act, a.act, a.M, a.K, p.nt / 2);
   if (rc) return rc;
   rc = w8 ? make_tmap_u8(&tm_w, a.weight, a.N, a.K, kBM) : make_tmap_w4(&tm_w, a.weight, a.N, a.K);
   if (rc) return rc;

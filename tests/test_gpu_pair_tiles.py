@@ -1,0 +1,35 @@
+"""Tiles of CTA pairs with 128 to 256 tokens: what the tile's tokens are follows the number of rounds, the result does not.  Against the same rows in pieces
+of at most 128 tokens, which take the single-CTA tiles: the same bits, for every tile size, ragged last tiles, one and several tiles per pair."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["chn", "grp", "w8"])
+@pytest.mark.parametrize("M,N", [(512, 4096), (600, 4096), (700, 4096), (890, 4096), (1000, 4096), (2500, 4096), (130, 28672), (200, 28672), (250, 28672), (1301, 6144), (4500, 4096)])
+def test_bits_of_small_tiles(dev, mode, M, N):
+    import qserve_backend.qgemm_w4a8_per_chn as chn
+    import qserve_backend.qgemm_w4a8_per_group as grp
+    import qserve_backend.qgemm_w8a8 as w8
+
+    K = 640 if mode != "chn" else 512
+    g = torch.Generator(device=dev).manual_seed(M + N)
+    ints = lambda lo, hi, *s: torch.randint(lo, hi, s, dtype=torch.int8, device=dev, generator=g)
+    half = lambda n, s: torch.rand(n, device=dev, generator=g).add(0.5).mul(s).half()
+    x, w = ints(-128, 128, M, K), ints(-128, 128, N, K if mode == "w8" else K // 2)
+    ws, xs, wz, xsum, s2, z2 = half(N, 2e-3), half(M, 1e-2), half(N, 1e-2), half(M, 1.0), ints(1, 17, K // 128, N), ints(-120, 1, K // 128, N)
+    got = []
+    for piece in (M, 100):
+        out = torch.full((M, N), float("nan"), dtype=torch.half, device=dev)
+        for a in range(0, M, piece):
+            r = slice(a, a + piece)
+            if mode == "chn":
+                chn.gemm_forward_cuda(x[r], w, ws, xs[r], wz, xsum[r], out[r])
+            elif mode == "grp":
+                grp.gemm_forward_cuda(x[r], w, z2, s2, ws, xs[r], out[r])
+            else:
+                w8.w8a8_gemm_forward_cuda(x[r], w, ws, xs[r], out[r])
+        assert torch.isfinite(out.float()).all()
+        got.append(out)
+    assert torch.equal(*got)
