@@ -27,6 +27,7 @@
 //     weight stream.
 //   * epilogue fused: acc*s1[n]*sa[m] - s1z[n]*asum[m] (per-channel) or acc*(s1[n]*sa[m]) (per-group, W8A8) -> fp16,
 //     IEEE fp32 in the reference's source order (bit-exact against the oracle).
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -1129,7 +1130,9 @@ int make_tmap_w4(CUtensorMap* m, const void* ptr, uint64_t N, uint64_t K, uint32
   return QS_OK;
 }
 
-int choose_split(int tiles, int kb_per_tile, int forced) {
+// resident(s): clusters of s CTAs of the kernel that the device holds at a time
+template <class Resident>
+int choose_split(int tiles, int kb_per_tile, int forced, Resident resident) {
   int s = 1;
   if (forced > 0) {
     s = forced;
@@ -1140,8 +1143,10 @@ int choose_split(int tiles, int kb_per_tile, int forced) {
   }
   if (s > 8) s = 8;
   while (s > 1 && kb_per_tile < s) s /= 2;
-  // split launches carry a receive buffer and run one CTA per SM: never more CTAs than SMs (a second wave costs more than it saves)
-  if (forced <= 0) while (s > 1 && tiles * s > num_sms()) s /= 2;
+  // split launches carry a receive buffer and mostly run one CTA per SM: never more CTAs than SMs, nor more clusters than the device holds (a GPC's SMs that
+  // are left over from whole clusters stay idle: 33 clusters of 4, 15 of 8), since a second wave costs more than the split saves.  Measured, 3584 K, per channel:
+  // 36 tiles at 16 tokens 10.2 us by 4 and 6.1 by 2, at 128 tokens 15.4 and 10.6; 16 tiles 8.6 by 8 and 4.8 by 4 (the last count that fits, 33: 6.1 by 4)
+  if (forced <= 0) while (s > 1 && (tiles * s > num_sms() || tiles > resident(s))) s /= 2;
   return s;
 }
 
@@ -1163,8 +1168,6 @@ int launch_gemm(const GemmArgs& a) {
   p.m_tiles = (a.M + NT - 1) / NT;
   p.kb_per_tile = (a.K + C::kSub * kBK - 1) / (C::kSub * kBK);  // pipeline stages (W4A8: of 256 K, the last one may be half zero-filled)
   const int tiles = n_tiles * p.m_tiles;
-  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.force_split) : 1;  // NT = 256: no room for the receive buffer
-
   CUtensorMap tm_act, tm_w;
   int rc = make_tmap_u8(&tm_act, a.act, a.M, a.K, NT);
   if (rc) return rc;
@@ -1181,8 +1184,33 @@ int launch_gemm(const GemmArgs& a) {
     done = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(tiles * p.split);
   cfg.blockDim = dim3(kNumThreads);
+  auto resident = [&](int split) {
+    // (W8A8's 32-token tiles: two CTAs per SM, whatever the query says, which counts one: 16 tiles 5.6 us by 8 and 6.5 by 4)
+    if (C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return num_sms() / split;
+    static std::atomic<int> held[2][kMaxDevices][4] = {};  // per (instantiation, device, split), as the attribute above; 0: not asked yet
+    std::atomic<int>& h = held[a.acc_out ? 1 : 0][device_ordinal()][split == 2 ? 1 : split == 4 ? 2 : 3];
+    int n = h.load(std::memory_order_relaxed);
+    if (n == 0) {
+      cudaLaunchAttribute cluster;
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      cluster.val.clusterDim.x = split;
+      cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+      cudaLaunchConfig_t ask = cfg;
+      ask.gridDim = dim3(tiles * split);
+      ask.dynamicSmemBytes = C::kSmemBytesSplit;
+      ask.attrs = &cluster;
+      ask.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &ask) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = num_sms() / split;
+      }
+      h.store(n, std::memory_order_relaxed);
+    }
+    return n;
+  };
+  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.force_split, resident) : 1;  // NT = 256: no room for the receive buffer
+  cfg.gridDim = dim3(tiles * p.split);
   cfg.dynamicSmemBytes = p.split > 1 ? C::kSmemBytesSplit : C::kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(a.stream);
   cudaLaunchAttribute attr[2];
