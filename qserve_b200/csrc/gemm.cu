@@ -583,71 +583,68 @@ struct PairCfg {
   static_assert(kSmemBytes <= 226 * 1024, "shared memory overflow");
 };
 
-// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and `cols` tokens from column col0 on, 32 (at last 16) at a
-// time; a warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum:
-// the tokens', m0: the tile's first token
-template <int MODE, bool ACC, int CH>
-__device__ __forceinline__ void pair_drain_chunk(const GemmParams& p, uint32_t trow, int tok0, int m0, int n, float ws, float wz, const float* s_asc,
-                                                 const float* s_asum) {
-  uint32_t r[CH];
-  if constexpr (CH == 32) tmem_ld_32x32b_x32(trow + tok0, r);
-  else tmem_ld_32x32b_x16(trow + tok0, r);
-  tmem_wait_ld();
+// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and `cols` tokens from column col0 on, 32 at a time; a
+// warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum: the
+// tokens', m0: the tile's first token
+template <int MODE, bool ACC>
+__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int cols, int m0, int n, float ws, float wz, const float* s_asc,
+                                           const float* s_asum) {
   const int tok_end = p.M - m0;
-  __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
-  if (tok0 + CH <= tok_end) {
-    // whole chunk inside M: no per-token branches, the scales come in as vectors, CH independent chains
-    float as[CH], am[CH];
+  // chunks that hold tokens (those past M cost the ragged tile 1 us); the shuffle shows the compiler that all of the warp's threads take as many
+  const int chunks = __shfl_sync(~0u, (min(cols, tok_end - col0) + 31) >> 5, 0);
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    const int tok0 = col0 + c * 32;
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(trow + tok0, r);
+    tmem_wait_ld();
+    __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
+    if (tok0 + 32 <= tok_end) {
+      // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
+      float as[32], am[32];
 #pragma unroll
-    for (int i = 0; i < CH; i += 4) {
-      const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
-      as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
-      if constexpr (MODE == kModeW4Chn) {
-        const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
-        am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
-      } else {
-        am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
+      for (int i = 0; i < 32; i += 4) {
+        const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
+        as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
+        if constexpr (MODE == kModeW4Chn) {
+          const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
+          am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
+        } else {
+          am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
+        }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
-      out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
-      if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
-      if (tok0 + i < tok_end) {
-        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
+      for (int i = 0; i < 32; ++i) {
+        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
         out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
         if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
+        if (tok0 + i < tok_end) {
+          const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
+          out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
+          if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+        }
       }
     }
   }
 }
-template <int MODE, bool ACC>
-__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int cols, int m0, int n, float ws, float wz, const float* s_asc,
-                                           const float* s_asum) {
-  int c = 0;
-#pragma unroll 1
-  for (; c + 16 < cols; c += 32) pair_drain_chunk<MODE, ACC, 32>(p, trow, col0 + c, m0, n, ws, wz, s_asc, s_asum);
-  if (c < cols) pair_drain_chunk<MODE, ACC, 16>(p, trow, col0 + c, m0, n, ws, wz, s_asc, s_asum);
-}
 // zero-fills an accumulator's columns [col0, col0 + cols) of the warp's 32 lanes
-__device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols) {
+__device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols, int nt) {
   auto eight = [&](int c) {
     tmem_st_16x128b_x2(trow + col0 + c, 0u, 0u, 0u, 0u);
     tmem_st_16x128b_x2(trow + col0 + c + (16u << 16), 0u, 0u, 0u, 0u);
   };
-  if (cols == 128) {  // (a loop takes 1 % of a tile of 4096 K longer)
+  if (nt == 256) {  // (a loop takes 1 % of a tile of 4096 K longer)
 #pragma unroll
     for (int c = 0; c < 128; c += 8) eight(c);
   } else {
 #pragma unroll 1
-    for (int c = 0; c < cols; c += 16) {
-      eight(c);
-      eight(c + 8);
+    for (int c = 0; c < cols; c += 32) {
+#pragma unroll
+      for (int k = 0; k < 32; k += 8) eight(c + k);
     }
   }
   tmem_wait_st();
@@ -655,7 +652,8 @@ __device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols) {
   __syncwarp();
 }
 
-template <int MODE, bool ACC>
+// FULL: tiles of 256 tokens, known to the compiler (per channel 28672 x 4096 at 1024 tokens 86.4 us, 87.0 without; 8192 x 512 at 512 7.8 and 7.9)
+template <int MODE, bool ACC, bool FULL>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) {
   using C = PairCfg<MODE>;
@@ -684,7 +682,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int total = p.m_tiles * ((p.N / kBM) >> 1);
   const int my_tiles = (total - pair + n_pairs - 1) / n_pairs;  // >= 1: the host launches at most `total` pairs
-  const int n_kb = p.kb_per_tile, nt = p.nt, nh = nt >> 1;
+  const int n_kb = p.kb_per_tile, nt = FULL ? 256 : p.nt, nh = nt >> 1;
   qs_trace(QS_K_GEMM, 0);
   if (threadIdx.x == 0) QS_PROF(0);
 
@@ -805,11 +803,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
     const bool unpacker = warp < 8;           // first / second warp of its lane quadrant
     const int quad = warp & 3;
     const int usel = unpacker ? 0 : 1;        // the 128-K sub-block of a stage this warp unpacks
-    const int col0 = unpacker ? 0 : nh;   // first accumulator column (token) of this warp's half
+    // accumulator columns (tokens) of this warp: half of them, in chunks of 32
+    const int first = (nt + 63) / 64 * 32, col0 = unpacker ? 0 : first, cols = unpacker ? first : nt - first;
     const int epi_tid = quad * 32 + lane;     // channel inside the tile
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     auto zero_fill = [&]() {
-      pair_zero(trow, col0, nh);
+      pair_zero(trow, col0, cols, nt);
       if (lane == 0) mbar_arrive_cluster(bar_zero, 0);
     };
     zero_fill();
@@ -885,7 +884,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       mbar_wait(bar_dfull, lt & 1);  // every MMA of the tile has retired
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(9);
       tc_fence_after();
-      pair_drain<MODE, ACC>(p, trow, col0, nh, m0, n, ws, wz, s_asc, s_asum);
+      pair_drain<MODE, ACC>(p, trow, col0, cols, m0, n, ws, wz, s_asc, s_asum);
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(10);
       if (lt + 1 < my_tiles) zero_fill();  // hands the accumulator back to the MMA issuers
       if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(11);
@@ -1011,10 +1010,10 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
     }
   } else if ((warp >= 2 && warp <= 5) || warp >= 8) {
     // a warp reaches the TMEM lanes 32 * (warp % 4) ..: the two warps of a quadrant take half of the token columns each
-    const int quad = warp & 3, col0 = warp < 8 ? 0 : nh, epi_tid = quad * 32 + lane;
+    const int first = (nt + 63) / 64 * 32, quad = warp & 3, col0 = warp < 8 ? 0 : first, cols = warp < 8 ? first : nt - first, epi_tid = quad * 32 + lane;
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     auto zero_fill = [&](int buf) {
-      pair_zero(trow + buf * NT, col0, nh);
+      pair_zero(trow + buf * NT, col0, cols, nt);
       if (lane == 0) mbar_arrive_cluster(&bar_zero[buf], 0);
     };
     zero_fill(0);
@@ -1029,7 +1028,7 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
       named_bar_sync(1, 256);
       mbar_wait(&bar_dfull[buf], (static_cast<uint32_t>(lt) >> 1) & 1u);
       tc_fence_after();
-      pair_drain<kModeW8, ACC>(p, trow + buf * NT, col0, nh, m0, n, ws, 0.f, s_asc, s_asc);
+      pair_drain<kModeW8, ACC>(p, trow + buf * NT, col0, cols, m0, n, ws, 0.f, s_asc, s_asc);
       if (lt + 2 < my_tiles) zero_fill(buf);
     }
   } else {
@@ -1132,17 +1131,17 @@ int make_tmap_w4(CUtensorMap* m, const void* ptr, uint64_t N, uint64_t K, uint32
 
 // resident(s): clusters of s CTAs of the kernel that the device holds at a time
 template <class Resident>
-int choose_split(int tiles, int kb_per_tile, int forced, Resident resident) {
+int choose_split(int tiles, int stages, int sub_blocks, int forced, Resident resident) {
   int s = 1;
   if (forced > 0) {
     s = forced;
   } else {
     const int sms = num_sms();
-    // smallest power of two that brings the CTA count to >= ~2/3 of the SMs; every CTA keeps >= 2 k-blocks
-    while (s < 8 && tiles * s < (2 * sms) / 3 && kb_per_tile / (2 * s) >= 1) s *= 2;
+    // smallest power of two that brings the CTA count to >= ~2/3 of the SMs; every CTA keeps >= 2 blocks of 128 K
+    while (s < 8 && tiles * s < (2 * sms) / 3 && sub_blocks / (4 * s) >= 1) s *= 2;
   }
   if (s > 8) s = 8;
-  while (s > 1 && kb_per_tile < s) s /= 2;
+  while (s > 1 && stages < s) s /= 2;
   // split launches carry a receive buffer and mostly run one CTA per SM: never more CTAs than SMs, nor more clusters than the device holds (a GPC's SMs that
   // are left over from whole clusters stay idle: 33 clusters of 4, 15 of 8), since a second wave costs more than the split saves.  Measured, 3584 K, per channel:
   // 36 tiles at 16 tokens 10.2 us by 4 and 6.1 by 2, at 128 tokens 15.4 and 10.6; 16 tiles 8.6 by 8 and 4.8 by 4 (the last count that fits, 33: 6.1 by 4)
@@ -1209,7 +1208,7 @@ int launch_gemm(const GemmArgs& a) {
     }
     return n;
   };
-  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.force_split, resident) : 1;  // NT = 256: no room for the receive buffer
+  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.K / kBK, a.force_split, resident) : 1;  // NT = 256: no room for the receive buffer
   cfg.gridDim = dim3(tiles * p.split);
   cfg.dynamicSmemBytes = p.split > 1 ? C::kSmemBytesSplit : C::kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(a.stream);
@@ -1228,20 +1227,51 @@ int launch_gemm(const GemmArgs& a) {
 // Tokens of a pair tile.  All pairs take a tile at a time, so the rounds count, and a round takes a share of its time whatever the tile's tokens: the group
 // scales' unpacking 0.71 of that of 256 tokens, per-channel weights 0.25, W8A8 0.57 (its operands' way out of L2), measured at 4736 tokens with 128 to 256 per
 // tile, 4096 x 4096.  4096 x 14336 at 512 tokens: 45 us with 256 per tile, 35 with 128; 4096 x 4096 at 4736: 76 with 256 (4.1 rounds), 70 with 224 (4.8).
-int pair_tokens(int M, int N, int mode) {
+// A smaller tile has to win by 2 % and, for short K, by up to 10 % more: a few tiles in a last round run faster than a full one, and SMs that are left free
+// take the next kernel's set-up (3584 x 2048 at 1024 tokens, 56 tiles of 256 11.4 us, 70 of 224 12.0).
+int pair_tokens(int M, int N, int K, int mode) {
   const float fixed = mode == kModeW4Grp ? 0.71f : mode == kModeW4Chn ? 0.25f : 0.57f;
   const int pairs = num_sms() / 2;
+  const float margin = 0.98f - 0.1f * std::min(1.f, 2048.f / static_cast<float>(K));
   int best = 256;
   float best_cost = 0.f;
   for (int nt = 256; nt >= 128; nt -= 32) {
     const long long tiles = static_cast<long long>((M + nt - 1) / nt) * (N / kBM / 2);
     const float cost = static_cast<float>((tiles + pairs - 1) / pairs) * (fixed + (1.f - fixed) * static_cast<float>(nt) / 256.f);
-    if (nt == 256 || cost < 0.98f * best_cost) {
+    if (nt == 256 || cost < margin * best_cost) {
       best = nt;
       best_cost = cost;
     }
   }
   return best;
+}
+
+// Whether CTA pairs are faster than the 128-token tiles of gemm_kernel.  A pair stages half of its tokens per SM and walks its tiles in one ring, so it wins
+// wherever the other kernel has one CTA per SM and no split over K (us, other kernel / pairs): per channel 12288 x 4096 at 65 to 128 tokens 17 / 13,
+// 4096 x 14336 at 257 41 / 28, 6144 x 4096 at 200 16.9 / 12.4; group scales 22 / 15, 60 / 40, 22.3 / 14.9; W8A8 at 128 16.5 / 15.3, at 257 37.7 / 32.2.
+// It does not
+//  - where gemm_kernel can split K over clusters, unless K is too short for that: below 512 tokens 4096 x 1024 at 140 7.2 / 6.6, 4096 x 2048 8.5 / 8.3,
+//    1024 x 1024 at 257 (split 4) 6.2 / 6.3; from 512 tokens on the pairs' tiles are full: 2048 x 4096 at 512 11.0 / 10.9, x 8192 15.8 / 17.1, 1024 x 1024
+//    at 512 (split 4) 6.6 / 5.9, x 2048 7.1 / 7.8 (W8A8 x 4096 at 600 11.7 / 12.7);
+//  - W4A8 with two CTAs per SM (at most 2 x SMs tiles) where the pairs take a second round: 12288 x 4096 at 300 19.2 / 21.1, 4096 x 4096 at 1100 18.2 / 20.2
+//    (at 400, 384 tiles, 33.4 / 22.5).  W8A8's tiles run one per SM there: 24.3 / 22.0;
+//  - calls of a few us, whose set-up counts: group scales with 512 K 12288 at 140 7.6 / 7.8, with 1024 K at 80 7.8 / 8.2, per channel with 512 K 18688 at 200
+//    8.3 / 9.3, W8A8 with 1024 K 6144 at 200 7.1 / 7.2, 9728 at 65 with 2048 K 10.1 / 10.2.
+bool pairs_pay(int M, int N, int K, int mode) {
+  if (M <= 64 || (N / kBM) % 2 != 0 || K < 512) return false;
+  const bool w8 = mode == kModeW8;
+  const int sms = num_sms(), t128 = (M + 127) / 128, tiles = (N / kBM) * t128;
+  if (2 * tiles <= sms) {
+    if (M <= 128) return false;
+    const int split = 10 * tiles < sms ? 8 : 9 * tiles < 2 * sms ? 4 : 2;  // about what choose_split takes
+    if (M < 512 || w8) return K * split <= 2048;
+    return (split == 2 ? K : K * split) < 8192;
+  }
+  if (M <= 128) return tiles < sms && K >= 2048 && (!w8 || M >= 96);
+  if (w8) return tiles > sms || K >= 2048;
+  const int nt = pair_tokens(M, N, K, mode);
+  if (tiles <= 2 * sms && 2 * ((M + nt - 1) / nt) * (N / kBM / 2) > sms) return false;
+  return M >= 512 || (tiles <= sms ? mode == kModeW4Chn || K >= 1024 : K >= 2048) || (tiles >= 2 * sms && t128 % 2 == 0);
 }
 
 // prefill: CTA pairs (cta_group::2), 256 channels x 128 to 256 tokens per pair
@@ -1261,7 +1291,7 @@ int launch_gemm_pair(const GemmArgs& a) {
   p.acc_out = static_cast<int32_t*>(a.acc_out);
   p.M = a.M; p.N = a.N; p.K = a.K;
   const int n_tiles = a.N / kBM;
-  p.nt = pair_tokens(a.M, a.N, MODE);
+  p.nt = pair_tokens(a.M, a.N, a.K, MODE);
   p.m_tiles = (a.M + p.nt - 1) / p.nt;
   p.kb_per_tile = (a.K + stage_k - 1) / stage_k;
   p.split = 1;
@@ -1273,10 +1303,11 @@ int launch_gemm_pair(const GemmArgs& a) {
   if (rc) return rc;
   auto kern = [&] {
     if constexpr (w8) return a.acc_out ? gemm_pair_w8_kernel<true> : gemm_pair_w8_kernel<false>;
-    else return a.acc_out ? gemm_pair_kernel<MODE, true> : gemm_pair_kernel<MODE, false>;
+    else if (p.nt == 256) return a.acc_out ? gemm_pair_kernel<MODE, true, true> : gemm_pair_kernel<MODE, false, true>;
+    else return a.acc_out ? gemm_pair_kernel<MODE, true, false> : gemm_pair_kernel<MODE, false, false>;
   }();
-  static bool attr_set[2][kMaxDevices] = {};
-  bool& done = attr_set[a.acc_out ? 1 : 0][device_ordinal()];
+  static bool attr_set[2][2][kMaxDevices] = {};
+  bool& done = attr_set[a.acc_out ? 1 : 0][p.nt == 256 ? 1 : 0][device_ordinal()];
   if (!done) {
     rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes), "cudaFuncSetAttribute(gemm pair smem)");
     if (rc) return rc;
@@ -1312,15 +1343,8 @@ int dispatch_gemm(const GemmArgs& a) {
   constexpr bool w8 = (MODE == kModeW8), grp = (MODE == kModeW4Grp);
   QS_REQUIRE(a.force_nt == 0 || a.force_nt == 32 || a.force_nt == 64 || a.force_nt == 128, "gemm: tile tokens must be 32, 64 or 128");
   {
-    static const bool no_pair = getenv("QS_GEMM_NO_PAIR") != nullptr;  // A/B hooks
-    static const int pair_min_m = getenv("QS_GEMM_PAIR_MIN_M") ? atoi(getenv("QS_GEMM_PAIR_MIN_M")) : 512;
-    // Below 512 tokens the pair kernel pays only if its 256-token tiles are as well filled as the 128-token ones (an even number of 128-token
-    // tiles: M in (128, 256] or (384, 512)) and there is at least one pair tile per TPC (measured: gate_up at M = 256
-    // 30.4 vs 35.5 us, at M = 320 58.1 vs 50.5; o_proj (16 pair tiles) at M = 256 16.6 vs 12.0).  W8A8: wherever the 128-token tiles are more than the SMs
-    // (28672 x 4096, M = 200 43 vs 65 us, 300 59 vs 72; 6144 x 4096, M = 400 25 vs 31, but M = 300, 144 tiles, 24.5 vs 22.5; 4096 x 4096, M = 400 22.5 vs 20.5)
-    const int t128 = (a.M + 127) / 128;
-    const bool small_ok = a.M > 128 && (w8 ? (a.N / kBM) * t128 > num_sms() : t128 % 2 == 0 && (a.N / kBM / 2) * ((a.M + 255) / 256) >= num_sms() / 2);
-    if (!no_pair && a.force_nt == 0 && a.force_split == 0 && (a.M >= pair_min_m || small_ok) && (a.N / kBM) % 2 == 0 && a.K >= 512) return launch_gemm_pair<MODE>(a);
+    static const bool no_pair = getenv("QS_GEMM_NO_PAIR") != nullptr;  // A/B hook
+    if (!no_pair && a.force_nt == 0 && a.force_split == 0 && pairs_pay(a.M, a.N, a.K, MODE)) return launch_gemm_pair<MODE>(a);
   }
   int nt = a.force_nt > 0 ? a.force_nt : 0;
   if (nt == 0) {
