@@ -538,7 +538,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 }
 
 // =============================================================================================
-// Prefill tiles (M >= 512, W4A8): a PAIR of CTAs on the two SMs of a TPC computes tiles of 256 channels x 128 to 256 tokens
+// Prompt tiles (from 65 tokens on where pairs_pay says so, W4A8): a PAIR of CTAs on the two SMs of a TPC computes tiles of 256 channels x 128 to 256 tokens
 // (pair_tokens, below; the figures here are those of 256) with cta_group::2 UMMAs,
 // persistently (one pair per TPC walks the tile list).
 //
