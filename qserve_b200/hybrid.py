@@ -106,16 +106,21 @@ class StepBatch:
     tile_row0: Optional[torch.Tensor] = None     # int32 [n_tiles] first row of the tile within its entry
     long_tokens: Optional[torch.Tensor] = None   # int32 [n_long] rows covered by tiles
     short_tokens: Optional[torch.Tensor] = None  # int32 [n_short] all other rows
-    seen_entry: Optional[torch.Tensor] = None    # the tiles again, those that see most positions last
-    seen_row0: Optional[torch.Tensor] = None
 
     # when `build` is told the page size: (slot, first position, tokens) of the entries of at least TILE_MIN tokens, for `context`
     page_size: int = 0
     long_spans: Sequence[tuple] = ()
     _contexts: dict = field(default_factory=dict)
+    # the tiles again, those that see most positions last; a batch made without them has them in the order of its tiles
+    seen_entry: Optional[torch.Tensor] = None
+    seen_row0: Optional[torch.Tensor] = None
 
     TILE_MIN = 16
     TILE_ROWS = 64
+
+    def __post_init__(self):
+        if self.seen_entry is None or self.seen_row0 is None:
+            self.seen_entry, self.seen_row0 = self.tile_entry, self.tile_row0
 
     @staticmethod
     def pack(entries: Sequence[tuple]):
@@ -157,7 +162,8 @@ class StepBatch:
         v = [d[i * T:(i + 1) * T] for i in range(5)] + [d[6 * T + i * E: 6 * T + (i + 1) * E] for i in range(4)]
         o = 6 * T + 4 * E
         t = [d[o + i * nt:o + (i + 1) * nt] for i in range(4)]
-        return StepBatch(T, E, *v, block_table, nt, n_long, n_short, t[0], t[1], d[5 * T:5 * T + n_long], d[5 * T + n_long:6 * T], t[2], t[3])
+        return StepBatch(T, E, *v, block_table, nt, n_long, n_short, t[0], t[1], d[5 * T:5 * T + n_long], d[5 * T + n_long:6 * T],
+                         seen_entry=t[2], seen_row0=t[3])
 
     @staticmethod
     def build(entries: Sequence[tuple], block_table: torch.Tensor, device: torch.device, page_size: int = 0) -> "StepBatch":
