@@ -35,9 +35,9 @@ int device_ordinal() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
   return dev;
 }
-int num_sms() {
+int num_sms() { return num_sms(device_ordinal()); }
+int num_sms(int dev) {
   static int sms[kMaxDevices] = {};
-  const int dev = device_ordinal();
   if (!sms[dev]) {
     int n = 0;
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);

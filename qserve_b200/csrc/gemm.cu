@@ -77,10 +77,17 @@ struct GemmParams {
   __half* out;               // [M, N]
   int32_t* acc_out;          // optional: raw INT32 accumulators [M, N] (parity tests)
   int M, N, K;
-  int m_tiles, kb_per_tile, split;
-  int nt;                    // pair kernels: tokens of a tile, a multiple of 32 up to 256
+  int m_tiles, kb_per_tile;
+  union {
+    int split;               // gemm_kernel: CTAs of a cluster that share a tile's K
+    int nt;                  // pair kernels: tokens of a tile, a multiple of 32 up to 256
+  };
   unsigned long long* prof;  // optional: 16 globaltimer stamps per CTA (tools/gemm_timeline.py)
 };
+// With two tensor maps, 352 bytes of a launch's parameters: with 360 the host takes longer over every launch.  16 x 4096 x 4096 called back to back is as
+// much the host's as the device's (5.1 us): the loop that issues the calls took 5.17 us a call (median of twelve processes) with 360 bytes and the device
+// asked for five times a call, now 5.02; where the host is the slower of the two, 5.45 to 5.55 and 5.23
+static_assert(sizeof(GemmParams) <= 96, "the launch's parameters grew");
 
 // WS = depth of the WEIGHT ring in shared memory.  Weights are static, so the producer streams them before the
 // programmatic-dependent-launch wait: everything that fits in the ring (plus the unpacked stages parked in tensor memory)
@@ -1131,12 +1138,11 @@ int make_tmap_w4(CUtensorMap* m, const void* ptr, uint64_t N, uint64_t K, uint32
 
 // resident(s): clusters of s CTAs of the kernel that the device holds at a time
 template <class Resident>
-int choose_split(int tiles, int stages, int sub_blocks, int forced, Resident resident) {
+int choose_split(int tiles, int stages, int sub_blocks, int forced, int sms, Resident resident) {
   int s = 1;
   if (forced > 0) {
     s = forced;
   } else {
-    const int sms = num_sms();
     // smallest power of two that brings the CTA count to >= ~2/3 of the SMs; every CTA keeps >= 2 blocks of 128 K
     while (s < 8 && tiles * s < (2 * sms) / 3 && sub_blocks / (4 * s) >= 1) s *= 2;
   }
@@ -1145,7 +1151,7 @@ int choose_split(int tiles, int stages, int sub_blocks, int forced, Resident res
   // split launches carry a receive buffer and mostly run one CTA per SM: never more CTAs than SMs, nor more clusters than the device holds (a GPC's SMs that
   // are left over from whole clusters stay idle: 33 clusters of 4, 15 of 8), since a second wave costs more than the split saves.  Measured, 3584 K, per channel:
   // 36 tiles at 16 tokens 10.2 us by 4 and 6.1 by 2, at 128 tokens 15.4 and 10.6; 16 tiles 8.6 by 8 and 4.8 by 4 (the last count that fits, 33: 6.1 by 4)
-  if (forced <= 0) while (s > 1 && (tiles * s > num_sms() || tiles > resident(s))) s /= 2;
+  if (forced <= 0) while (s > 1 && (tiles * s > sms || tiles > resident(s))) s /= 2;
   return s;
 }
 
@@ -1174,8 +1180,10 @@ int launch_gemm(const GemmArgs& a) {
   if (rc) return rc;
 
   auto kern = a.acc_out ? gemm_kernel<MODE, NT, WS, AS, true> : gemm_kernel<MODE, NT, WS, AS, false>;
+  // asked for once: calls of a few us are as much the host's as the device's, and a question takes 25 ns
+  const int dev = device_ordinal(), sms = num_sms(dev);
   static bool attr_set[2][kMaxDevices] = {};  // per (instantiation, device): the attribute is a per-device property of the function
-  bool& done = attr_set[a.acc_out ? 1 : 0][device_ordinal()];
+  bool& done = attr_set[a.acc_out ? 1 : 0][dev];
   if (!done) {
     rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSplitFits ? C::kSmemBytesSplit : C::kSmemBytes),
                     "cudaFuncSetAttribute(gemm smem)");
@@ -1186,9 +1194,9 @@ int launch_gemm(const GemmArgs& a) {
   cfg.blockDim = dim3(kNumThreads);
   auto resident = [&](int split) {
     // (W8A8's 32-token tiles: two CTAs per SM, whatever the query says, which counts one: 16 tiles 5.6 us by 8 and 6.5 by 4)
-    if (C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return num_sms() / split;
+    if (C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return sms / split;
     static std::atomic<int> held[2][kMaxDevices][4] = {};  // per (instantiation, device, split), as the attribute above; 0: not asked yet
-    std::atomic<int>& h = held[a.acc_out ? 1 : 0][device_ordinal()][split == 2 ? 1 : split == 4 ? 2 : 3];
+    std::atomic<int>& h = held[a.acc_out ? 1 : 0][dev][split == 2 ? 1 : split == 4 ? 2 : 3];
     int n = h.load(std::memory_order_relaxed);
     if (n == 0) {
       cudaLaunchAttribute cluster;
@@ -1202,13 +1210,13 @@ int launch_gemm(const GemmArgs& a) {
       ask.numAttrs = 1;
       if (cudaOccupancyMaxActiveClusters(&n, kern, &ask) != cudaSuccess || n <= 0) {
         cudaGetLastError();
-        n = num_sms() / split;
+        n = sms / split;
       }
       h.store(n, std::memory_order_relaxed);
     }
     return n;
   };
-  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.K / kBK, a.force_split, resident) : 1;  // NT = 256: no room for the receive buffer
+  p.split = C::kSplitFits ? choose_split(tiles, p.kb_per_tile, a.K / kBK, a.force_split, sms, resident) : 1;  // NT = 256: no room for the receive buffer
   cfg.gridDim = dim3(tiles * p.split);
   cfg.dynamicSmemBytes = p.split > 1 ? C::kSmemBytesSplit : C::kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(a.stream);
@@ -1294,7 +1302,6 @@ int launch_gemm_pair(const GemmArgs& a) {
   p.nt = pair_tokens(a.M, a.N, a.K, MODE);
   p.m_tiles = (a.M + p.nt - 1) / p.nt;
   p.kb_per_tile = (a.K + stage_k - 1) / stage_k;
-  p.split = 1;
   p.prof = static_cast<unsigned long long*>(a.prof);
   CUtensorMap tm_act, tm_w;
   int rc = make_tmap_u8(&tm_act, a.act, a.M, a.K, p.nt / 2);

@@ -10,6 +10,7 @@ bool pdl_enabled();
 constexpr int kMaxDevices = 64;
 int device_ordinal();
 int num_sms();
+int num_sms(int dev);  // dev: what device_ordinal() said
 
 struct GemmArgs {
   const void* act = nullptr;        // int8 [M, K]
