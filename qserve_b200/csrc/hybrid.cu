@@ -1547,25 +1547,23 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
     if (int rc = column_scan(scan, kScanDelta, s)) return rc;
   } else
   // rows of a column per thread: all of them up to 64 (a warp then reads q / k as broadcasts), 64 above
-#define QS_SCAN_AS(DP, PARTS, CH, CPT, KERNEL)                                                                                                           \
+#define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
   do {                                                                                                                                        \
     constexpr int cols = 128 / PARTS * CPT;                                                                                                   \
     const size_t sm = (size_t)2 * CH * (2 * PARTS * (DP / PARTS + 4) + cols + 4) * sizeof(float);                                             \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
-    auto kern = KERNEL;                             \
+    auto kern = vec ? delta_scan_kernel<DP, PARTS, CH, CPT, true> : delta_scan_kernel<DP, PARTS, CH, CPT, false>;                             \
     if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);                                     \
     kern<<<grid, 128, sm, s>>>(o_raw, prep, state, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                              \
   } while (0)
-#define QS_SCAN(DP, PARTS, CH, CPT) QS_SCAN_AS(DP, PARTS, CH, CPT, (vec ? delta_scan_kernel<DP, PARTS, CH, CPT, true> : delta_scan_kernel<DP, PARTS, CH, CPT, false>))
   // two adjacent columns per thread where the head has the columns for it: a q / k word read from shared memory then feeds two columns
   // (the scan is bound by shared-memory bandwidth: every thread reads its rows' q and k for every token)
   if (D <= 16) QS_SCAN(16, 1, 16, 1);
   else if (D <= 32) QS_SCAN(32, 1, 16, 1);
   else if (D <= 64) { if (Dv >= 128) QS_SCAN(64, 2, 16, 2); else QS_SCAN(64, 2, 16, 1); }
-  else if (D <= 128) { if (Dv >= 64) QS_SCAN_AS(128, 8, 16, 2, (delta_scan_kernel<128, 8, 16, 2, false>)); else QS_SCAN(128, 4, 16, 1); }
+  else if (D <= 128) { if (Dv >= 64) QS_SCAN(128, 8, 16, 2); else QS_SCAN(128, 4, 16, 1); }  // a state off a 16-byte boundary
   else QS_SCAN(256, 8, 8, 1);
 #undef QS_SCAN
-#undef QS_SCAN_AS
   const int warps = T * H, gate_at = 2 * G * D + H * Dv;
   if (Dv == 128 && stride % 4 == 0 && gate_at % 4 == 0 && out_stride % 4 == 0 && al(proj, 4 * sizeof(ST)) && al(out, 4 * sizeof(ST)) && al(o_raw, 16) && al(norm_w, 16))
     delta_gate_out128_kernel<ST><<<(warps + 3) / 4, 128, 0, s>>>((ST*)out, out_stride, o_raw, (const ST*)proj + gate_at, stride, norm_w, T, H, eps);

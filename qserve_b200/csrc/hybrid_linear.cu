@@ -309,16 +309,15 @@ int launch_scan(float* o_raw, const float* prep, float* state, const float* head
     if (MODE == kScanTokenDecay) a.q = H * Dv + G * D, a.g = H * Dv, a.a = a.v = 0, a.n0 = H * Dv + 2 * G * D, a.n1 = a.n0 + H;
     if (column_scan_takes(a)) return column_scan(a, MODE, s);
   }
-#define QS_SCAN_AS(DP, PARTS, CH, CPT, KERNEL)                                                                                                           \
+#define QS_SCAN(DP, PARTS, CH, CPT)                                                                                                           \
   do {                                                                                                                                        \
     constexpr int cols = 128 / PARTS * CPT;                                                                                                   \
     const size_t smb = (size_t)2 * CH * (NVEC * PARTS * (DP / PARTS + 4) + cols + (MODE == kScanTokenDecay ? 4 : 0)) * sizeof(float);            \
     dim3 grid(E, H, (Dv + cols - 1) / cols);                                                                                                  \
-    auto kern = KERNEL;                 \
+    auto kern = vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>;                 \
     if (smb > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);                                   \
     kern<<<grid, 128, smb, s>>>(o_raw, prep, state, head_decay, entry_start, entry_len, entry_slot, entry_pos0, H, G, D, Dv);                 \
   } while (0)
-#define QS_SCAN(DP, PARTS, CH, CPT) QS_SCAN_AS(DP, PARTS, CH, CPT, (vec ? linear_scan_kernel<DP, PARTS, CH, CPT, MODE, true> : linear_scan_kernel<DP, PARTS, CH, CPT, MODE, false>))
   // rows of a column per thread: all of them up to 32, 32 or 16 above (the parts of a column meet through shuffles).  Long runs of tokens
   // (prompt portions) take two adjacent columns per thread where the head has the columns for it: a q / g word read from shared memory then
   // feeds two columns; steps of mostly single tokens are bound by reading and writing the state and keep one column per thread
@@ -326,14 +325,13 @@ int launch_scan(float* o_raw, const float* prep, float* state, const float* head
   else if (D <= 32) QS_SCAN(32, 1, 16, 1);
   else if (D <= 64) { if (Dv >= 128 && long_runs) QS_SCAN(64, 2, 16, 2); else QS_SCAN(64, 2, 16, 1); }
   // (three row vectors per token: chunks of 8 tokens keep a block's staging near 32 KB, so that as many blocks share an SM as with two)
-  else if (D <= 128) {  // (long runs of rows, values and state in 16-byte words do not come here)
-    if (Dv >= 64 && long_runs) { if (NVEC == 3) QS_SCAN_AS(128, 8, 8, 2, (linear_scan_kernel<128, 8, 8, 2, MODE, false>)); else QS_SCAN_AS(128, 8, 16, 2, (linear_scan_kernel<128, 8, 16, 2, MODE, false>)); }
+  else if (D <= 128) {  // (long runs come here where the state lies off a 16-byte boundary or a size is no multiple of 4)
+    if (Dv >= 64 && long_runs) { if (NVEC == 3) QS_SCAN(128, 8, 8, 2); else QS_SCAN(128, 8, 16, 2); }
     else QS_SCAN(128, 4, 16, 1);
   }
   else if (D <= 256) QS_SCAN(256, 8, 8, 1);
   else QS_SCAN(512, 16, 4, 1);
 #undef QS_SCAN
-#undef QS_SCAN_AS
   return check_cuda(cudaGetLastError(), "hyb linear scan");
 }
 
