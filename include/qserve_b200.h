@@ -254,8 +254,9 @@ QS_API int qs_hyb_attention(void* out, int64_t out_stride, const void* q, int64_
                             void* stream);
 /* The same attention on the fast kernels (bfloat16 storage, dim and vdim multiples of 16, vdim in {32, 64, 96, 128, 256}, heads / kv_heads <= 16):
  * entries of at least 16 tokens run as 64-row tiles on the tensor cores (tile_entry / tile_row0: entry and first row within it of every tile;
- * long_tokens: their token rows), the tokens listed in short_tokens one by one, the query heads of a key/value head as the rows of a
- * tensor-core tile and the keys shared out over several blocks.  scratch: fp32, qs_hyb_attention_scratch_floats elements.
+ * long_tokens: their token rows; any order, the tiles listed last start first, so a list by how many positions the tiles see is the fastest),
+ * the tokens listed in short_tokens one by one, the query heads of a key/value head as the rows of a tensor-core tile and the keys shared out
+ * over several blocks.  scratch: fp32, qs_hyb_attention_scratch_floats elements.
  * qs_hyb_attention_fast_supported returns 1 if the shape qualifies. */
 QS_API int qs_hyb_attention_fast_supported(int dtype, int heads, int kv_heads, int maps, int dim, int vdim, int64_t q_stride);
 /* fp32 elements of scratch that qs_hyb_attention_fast needs for a step of `tokens` tokens */

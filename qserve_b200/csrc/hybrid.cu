@@ -432,7 +432,9 @@ __global__ void __launch_bounds__(128, KT == 32 ? 3 : 2) tile_attention_kernel(
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smraw);
   __nv_bfloat16* Ks = Qs + kTileQ * SD;
   __nv_bfloat16* Vs = Ks + 2 * KT * SD;  // two key buffers, then two value buffers
-  const int tile = blockIdx.x, hm = blockIdx.y, h = hm / maps, m = hm - h * maps, g = h / (H / G);
+  // the last tiles of the list are the longest (of an entry always, of the list where the caller has sorted it): they go first, all heads of a tile together
+  const int heads = H * maps, walk = blockIdx.x / heads, hm = blockIdx.x - walk * heads, tile = gridDim.x / heads - 1 - walk;
+  const int h = hm / maps, m = hm - h * maps, g = h / (H / G);
   const int e = tile_entry[tile], r0 = tile_row0[tile];
   const int n_rows = min(kTileQ, entry_len[e] - r0);
   const int tok0 = entry_start[e] + r0, qpos0 = entry_pos0[e] + r0;
@@ -1466,7 +1468,7 @@ int launch_tiles(float* scratch, const void* q, long long q_stride, const void* 
     if (int rc = check_cuda(cudaFuncSetAttribute(tile_attention_kernel<NVT, 3, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "tile attention smem")) return rc;
     attr_set[device_ordinal()] = true;
   }
-  tile_attention_kernel<NVT, 3, KT><<<dim3(n_tiles, H * maps), 128, smem, s>>>(scratch, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kpool,
+  tile_attention_kernel<NVT, 3, KT><<<n_tiles * H * maps, 128, smem, s>>>(scratch, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kpool,
       (const __nv_bfloat16*)vpool, tile_entry, tile_row0, entry_start, entry_len, entry_slot, entry_pos0, block_table, max_blocks, H, G, maps, D, scale, page, chunk, window, sinks,
       ex.keep_first, ex.slopes, cap_in(ex, scale), cap_out(ex));
   return check_cuda(cudaGetLastError(), "hyb_attention tiles");

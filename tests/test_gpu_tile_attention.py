@@ -93,3 +93,37 @@ def test_shapes_that_stay_on_the_general_tiles(dev, H, G, page, D, scale):
 def test_tiles_without_the_short_portions(dev):
     """A call that lists the tiles of a mixed step alone: its token rows go past the number of rows it lists."""
     _run(dev, 4, 2, 2, [3, 9, 130, 1, 70], [0, 70, 5, 640, 0], 64, tiles_only=True)
+
+
+def test_the_longest_tiles_start_first(dev):
+    """Shapes that stay on the general tiles (three query heads per key/value head): a list of tiles by how many positions they see is faster than the same
+    list backwards (1.2 to 1.4 times; the other way about where the kernel starts with the first of the list), and every order gives the same bits."""
+    from qserve_b200._lib import check, lib
+    from qserve_b200.hybrid import StepBatch
+
+    H, G, lens, page, D = 6, 2, [2048, 1843, 1570, 1297], 64, 128
+    g, E, T, blocks = torch.Generator(device=dev).manual_seed(5), len(lens), sum(lens), 32
+    table = torch.arange(E * blocks, dtype=torch.int32, device=dev).view(E, blocks)
+    r = lambda *s: torch.randn(*s, device=dev, generator=g).to(BF)
+    q, k, v, out = r(T, H * D), r(E * blocks, page, G, D), r(E * blocks, page, G, D), torch.zeros(T, H * D, dtype=BF, device=dev)
+    b = StepBatch.build([(e, 0, -1, [1] * n) for e, n in enumerate(lens)], table, dev)
+    scratch = torch.zeros(int(lib.qs_hyb_attention_scratch_floats(T, H, G, 1, D)), device=dev)
+    p, us, outs = lambda t: t.data_ptr(), [], []
+    for te, tr in ((b.seen_entry, b.seen_row0), (b.seen_entry.flip(0).contiguous(), b.seen_row0.flip(0).contiguous())):
+        took = []
+        for _ in range(6):
+            a, e = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(5):
+                check(lib.qs_hyb_attention_fast(p(out), out.stride(0), p(q), q.stride(0), p(k), p(v), p(b.tok_slot), p(b.tok_pos), p(table), blocks, p(te), p(tr),
+                                                b.n_tiles, p(b.long_tokens), b.n_long, None, 0, p(b.entry_start), p(b.entry_len), p(b.entry_slot), p(b.entry_pos0),
+                                                p(scratch), H, G, 1, D, D, D ** -0.5, 0.0, 1.0, 1e-5, 0, page, 0, 0, None, None, 0,
+                                                torch.cuda.current_stream().cuda_stream))
+            e.record()
+            e.synchronize()
+            took.append(a.elapsed_time(e))
+        us.append(min(took) * 200)
+        outs.append(out.clone())
+    print(us)
+    assert torch.equal(*outs)
+    assert us[0] < 0.95 * us[1], us
