@@ -12,8 +12,11 @@
 //                    operand), accumulating in a third TMEM region
 // S, P and O share no TMEM columns (64 + 32 + 128 of the CTA's 256), so the next block's S is computed while this block's softmax goes on, and P V while
 // the next softmax does.  Blocks of 128 keys left room for P only over S, so the next S waited for P V: 8 prompts of 539 .. 1024 tokens x 32 heads 103 us,
-// then 89; with the longest query blocks of all sequences first and whole rows stored 86.  2 x 4096 tokens 374 -> 271 us (0.73 -> 1.01 PFLOP/s), 8192 tokens
-// 674 -> 489.
+// then 89; with the longest query blocks of all sequences first and whole rows stored 86, with two blocks in the first step 3 % less.  2 x 4096 tokens
+// 374 -> 271 us (0.73 -> 1.01 PFLOP/s), 8192 tokens 674 -> 489.
+// The first step takes two blocks (S in 128 columns, P in 2 x 32: nothing is there to overlap with yet): sequences of 65 to 128 tokens have one step, as with
+// blocks of 128 keys.  40 x 100 tokens x 32 heads: 31.3 us with blocks of 128, 34.6 with one block in every step, now 30.7; calls whose sequences all have one query
+// block take a form without the walk.
 // The O accumulator is rescaled only when a row's maximum has grown by more than 2^8 since the last rescale (the sum uses the same stale
 // maximum, so the quotient is exact up to rounding); the decision is taken per warp because tcgen05.ld/st are warp-collective.
 // 256 TMEM columns and 96 KB of shared memory per CTA: two CTAs per SM, one's softmax overlaps the other's MMAs.  K and V are double-buffered.
@@ -37,10 +40,12 @@ constexpr int kThreads = 192;   // warps 0..3 softmax / epilogue, warp 4 TMA pro
 constexpr int kTileBytes = kBQ * kD * 2;      // 32 KB: two swizzled [128 rows x 64 halfs] sub-tiles
 constexpr int kSubBytes = kTileBytes / 2;     // 16 KB
 constexpr int kKvBytes = kBKV * kD * 2;       // 16 KB: a K or V block, two sub-tiles of 64 rows
-constexpr int kKvSub = kKvBytes / 2;
+constexpr int kKvSub = kKvBytes / 2;          // a sub-tile's two buffers lie side by side: both blocks are the rows of one operand
 constexpr int kOffQ = 0, kOffK = kTileBytes, kOffV = kOffK + 2 * kKvBytes, kOffBar = kOffV + 2 * kKvBytes;
 constexpr int kSmemBytes = kOffBar + 128;
-constexpr uint32_t kTmemCols = 256, kColP = 64, kColO = 128;  // S: columns [0, 64), P: [64, 96), O: [128, 256)
+constexpr uint32_t kTmemCols = 256;
+// S: columns [0, 64), of the first two blocks [0, 128); P: [64, 96), of the second block [96, 128); O: [128, 256)
+constexpr uint32_t kColP = 64, kColP1 = 96, kColO = 128;
 constexpr float kRescaleThreshold = 8.f;      // log2 units
 
 // kind::f16 instruction descriptor: D = f32, A = B = f16, A K-major; B K-major (S = Q K^T) or MN-major (O = P V)
@@ -109,6 +114,8 @@ struct PrefillAttnParams {
   int q_blocks;           // query blocks of the longest sequence, as far as this launch goes
 };
 
+// ONE: no sequence of the call has more than one query block
+template <bool ONE>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const PrefillAttnParams p) {
@@ -123,11 +130,12 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   const int hkv = h / (p.num_heads / p.num_kv_heads);
   // causal, q and k positions coincide: the key blocks up to the query block's last row, as far as the sequence goes
   const int n_kb = (min((qb + 1) * kBQ, seq_len) + kBKV - 1) / kBKV;
+  const int n_steps = ONE ? 1 : max(1, n_kb - 1);  // the first one takes two blocks
 
   uint8_t* s_q = smem + kOffQ;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kOffBar);
   uint64_t* bar_q = bar + 0;       // Q tile landed
-  uint64_t* bar_s = bar + 1;       // S complete in tensor memory
+  uint64_t* bar_s = bar + 1;       // a step's S complete in tensor memory
   uint64_t* bar_read = bar + 2;    // S read by the four softmax warps (4 arrivals): the next one may follow
   uint64_t* bar_p = bar + 3;       // P written by the four softmax warps (4 arrivals)
   uint64_t* bar_o = bar + 4;       // O += P V retired: O may be rescaled / read, P overwritten
@@ -160,59 +168,72 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       mbar_expect_tx(bar_q, kTileBytes);
       tma_load_2d(s_q, &tmap_q, h * kD, q_row, bar_q);
       tma_load_2d(s_q + kSubBytes, &tmap_q, h * kD + 64, q_row, bar_q);
-      for (int j = 0; j < n_kb; ++j) {
+      auto ring = [&](int j, const CUtensorMap* map, int off, uint64_t* full, uint64_t* freed) {
         const int k_row = seq_start + j * kBKV, st = j & 1;
-        const uint32_t ph = (static_cast<uint32_t>(j) >> 1) & 1u;
-        uint8_t *kb = smem + kOffK + st * kKvBytes, *vb = smem + kOffV + st * kKvBytes;
-        mbar_wait(&bar_kfree[st], ph ^ 1u);  // a fresh barrier passes the wait on the "previous" phase
-        mbar_expect_tx(&bar_kfull[st], kKvBytes);
-        tma_load_2d(kb, &tmap_k, hkv * kD, k_row, &bar_kfull[st]);
-        tma_load_2d(kb + kKvSub, &tmap_k, hkv * kD + 64, k_row, &bar_kfull[st]);
-        mbar_wait(&bar_vfree[st], ph ^ 1u);
-        mbar_expect_tx(&bar_vfull[st], kKvBytes);
-        tma_load_2d(vb, &tmap_v, hkv * kD, k_row, &bar_vfull[st]);
-        tma_load_2d(vb + kKvSub, &tmap_v, hkv * kD + 64, k_row, &bar_vfull[st]);
+        uint8_t* buf = smem + off + st * kKvSub;
+        mbar_wait(&freed[st], ((static_cast<uint32_t>(j) >> 1) & 1u) ^ 1u);  // a fresh barrier passes the wait on the "previous" phase
+        mbar_expect_tx(&full[st], kKvBytes);
+        tma_load_2d(buf, map, hkv * kD, k_row, &full[st]);
+        tma_load_2d(buf + 2 * kKvSub, map, hkv * kD + 64, k_row, &full[st]);
+      };
+      ring(0, &tmap_k, kOffK, bar_kfull, bar_kfree);
+      for (int j = 0; j < n_kb; ++j) {
+        if (j + 1 < n_kb) ring(j + 1, &tmap_k, kOffK, bar_kfull, bar_kfree);
+        ring(j, &tmap_v, kOffV, bar_vfull, bar_vfree);
       }
     }
   } else if (warp == 5) {
     // ===================================== MMA issuer =====================================
     if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_f16(kBQ, kBKV, 0u);
+      constexpr uint32_t idesc_qk = umma_idesc_f16(kBQ, kBKV, 0u), idesc_qk2 = umma_idesc_f16(kBQ, 2 * kBKV, 0u);
       constexpr uint32_t idesc_pv = umma_idesc_f16(kBQ, kD, 1u);
-      auto products = [&](int j, uint32_t at) {  // Q K^T of block j
-        const int st = j & 1;
-        mbar_wait(&bar_kfull[st], (static_cast<uint32_t>(j) >> 1) & 1u);
+      auto products = [&](int st, uint32_t idesc) {  // Q K^T of the block in buffer st, or of the blocks in both
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks) {
           const uint64_t adesc = umma_desc_sw128(smem_u32(s_q + (ks >> 2) * kSubBytes)) + (ks & 3) * 2;
-          const uint64_t bdesc = umma_desc_sw128(smem_u32(smem + kOffK + st * kKvBytes + (ks >> 2) * kKvSub)) + (ks & 3) * 2;
-          umma_f16_ss(at, adesc, bdesc, idesc_qk, ks > 0 ? 1u : 0u);
+          const uint64_t bdesc = umma_desc_sw128(smem_u32(smem + kOffK + st * kKvSub + (ks >> 2) * 2 * kKvSub)) + (ks & 3) * 2;
+          umma_f16_ss(tmem_s, adesc, bdesc, idesc, ks > 0 ? 1u : 0u);
         }
-      };
-      auto scores = [&](int j) {  // S of block j
-        if (j > 0) mbar_wait(bar_read, static_cast<uint32_t>(j - 1) & 1u);
-        products(j, tmem_s);
-        // the first maximum is that of two blocks: the second one's scores, into the columns where O will be, for their maximum alone
-        if (j == 0 && n_kb > 1) products(1, tmem_s + kColO);
         umma_commit(bar_s);
-        umma_commit(&bar_kfree[j & 1]);
       };
-      mbar_wait(bar_q, 0);
-      scores(0);
-      for (int j = 0; j < n_kb; ++j) {
-        if (j + 1 < n_kb) scores(j + 1);  // while the softmax of block j goes on
+      // O += P V of block j: A = P (fp16 pairs, 8 TMEM columns per 16 keys), B = V rows [key][dim] = MN-major, 16 keys (2 KB) per instruction
+      auto weighted = [&](int j, uint32_t weights) {
         const int st = j & 1;
-        mbar_wait(bar_p, static_cast<uint32_t>(j) & 1u);
         mbar_wait(&bar_vfull[st], (static_cast<uint32_t>(j) >> 1) & 1u);
         tc_fence_after();
-        // O += P V: A = P (fp16 pairs, 8 TMEM columns per 16 keys), B = V rows [key][dim] = MN-major, 16 keys (2 KB) per instruction
 #pragma unroll
         for (int kk = 0; kk < kBKV / 16; ++kk) {
-          const uint64_t bdesc = umma_desc_sw128_mn(smem_u32(smem + kOffV + st * kKvBytes + kk * 2048), kKvSub);
-          umma_f16_ts(tmem_s + kColO, tmem_s + kColP + kk * 8, bdesc, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          const uint64_t bdesc = umma_desc_sw128_mn(smem_u32(smem + kOffV + st * kKvSub + kk * 2048), 2 * kKvSub);
+          umma_f16_ts(tmem_s + kColO, weights + kk * 8, bdesc, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
         }
         umma_commit(&bar_vfree[st]);
+      };
+      mbar_wait(bar_q, 0);
+      mbar_wait(&bar_kfull[0], 0);
+      if (n_kb > 1) {
+        mbar_wait(&bar_kfull[1], 0);
+        products(0, idesc_qk2);
+        umma_commit(&bar_kfree[1]);
+      } else {
+        products(0, idesc_qk);
+      }
+      umma_commit(&bar_kfree[0]);
+      for (int i = 0; i < n_steps; ++i) {
+        if (i + 1 < n_steps) {  // the next step's S (block i + 2), while this step's softmax goes on
+          const int st = i & 1;
+          mbar_wait(bar_read, static_cast<uint32_t>(i) & 1u);
+          mbar_wait(&bar_kfull[st], ((static_cast<uint32_t>(i) + 2) >> 1) & 1u);
+          products(st, idesc_qk);
+          umma_commit(&bar_kfree[st]);
+        }
+        mbar_wait(bar_p, static_cast<uint32_t>(i) & 1u);
+        if (i == 0) {
+          weighted(0, tmem_s + kColP);
+          if (n_kb > 1) weighted(1, tmem_s + kColP1);
+        } else {
+          weighted(i + 1, tmem_s + kColP);
+        }
         umma_commit(bar_o);
       }
     }
@@ -223,128 +244,187 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     const int q_pos = qb * kBQ + row;  // position inside the sequence
     float m_used = -CUDART_INF_F;      // the maximum the accumulated O and l are expressed against (log2 domain, scaled)
     float l = 0.f;
-    // A row's largest weight against the maximum that is used is exactly 1 and rounds to fp16 without an error; the first 128 keys hold it more often than
-    // the first 64 (error against 64 bits 0.6 % larger with the first block's own maximum), so the second block's scores have a say in the first maximum
-    float second = -CUDART_INF_F;
-    if (n_kb > 1) {
-      mbar_wait(bar_s, 0);
-      tc_fence_after();
-      uint32_t r[2][32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_o + c * 32, r[c]);
-      tmem_wait_ld();
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (kBKV + c * 32 + i <= q_pos) second = fmaxf(second, __uint_as_float(r[c][i]));
-    }
-    for (int j = 0; j < n_kb; ++j) {
-      const uint32_t ph = static_cast<uint32_t>(j) & 1u;
-      mbar_wait(bar_s, ph);
-      tc_fence_after();
-      // ---- the whole S row (64 fp32) comes into registers with ONE TMEM round trip ----
-      uint32_t r[kBKV / 32][32];
-#pragma unroll
-      for (int c = 0; c < kBKV / 32; ++c) tmem_ld_32x32b_x32(t_s + c * 32, r[c]);
+    using Row = uint32_t[2][32];       // of S: 64 fp32
+    Row r;
+    uint32_t pk[32];                   // its weights
+    auto fetch = [&](Row& x, uint32_t from) {
+      tmem_ld_32x32b_x32(from, x[0]);
+      tmem_ld_32x32b_x32(from + 32, x[1]);
+    };
+    auto fetched = [&]() {
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_read);
+    };
+    auto mask = [&](Row& x, int j) {
       if (j * kBKV + kBKV - 1 > qb * kBQ + warp * 32) {  // warp-uniform: the block reaches past the warp's first row
 #pragma unroll
-        for (int c = 0; c < kBKV / 32; ++c)
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (j * kBKV + c * 32 + i > q_pos) r[c][i] = 0xff800000u;  // -inf: exp2 turns it into an exact 0
+            if (j * kBKV + c * 32 + i > q_pos) x[c][i] = 0xff800000u;  // -inf: exp2 turns it into an exact 0
       }
-      float top[4] = {second, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-      second = -CUDART_INF_F;
+    };
+    auto largest = [&](const Row& x, float m) {
+      float top[4] = {m, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-      for (int c = 0; c < kBKV / 32; ++c)
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], __uint_as_float(r[c][i]));
-      const float m_blk = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * p.scale_log2;
-      // ---- lazy rescale of O and l (warp-uniform decision) ----
-      const bool grow = (m_blk - m_used) > kRescaleThreshold;  // true on the first block (m_used = -inf; every row sees its first key there)
-      auto retired = [&]() {  // the previous O += P V
-        if (j > 0) {
-          mbar_wait(bar_o, ph ^ 1u);
-          tc_fence_after();
-        }
-      };
-      if (__any_sync(0xffffffffu, grow)) {
-        retired();
-        const float m_new = grow ? m_blk : m_used;
-        const float alpha = (m_used == -CUDART_INF_F) ? 0.f : ex2_approx(m_used - m_new);  // 1 for rows that keep their maximum
-        if (j > 0) {
-#pragma unroll 1
-          for (int c = 0; c < kD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32b_x32(t_o + c * 32, o);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32b_x32(t_o + c * 32, o);
-          }
-        }
-        l *= alpha;
-        m_used = m_new;
-      }
-      // ---- P = exp2(s * scale - m_used), rounded to fp16 ----
-      uint32_t pk[32];
+        for (int i = 0; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], __uint_as_float(x[c][i]));
+      return fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+    };
+    auto weights = [&](const Row& x) {  // P = exp2(s * scale - m_used), rounded to fp16
 #pragma unroll
       for (int i = 0; i < 64; i += 2) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(r[i >> 5][i & 31]), p.scale_log2, -m_used));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(r[i >> 5][(i & 31) + 1]), p.scale_log2, -m_used));
+        const float p0 = ex2_approx(fmaf(__uint_as_float(x[i >> 5][i & 31]), p.scale_log2, -m_used));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(x[i >> 5][(i & 31) + 1]), p.scale_log2, -m_used));
         const __half2 h2 = __floats2half2_rn(p0, p1);
         // the row sum is taken over the ROUNDED probabilities: numerator (the MMA sees fp16 P) and denominator then agree
         const float2 f = __half22float2(h2);
         l += f.x + f.y;
         pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
       }
-      retired();
-      tmem_st_32x32b_x32(t_s + kColP, pk);
+    };
+    auto stored = [&]() {
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_p);
-    }
-    // ---- epilogue: O / l -> fp16 ----
-    mbar_wait(bar_o, static_cast<uint32_t>(n_kb - 1) & 1u);
+    };
+    // The first step takes two blocks; the second one's scores lie where P will be (a warp has read its lanes of them before it writes P).  A row's largest
+    // weight against the maximum that is used is exactly 1 and rounds to fp16 without an error; the first 128 keys hold it more often than the first 64
+    // (error against 64 bits 0.6 % larger with the first block's own maximum).  With more steps to come the second block's scores are read twice, for their
+    // maximum and for their weights: with both rows held (152 registers) a step of one long and many short prompts took up to 1.4 times as long (20 x 64 and
+    // 2048 tokens: 130 us, 89 with 127 registers)
+    mbar_wait(bar_s, 0);
     tc_fence_after();
-    const float inv = 1.f / l;
-    // through shared memory (every product has retired: the K and V buffers are free), so that half a warp stores a whole row; a lane per row touched 32
-    // lines with every store
-    constexpr int kPitch = kD * 2 + 16;
-    uint8_t* mine = smem + kOffK + warp * 32 * kPitch;
-    static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the K and V buffers");
-#pragma unroll 1
-    for (int c = 0; c < kD / 32; c += 2) {
-      uint32_t r[2][32];
-      tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
-      tmem_ld_32x32b_x32(t_o + c * 32 + 32, r[1]);
+    if constexpr (ONE) {
+      Row r1;
+      fetch(r, t_s);
+      if (n_kb > 1) fetch(r1, t_s + kBKV);
       tmem_wait_ld();
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        uint4 o;
-        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t* x = &r[v >> 2][(v & 3) * 8 + 2 * e];
-          const __half2 h2 = __floats2half2_rn(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv);
-          ow[e] = *reinterpret_cast<const uint32_t*>(&h2);
-        }
-        *reinterpret_cast<uint4*>(mine + lane * kPitch + c * 64 + v * 16) = o;
+      mask(r, 0);
+      float m = largest(r, -CUDART_INF_F);
+      if (n_kb > 1) {
+        mask(r1, 1);
+        m = largest(r1, m);
+      }
+      m_used = m * p.scale_log2;
+      weights(r);
+      tmem_st_32x32b_x32(t_s + kColP, pk);
+      if (n_kb > 1) {
+        weights(r1);
+        tmem_st_32x32b_x32(t_s + kColP1, pk);
+      }
+    } else {
+      float m = -CUDART_INF_F;
+      if (n_kb > 1) {
+        fetch(r, t_s + kBKV);
+        tmem_wait_ld();
+        mask(r, 1);
+        m = largest(r, m);
+      }
+      fetch(r, t_s);
+      fetched();
+      mask(r, 0);
+      m_used = largest(r, m) * p.scale_log2;
+      weights(r);
+      if (n_kb > 1) {
+        fetch(r, t_s + kBKV);
+        tmem_wait_ld();
+        mask(r, 1);
+        tmem_st_32x32b_x32(t_s + kColP, pk);
+        weights(r);
+        tmem_st_32x32b_x32(t_s + kColP1, pk);
+      } else {
+        tmem_st_32x32b_x32(t_s + kColP, pk);
       }
     }
-    __syncwarp();
-    const int pos0 = qb * kBQ + warp * 32 + (lane >> 4);
-    __half* dst = p.out + static_cast<long long>(seq_start + pos0) * p.out_stride + h * kD + (lane & 15) * 8;
+    stored();
+    for (int i = 1; i < n_steps; ++i) {
+      const uint32_t ph = static_cast<uint32_t>(i) & 1u;
+      mbar_wait(bar_s, ph);
+      tc_fence_after();
+      fetch(r, t_s);  // ONE TMEM round trip
+      fetched();
+      mask(r, i + 1);
+      const float m_blk = largest(r, -CUDART_INF_F) * p.scale_log2;
+      // ---- lazy rescale of O and l (warp-uniform decision) ----
+      const bool grow = (m_blk - m_used) > kRescaleThreshold;
+      auto retired = [&]() {  // the previous O += P V
+        mbar_wait(bar_o, ph ^ 1u);
+        tc_fence_after();
+      };
+      if (__any_sync(0xffffffffu, grow)) {
+        retired();
+        const float m_new = grow ? m_blk : m_used;
+        const float alpha = (m_used == -CUDART_INF_F) ? 0.f : ex2_approx(m_used - m_new);  // 1 for rows that keep their maximum
+#pragma unroll 1
+        for (int c = 0; c < kD / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32b_x32(t_o + c * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 32; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+          tmem_st_32x32b_x32(t_o + c * 32, o);
+        }
+        l *= alpha;
+        m_used = m_new;
+      }
+      weights(r);
+      retired();
+      tmem_st_32x32b_x32(t_s + kColP, pk);
+      stored();
+    }
+    // ---- epilogue: O / l -> fp16 ----
+    mbar_wait(bar_o, static_cast<uint32_t>(n_steps - 1) & 1u);
+    tc_fence_after();
+    const float inv = 1.f / l;
+    auto eight = [&](const uint32_t* x) {  // eight outputs
+      uint4 o;
+      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __half2 h2 = __floats2half2_rn(__uint_as_float(x[2 * e]) * inv, __uint_as_float(x[2 * e + 1]) * inv);
+        ow[e] = *reinterpret_cast<const uint32_t*>(&h2);
+      }
+      return o;
+    };
+    if (ONE && qb * kBQ + warp * 32 + 32 > seq_len) {
+      // the warp's rows end with the sequence, as most do where sequences are this short: a lane stores its row (300
+      // sequences of 30 tokens x 32 heads: 159 us through shared memory, so 139; where all 32 rows are there, 40 x 128 tokens, 39.8 and 37.6)
+      __half* dst = p.out + static_cast<long long>(seq_start + q_pos) * p.out_stride + h * kD;
+#pragma unroll 1
+      for (int c = 0; c < kD / 32; ++c) {
+        tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
+        tmem_wait_ld();
+        if (q_pos < seq_len) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) *reinterpret_cast<uint4*>(dst + c * 32 + v * 8) = eight(r[0] + v * 8);
+        }
+      }
+    } else {
+      // through shared memory (every product has retired: the K and V buffers are free), so that half a warp stores a whole row; a lane per row touched 32
+      // lines with every store
+      constexpr int kPitch = kD * 2 + 16;
+      uint8_t* mine = smem + kOffK + warp * 32 * kPitch;
+      static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the K and V buffers");
+#pragma unroll 1
+      for (int c = 0; c < kD / 32; c += 2) {
+        fetch(r, t_o + c * 32);
+        tmem_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 8; ++v) *reinterpret_cast<uint4*>(mine + lane * kPitch + c * 64 + v * 16) = eight(r[v >> 2] + (v & 3) * 8);
+      }
+      __syncwarp();
+      const int pos0 = qb * kBQ + warp * 32 + (lane >> 4);
+      __half* dst = p.out + static_cast<long long>(seq_start + pos0) * p.out_stride + h * kD + (lane & 15) * 8;
 #pragma unroll 8
-    for (int r = 0; r < 32; r += 2)
-      if (pos0 + r < seq_len)
-        *reinterpret_cast<uint4*>(dst + static_cast<long long>(r) * p.out_stride) = *reinterpret_cast<const uint4*>(mine + (r + (lane >> 4)) * kPitch + (lane & 15) * 16);
+      for (int k = 0; k < 32; k += 2)
+        if (pos0 + k < seq_len)
+          *reinterpret_cast<uint4*>(dst + static_cast<long long>(k) * p.out_stride) = *reinterpret_cast<const uint4*>(mine + (k + (lane >> 4)) * kPitch + (lane & 15) * 16);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -405,10 +485,12 @@ int prefill_attention(const PrefillAttnArgs& a) {
   if (rc) return rc;
   rc = make_tmap_f16(&tv, a.v, a.num_tokens, static_cast<uint64_t>(a.num_kv_heads) * kD, a.v_stride, kBKV);
   if (rc) return rc;
-  static bool attr_set[kMaxDevices] = {};
-  bool& done = attr_set[device_ordinal()];
+  const bool one = a.max_seqlen <= kBQ;
+  auto kern = one ? prefill_attention_kernel<true> : prefill_attention_kernel<false>;
+  static bool attr_set[2][kMaxDevices] = {};
+  bool& done = attr_set[one ? 1 : 0][device_ordinal()];
   if (!done) {
-    rc = check_cuda(cudaFuncSetAttribute(prefill_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "cudaFuncSetAttribute(prefill attention)");
+    rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "cudaFuncSetAttribute(prefill attention)");
     if (rc) return rc;
     done = true;
   }
@@ -432,7 +514,7 @@ int prefill_attention(const PrefillAttnArgs& a) {
   for (int left = (a.max_seqlen + kBQ - 1) / kBQ; left > 0; left -= kMaxZ) {
     p.q_blocks = left;
     cfg.gridDim = dim3(a.num_heads, a.batch, left < kMaxZ ? left : kMaxZ);
-    rc = check_cuda(cudaLaunchKernelEx(&cfg, prefill_attention_kernel, tq, tk, tv, p), "prefill attention launch");
+    rc = check_cuda(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p), "prefill attention launch");
     if (rc) return rc;
   }
   return QS_OK;

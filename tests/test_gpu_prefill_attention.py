@@ -121,3 +121,16 @@ def test_empty_and_argument_errors(dev):
         backend.flash_attn_varlen_func(q[:, :, :64], k[:, :, :64], v[:, :, :64], cu_d, cu_d, 64, 64, causal=True)
     with pytest.raises(RuntimeError):
         backend.flash_attn_varlen_func(q, k, v, cu_d, cu_d, 64, 64, causal=True, window_size=(128, 0))
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 2), (32, 8)])
+def test_one_query_block_has_the_bits_of_many(dev, hq, hkv):
+    """Calls whose sequences all fit one block of 128 queries take a form of the kernel of their own; a longer neighbour sends them to the general one.  Lengths
+    around the warps' 32 rows and the 64-key blocks, scores far enough apart that maxima differ between the blocks."""
+    from qserve_b200 import backend
+    lens = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 100, 127, 128, 2]
+    q, k, v, _, cu = _inputs(lens + [300], hq, hkv, 5 + hq, dev, sigma=2.5)
+    T, n = sum(lens), len(lens)
+    many = backend.flash_attn_varlen_func(q, k, v, cu, cu, 300, 300, dropout_p=0.0, causal=True)
+    one = backend.flash_attn_varlen_func(q[:T], k[:T], v[:T], cu[:n + 1].contiguous(), cu[:n + 1].contiguous(), 128, 128, dropout_p=0.0, causal=True)
+    assert torch.isfinite(one.float()).all() and torch.equal(one, many[:T])
