@@ -124,6 +124,49 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
   return d;
 }
 
+// What a head group's last CTA does with the splits' partial rows.  One warp per head, lane = split for the weights (nsplit <= 32), lane = 4 dims for the sum:
+// the maxima and sums of all splits arrive in one round trip to L2 and the partial rows of eight splits are in flight together, also where the last batch has
+// fewer (one after the other they cost a round trip each: 4 sequences of 1081 to 2000 tokens, six or eight splits, INT4: 13.1 us, now 11.5; walking all the splits
+// so kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits).  The sums run over the splits in order.  A call:
+// inlined, the eight rows' registers made the main loop spill (INT8, 64 sequences of up to 1024 tokens 32.4 us, 31.6 so).
+__device__ __noinline__ void merge_splits(__half* __restrict__ out, const float* ws_part, int row0, int Gc, int nsplit, int used) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < Gc; r += kWarps) {
+    const float* pr = ws_part + static_cast<size_t>(row0 + r) * nsplit * (kD + 2);
+    const float ms = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD) : -CUDART_INF_F;
+    const float ls = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD + 1) : 0.f;
+    float M = ms;
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
+    const float e = (ms == -CUDART_INF_F) ? 0.f : exp2f(ms - M);
+    float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = 0; s0 < used; s0 += 8) {
+      float2 x[8], y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = y[k] = make_float2(0.f, 0.f);
+        if (s0 + k < used) {
+          const float2* row = reinterpret_cast<const float2*>(pr + (s0 + k) * (kD + 2));  // 130 floats per split: 8-byte aligned
+          x[k] = __ldcg(row + lane);
+          y[k] = __ldcg(row + 32 + lane);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (s0 + k >= used) break;
+        const float w = __shfl_sync(0xffffffffu, e, s0 + k);
+        L = fmaf(__shfl_sync(0xffffffffu, ls, s0 + k), w, L);
+        acc[0] = fmaf(x[k].x, w, acc[0]); acc[1] = fmaf(x[k].y, w, acc[1]);
+        acc[2] = fmaf(y[k].x, w, acc[2]); acc[3] = fmaf(y[k].y, w, acc[3]);
+      }
+    }
+    const float inv = __fdividef(1.f, L + 1.e-6f);
+    __half2* o2 = reinterpret_cast<__half2*>(out + static_cast<size_t>(row0 + r) * kD);
+    o2[lane] = __floats2half2_rn(acc[0] * inv, acc[1] * inv);
+    o2[32 + lane] = __floats2half2_rn(acc[2] * inv, acc[3] * inv);
+  }
+}
+
 template <int BITS>
 __global__ void __launch_bounds__(kAttnThreadsV2, 4)
 decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restrict__ k_in, const __half* __restrict__ v_in, long long q_stride,
@@ -177,8 +220,8 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   const long long* vptrs = kv_pointers + (static_cast<size_t>(b) * 2 + 1) * max_blocks;
   const int n_pages = (tlen + kPageTokens - 1) / kPageTokens;
   const int pps = nsplit > 1 ? (n_pages + nsplit - 1) / nsplit : n_pages;  // no division ahead of the first copy where there are no splits
-  // splits that hold pages: a CTA beyond them leaves empty partial rows behind and takes no part in the merge (with a prologue and a place in the merge of
-  // its own it was the last to finish where it did not fit the first wave)
+  // splits that hold pages: a CTA beyond them leaves an empty partial row behind, so that every split of the call has one, and takes no part in the merge (with
+  // a prologue and a place in the merge of its own it was the last to finish where it did not fit the first wave)
   const int used = nsplit > 1 ? max(1, (n_pages + pps - 1) / max(pps, 1)) : 1;
   if (split >= used) {
     pdl_wait();
@@ -680,33 +723,8 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     __syncthreads();
     final_written = (s_last != 0);
     if (s_last) {
-      // One warp per head, lane = split for the weights (nsplit <= 32), lane = 4 dims for the sum: the maxima and sums of all splits arrive in one
-      // round trip to L2 and the partial rows of several splits are in flight together.  (Walking the splits one dependent load after the other
-      // kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits.)  The sums run over the splits in order.
       __threadfence();
-      for (int r = warp; r < Gc; r += kWarps) {
-        const float* pr = ws_part + (static_cast<size_t>(b) * num_heads + h0 + r) * nsplit * (kD + 2);
-        const float ms = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD) : -CUDART_INF_F;
-        const float ls = (lane < used) ? __ldcg(pr + lane * (kD + 2) + kD + 1) : 0.f;
-        float M = ms;
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
-        const float e = (ms == -CUDART_INF_F) ? 0.f : exp2f(ms - M);
-        float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int sp = 0; sp < used; ++sp) {
-          const float2* row = reinterpret_cast<const float2*>(pr + sp * (kD + 2));  // 130 floats per split: 8-byte aligned
-          const float2 x = __ldcg(row + lane), y = __ldcg(row + 32 + lane);
-          const float w = __shfl_sync(0xffffffffu, e, sp);
-          L = fmaf(__shfl_sync(0xffffffffu, ls, sp), w, L);
-          acc[0] = fmaf(x.x, w, acc[0]); acc[1] = fmaf(x.y, w, acc[1]);
-          acc[2] = fmaf(y.x, w, acc[2]); acc[3] = fmaf(y.y, w, acc[3]);
-        }
-        const float inv = __fdividef(1.f, L + 1.e-6f);
-        __half2* o2 = reinterpret_cast<__half2*>(out + (static_cast<size_t>(b) * num_heads + h0 + r) * kD);
-        o2[lane] = __floats2half2_rn(acc[0] * inv, acc[1] * inv);
-        o2[32 + lane] = __floats2half2_rn(acc[2] * inv, acc[3] * inv);
-      }
+      merge_splits(out, ws_part, b * num_heads + h0, Gc, nsplit, used);
     }
   }
   if (q_out != nullptr && final_written) {

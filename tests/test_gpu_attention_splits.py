@@ -52,3 +52,17 @@ def test_splits_fill_the_machine(dev, bits, B, Hq, Hkv, ctx):
     slots = 4 * torch.cuda.get_device_properties(dev).multi_processor_count
     want = min(32, -(-ctx // 256), -(-slots // blocks)) if 2 * blocks <= slots and ctx > 512 else 0
     assert int((~rows.isnan()).sum()) == B * Hq * want * 130
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("lens", [[2049, 1980, 1700, 1500, 1100, 650, 300, 70, 1], [4097, 4000, 3300, 2900, 2500, 2100], [8193, 7000, 6500, 6000]])
+def test_every_number_of_splits_with_pages(dev, bits, lens):
+    """The merge takes eight splits' rows at a time: sequences of one call that leave it one to nine, 11 to 17 and 23 to 32 of them."""
+    rng = np.random.default_rng(sum(lens) + bits)
+    B, Hq, Hkv = len(lens), 4, 1
+    kp, vp, bt, q, k, v = _mk(rng, B, Hq, Hkv, lens, bits)
+    out, _, _ = _run_gpu(dev, kp, vp, bt, q, k, v, lens, bits)
+    exact = kv.decode_attention(q, k, v, kp, vp, bt, lens, ROPE, faithful=False).astype(np.float32)
+    got = out.astype(np.float32)
+    assert np.isfinite(got).all()
+    assert np.abs(got - exact).max() <= 3e-3 * max(1.0, float(np.abs(exact).max()))
