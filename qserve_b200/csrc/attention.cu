@@ -16,6 +16,8 @@
 // INT8 quantisation of the output row (single_query_attention_quant).
 #include <math_constants.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "launch.h"
 
@@ -90,17 +92,18 @@ constexpr int kOStride = kD + 4;  // floats per (warp, head) row of the merge bu
 
 // A warp consumes 32-token slices of the 64-token pages of one kv head.  Each warp owns a private ring of kSlots slots, filled by its lane 0 with
 // cp.async.bulk copies and guarded by one "full" mbarrier per slot (the refill of a slot is issued by the same warp right after it has consumed it, so no
-// "empty" barrier and no producer warp are needed).  INT4: a slot holds a whole slice, K codes | V codes | K scales | K zeros | V scales | V zeros, and the
-// ring two.  INT8: a slot holds one half of a slice, first K, then V (codes | scales | zeros), and the ring three: 135 KB are on their way per SM where two
-// whole slices take so much that only three CTAs fit, and 64 sequences x 8 heads need a second wave (45 us, now 34; INT4 with slots of halves: 3 % slower,
-// its CTAs fit either way and a wait more per slice is what remains).
+// "empty" barrier and no producer warp are needed).  A slot holds a whole slice, K codes | V codes | K scales | K zeros | V scales | V zeros, and the ring
+// two; or, INT8 in calls of more than three CTAs per SM, one half of a slice, first K, then V (codes | scales | zeros), and the ring three: 135 KB are on
+// their way per SM where two whole slices take so much that only three CTAs fit, and 64 sequences x 8 heads need a second wave (45 us, now 34).  Where CTAs
+// fit either way a wait more per slice is what remains of the halves: INT4 3 % slower, INT8 (1 x 300 tokens x 8
+// heads) 9.2 us and 7.9 in whole slices, whose three CTAs have 168 registers each.
 constexpr int kSliceTokens = 32;
-template <int BITS>
+template <int BITS, int PER>  // PER: slots of a slice
 struct StageLayout {
   static constexpr int kCodes = kPageTokens * kD * BITS / 8;       // bytes of K (or V) codes of one head-page
   static constexpr int kSliceCodes = kSliceTokens * kD * BITS / 8;  // ... of one 32-token slice
-  static constexpr int kPerSlice = BITS == 4 ? 1 : 2;               // slots of a slice
-  static constexpr int kSlots = BITS == 4 ? 2 : 3;
+  static constexpr int kPerSlice = PER;
+  static constexpr int kSlots = PER == 1 ? 2 : 3;
   static constexpr int kOffV = kPerSlice == 1 ? kSliceCodes : 0;    // V codes in their slot
   static constexpr int kOffKm = kPerSlice == 1 ? 2 * kSliceCodes : kSliceCodes;  // fp16 K scales [32] | zeros [32]
   static constexpr int kOffVm = kPerSlice == 1 ? kOffKm + 128 : kOffKm;
@@ -167,14 +170,14 @@ __device__ __noinline__ void merge_splits(__half* __restrict__ out, const float*
   }
 }
 
-template <int BITS>
-__global__ void __launch_bounds__(kAttnThreadsV2, 4)
+template <int BITS, int PER>
+__global__ void __launch_bounds__(kAttnThreadsV2, BITS == 8 && PER == 1 ? 3 : 4)
 decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restrict__ k_in, const __half* __restrict__ v_in, long long q_stride,
                         long long k_stride, long long v_stride, const long long* __restrict__ kv_pointers, const int* __restrict__ lengths,
                         __half* __restrict__ out, int num_heads, int num_kv_heads, int max_blocks, PageGeom pg, float rotary_base, int rotary_dim,
                         int timestep, int nsplit, float* __restrict__ ws_part, uint32_t* __restrict__ ws_cnt, uint32_t* __restrict__ tok_cnt, int8_t* __restrict__ q_out,
                         __half* __restrict__ q_scale, __half* __restrict__ q_sum, unsigned long long* __restrict__ prof) {
-  using SL = StageLayout<BITS>;
+  using SL = StageLayout<BITS, PER>;
   constexpr int R = SL::kSlots;
   const int G = num_heads / num_kv_heads;
   const int gparts = (G + kMaxG - 1) / kMaxG;
@@ -1048,9 +1051,12 @@ int decode_attention(const DecodeAttnArgs& a) {
     out = static_cast<uint8_t*>(a.workspace) + kAttnCounterBytes + part_bytes;
   }
   dim3 grid(gx, a.batch, nsplit);
-  auto run = [&](auto kern, size_t smem) {
-    static bool attr_done[2][kMaxDevices] = {};
-    bool& done = attr_done[a.int4_kv ? 0 : 1][device_ordinal()];
+  auto run = [&](auto bits, auto per) {
+    constexpr int kBits = decltype(bits)::value, kPer = decltype(per)::value;
+    auto kern = decode_attention_kernel<kBits, kPer>;
+    constexpr size_t smem = static_cast<size_t>(kWarps) * StageLayout<kBits, kPer>::kWarpBytes;
+    static bool attr_done[kMaxDevices] = {};  // of this instantiation
+    bool& done = attr_done[device_ordinal()];
     if (!done) {
       int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "attention smem attribute");
       if (rc) return rc;
@@ -1076,8 +1082,12 @@ int decode_attention(const DecodeAttnArgs& a) {
                       part, cnt, tok_cnt, static_cast<int8_t*>(a.q_out), static_cast<__half*>(a.q_scale), static_cast<__half*>(a.q_sum), static_cast<unsigned long long*>(a.prof)), "single_query_attention");
   };
   QS_REQUIRE(a.tokens_per_block == kPageTokens, "single_query_attention: tokens_per_block=%d, only 64 is supported (cache_engine block_size)", a.tokens_per_block);
-  return a.int4_kv ? run(decode_attention_kernel<4>, static_cast<size_t>(kWarps) * StageLayout<4>::kWarpBytes)
-                   : run(decode_attention_kernel<8>, static_cast<size_t>(kWarps) * StageLayout<8>::kWarpBytes);
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  if (a.int4_kv) return run(std::integral_constant<int, 4>{}, One{});
+  // INT8: halves where whole slices, three CTAs per SM, would need a second wave
+  const bool fits = static_cast<long long>(ctas) * nsplit <= 3ll * num_sms();
+  return fits ? run(std::integral_constant<int, 8>{}, One{}) : run(std::integral_constant<int, 8>{}, Two{});
 }
 
 int prefill_rope_append(const PrefillAppendArgs& a) {

@@ -3,6 +3,7 @@ through its ring more than 32 slices and fetches its page pointers again (INT8: 
 of the float64 attention over the same cache."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import kv
 from tests.test_gpu_attention import ROPE, _mk, _run_gpu
@@ -26,3 +27,21 @@ def test_walks_past_a_batch_of_pointers(dev, bits, long):
     got = out.astype(np.float32)
     assert np.isfinite(got).all()
     assert np.abs(got - exact).max() <= 3e-3 * max(1.0, float(np.abs(exact).max()))
+
+
+@pytest.mark.parametrize("ctx", [1, 33, 64, 65, 190, 300, 512])
+def test_whole_slices_and_halves(dev, ctx):
+    """INT8 calls of up to three blocks per multiprocessor fetch whole slices, larger ones halves: the same sequences give the same bits in either."""
+    rng = np.random.default_rng(ctx)
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    few, H = 5, 8
+    many = 3 * sms // H + 1
+    lens = ([ctx, 1, max(1, ctx - 63), ctx // 2 + 1, ctx] * (-(-many // few)))[:many]
+    kp, vp, bt, q, k, v = _mk(rng, many, H, H, lens, 8, pages=1 + sum((n + 63) // 64 for n in lens))
+    own, at = 1 + rng.permutation(sum((n + 63) // 64 for n in lens)), 0
+    for b, n in enumerate(lens):
+        bt[b, :(n + 63) // 64] = own[at:at + (n + 63) // 64]
+        at += (n + 63) // 64
+    halves, k1, v1 = _run_gpu(dev, kp, vp, bt, q, k, v, lens, 8)
+    whole, _, _ = _run_gpu(dev, kp, vp, bt[:few], q[:few], k[:few], v[:few], lens[:few], 8)
+    assert np.isfinite(halves.astype(np.float32)).all() and np.array_equal(whole.view(np.uint16), halves[:few].view(np.uint16))
