@@ -1168,7 +1168,7 @@ __global__ void __launch_bounds__(kPrepThreads) delta_prepare_kernel(
 // and the window of inputs in registers, the unit length is a warp sum, and nothing is loaded twice.  (One block per (token, unit) read every
 // input `taps` times with 2-byte accesses and met in shared memory for every unit: 6758 tokens, 24 units of 128, 253 us; now 56, floor 22.)
 template <typename ST, int TAPS>
-__global__ void __launch_bounds__(128, 6) delta_prepare_walk_kernel(float* __restrict__ prep, const ST* __restrict__ proj, long long stride,
+__global__ void __launch_bounds__(128, TAPS == 4 ? 6 : 0) delta_prepare_walk_kernel(float* __restrict__ prep, const ST* __restrict__ proj, long long stride,
                                                                  const float* __restrict__ conv_w, float* __restrict__ conv_state,
                                                                  const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                                                  const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,

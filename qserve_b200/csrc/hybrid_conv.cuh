@@ -137,8 +137,9 @@ __device__ __forceinline__ ConvWalk<ST, V, TAPS> conv_walk(const float* w, const
 
 // Rows t0 .. t1 - 1 at channels c .. c + V - 1 in order, `use(t, y)` takes each.  The inputs and tables of N rows are fetched together: one at a time,
 // every row waited for its own load.  A walk of one row (conv_run) takes N = 1: the other rows' code costs registers (256 rows of 6144 channels: 21 us
-// with N = 4, 19 with 1; single tokens of 64 sequences 6.9).  Prompts wait for memory with few warps in flight: kernels that walk ask for six blocks per SM (four
-// rows in 85 registers; five: 6758 rows of 6144 channels 81 us, six 75, eight spill; the next four rows ahead of these: 83 to 99).
+// with N = 4, 19 with 1; single tokens of 64 sequences 6.9).  Prompts wait for memory with few warps in flight: the walks of four rows with four taps, which
+// take 92 to 96 registers by themselves, ask for six blocks per SM (80 registers; five: 6758 rows of 6144 channels 81 us, six 75, eight spill; the next four
+// rows ahead of these: 83 to 99).  The others do not: they need fewer, and where six blocks are asked for the compiler spends up to 85 on them.
 template <typename ST, int V, int N = 4, typename Walk, typename Use>
 __device__ __forceinline__ void conv_rows(Walk& walk, const ST* __restrict__ in, long long stride, const float* __restrict__ in_bias, const ConvTables& tab,
                                           int t0, int t1, int c, bool shift, Use use) {
