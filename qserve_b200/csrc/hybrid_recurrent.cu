@@ -423,7 +423,9 @@ int launch_state_space(void* out, long long out_stride, float* prep, float* o_ra
   const size_t smb = (size_t)part * sizeof(float);
   const int vec = part % 4 == 0 && stride % 4 == 0 && out_stride % 4 == 0 && aligned(proj, 4 * sizeof(ST)) && aligned(out, 4 * sizeof(ST)) &&
                   aligned(o_raw, 16) && aligned(norm_w, 16);
-  if (vec && part <= 512) {
+  // (steps of few tokens wait for one chain after the other: with a warp for 512 numbers it is longer than with 128 threads, 16 tokens of 8 parts 11.0 us with the
+  // scan, 9.6 so; level from about 16 parts per SM on)
+  if (vec && part <= 512 && (long long)T * norm_groups >= 16ll * num_sms()) {
     ssd_out_warp_kernel<ST><<<(T * norm_groups + 3) / 4, 128, 0, s>>>((ST*)out, out_stride, o_raw, proj, stride, norm_w, out_scale, eps, inner, part, norm_groups, T);
     return check_cuda(cudaGetLastError(), "hyb_state_space");
   }
