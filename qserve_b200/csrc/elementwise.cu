@@ -774,7 +774,11 @@ __global__ void __launch_bounds__(256, kSiluCtas) silu_and_mul_kernel(__half* __
   qs_trace(QS_K_SILU, 1);
   const unsigned vpr = d / 8;  // vectors per output row
   const unsigned stride = gridDim.x * blockDim.x;
-  const unsigned row_step = stride / vpr, col_step = stride - row_step * vpr;
+  unsigned row_step = 0, col_step = 0;
+  if (n_vec > stride) {  // calls of one vector per thread do without the division (128 rows of 2 x 11008: 4.1 us with it, 3.7 without)
+    row_step = stride / vpr;
+    col_step = stride - row_step * vpr;
+  }
   const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned row = first / vpr, col = first - row * vpr;
   auto one = [&](uint4& x, uint4& y) {  // the vector at (row, col), then on to the thread's next one
