@@ -1171,10 +1171,11 @@ __global__ void __launch_bounds__(kThreads) norm_quant_fast_kernel(int8_t* __res
 // Prompts: the row operations of up to 4096 columns with 128 threads (norm) or a warp (quantisation) per row.  With 512 threads per row four rows are in
 // work per SM, each a chain of a load and three to five block barriers with 16 bytes per thread on their way; with these 16 rows are.
 // 5000 rows of 4096: norm 34.6 -> 24.1 us (61 MB), with the sum 46 -> 29, 6108 rows quantised with the sum 28.3 -> 19.7.  Below the limits a row per 512
-// threads is level or better: 592 rows are in work at once there.  (A warp per row for the norm as well: 18 us where 512 rows take 10, 5000 take 33.)
+// threads is level or better: 592 rows are in work at once there (four on each of 148 SMs; quantised with the sum, 1250 and 1300 rows of 2048 take 5.65 us so
+// and 5.8 to 6.2 by warps, 1500 of 4096 7.7 and 7.2).  (A warp per row for the norm as well: 18 us where 512 rows take 10, 5000 take 33.)
 // ------------------------------------------------------------------------------------------------
 constexpr int kRowVecs = 16;  // 16-byte vectors of a lane: a warp holds the row
-constexpr int kNormRowMin = 592, kQuantRowMin = 1184;
+constexpr int kNormRowMin = 592, kQuantRowMin = 1184, kQuantSumRowMin = 1400;
 
 // Same bits as norm_quant_fast_kernel<false, false, 1>: thread (warp k, lane l) holds what threads 32 (4 k + i) + l, i = 0 .. 3, hold there, and the sums go
 // through the same tree (the lanes of each of the 16 warps, then the warps).
@@ -1418,7 +1419,7 @@ int quant_per_token(void* out_q, const void* in, void* input_sum, void* scale, i
       return launch(kern, dim3(tokens), dim3(kThreads), 0, stream, "invoke_quant", static_cast<int8_t*>(out_q), static_cast<const __half*>(in),
                     static_cast<__half*>(input_sum), static_cast<__half*>(scale), hidden);
     };
-    if (nvec <= 32 * kRowVecs && tokens >= kQuantRowMin)
+    if (nvec <= 32 * kRowVecs && tokens >= (input_sum != nullptr ? kQuantSumRowMin : kQuantRowMin))
       return launch(quant_rows_kernel, dim3((tokens + 3) / 4), dim3(128), 0, stream, "invoke_quant", static_cast<int8_t*>(out_q), static_cast<const __half*>(in),
                     static_cast<__half*>(input_sum), static_cast<__half*>(scale), hidden, tokens);
     if (nvec <= kThreads) return go(quant_per_token_fast_kernel<1>);

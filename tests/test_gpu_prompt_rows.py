@@ -39,6 +39,12 @@ def test_many_rows_have_the_bits_of_few(dev, rows, H):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("H", [8, 1032, 4096])
+@pytest.mark.parametrize("rows", [1399, 1400])
+def test_many_rows_with_the_sum(dev, rows, H):
+    test_many_rows_have_the_bits_of_few(dev, rows, H)  # quantisation with the sum: a warp per row from 1400 rows on
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("Hq,Hkv", [(1, 1), (3, 3), (32, 8), (40, 8), (32, 32)])
 def test_append_of_an_unaligned_buffer(dev, bits, Hq, Hkv):
