@@ -130,8 +130,9 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
 // What a head group's last CTA does with the splits' partial rows.  One warp per head, lane = split for the weights (nsplit <= 32), lane = 4 dims for the sum:
 // the maxima and sums of all splits arrive in one round trip to L2 and the partial rows of eight splits are in flight together, also where the last batch has
 // fewer (one after the other they cost a round trip each: 4 sequences of 1081 to 2000 tokens, six or eight splits, INT4: 13.1 us, now 11.5; walking all the splits
-// so kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits).  The sums run over the splits in order.  A call:
-// inlined, the eight rows' registers made the main loop spill (INT8, 64 sequences of up to 1024 tokens 32.4 us, 31.6 so).
+// so kept the last CTA of a sequence busy for about 25 of 44 us at 4 sequences x 8000 tokens, 19 splits).  Full batches go without the rest's conditions (4 x
+// 8000, INT8: 22.4 us with them, 21.9).  The sums run over the splits in order.  A call: inlined, the rows' registers are the main loop's as well (INT8, 64
+// sequences of up to 1024 tokens 32.1 us, 31.2 so).
 __device__ __noinline__ void merge_splits(__half* __restrict__ out, const float* ws_part, int row0, int Gc, int nsplit, int used) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int r = warp; r < Gc; r += kWarps) {
@@ -143,12 +144,12 @@ __device__ __noinline__ void merge_splits(__half* __restrict__ out, const float*
     for (int m = 16; m >= 1; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
     const float e = (ms == -CUDART_INF_F) ? 0.f : exp2f(ms - M);
     float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s0 = 0; s0 < used; s0 += 8) {
+    auto rows = [&](int s0, int n) {
       float2 x[8], y[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         x[k] = y[k] = make_float2(0.f, 0.f);
-        if (s0 + k < used) {
+        if (k < n) {
           const float2* row = reinterpret_cast<const float2*>(pr + (s0 + k) * (kD + 2));  // 130 floats per split: 8-byte aligned
           x[k] = __ldcg(row + lane);
           y[k] = __ldcg(row + 32 + lane);
@@ -156,13 +157,16 @@ __device__ __noinline__ void merge_splits(__half* __restrict__ out, const float*
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        if (s0 + k >= used) break;
+        if (k >= n) break;
         const float w = __shfl_sync(0xffffffffu, e, s0 + k);
         L = fmaf(__shfl_sync(0xffffffffu, ls, s0 + k), w, L);
         acc[0] = fmaf(x[k].x, w, acc[0]); acc[1] = fmaf(x[k].y, w, acc[1]);
         acc[2] = fmaf(y[k].x, w, acc[2]); acc[3] = fmaf(y[k].y, w, acc[3]);
       }
-    }
+    };
+    int s0 = 0;
+    for (; s0 + 8 <= used; s0 += 8) rows(s0, 8);
+    if (s0 < used) rows(s0, used - s0);
     const float inv = __fdividef(1.f, L + 1.e-6f);
     __half2* o2 = reinterpret_cast<__half2*>(out + static_cast<size_t>(row0 + r) * kD);
     o2[lane] = __floats2half2_rn(acc[0] * inv, acc[1] * inv);
