@@ -36,11 +36,10 @@ def _report(name, acc_g, acc_o, out_g, out_o):
 SHAPES = [  # (M, N, K)
     (16, 128, 128), (1, 256, 256), (16, 4096, 4096), (33, 384, 512), (64, 256, 1024), (64, 4096, 4096),
     (100, 512, 640), (128, 256, 256), (200, 384, 384), (256, 256, 512), (300, 256, 256), (700, 384, 256),
-    # prefill tiles: M >= 512 with an even number of channel tiles takes the CTA-pair kernel (cta_group::2, 256-token tiles, persistent), an odd number or
-    # K < 512 the 128-token tiles; ragged last token block, K % 256 == 128, several tiles per persistent pair
+    # CTA pairs (cta_group::2, persistent): 128-token tiles per channel, 256 with group scales (W8A8 splits K instead); K below 512 keeps the 128-token tiles of
+    # one CTA; ragged last token block, K % 256 == 128
     (1000, 512, 1152), (513, 1024, 384), (2048, 768, 512),
-    # 128 < M < 512 takes the pair kernel only when its 256-token tiles are well filled AND there is a pair tile per TPC (wide layers):
-    # one partial 256-token tile (192 tokens), two tiles with a ragged second one (448)
+    # pairs below 512 tokens, one partial tile (192 tokens) and a ragged last one (448): 192-token tiles per channel, 256 with group scales, 256 and 160 in W8A8
     (192, 19200, 512), (448, 9728, 640),
 ]
 
@@ -147,7 +146,7 @@ def test_llama3_8b_layer_shapes_decode_b64(dev):
         assert np.array_equal(bits16(np_of(out)), bits16(out_o)), (K, N)
 
 
-CONFIG_SHAPES = [  # BASELINE.json configs 3-5 (SURVEY.md 8d): (mode, M, N, K)
+CONFIG_SHAPES = [  # (mode, M, N, K)
     ("grp", 64, 6144, 4096), ("grp", 64, 4096, 14336),                                  # 3: Llama-3-8B g128, decode batch 64
     ("w8", 128, 6144, 4096), ("w8", 128, 28672, 4096), ("w8", 128, 4096, 14336),        # 4: Mistral-7B W8A8, decode batch 128
     ("chn", 64, 6144, 8192), ("chn", 64, 8192, 2048), ("chn", 64, 12288, 8192), ("chn", 64, 8192, 6144),  # 5: Qwen1.5-72B, TP=4 shards
@@ -233,3 +232,51 @@ def test_invalid_shapes_raise(dev):
     with pytest.raises(RuntimeError):  # K not a multiple of 128
         op.gemm_forward_cuda(i8(4, 64), i8(128, 32), h(128), h(4), h(128), h(4), h(4, 128))
     op.gemm_forward_cuda(i8(0, 128), i8(128, 64), h(128), h(0), h(128), h(0), h(0, 128))  # empty batch is a no-op
+
+
+# What the choice of tiles gives calls on a B200's 148 multiprocessors: every number of tokens of a CTA pair's tile, ragged last tiles, one tile per pair and
+# (the last of each kind of weights) several.  A tile's tokens show in the number of blocks, 2 x min(tiles, 74).
+PAIR_TILES = [
+    ("chn", 641, 768, 4096, 128), ("chn", 513, 3840, 4096, 160), ("chn", 641, 3840, 4096, 192), ("chn", 961, 3328, 4096, 224), ("chn", 449, 6400, 4096, 256), ("chn", 580, 9728, 512, 256),
+    ("grp", 2049, 256, 4096, 128), ("grp", 897, 1280, 14336, 160), ("grp", 641, 768, 4096, 192), ("grp", 961, 3328, 14336, 224), ("grp", 449, 6400, 4096, 256), ("grp", 393, 9728, 512, 256),
+    ("w8", 129, 4864, 4096, 128), ("w8", 513, 3840, 14336, 160), ("w8", 641, 3328, 4096, 192), ("w8", 961, 3328, 14336, 224), ("w8", 449, 6400, 4096, 256), ("w8", 495, 9728, 512, 256),
+]
+
+
+@pytest.mark.parametrize("mode,M,N,K,tokens", PAIR_TILES)
+def test_every_pair_tile(dev, mode, M, N, K, tokens):
+    from qserve_b200._lib import lib
+    import qserve_backend.qgemm_w4a8_per_chn as opc
+    import qserve_backend.qgemm_w4a8_per_group as opg
+    import qserve_backend.qgemm_w8a8 as op8
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("the choice of tiles follows the number of multiprocessors")
+    rng = np.random.default_rng(M + N + K)
+    aq, sa, asum = _acts(rng, M, K)
+    if mode == "chn":
+        q, qw, s1, s1z = w4a8.synth_per_channel(rng, N, K)
+        want, acc_o = w4a8.gemm_w4a8_per_chn(aq, qw, s1, sa, s1z, asum, return_acc=True)
+        op, args = opc.gemm_forward_cuda, (aq, qw, s1, sa, s1z, asum)
+    elif mode == "grp":
+        q, qw, s1, s2s, s2z = w4a8.synth_per_group(rng, N, K)
+        want, acc_o = w4a8.gemm_w4a8_per_group(aq, qw, s2z, s2s, s1, sa, return_acc=True)
+        op, args = opg.gemm_forward_cuda, (aq, qw, s2z, s2s, s1, sa)
+    else:
+        w, sw = rng.integers(-128, 128, size=(N, K), dtype=np.int8), rng.uniform(0.001, 0.01, size=N).astype(np.float16)
+        want, acc_o = w4a8.gemm_w8a8(aq, w, sw, sa, return_acc=True)
+        op, args = op8.w8a8_gemm_forward_cuda, (aq, w, sw, sa)
+    out, acc = torch.full((M, N), float("nan"), dtype=torch.half, device=dev), torch.zeros((M, N), dtype=torch.int32, device=dev)
+    args = [to_dev(a, dev) for a in args]
+    stamps = torch.zeros(16 * 4096, dtype=torch.int64, device=dev)  # 16 per block, for more blocks than any tiles would have here
+    lib.qs_gemm_set_profile_buffer(stamps.data_ptr())
+    try:
+        op(*args, out, _acc_out=acc)
+        torch.cuda.synchronize()
+    finally:
+        lib.qs_gemm_set_profile_buffer(None)
+    plain = torch.full((M, N), float("nan"), dtype=torch.half, device=dev)
+    op(*args, plain)
+    blocks = int((stamps.view(-1, 16)[:, 0] != 0).sum())
+    assert blocks == 2 * min(74, -(-M // tokens) * (N // 256))
+    assert np.array_equal(np_of(acc), acc_o)
+    assert np.array_equal(bits16(np_of(out)), bits16(want)) and np.array_equal(bits16(np_of(plain)), bits16(want))

@@ -1,5 +1,6 @@
 """Tiles of CTA pairs with 128 to 256 tokens: what the tile's tokens are follows the number of rounds, the result does not.  Against the same rows in pieces
-of at most 100 or 64 tokens, which take the single-CTA tiles: the same bits, for every tile size, ragged last tiles, one and several tiles per pair."""
+of at most 100 or 64 tokens, which take the single-CTA tiles: the same bits, for the sizes that calls with short K get (per channel 128, 192 and 256 tokens,
+group scales 256, W8A8 160 and 256; every size in test_gpu_gemm.py), ragged last tiles, one and several tiles per pair, and where pairs begin."""
 import pytest
 import torch
 

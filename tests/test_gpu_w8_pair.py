@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (512, 256, 512), (513, 512, 640), (1000, 4096, 1152),   # pairs
+    (512, 256, 512), (513, 512, 640),                        # split, above 512 tokens as well
+    (1000, 4096, 1152), (600, 4096, 640),                    # pairs: tiles of 256 tokens, of 160
     (2100, 4096, 512), (3000, 8192, 512), (4500, 8192, 640),  # several tiles per pair: two, six and eight
     (129, 28672, 512), (300, 28672, 640), (400, 6144, 512),  # pairs below 512 tokens
     (128, 28672, 640), (65, 19200, 512),                     # two CTAs per multiprocessor
