@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Condense an `ncu --metrics gpu__time_duration.sum --csv` launch list of one decode step into per-kernel counts / times / shares.
-usage: python tools/launches_summary.py gpurun_out/launches.csv > profiles/rNN_launches_summary.txt"""
+usage: python tools/launches_summary.py launches.csv > profiles/launches_summary.txt"""
 import collections
 import csv
 import sys

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Condense an .ncu-rep (ncu --set full) into the handful of numbers the roofline discussion needs.
-usage: python tools/ncu_summary.py report.ncu-rep [> profiles/rNN_<kernel>.txt]"""
+usage: python tools/ncu_summary.py report.ncu-rep [> profiles/<kernel>.txt]"""
 import csv
 import subprocess
 import sys

@@ -1,4 +1,4 @@
-// Micro-benchmark (prepared in round 1, not yet run): per-operation cost, seen by ONE thread, of the synchronisation
+// Micro-benchmark: per-operation cost, seen by ONE thread, of the synchronisation
 // primitives that pace the GEMM main loop -- mbarrier.try_wait / test_wait on a completed phase, mbarrier.arrive,
 // tcgen05.commit with no MMA outstanding, tcgen05.fence -- and the latency of a programmatic-dependent-launch boundary
 // (chain of trivial kernels: trigger at entry, griddepcontrol.wait, exit).
