@@ -87,7 +87,7 @@ QS_API int qs_gemm_force_tile_tokens(int nt);
 /* profiling hook: device buffer of 16 x uint64 per CTA receiving %globaltimer stamps of the GEMM phases; NULL disables */
 QS_API int qs_gemm_set_profile_buffer(void* dev_buffer);
 /* step tracing: u64 buffer [0] = record count (zero it), then `capacity_records` x (kernel_id << 8 | phase, %globaltimer);
- * block 0 of every kernel logs entry (0), dependency resolved (1) and exit (2); NULL disables (tools/step_timeline.py) */
+ * block 0 of every kernel logs entry (0), dependency resolved (1) and exit (2); NULL disables */
 QS_API int qs_set_trace_buffer(void* dev_buffer, unsigned capacity_records);
 
 /* ---------------------------------------------------------------------------------------------------------

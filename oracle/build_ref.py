@@ -8,7 +8,7 @@ The reference's own build (`kernels/setup.py`) refuses compute capability 10.0
 sources where they lie under /root/reference (never copied into this repo) with
 the reference's own flags (kernels/setup.py:19-36) and only the arch changed to
 `-gencode arch=compute_100a,code=sm_100a`.  Outputs go to oracle/_ref/ (git-ignored,
-but shipped to the GPU box by gpurun).  Each module is renamed
+but it travels with the tree).  Each module is renamed
 `ref_<name>` through -DTORCH_EXTENSION_NAME so it can be imported next to the
 product's `qserve_backend.<name>`.
 

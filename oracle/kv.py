@@ -51,7 +51,7 @@ class PagePool:
             self.randomize(rng)
 
     def randomize(self, rng, scale_range=(0.01, 0.1), zero_range=(0.0, None)):
-        """random codes, scale~U(0.01,0.1), zero~U(0,15|255) fp16."""
+        """Random codes, scale~U(0.01,0.1), zero~U(0,15|255) fp16."""
         n = self.data.shape[0]
         self.data[:, : self.cb] = rng.integers(0, 256, size=(n, self.cb), dtype=np.uint8)
         zmax = zero_range[1] if zero_range[1] is not None else (15.0 if self.bits == 4 else 255.0)
@@ -341,7 +341,7 @@ def decode_attention(q, k, v, kpool: PagePool, vpool: PagePool, block_tables, le
 
 
 # ------------------------------------------------------------------------------------------------
-#  prefill attention: what `flash_attn_varlen_func(q, k, v, cu_seqlens, ..., causal=True)` computes at
+# Prefill attention: what `flash_attn_varlen_func(q, k, v, cu_seqlens, ..., causal=True)` computes at
 # llama_w4a8_unpad.py:232 on the rotated q / k of the packed qkv buffer -- un-quantised K / V, causal, grouped-query.
 # Reference for the B200 prefill kernel of the next round; float64, no rounding model (flash-attn is third-party and unpinned).
 # ------------------------------------------------------------------------------------------------

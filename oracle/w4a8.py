@@ -40,7 +40,7 @@ def pack_w4(q: np.ndarray) -> np.ndarray:
 
 
 def unpack_w4(qweight: np.ndarray) -> np.ndarray:
-    """Inverse of pack_w4 (SURVEY.md Appendix A1; consumer gemm_cuda.cu:286-298).
+    """Inverse of pack_w4 (consumer gemm_cuda.cu:286-298).
 
     View qweight as P[N/32][K/32][32 lanes][16 B]; for lane t = c*4+e and byte j = d*8+b*4+f:
       low  nibble = q[n32*32 + b*8 + c     ][k32*32 + d*16 + e*4 + f]
@@ -205,7 +205,7 @@ def dequant_then_matmul_per_chn(a_q, qweight, s1, s1z, ascales):
 
 
 # --------------------------------------------------------------------------------------
-# synthetic weight generators used by tests and bench (SURVEY.md section 8d)
+# synthetic weight generators used by tests and bench
 # --------------------------------------------------------------------------------------
 
 

@@ -51,7 +51,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------
-// step tracing (tools/step_timeline.py): block (0,0,0) of every kernel logs %globaltimer at entry, after the PDL wait and
+// step tracing: block (0,0,0) of every kernel logs %globaltimer at entry, after the PDL wait and
 // at exit into a device buffer [0] = record count, then records of 2 x u64: (kernel_id << 8 | phase), time.  Off by default.
 // ---------------------------------------------------------------------------------------------
 static __device__ unsigned long long* g_qs_trace = nullptr;
@@ -218,7 +218,6 @@ __device__ __forceinline__ void umma_i8_ts_2cta(uint32_t d_tmem, uint32_t a_tmem
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// arrive (once all previously issued MMAs of this thread have completed) on the mbarrier at this CTA-relative offset in BOTH CTAs of the pair
 // the same with A (this CTA's half of its rows, the peer's at the same place) from shared memory
 __device__ __forceinline__ void umma_i8_ss_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -229,6 +228,7 @@ __device__ __forceinline__ void umma_i8_ss_2cta(uint32_t d_tmem, uint64_t a_desc
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// arrive (once all previously issued MMAs of this thread have completed) on the mbarrier at this CTA-relative offset in BOTH CTAs of the pair
 __device__ __forceinline__ void umma_commit_2cta(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                "h"(static_cast<uint16_t>(3))

@@ -14,7 +14,7 @@
 //     reference's exact 32-bit multiply + vadd4), and write INT8 rows straight into TENSOR MEMORY with
 //     tcgen05.st.16x128b -- the mma.sync B-fragment order of the checkpoint is exactly the 16x128b TMEM store
 //     pattern, so no shuffle and no shared-memory round trip is needed.
-//   * two issuer threads (warps 1 and 7: even / odd 256-K stages) issue tcgen05.mma.kind::i8 with A (weights) from TMEM and
+//   * two issuer threads (warps 1 and 7: even / odd stages, of 256 K in W4A8 and 128 in W8A8) issue tcgen05.mma.kind::i8 with A (weights) from TMEM and
 //     B (INT8 activations, TMA-loaded with the 128-byte swizzle) from shared memory; INT32 accumulators live in TMEM and are
 //     zero-filled up front so that every MMA accumulates (the integer result cannot depend on how the two streams interleave).
 //   * weights and activations travel in separate rings: the weight producer never waits for the previous kernel, so with
@@ -82,7 +82,7 @@ struct GemmParams {
     int split;               // gemm_kernel: CTAs of a cluster that share a tile's K
     int nt;                  // pair kernels: tokens of a tile, a multiple of 32 up to 256
   };
-  unsigned long long* prof;  // optional: 16 globaltimer stamps per CTA (tools/gemm_timeline.py)
+  unsigned long long* prof;  // optional: 16 globaltimer stamps per CTA
 };
 // With two tensor maps, 352 bytes of a launch's parameters: with 360 the host takes longer over every launch.  16 x 4096 x 4096 called back to back is as
 // much the host's as the device's (5.1 us): the loop that issues the calls took 5.17 us a call (median of twelve processes) with 360 bytes and the device
@@ -550,7 +550,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 // persistently (one pair per TPC walks the tile list).
 //
 // Why: with 128-token tiles every CTA pulls its whole 128 x K weight band AND its whole 128 x K activation band out of L2: M = 4096 x N = 28672 x
-// K = 4096 moves 5.5 GB L2 -> SM in 413 us = 13 TB/s, which IS the chip's L2 throughput (~6300 B/clk, B300_MICROARCH.md) -- the tensor pipe idles
+// K = 4096 moves 5.5 GB L2 -> SM in 413 us = 13 TB/s, which IS the chip's L2 throughput (~6300 B/clk) -- the tensor pipe idles
 // at 52 %.  In a CTA pair each SM unpacks its own 128 channels into its own tensor memory (A operand) but stages only HALF of the 256 tokens of
 // the activation tile (B operand); the 2-CTA MMA reads the other half from the peer SM.  L2 -> SM traffic halves (2.7 GB for the shape above).
 // The first version of this kernel (one tile per launch-time CTA pair, 1 pair per TPC because of its 512 TMEM columns) lost all of that again to
@@ -743,7 +743,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
       }
     }
   } else if (warp == 6) {
-    // ===================================== activation producer: this CTA's 128 of the tile's 256 tokens =====================================
+    // ===================================== activation producer: this CTA's half of the tile's tokens =====================================
     if (lane == 0) {
       pdl_wait();
       qs_trace(QS_K_GEMM, 1, 6 * 32);
@@ -909,7 +909,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
 }
 
 // =============================================================================================
-// The same for W8A8: nothing to unpack, so both operands come from shared memory as TMA delivers them (A: each CTA its 128 channels, B: each CTA half of the
+// The same for W8A8: nothing to unpack, so both operands come from shared memory as TMA delivers them (A: each CTA its 128 channels, B: each CTA half of
 // the tile's tokens), tensor memory holds two accumulators, and a tile's epilogue runs under the next tile's products.
 // Roles per CTA: warp 0 weight producer (never waits for the previous kernel) | warp 6 activation producer | leader's warps 1 and 7: MMA issuers (even / odd
 // stages) | warps 2..5 and 8..11 epilogue.  One ring of 128-K stages for both operands; both CTAs' copies signal the leader's "full" barrier.
@@ -1267,14 +1267,15 @@ int pair_tokens(int M, int N, int K, int mode) {
 //  - W4A8 with two CTAs per SM (at most 2 x SMs tiles) where the pairs take a second round: 12288 x 4096 at 300 19.2 / 21.1, 4096 x 4096 at 1100 18.2 / 20.2
 //    (at 400, 384 tiles, 33.4 / 22.5).  W8A8's tiles run one per SM there: 24.3 / 22.0;
 //  - calls of a few us, whose set-up counts: group scales with 512 K 12288 at 140 7.6 / 7.8, with 1024 K at 80 7.8 / 8.2, per channel with 512 K 18688 at 200
-//    8.3 / 9.3, W8A8 with 1024 K 6144 at 200 7.1 / 7.2, 9728 at 65 with 2048 K 10.1 / 10.2.
+//    8.3 / 9.3, W8A8 with 1024 K 6144 at 200 7.1 / 7.2, 9728 at 65 with 2048 K 10.1 / 10.2.  An even number of 128-token tiles on two CTAs per SM and more is no
+//    such call: per channel 512 K 28672 at 256 14.0 / 11.2, 1024 K 12288 at 448 14.9 / 11.7, group scales 640 K 9728 at 448 13.9 / 11.0.
 bool pairs_pay(int M, int N, int K, int mode) {
   if (M <= 64 || (N / kBM) % 2 != 0 || K < 512) return false;
   const bool w8 = mode == kModeW8;
   const int sms = num_sms(), t128 = (M + 127) / 128, tiles = (N / kBM) * t128;
   if (2 * tiles <= sms) {
     if (M <= 128) return false;
-    const int split = 10 * tiles < sms ? 8 : 9 * tiles < 2 * sms ? 4 : 2;  // about what choose_split takes
+    const int split = 10 * tiles < sms ? 8 : 9 * tiles < 2 * sms ? 4 : 2;  // what choose_split takes (33 clusters of 4 and 15 of 8 are resident; the number of tiles is even)
     if (M < 512 || w8) return K * split <= 2048;
     return (split == 2 ? K : K * split) < 8192;
   }
@@ -1349,7 +1350,9 @@ int dispatch_gemm(const GemmArgs& a) {
   QS_REQUIRE(a.K % kBK == 0, "gemm: K=%d must be a multiple of %d", a.K, kBK);
   QS_REQUIRE((reinterpret_cast<uintptr_t>(a.act) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.weight) & 15) == 0, "gemm: operands must be 16-byte aligned");
   QS_REQUIRE(a.force_split == 0 || a.force_split == 1 || a.force_split == 2 || a.force_split == 4 || a.force_split == 8, "gemm: split must be 1, 2, 4 or 8");
-  // weight-ring depths (256-K stages) chosen so that NT <= 128 fits two CTAs per SM (<= 113 KB smem, <= 256 TMEM columns)
+  // weight-ring depths (stages of 256 K, W8A8 of 128) chosen so that tiles of up to 128 tokens fit two CTAs per SM (<= 113 KB smem, <= 256 TMEM columns) where
+  // nothing else is said.  W8A8 up to 64 tokens, stages of 256 and now of 128 K: 4096 x 4096 at 16 tokens 6.9 and 6.5 us, 12288 x 4096 15.6 and 14.5, at 64 16.7 and
+  // 15.6, 4096 x 14336 at 16 16.0 and 15.2
   constexpr bool w8 = (MODE == kModeW8), grp = (MODE == kModeW4Grp);
   QS_REQUIRE(a.force_nt == 0 || a.force_nt == 32 || a.force_nt == 64 || a.force_nt == 128, "gemm: tile tokens must be 32, 64 or 128");
   {

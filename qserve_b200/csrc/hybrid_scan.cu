@@ -68,7 +68,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 
 constexpr int kParts = 8, kRows = 16, kSeg = kRows + 4;  // a part's segment of a staged row vector is padded: the parts hit different banks
 constexpr int kVec = kParts * kSeg;                      // floats of a staged row vector
-constexpr int kThreads = 128, kSms = 148;
+constexpr int kThreads = 128, kSms = 148;  // (the device deals the units by kSms as well: a B200's)
 
 constexpr int scan_vectors(int mode) { return mode == kScanChannelDecay ? 3 : 2; }
 constexpr int scan_chunk(int mode) { return mode == kScanChannelDecay ? 8 : 12; }  // tokens of a staged chunk: two chunks stay below 40 KB
@@ -450,7 +450,8 @@ int launch_mode(const ScanArgs& p, cudaStream_t s) {
   // The narrowest blocks of which each SM holds two.  A step costs a warp about 140 cycles and 110 more per column of a thread: few units want short
   // steps, many want few instructions per element.  us of the whole layer with 1 / 2 / 4 columns, width 2048 unless said: delta rule, 1 x 2048 tokens of
   // width 1024: 355 / 439 / 648, 2 x 1000: 280 / 292 / 396, 4 x 2048: 869 / 771 / 878, 8 x 1000: 838 / 703 / 654; state space, 1 x 2048 of width 1024:
-  // 290 / 339 / 502, 2 x 1000: 372 / 312 / 357, 4 x 2048: 1180 / 1105 / 1035.
+  // 290 / 339 / 502, 2 x 1000: 372 / 312 / 357, 4 x 2048: 1180 / 1105 / 1035.  The delta rule's single tokens take the same rule; the kernel before this one
+  // and this one, 16 heads of 128 x 128: 8 tokens 17.1 / 13.7, 64 61.8 / 42.0, 256 210 / 126 (no other width has been measured for them).
   if (blocks(1) <= 2 * kSms) return launch<MODE, 1>(p, s);
   if (blocks(2) <= 2 * kSms) return launch<MODE, 2>(p, s);
   return launch<MODE, 4>(p, s);

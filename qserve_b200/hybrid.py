@@ -150,7 +150,7 @@ class StepBatch:
             r += n
         lists[:] = torch.tensor(longs + shorts, dtype=torch.int32)
         if nt:
-            # once in the entries' order, once by how many positions their rows see: the attention kernels start with the last
+            # once in the entries' order, once by how many positions their rows see: the attention kernels start with the last of a list
             seen = sorted(tiles, key=lambda t: entries[t[0]][1] + t[1])
             host[6 * T + 4 * E:] = torch.tensor([x[k] for x2 in (tiles, seen) for k in (0, 1) for x in x2], dtype=torch.int32)
         return host, (T, E, nt, len(longs), len(shorts))

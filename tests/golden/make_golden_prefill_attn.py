@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Golden vector for the prompt-phase attention: the output of flash-attn itself (the third-party kernel the reference calls at
-llama_w4a8_unpad.py:232-242) on a small ragged batch.  Needs a GPU and the image's flash_attn; run on the GPU box:
-    python tests/golden/make_golden_prefill_attn.py gpurun_out/prefill_attn_flash.npz
+llama_w4a8_unpad.py:232-242) on a small ragged batch.  Needs a GPU and flash_attn:
+    python tests/golden/make_golden_prefill_attn.py prefill_attn_flash.npz
 and copy the result to tests/golden/.  tests/test_oracle_prefill_attention.py pins oracle/prefill_attention.py against it."""
 import sys
 

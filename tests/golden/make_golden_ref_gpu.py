@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Capture golden vectors from the UNMODIFIED reference CUDA kernels (oracle/_ref, built by oracle/build_ref.py for
-sm_100a) on a B200:  gpurun -- python tests/golden/make_golden_ref_gpu.py
-Writes gpurun_out/golden_ref/*.npz; the files are then committed under tests/golden/ref_*.npz and pin the CPU oracle
+sm_100a) on a B200:  python tests/golden/make_golden_ref_gpu.py
+The files it writes are then committed under tests/golden/ref_*.npz and pin the CPU oracle
 (tests/test_oracle_vs_reference_golden.py).  Inputs are seeded; every output of the reference kernels is stored."""
 import os
 import sys

@@ -29,7 +29,7 @@ def test_library_exports_every_declared_symbol():
 
 
 def test_dropin_module_surface():
-    """module and function names of the seven reference extensions."""
+    """Module and function names of the seven reference extensions."""
     import qserve_backend as qb
 
     want = {

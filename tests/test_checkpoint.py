@@ -1,4 +1,4 @@
-"""CPU: the checkpoint converter / loader (qserve_b200/checkpoint.py, SURVEY.md 8f-1) against golden vectors produced by the
+"""CPU: the checkpoint converter / loader (qserve_b200/checkpoint.py) against golden vectors produced by the
 reference's own `from_linear` (tests/golden/make_golden_pack.py) and against the oracle's packer."""
 import glob
 import os

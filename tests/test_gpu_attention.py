@@ -1,6 +1,6 @@
 """GPU parity: KV4 / KV8 paged decode attention, prefill RoPE+append and padding offsets vs the CPU oracle.
 
-Stated tolerances (floating point, SURVEY.md 8c: the reference itself is order dependent here)
+Stated tolerances (floating point: the reference itself is order dependent here)
   * attention output: max |out - exact| <= 3e-3 * max(1, max|out|), where `exact` is the float64 attention over the
     same quantised cache (oracle faithful=False); the reference-faithful oracle (fp16 partial dots, fp16 logits,
     fp16 tree reduction of the output) is itself only within 1e-2 of `exact` (measured: 7e-3 with KV8), and our kernel
@@ -197,9 +197,9 @@ def test_attention_argument_errors(dev):
 
 
 def test_multi_wave_launches_are_stable(dev):
-    """Regression (round 2): more CTAs than resident slots (4 per SM).  A late CTA of a multi-wave launch does not sit in
-    griddepcontrol.wait, so its warps reach their first bulk copy immediately; in round 1 thread 0 initialised every warp's
-    ring barriers without a block barrier, and a warp that armed its ring first lost its transaction count and hung (one
+    """Regression: more CTAs than resident slots (4 per SM).  A late CTA of a multi-wave launch does not sit in
+    griddepcontrol.wait, so its warps reach their first bulk copy immediately; when thread 0 initialised every warp's
+    ring barriers without a block barrier, a warp that armed its ring first lost its transaction count and hung (one
     warp in ~1e8 slices: seen only at Qwen1.5-72B size, 4096 CTAs per launch).  Many back-to-back launches must all finish
     and reproduce the first result bit for bit."""
     import qserve_backend.fused_attention as fa

@@ -1,6 +1,6 @@
-"""Tensor parallelism on real GPUs (needs >= 2 devices: run with `gpurun --gpus 2 -- python -m pytest tests/test_gpu_tp.py -m gpu`).
+"""Tensor parallelism on real GPUs (needs >= 2 devices).
 
-SURVEY.md 8e parity rule, checked over NCCL on two B200s:
+The parity rule, checked over NCCL on two B200s:
   * per-token quantisation with the max-all-reduced amax gives every rank exactly its K slice of the single-GPU codes, the
     same scale, and the local shard's activation sum;
   * the INT32 accumulators of the row-parallel GEMM shards, sum-all-reduced, are BIT-identical to the single-GPU accumulators;
@@ -129,7 +129,7 @@ def _worker(rank, world, port, precision, q):
 @pytest.mark.parametrize("precision", ["w4a8kv4", "w4a8kv4-g128", "w8a8kv8"])
 def test_tp2_parity_rule_nccl(precision):
     if not torch.cuda.is_available() or torch.cuda.device_count() < 2:
-        pytest.skip("needs >= 2 CUDA devices (gpurun --gpus 2)")
+        pytest.skip("needs >= 2 CUDA devices")
     import torch.multiprocessing as mp
 
     ctx = mp.get_context("spawn")

@@ -222,8 +222,8 @@ def test_live_gemm_w8a8_config4(dev, K, N):
 def test_live_decode_attention_full_size(dev, bits, B, ctx):
     """Config 2 (KV4, B=64, ctx=1024, 32 q heads / 8 kv heads) and config 4 (KV8, B=128): every one of the B x 32 heads is
     compared with the reference kernel's output on identical pages, and the appended K/V slots byte for byte.
-    Bar: |ours - ref| <= 1e-2 * max(1, |ref|) (fp16 logits / fp16 probabilities make the reference itself order dependent,
-    SURVEY.md 8c); additionally our error against float64 attention over the same cache must not exceed the reference's by
+    Bar: |ours - ref| <= 1e-2 * max(1, |ref|) (fp16 logits / fp16 probabilities make the reference order dependent by
+    itself); additionally our error against float64 attention over the same cache must not exceed the reference's by
     more than 1e-3 (we accumulate in fp32 where the reference rounds p to fp16)."""
     ref, qb = _ref("fused_attention"), _qb()
     from qserve_b200.decode import DecodeRunner

@@ -34,7 +34,7 @@ def test_pack_unpack_roundtrip_property(rng):
 
 
 def test_pack_layout_formula(rng):
-    """lane t = c*4+e, byte j = d*8+b*4+f of a 32x32 tile."""
+    """The checkpoint layout: lane t = c*4+e, byte j = d*8+b*4+f of a 32x32 tile."""
     q = rng.integers(0, 16, size=(64, 64), dtype=np.uint8)
     P = w4a8.pack_w4(q).view(np.uint8).reshape(2, 2, 32, 16)
     for _ in range(200):
@@ -61,7 +61,7 @@ def test_config1_plumbing_per_channel_vs_dequant_matmul(rng):
     qw, s1h, s1z = w4a8.pack_per_channel(q, s1, z)
     x = rng.standard_normal((M, K)).astype(np.float16)
     aq, sa, _ = ops.quant_per_token(x)
-    asum = (sa.astype(np.float32) * aq.astype(np.int32).sum(axis=1)).astype(np.float16)  # asum = sa * sum(a_q) (SURVEY 8d-1)
+    asum = (sa.astype(np.float32) * aq.astype(np.int32).sum(axis=1)).astype(np.float16)  # asum = sa * sum(a_q)
     out, acc = w4a8.gemm_w4a8_per_chn(aq, qw, s1h, sa, s1z, asum, return_acc=True)
     ref = w4a8.dequant_then_matmul_per_chn(aq, qw, s1h, s1z, sa)
     assert np.array_equal(acc, w4a8.int_matmul(aq, q))
