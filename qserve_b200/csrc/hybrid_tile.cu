@@ -293,31 +293,48 @@ __global__ void __launch_bounds__(kThreads, 2) umma_tile_kernel(const __grid_con
     mbar_wait(bar_o, static_cast<uint32_t>(n_walk - 1) & 1u);
     tc_fence_after();
     const float inv = 1.f / l;
-    // Through shared memory (every product has retired: the buffers are free), so that a warp stores whole rows; a lane per row touched 32 lines with every
-    // store
-    constexpr int kPitch = kD * 4 + 16;
-    uint8_t* mine = sm + kOffK + warp * 32 * kPitch;
-    static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the key, value and weight buffers");
-#pragma unroll 1
-    for (int c = 0; c < kD / 32; c += 2) {
-      uint32_t r[2][32];
-      tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
-      tmem_ld_32x32b_x32(t_o + c * 32 + 32, r[1]);
-      tmem_wait_ld();
-#pragma unroll
-      for (int v = 0; v < 16; ++v) {
-        const uint32_t* x = &r[v >> 3][(v & 7) * 4];
-        *reinterpret_cast<float4*>(mine + lane * kPitch + c * 128 + v * 16) =
-            make_float4(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv, __uint_as_float(x[2]) * inv, __uint_as_float(x[3]) * inv);
-      }
-    }
-    __syncwarp();
     const int row0 = (warp & 1) * 32;
-    float* dst = p.a_out + ((static_cast<size_t>(tok0 + row0) * p.H + h) * p.maps + m) * kD + lane * 4;
-    const size_t step = static_cast<size_t>(p.H) * p.maps * kD;
+    if (row0 + 32 > n_rows) {
+      // the warp's rows end with the portion: a lane stores its row (64 portions of 16 tokens x 16 heads x 2 maps: 35.9 us through shared memory,
+      // 33.3 so)
+      float* dst = p.a_out + ((static_cast<size_t>(tok0 + row) * p.H + h) * p.maps + m) * kD;
+#pragma unroll 1
+      for (int c = 0; c < (row0 < n_rows ? kD / 32 : 0); ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(t_o + c * 32, r);
+        tmem_wait_ld();
+        if (row < n_rows) {
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<float4*>(dst + c * 32 + v * 4) = make_float4(__uint_as_float(r[v * 4]) * inv, __uint_as_float(r[v * 4 + 1]) * inv,
+                                                                           __uint_as_float(r[v * 4 + 2]) * inv, __uint_as_float(r[v * 4 + 3]) * inv);
+        }
+      }
+    } else {
+      // Through shared memory (every product has retired: the buffers are free), so that a warp stores whole rows; a lane per row touched 32 lines with every
+      // store
+      constexpr int kPitch = kD * 4 + 16;
+      uint8_t* mine = sm + kOffK + warp * 32 * kPitch;
+      static_assert(4 * 32 * kPitch <= kOffBar - kOffK, "the rows fit the key, value and weight buffers");
+#pragma unroll 1
+      for (int c = 0; c < kD / 32; c += 2) {
+        uint32_t r[2][32];
+        tmem_ld_32x32b_x32(t_o + c * 32, r[0]);
+        tmem_ld_32x32b_x32(t_o + c * 32 + 32, r[1]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 16; ++v) {
+          const uint32_t* x = &r[v >> 3][(v & 7) * 4];
+          *reinterpret_cast<float4*>(mine + lane * kPitch + c * 128 + v * 16) =
+              make_float4(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv, __uint_as_float(x[2]) * inv, __uint_as_float(x[3]) * inv);
+        }
+      }
+      __syncwarp();
+      float* dst = p.a_out + ((static_cast<size_t>(tok0 + row0) * p.H + h) * p.maps + m) * kD + lane * 4;
+      const size_t step = static_cast<size_t>(p.H) * p.maps * kD;
 #pragma unroll 16
-    for (int r = 0; r < 32; ++r)
-      if (row0 + r < n_rows) *reinterpret_cast<float4*>(dst + r * step) = *reinterpret_cast<const float4*>(mine + r * kPitch + lane * 16);
+      for (int r = 0; r < 32; ++r) *reinterpret_cast<float4*>(dst + r * step) = *reinterpret_cast<const float4*>(mine + r * kPitch + lane * 16);
+    }
   }
   tc_fence_before();
   __syncthreads();
