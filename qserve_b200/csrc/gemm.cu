@@ -1372,8 +1372,11 @@ int dispatch_gemm(const GemmArgs& a) {
     // W8A8 at 65..128 tokens: layers that want a split run one CTA per SM beside the receive buffer and take a deeper activation ring
     const int tiles = (a.N / kBM) * ((a.M + 127) / 128);
     if (a.force_split != 1 && tiles * 2 <= num_sms()) return launch_gemm<MODE, 128, 4, 4>(a);
-    // one CTA per SM at most: it may as well have all of the shared memory
-    if (tiles <= num_sms()) return launch_gemm<MODE, 128, 8, 4>(a);
+    // One CTA per SM at most: it may as well have all of the shared memory.  With long K also where two per SM leave the second half of a last round empty (an odd
+    // number of 128-channel tiles, which pairs do not take; us, two per SM / one): 22144 x 8576 at 162 tokens, 346 tiles, 74.0 / 69.6, 12416 x 8576 at 500 77.1 /
+    // 69.9; at 4096 K the second CTA's set-up under the first one's products is worth more, 22144 at 162 37.5 / 39.5
+    const int sms = num_sms(), one = (tiles + sms - 1) / sms, two = (tiles + 2 * sms - 1) / (2 * sms);
+    if (tiles <= sms || (a.K >= 6144 && one < 2 * two)) return launch_gemm<MODE, 128, 8, 4>(a);
   }
   return launch_gemm<MODE, 128, (w8 ? 4 : 2), 2>(a);
 }

@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
     (300, 6144, 512), (200, 6144, 640), (100, 12800, 512),   # one
     (100, 4096, 4096), (128, 6144, 1152), (66, 128, 2048),   # split
     (64, 6144, 640), (33, 28672, 512), (1, 128, 128), (17, 256, 384),
+    (300, 16256, 6144), (500, 12416, 6144), (300, 16256, 6016), (520, 16256, 6144),  # an odd number of channel tiles: one and two CTAs per multiprocessor
 ])
 def test_against_64_bits(dev, M, N, K):
     import qserve_backend.qgemm_w8a8 as w8
