@@ -124,6 +124,5 @@ def test_the_longest_tiles_start_first(dev):
             took.append(a.elapsed_time(e))
         us.append(min(took) * 200)
         outs.append(out.clone())
-    print(us)
     assert torch.equal(*outs)
     assert us[0] < 0.95 * us[1], us
