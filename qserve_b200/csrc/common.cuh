@@ -247,6 +247,13 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
 }
 // named barrier over `threads` threads (a multiple of 32) of the CTA; id 0 is __syncthreads
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Registers per thread of the warpgroup from here on (every warp of four neighbours executes it).  What the warpgroups of a block take together has to stay
+// within its launch's threads x registers per thread: an increase beyond that waits for good.
+template <bool UP, int N>
+__device__ __forceinline__ void set_max_regs() {
+  if constexpr (UP) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+  else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
 // arrive on the mbarrier at the same CTA-relative offset in CTA `rank` of the cluster.  Default semantics (release at CTA scope) on purpose:
 // `.release.cluster` (with `try_wait.acquire.cluster` behind the wait) costs ~1 us per pipeline stage.  The data these barriers guard is tensor memory / TMA-written shared memory, ordered by tcgen05.wait::st +
 // tcgen05.fence::before_thread_sync on the producer side and tcgen05.fence::after_thread_sync on the consumer side, not by generic-proxy fences;

@@ -55,7 +55,7 @@ constexpr bool kPairCvt = QS_PAIR_CVT != 0;
 #define QS_DECODE_CVT 1
 #endif
 constexpr bool kDecodeCvt = QS_DECODE_CVT != 0;  // the same choice for the epilogue of gemm_kernel
-constexpr int kPairThreads = 384;  // gemm_pair_kernel: the 8 warps of gemm_kernel + 4 more epilogue warps
+constexpr int kPairThreads = 384, kPairRoundsThreads = 640;  // CTAs of the pair kernels; with warps of their own for the epilogue (W4A8, tiles in several rounds)
 // warp roles: 0 weight producer | 1 TMEM owner + MMA issuer (even stages) | 2..5 unpack + TMEM epilogue | 6 activation producer |
 // 7 MMA issuer (odd stages).
 // All eight warps take part in the final reduce / scale / store phase.
@@ -193,7 +193,6 @@ __device__ __forceinline__ float epilogue_one(int32_t acc, float ws, float wsz, 
 // with the s8 zero.  vadd4 is four to five integer operations, which made this loop the bound of group scales.  Where 15 s + (z ^ 128) <= 255 no byte of
 // q s + (z ^ 128) leaves its place, whatever the codes: multiply and add are one instruction, and flipping the bytes' top bits gives q s + z mod 256.  That
 // holds for every weight whose dequantised range [z, 15 s + z] is a byte's; a block in which a lane's channel has another range goes the long way, same bits.
-// us, the long way for all / now: 28672 x 4096 at 16 tokens 19.5 / 16.5, at 64 21.0 / 18.0, at 5000 451 / 420; 4096 x 4096 at 16 7.1 / 6.8 (per channel 6.5).
 template <int MODE>
 __device__ __forceinline__ void unpack_block(const uint8_t* wsrc, uint32_t tdst, uint32_t sc4, uint32_t zp4) {
   uint32_t sc[4] = {}, zb[4] = {};
@@ -575,12 +574,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant_
 // at 52 %.  In a CTA pair each SM unpacks its own 128 channels into its own tensor memory (A operand) but stages only HALF of the 256 tokens of
 // the activation tile (B operand); the 2-CTA MMA reads the other half from the peer SM.  L2 -> SM traffic halves (2.7 GB for the shape above).
 // The first version of this kernel (one tile per launch-time CTA pair, 1 pair per TPC because of its 512 TMEM columns) lost all of that again to
-// un-overlapped per-tile fill / drain (24 us per tile for 8.3 us of MMA work), hence the persistent form: operand rings run
-// across tile boundaries, the only exposed per-tile cost is the accumulator drain (TMEM -> registers -> global, no shared-memory staging).
+// un-overlapped per-tile fill / drain (24 us per tile for 8.3 us of MMA work), hence the persistent form: operand rings run across tile boundaries.
 //
-// Roles per CTA (384 threads): warp 0 weight producer | warp 1 TMEM allocator, leader: MMA issuer (even stages) | warps 2..5 unpack + epilogue |
-// warp 6 activation producer (both CTAs signal the LEADER's "full" barrier: cta_group::2 TMA) | warp 7 leader: MMA issuer (odd stages) |
-// warps 8..11 epilogue only (a lone warp per scheduler issues one instruction per clock: four warps needed 9 us to drain a tile, eight 2 x fewer).
+// 256 accumulator columns and the ring of unpacked weights fill tensor memory, so a tile's products wait until the accumulator has been read.  Where the pairs
+// take several tiles (ROUNDS), eight warps of their own hold it in registers (128 a thread, setmaxnreg), hand the columns back 0.5 us after the last product and
+// convert and store under the next tile's products, while the unpack warps go on as well; with the unpack warps converting and storing first, a tile took 4 us
+// that were not products (12.5 for 8.5 of products).  us, that way / this: per channel 28672 x 4096 at 5000 tokens 414 / 367, 6144 x 4096 at 6108 117 / 104,
+// 28672 x 4096 at 250 31.1 / 29.1; group scales 410 / 381, 118 / 108, 29.9 / 28.8; 28672 x 512 at 2048 58.0 / 50.0 and 58.9 / 47.7.  Calls of one round have no
+// next tile, and 256 threads more to set up (512 tokens, 4096 x 4096: 11.4 / 12.1); nor do two rounds of smaller tiles pay for them (1300 tokens 20.8 / 21.3).
+// ncu, 2000 tokens: tensor pipe 81 % active while an SM works, L2 -> SM 11 TB/s, which is what a stage now waits for.
+//
+// Roles per CTA: warp 0 weight producer | warp 1 TMEM allocator, leader: MMA issuer (even stages) | warp 2 activation producer (both CTAs signal the LEADER's
+// "full" barrier: cta_group::2 TMA) | warp 3 leader: MMA issuer (odd stages) | warps 4..11 unpack, two per lane quadrant (group scales are bound by their integer
+// work: 4 -> 8 warps), without ROUNDS also the epilogue | warps 12..19, ROUNDS: epilogue (a lone warp per scheduler issues one instruction per clock: four warps
+// needed 9 us to drain a tile, eight less than half).
 // Only the even CTA of the pair (the leader) issues MMAs; its commits are multicast to the "empty" barriers of both CTAs.  All rings have even
 // depth (two alternating issuers, see gemm_kernel).  The accumulator is zero-filled by the epilogue warps (tcgen05.st) and every MMA accumulates:
 // the two issuers' first instructions of a tile are not ordered against each other.
@@ -611,54 +618,47 @@ struct PairCfg {
   static_assert(kSmemBytes <= 226 * 1024, "shared memory overflow");
 };
 
-// Accumulators of a pair tile -> fp16 output: a thread holds one channel (TMEM lane of `trow`) and `cols` tokens from column col0 on, 32 at a time; a
-// warp's store covers 32 consecutive channels of one token = 64 B (two full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum: the
-// tokens', m0: the tile's first token
+// 32 accumulators of a pair tile (this thread's channel, tokens tok0 ..) -> fp16 output; a warp's store covers 32 consecutive channels of one token = 64 B (two
+// full sectors).  ws, wz: the channel's scale and scaled zero, s_asc, s_asum: the tokens', m0: the tile's first token
 template <int MODE, bool ACC>
-__device__ __forceinline__ void pair_drain(const GemmParams& p, uint32_t trow, int col0, int cols, int m0, int n, float ws, float wz, const float* s_asc,
-                                           const float* s_asum) {
+__device__ __forceinline__ void pair_finish(const GemmParams& p, const uint32_t (&r)[32], int tok0, int m0, int n, float ws, float wz, const float* s_asc,
+                                            const float* s_asum) {
   const int tok_end = p.M - m0;
-  // chunks that hold tokens (those past M cost the ragged tile 1 us); the shuffle shows the compiler that all of the warp's threads take as many
-  const int chunks = __shfl_sync(~0u, (min(cols, tok_end - col0) + 31) >> 5, 0);
-#pragma unroll 1
-  for (int c = 0; c < chunks; ++c) {
-    const int tok0 = col0 + c * 32;
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(trow + tok0, r);
-    tmem_wait_ld();
-    __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
-    if (tok0 + 32 <= tok_end) {
-      // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
-      float as[32], am[32];
+  __half* out = p.out + static_cast<size_t>(m0 + tok0) * p.N + n;
+  if (tok0 + 32 <= tok_end) {
+    // whole chunk inside M: no per-token branches, the scales come in as vectors, 32 independent chains
+    float as[32], am[32];
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
-        as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
-        if constexpr (MODE == kModeW4Chn) {
-          const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
-          am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
-        } else {
-          am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
-        }
+    for (int i = 0; i < 32; i += 4) {
+      const float4 a4 = *reinterpret_cast<const float4*>(s_asc + tok0 + i);
+      as[i] = a4.x; as[i + 1] = a4.y; as[i + 2] = a4.z; as[i + 3] = a4.w;
+      if constexpr (MODE == kModeW4Chn) {
+        const float4 m4 = *reinterpret_cast<const float4*>(s_asum + tok0 + i);
+        am[i] = m4.x; am[i + 1] = m4.y; am[i + 2] = m4.z; am[i + 3] = m4.w;
+      } else {
+        am[i] = am[i + 1] = am[i + 2] = am[i + 3] = 0.f;
       }
+    }
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
+    for (int i = 0; i < 32; ++i) {
+      const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, as[i], am[i]);
+      out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
+      if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
+      if (tok0 + i < tok_end) {
+        const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
         out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
         if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {  // (fully unrolled: a dynamic index would push r[] into local memory for the fast path as well)
-        if (tok0 + i < tok_end) {
-          const float o = epilogue_one<MODE, kPairCvt>(static_cast<int32_t>(r[i]), ws, wz, s_asc[tok0 + i], s_asum[tok0 + i]);
-          out[static_cast<size_t>(i) * p.N] = __float2half_rn(o);
-          if constexpr (ACC) p.acc_out[static_cast<size_t>(m0 + tok0 + i) * p.N + n] = static_cast<int32_t>(r[i]);
-        }
       }
     }
   }
 }
+// chunks of 32 columns from col0 on that hold tokens (those past M cost the ragged tile 1 us); the shuffle shows the compiler that all of the warp's threads
+// take as many
+__device__ __forceinline__ int pair_chunks(int tok_end, int col0, int cols) { return __shfl_sync(~0u, (min(cols, tok_end - col0) + 31) >> 5, 0); }
 // zero-fills an accumulator's columns [col0, col0 + cols) of the warp's 32 lanes
 __device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols, int nt) {
   auto eight = [&](int c) {
@@ -681,8 +681,8 @@ __device__ __forceinline__ void pair_zero(uint32_t trow, int col0, int cols, int
 }
 
 // FULL: tiles of 256 tokens, known to the compiler (per channel 28672 x 4096 at 1024 tokens 86.4 us, 87.0 without; 8192 x 512 at 512 7.8 and 7.9)
-template <int MODE, bool ACC, bool FULL>
-__global__ void __launch_bounds__(kPairThreads, 1)
+template <int MODE, bool ACC, bool FULL, bool ROUNDS>
+__global__ void __launch_bounds__(ROUNDS ? kPairRoundsThreads : kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) {
   using C = PairCfg<MODE>;
   constexpr int NT = C::NT, WS = C::WS, AS = C::AS, TA = C::TA;
@@ -736,6 +736,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
   auto tile_m = [&](int lt) { return (pair + lt * n_pairs) % p.m_tiles; };
   auto tile_n = [&](int lt) { return 2 * ((pair + lt * n_pairs) / p.m_tiles) + static_cast<int>(rank); };
 
+  // 4 x 48 + 8 x 64 + 8 x 152 registers of 32 lanes: the 61440 that 640 threads are launched with
+  if (ROUNDS && warp < 4) set_max_regs<false, 48>();
   if (warp == 0) {
     // ===================================== weight producer (static data: never waits for the previous kernel) =====================================
     if (lane == 0) {
@@ -763,11 +765,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         }
       }
     }
-  } else if (warp == 6) {
+  } else if (warp == 2) {
     // ===================================== activation producer: this CTA's half of the tile's tokens =====================================
     if (lane == 0) {
       pdl_wait();
-      qs_trace(QS_K_GEMM, 1, 6 * 32);
+      qs_trace(QS_K_GEMM, 1, 2 * 32);
       int s = 0;
       uint32_t ph = 0;
       for (int lt = 0; lt < my_tiles; ++lt) {
@@ -782,9 +784,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         }
       }
     }
-  } else if (leader && (warp == 1 || warp == 7)) {
-    // ===================================== leader: two MMA issuers (even / odd iterations), 256 x nt x 32 INT8 UMMAs over both SMs ==========
-    if (lane == 0) {
+  } else if (warp < 4) {
+    if (leader && lane == 0) {
+      // =================================== leader: two MMA issuers (even / odd iterations), 256 x nt x 32 INT8 UMMAs over both SMs ==========
       const uint32_t idesc = umma_idesc_i8(2 * kBM, nt, 1u, 1u);
       const int g_end = my_tiles * n_kb;
       int it = (warp == 1) ? 0 : 1;  // iteration inside the current tile
@@ -824,60 +826,48 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         }
       }
     }
-  } else if ((warp >= 2 && warp <= 5) || warp >= 8) {
-    // ===================================== unpack + epilogue: warps 2..5 and 8..11, both CTAs =====================================
-    // A warp reaches the TMEM lanes 32 * (warp % 4) ..: the two warps of a lane quadrant split every stage's two 128-K sub-blocks (unpack) and the
-    // 256 token columns (epilogue).  (Per-group mode is bound by the integer work of the level-2 dequantisation in this loop: 4 -> 8 warps.)
-    const bool unpacker = warp < 8;           // first / second warp of its lane quadrant
-    const int quad = warp & 3;
-    const int usel = unpacker ? 0 : 1;        // the 128-K sub-block of a stage this warp unpacks
-    // accumulator columns (tokens) of this warp: half of them, in chunks of 32
-    const int first = (nt + 63) / 64 * 32, col0 = unpacker ? 0 : first, cols = unpacker ? first : nt - first;
+  } else {
+    // ===================================== unpack: warps 4 to 11; epilogue: warps 12 to 19, or 4 to 11 again; both CTAs =====================================
+    // A warp reaches the TMEM lanes 32 * (warp % 4) ..: the two unpack warps of a lane quadrant take one of a stage's two 128-K sub-blocks each, the two
+    // epilogue warps half of the accumulator's columns (tokens) each, in chunks of 32
+    static_assert(kSub == 2, "two warps per lane quadrant take one sub-block each");
+    const bool unpacks = warp < 12;
+    const int quad = warp & 3, half = ((warp >> 2) - 1) & 1;
+    const int first = (nt + 63) / 64 * 32, col0 = half == 0 ? 0 : first, cols = half == 0 ? first : nt - first;
     const int epi_tid = quad * 32 + lane;     // channel inside the tile
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     auto zero_fill = [&]() {
       pair_zero(trow, col0, cols, nt);
       if (lane == 0) mbar_arrive_cluster(bar_zero, 0);
     };
-    zero_fill();
     int s = 0, ta = 0;
     uint32_t ph = 0, pha = 0;
-    for (int lt = 0; lt < my_tiles; ++lt) {
-      const int m_tile = tile_m(lt), n_tile = tile_n(lt);
-      {
-        for (int it = 0; it < n_kb; ++it) {
-          mbar_wait(&bar_wfull[s], ph);
-          mbar_wait(&bar_aempty[ta], pha ^ 1);
-          tc_fence_after();
-          static_assert(kSub == 2, "two warps per lane quadrant take one sub-block each");
-          {
-            const int u = usel;
-            const uint8_t* wsrc = s_w + s * C::kWBytes + u * C::kWSub + quad * 2048 + lane * 16;
-            const uint32_t tdst = trow + NT + ta * C::kAStageCols + u * (kBK / 4);
-            uint32_t sc4 = 0, zp4 = 0;
-            if constexpr (MODE == kModeW4Grp) {
-              const uint8_t* s2 = s_s2 + s * C::kS2Bytes + u * C::kS2Sub + quad * 32 + (lane >> 2) * 4;
-              sc4 = *reinterpret_cast<const uint32_t*>(s2);
-              zp4 = *reinterpret_cast<const uint32_t*>(s2 + kBM);
-            }
-            unpack_block<MODE>(wsrc, tdst, sc4, zp4);
-          }
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_cluster(&bar_afull[ta], 0);  // the leader's barrier counts the unpack warps of both CTAs
-            mbar_arrive(&bar_wempty[s]);
-          }
-          if (++s == WS) { s = 0; ph ^= 1; }
-          if (++ta == TA) { ta = 0; pha ^= 1; }
-          if (epi_tid == 0 && lt == 0 && it == 8) QS_PROF(14);
+    auto unpack = [&](int stages) {
+      for (; stages > 0; --stages) {
+        mbar_wait(&bar_wfull[s], ph);
+        mbar_wait(&bar_aempty[ta], pha ^ 1);
+        tc_fence_after();
+        const uint8_t* wsrc = s_w + s * C::kWBytes + half * C::kWSub + quad * 2048 + lane * 16;
+        uint32_t sc4 = 0, zp4 = 0;
+        if constexpr (MODE == kModeW4Grp) {
+          const uint8_t* s2 = s_s2 + s * C::kS2Bytes + half * C::kS2Sub + quad * 32 + (lane >> 2) * 4;
+          sc4 = *reinterpret_cast<const uint32_t*>(s2);
+          zp4 = *reinterpret_cast<const uint32_t*>(s2 + kBM);
         }
-        if (epi_tid == 0 && lt == 0) QS_PROF(8);
+        unpack_block<MODE>(wsrc, trow + NT + ta * C::kAStageCols + half * (kBK / 4), sc4, zp4);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_cluster(&bar_afull[ta], 0);  // the leader's barrier counts the unpack warps of both CTAs
+          mbar_arrive(&bar_wempty[s]);
+        }
+        if (++s == WS) { s = 0; ph ^= 1; }
+        if (++ta == TA) { ta = 0; pha ^= 1; }
       }
-      // ------------------------------ epilogue: this CTA's 128 channels x nt tokens, TMEM -> registers -> global ------------------------------
-      pdl_wait();
-      const int m0 = m_tile * nt;
+    };
+    auto finish = [&](int lt) {
+      const int m0 = tile_m(lt) * nt;
       float* s_asc = s_row + (lt & 1) * 2 * NT;  // double-buffered by tile parity: a fast warp may already fill the next tile's values
       float* s_asum = s_asc + NT;
       {
@@ -886,21 +876,59 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
         s_asc[j] = ok ? __half2float(p.ascales[m0 + j]) : 0.f;
         if constexpr (MODE == kModeW4Chn) s_asum[j] = ok ? __half2float(p.a_ssums[m0 + j]) : 0.f;
       }
-      const int n = n_tile * kBM + epi_tid;
+      const int n = tile_n(lt) * kBM + epi_tid;
       const float ws = __half2float(__ldg(p.wscales + n));
       float wz = 0.f;
       if constexpr (MODE == kModeW4Chn) wz = __half2float(__ldg(p.w_szs + n));
       named_bar_sync(1, 256);  // the eight epilogue warps: per-token scales visible
       mbar_wait(bar_dfull, lt & 1);  // every MMA of the tile has retired
-      if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(9);
+      if (epi_tid == 0 && half == 0 && lt == 0) QS_PROF(9);
       tc_fence_after();
-      pair_drain<MODE, ACC>(p, trow, col0, cols, m0, n, ws, wz, s_asc, s_asum);
-      if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(10);
-      if (lt + 1 < my_tiles) zero_fill();  // hands the accumulator back to the MMA issuers
-      if (epi_tid == 0 && lt == 0 && unpacker) QS_PROF(11);
+      const int chunks = pair_chunks(p.M - m0, col0, cols);
+      if (ROUNDS && lt + 1 < my_tiles) {
+        // all of the warp's accumulators into registers, and the columns back to the issuers; converting and storing goes on under the next tile's products
+        uint32_t r[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(trow + col0 + c * 32, r[c]);  // (columns past the tile's are loaded and left: col0 + 128 <= 256)
+        tmem_wait_ld();
+        zero_fill();
+        if (epi_tid == 0 && half == 0 && lt == 0) QS_PROF(11);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c < chunks) pair_finish<MODE, ACC>(p, r[c], col0 + c * 32, m0, n, ws, wz, s_asc, s_asum);
+      } else {
+        // nothing else to do for these warps meanwhile, and a loop has a quarter of the instructions to fetch
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(trow + col0 + c * 32, r);
+          tmem_wait_ld();
+          pair_finish<MODE, ACC>(p, r, col0 + c * 32, m0, n, ws, wz, s_asc, s_asum);
+        }
+      }
+      if (epi_tid == 0 && half == 0 && lt == 0) QS_PROF(10);
+    };
+    if constexpr (ROUNDS) {
+      if (unpacks) {
+        set_max_regs<false, 64>();
+        unpack(my_tiles * n_kb);
+        pdl_wait();
+      } else {
+        zero_fill();
+        set_max_regs<true, 152>();
+        pdl_wait();
+        for (int lt = 0; lt < my_tiles; ++lt) finish(lt);
+      }
+    } else {
+      zero_fill();
+      for (int lt = 0; lt < my_tiles; ++lt) {
+        unpack(n_kb);
+        if (epi_tid == 0 && half == 0 && lt == 0) QS_PROF(8);
+        pdl_wait();
+        finish(lt);
+        if (lt + 1 < my_tiles) zero_fill();  // hands the accumulator back to the MMA issuers
+      }
     }
-  } else {
-    pdl_wait();
   }
 
   tc_fence_before();
@@ -1038,7 +1066,14 @@ gemm_pair_w8_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_c
       named_bar_sync(1, 256);
       mbar_wait(&bar_dfull[buf], (static_cast<uint32_t>(lt) >> 1) & 1u);
       tc_fence_after();
-      pair_drain<kModeW8, ACC>(p, trow + buf * NT, col0, cols, m0, n, ws, 0.f, s_asc, s_asc);
+      const int chunks = pair_chunks(p.M - m0, col0, cols);
+#pragma unroll 1
+      for (int c = 0; c < chunks; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(trow + buf * NT + col0 + c * 32, r);
+        tmem_wait_ld();
+        pair_finish<kModeW8, ACC>(p, r, col0 + c * 32, m0, n, ws, 0.f, s_asc, s_asc);
+      }
       if (lt + 2 < my_tiles) zero_fill(buf);
     }
   } else {
@@ -1316,23 +1351,26 @@ int launch_gemm_pair(const GemmArgs& a) {
   if (rc) return rc;
   rc = w8 ? make_tmap_u8(&tm_w, a.weight, a.N, a.K, kBM) : make_tmap_w4(&tm_w, a.weight, a.N, a.K);
   if (rc) return rc;
+  // persistent: one CTA pair per TPC walks the (m fastest) tile list with stride = number of pairs
+  const int total_pairs = (n_tiles / 2) * p.m_tiles, pairs = std::min(total_pairs, num_sms() / 2);
+  const bool full = p.nt == 256, rounds = total_pairs > (full ? 1 : 2) * pairs;
   auto kern = [&] {
     if constexpr (w8) return a.acc_out ? gemm_pair_w8_kernel<true> : gemm_pair_w8_kernel<false>;
-    else if (p.nt == 256) return a.acc_out ? gemm_pair_kernel<MODE, true, true> : gemm_pair_kernel<MODE, false, true>;
-    else return a.acc_out ? gemm_pair_kernel<MODE, true, false> : gemm_pair_kernel<MODE, false, false>;
+    else if (rounds) return full ? (a.acc_out ? gemm_pair_kernel<MODE, true, true, true> : gemm_pair_kernel<MODE, false, true, true>)
+                                 : (a.acc_out ? gemm_pair_kernel<MODE, true, false, true> : gemm_pair_kernel<MODE, false, false, true>);
+    else return full ? (a.acc_out ? gemm_pair_kernel<MODE, true, true, false> : gemm_pair_kernel<MODE, false, true, false>)
+                     : (a.acc_out ? gemm_pair_kernel<MODE, true, false, false> : gemm_pair_kernel<MODE, false, false, false>);
   }();
-  static bool attr_set[2][2][kMaxDevices] = {};
-  bool& done = attr_set[a.acc_out ? 1 : 0][p.nt == 256 ? 1 : 0][device_ordinal()];
+  static bool attr_set[2][2][2][kMaxDevices] = {};
+  bool& done = attr_set[a.acc_out ? 1 : 0][full ? 1 : 0][rounds ? 1 : 0][device_ordinal()];
   if (!done) {
     rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes), "cudaFuncSetAttribute(gemm pair smem)");
     if (rc) return rc;
     done = true;
   }
   cudaLaunchConfig_t cfg{};
-  // persistent: one CTA pair per TPC walks the (m fastest) tile list with stride = number of pairs
-  const int total_pairs = (n_tiles / 2) * p.m_tiles;
-  cfg.gridDim = dim3(2 * std::min(total_pairs, num_sms() / 2));
-  cfg.blockDim = dim3(kPairThreads);
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(!w8 && rounds ? kPairRoundsThreads : kPairThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(a.stream);
   cudaLaunchAttribute attr[2];
