@@ -8,7 +8,7 @@
 // B200 design: the reference launches one CTA per *query* head and therefore streams every KV head
 // Hq/Hkv times; here one CTA (4 warps) owns a (sequence, KV head, context split) and serves all query heads of the GQA
 // group from a single pass over the pages, so HBM traffic is the algorithmic minimum.  Every warp streams its own 32-token
-// slices of the pages with cp.async.bulk into a private shared-memory ring; the (<= 8 heads) x 32-token QK^T and PV
+// slices of the pages with cp.async into a private shared-memory ring; the (<= 8 heads) x 32-token QK^T and PV
 // products run as mma.sync m16n8k16 on "biased" operands (0x6400 | code = 1024 + code in fp16: one LOP3 per two codes, the
 // constant parts are removed after the MMA), per-token scale / zero are folded into the logits and probabilities, the
 // softmax is an online (flash-decoding) softmax with lazy rescaling, and context splits are merged by the last-arriving
@@ -52,6 +52,16 @@ __device__ __forceinline__ unsigned long long attn_gtime() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)::"memory");
   return t;
 }
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+// four 8 x 8 matrices of 16-bit words, transposed: lane 8 m + r gives the address of row r of matrix m, thread t gets (rows 2 (t % 4), + 1; column t / 4) of each
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t smem) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem) : "memory");
+}
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -90,13 +100,18 @@ constexpr int kAttnThreadsV2 = kAttnConsumers;  // no dedicated producer warp: e
 constexpr int kPageTokens = 64;
 constexpr int kOStride = kD + 4;  // floats per (warp, head) row of the merge buffer
 
-// A warp consumes 32-token slices of the 64-token pages of one kv head.  Each warp owns a private ring of kSlots slots, filled by its lane 0 with
-// cp.async.bulk copies and guarded by one "full" mbarrier per slot (the refill of a slot is issued by the same warp right after it has consumed it, so no
-// "empty" barrier and no producer warp are needed).  A slot holds a whole slice, K codes | V codes | K scales | K zeros | V scales | V zeros, and the ring
-// two; or, INT8 in calls of more than three CTAs per SM, one half of a slice, first K, then V (codes | scales | zeros), and the ring three: 135 KB are on
-// their way per SM where two whole slices take so much that only three CTAs fit, and 64 sequences x 8 heads need a second wave (45 us, now 34).  Where CTAs
-// fit either way a wait more per slice is what remains of the halves: INT4 3 % slower, INT8 (1 x 300 tokens x 8
-// heads) 9.2 us and 7.9 in whole slices, whose three CTAs have 168 registers each.
+// A warp consumes 32-token slices of the 64-token pages of one kv head, out of a private ring of kSlots slots that its lanes fill with cp.async, one group per
+// slot (the refill of a slot is issued by the same warp right after it has consumed it, so neither barriers nor a producer warp are needed).  A slot holds a
+// whole slice, K codes | V codes | K scales | K zeros | V scales | V zeros, and the ring two; or, INT8 in calls of more than three CTAs per SM, one half of a
+// slice, first K, then V (codes | scales | zeros), and the ring three: 135 KB are on their way per SM where two whole slices take so much that only three CTAs
+// fit, and 64 sequences x 8 heads need a second wave (45 us, with halves 34).  Where CTAs fit either way a wait more per slice is what remains of the halves:
+// INT4 3 % slower, INT8 (1 x 300 tokens x 8 heads) 9.2 us and 7.9 in whole slices, whose three CTAs have 168 registers each.
+//
+// The main loop is bound by its instructions (issue slots 45 % busy, the integer pipe as much, with four warps per scheduler to hide a slice's chain).  One lane's
+// cp.async.bulk copies with an mbarrier per slot took 60 of them per slice; with all lanes copying 16 bytes each it is 25, the lanes choose where their words
+// go, and V comes out of shared memory through transposing loads that bring two tokens of one dim together: INT8 operands of V take one instruction per two
+// codes instead of two, INT4's five per eight instead of six.  us, bulk copies / this: 64 sequences of up to 1024 tokens, 8 heads, INT4 23.2 / 20.0, INT8 31.5 /
+// 25.9; 128 sequences INT8 56.7 / 46.3; 4 of up to 8000 INT4 16.8 / 15.4, INT8 22.2 / 18.7; 1 of 100 5.6 / 5.4.
 constexpr int kSliceTokens = 32;
 template <int BITS, int PER>  // PER: slots of a slice
 struct StageLayout {
@@ -110,6 +125,14 @@ struct StageLayout {
   static constexpr int kBytes = kOffVm + 128;
   static constexpr int kWarpBytes = kSlots * kBytes;  // private ring of one warp (also holds its partial O^T at the end)
   static_assert(kWarpBytes >= kMaxG * kOStride * 4, "the per-warp ring must hold the warp's partial output");
+  static_assert(kBytes % 128 == 0, "the places of a slot are counted from a line of 128 bytes");
+  // Where 16-byte word c of a token's row belongs: a permutation inside lines of 128 bytes that lets K reads (a quarter warp: all of rows p and p + 4, or every
+  // other word of them) and V reads (one word of eight neighbouring rows) meet every bank once.
+  static constexpr int kRow = kD * BITS / 8;  // bytes of a token's row
+  static __device__ __forceinline__ uint32_t place(int row, int c) {
+    if constexpr (BITS == 4) return (row >> 1) * 128 + (((row ^ (row >> 2)) & 1) * 4 + (c ^ ((row >> 1) & 3))) * 16;
+    else return row * 128 + (c ^ (((row >> 2) & 1) | ((row & 3) << 1))) * 16;
+  }
 };
 
 // full m16n8k16: all four A registers and all four accumulators carry data
@@ -202,25 +225,15 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   __shared__ float s_m[kWarps + 1][kMaxG], s_l[kWarps + 1][kMaxG];
   __shared__ float s_f[kWarps + 1][kMaxG];                                // merge weights exp2(m_w - M) [* 1 / L]
   __shared__ float2 s_meta[kWarps][2][kSliceTokens];                     // per token (scale, c) of the slice in flight: K pre-multiplied by sm_scale
-  __shared__ __align__(8) uint64_t s_full[kWarps][R];
   __shared__ uint32_t s_last;
 
-  // Every warp initialises the barriers of ITS OWN ring (lane 0, the lane that later arms them and issues the copies), so no block-wide
-  // barrier is needed between initialisation and first use.  With thread 0 initialising all rings and no barrier, a late CTA
-  // of a multi-wave launch (64 kv heads x 64 sequences = 4096 CTAs at Qwen1.5-72B), which does not sit in griddepcontrol.wait, could arm a ring ahead
-  // of its initialisation, which then wiped the pending transaction count: that warp waited forever (one in ~10^8 slices).
-  if (lane == 0) {
-    for (int i = 0; i < R; ++i) mbar_init(&s_full[warp][i], 1);
-    fence_barrier_init();
-  }
-  __syncwarp();
 #define ATTN_PROF(slot) do { if (prof) prof[((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 16 + (slot)] = attn_gtime(); } while (0)
   if (threadIdx.x == 0) ATTN_PROF(0);
   qs_trace(QS_K_ATTN, 0);
   if (threadIdx.x == 0) pdl_launch_dependents();  // dependents may become resident (and prefetch static data) right away
 
   // The sequence lengths and the page-pointer table are prepared by the host side before the step (model_runner.py:506-530):
-  // they are read BEFORE the dependency wait, so that the chain length -> page pointers -> first bulk copy (two dependent
+  // they are read BEFORE the dependency wait, so that the chain length -> page pointers -> first copy (two dependent
   // global round trips) overlaps the tail of the preceding qkv GEMM.  Page CONTENTS and q/k/v are only touched after the wait.
   const int tlen = lengths ? lengths[b] - 1 : timestep;  // tokens already in the cache (Template.hpp:901: length_per_sample ? len - 1 : timestep)
   const long long* kptrs = kv_pointers + (static_cast<size_t>(b) * 2 + 0) * max_blocks;
@@ -246,42 +259,38 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   const int my_first = p_begin + (warp >> 1);
   const int n_my = (p_end > my_first) ? (p_end - my_first + 1) / 2 : 0;
   uint8_t* my_ring = s_ring + warp * SL::kWarpBytes;
-  uint64_t* my_full = &s_full[warp][0];
   const int zoff = pg.num_kv_heads * pg.tokens_per_block * 2;  // bytes from a scale row to the zero row
   long long kp_l = 0, vp_l = 0;  // lane l: page pointers of this warp's pages (batch * 32 + l); K runs ahead of V
   auto load_ptrs = [&](long long& ptr, const long long* table, int j0) {
     const int pidx = my_first + 2 * (j0 + lane);
     ptr = (pidx < p_end) ? table[pidx] : 0;
   };
-  // all lanes call; lane 0 issues the copies of this warp's u-th slot contents into slot `slot`: slice u, or half u & 1 of slice u >> 1
+  // all lanes call: the copies of this warp's u-th slot contents into slot `slot`: slice u, or half u & 1 of slice u >> 1.  A copy instruction takes 512
+  // consecutive bytes of codes; lane_at is where the lane's 16 bytes belong (see StageLayout).
   const int units = SL::kPerSlice * n_my;
+  const uint32_t ring = smem_u32(my_ring), lane_at = SL::place(lane * 16 / SL::kRow, lane * 16 % SL::kRow / 16);
+  const uint32_t codes_off = hk * SL::kCodes + hslice * SL::kSliceCodes + lane * 16;
+  const uint32_t meta_off = pg.code_bytes + hk * 128 + hslice * 64 + ((lane >> 2) & 1) * zoff + (lane & 3) * 16;  // four lanes per row of scales or zeros
+  auto copy = [&](uint32_t dst, const uint8_t* page) {
+#pragma unroll
+    for (int i = 0; i < SL::kSliceCodes / 512; ++i) cp_async16(dst + i * 512 + (BITS == 8 && (i & 1) ? lane_at ^ 16u : lane_at), page + codes_off + i * 512);
+  };
   auto issue = [&](int u, int slot) {
     const int j = u / SL::kPerSlice;
-    auto copy = [&](const uint8_t* page, int codes_at, int meta_at) {
-      uint8_t* dst = my_ring + slot * SL::kBytes;
-      bulk_copy_g2s(dst + codes_at, page + static_cast<size_t>(hk) * SL::kCodes + hslice * SL::kSliceCodes, SL::kSliceCodes, &my_full[slot]);
-      const uint8_t* meta = page + pg.code_bytes + hk * 128 + hslice * 64;
-      bulk_copy_g2s(dst + meta_at, meta, 64, &my_full[slot]);
-      bulk_copy_g2s(dst + meta_at + 64, meta + zoff, 64, &my_full[slot]);
-    };
+    const uint32_t dst = ring + slot * SL::kBytes;
     if constexpr (SL::kPerSlice == 1) {
-      const long long kp = __shfl_sync(0xffffffffu, kp_l, j & 31), vp = __shfl_sync(0xffffffffu, vp_l, j & 31);
-      if (lane == 0) {
-        fence_proxy_async();  // the slot was last read through the generic proxy
-        mbar_expect_tx(&my_full[slot], SL::kBytes);
-        copy(reinterpret_cast<const uint8_t*>(kp), 0, SL::kOffKm);
-        copy(reinterpret_cast<const uint8_t*>(vp), SL::kOffV, SL::kOffVm);
-      }
+      const uint8_t* kp = reinterpret_cast<const uint8_t*>(__shfl_sync(0xffffffffu, kp_l, j & 31));
+      const uint8_t* vp = reinterpret_cast<const uint8_t*>(__shfl_sync(0xffffffffu, vp_l, j & 31));
+      copy(dst, kp);
+      copy(dst + SL::kOffV, vp);
+      if (lane < 16) cp_async16(dst + SL::kOffKm + lane * 16, (lane < 8 ? kp : vp) + meta_off);
     } else {
-      const long long ptr = __shfl_sync(0xffffffffu, (u & 1) ? vp_l : kp_l, j & 31);
-      if (lane == 0) {
-        fence_proxy_async();
-        mbar_expect_tx(&my_full[slot], SL::kBytes);
-        copy(reinterpret_cast<const uint8_t*>(ptr), 0, SL::kOffKm);
-      }
+      const uint8_t* page = reinterpret_cast<const uint8_t*>(__shfl_sync(0xffffffffu, (u & 1) ? vp_l : kp_l, j & 31));
+      copy(dst, page);
+      if (lane < 8) cp_async16(dst + SL::kOffKm + lane * 16, page + meta_off);
     }
   };
-  // what follows u into its slot, once every lane is done with u
+  // what follows u into its slot, once every lane is done with u; a group per unit, also where nothing follows: the waits count groups
   auto refill = [&](int u, int slot) {
     __syncwarp();
     const int next = u + R, j = next / SL::kPerSlice;
@@ -292,6 +301,11 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       }
       issue(next, slot);
     }
+    cp_async_commit();
+  };
+  auto arrived = [&]() {  // the oldest unit on its way
+    cp_async_wait<R - 1>();
+    __syncwarp();
   };
   load_ptrs(kp_l, kptrs, 0);
   load_ptrs(vp_l, vptrs, 0);
@@ -320,7 +334,11 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       }
     }
     const __half vnew = vg[threadIdx.x];
-    for (int u = 0; u < R && u < units; ++u) issue(u, u);  // the cache stream starts before the new-token work below
+#pragma unroll
+    for (int u = 0; u < R; ++u) {  // the cache stream starts before the new-token work below
+      if (u < units) issue(u, u);
+      cp_async_commit();
+    }
     if (threadIdx.x == 0) ATTN_PROF(3);
     float sn, cs;
     {
@@ -428,7 +446,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     }
 
     const float sm_scale = rsqrtf(static_cast<float>(kD)) * 1.4426950408889634f;  // 1/sqrt(D) * log2(e)
-    // O^T accumulators: m-tile i (dims 16g + 2i, 16g + 2i + 1) x heads (2q4, 2q4+1)
+    // O^T accumulators: m-tile i (INT4 dims 32 (i / 2) + 4 g + 2 (i % 2) and the next one, INT8 16 i + 2 g and the next one) x heads (2q4, 2q4+1)
     float o[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
@@ -438,17 +456,17 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
 
     // S^T = K Q^T: A rows g / g+8 <-> chunk tokens tokA / 8+tokA (the permutation keeps the V row reads at a 2-way conflict)
     const int tokA = (g & 1) * 4 + (g >> 1);
-    constexpr int kRow = kD * BITS / 8;  // bytes per token row
+    const uint32_t k_at = SL::place(tokA, BITS == 4 ? q4 : 2 * q4);                                                // + 512 or 1024 bytes: tokens 8 on
+    const uint32_t v_at = SL::place((lane & 1) * 4 + ((lane >> 1) & 3) + (lane & 8), lane >> 4) + SL::kOffV;  // matrices: tokens 0 .. 7, 8 .. 15, next word
     // warp w consumes tokens [32 (w & 1), +32) of the pages whose index has parity (w >> 1): two 16-token MMA chunks per
     // iteration share one barrier wait, one max reduction and one set of address computations
     const int hbase = hslice * kSliceTokens;
     int s = 0;  // the slot at hand
-    uint32_t ph = 0;
-    auto advance = [&]() { if (++s == R) { s = 0; ph ^= 1; } };
+    auto advance = [&]() { if (++s == R) s = 0; };
     if (threadIdx.x == 0) ATTN_PROF(4);
     for (int j = 0; j < n_my; ++j) {
       const int pidx = my_first + 2 * j;
-      mbar_wait(&my_full[s], ph);
+      arrived();
       if (threadIdx.x == 0 && j == 0) ATTN_PROF(5);
       const uint8_t* st = my_ring + s * SL::kBytes;
       const int t0 = pidx * kPageTokens + hbase;  // first token of this warp's 32-token slice
@@ -480,10 +498,10 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
         // ---- S^T (2 x 16 tokens x 8 heads) on biased codes: 16 MMAs ----
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const uint8_t* krow = st + (c * kChunk + tokA) * kRow;
+          const uint8_t* krow = st + c * kChunk * SL::kRow + k_at;
           if constexpr (BITS == 4) {
-            const uint4 ka = *reinterpret_cast<const uint4*>(krow + q4 * 16);
-            const uint4 kb = *reinterpret_cast<const uint4*>(krow + 8 * kRow + q4 * 16);
+            const uint4 ka = *reinterpret_cast<const uint4*>(krow);
+            const uint4 kb = *reinterpret_cast<const uint4*>(krow + 8 * SL::kRow);
             const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb.x, kb.y, kb.z, kb.w};
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
@@ -494,8 +512,9 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
                        lop3_and_or(ta, 0x00f000f0u, kMagic), lop3_and_or(tb, 0x00f000f0u, kMagic), qb0[2 * w + 1], qb1[2 * w + 1]);
             }
           } else {
-            const uint4 ka0 = *reinterpret_cast<const uint4*>(krow + q4 * 32), ka1 = *reinterpret_cast<const uint4*>(krow + q4 * 32 + 16);
-            const uint4 kb0 = *reinterpret_cast<const uint4*>(krow + 8 * kRow + q4 * 32), kb1 = *reinterpret_cast<const uint4*>(krow + 8 * kRow + q4 * 32 + 16);
+            const uint8_t* krow1 = st + c * kChunk * SL::kRow + (k_at ^ 16u);  // word 2 q4 + 1
+            const uint4 ka0 = *reinterpret_cast<const uint4*>(krow), ka1 = *reinterpret_cast<const uint4*>(krow1);
+            const uint4 kb0 = *reinterpret_cast<const uint4*>(krow + 8 * SL::kRow), kb1 = *reinterpret_cast<const uint4*>(krow1 + 8 * SL::kRow);
             const uint32_t wa[8] = {ka0.x, ka0.y, ka0.z, ka0.w, ka1.x, ka1.y, ka1.z, ka1.w};
             const uint32_t wb[8] = {kb0.x, kb0.y, kb0.z, kb0.w, kb1.x, kb1.y, kb1.z, kb1.w};
 #pragma unroll
@@ -510,7 +529,7 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       if constexpr (SL::kPerSlice == 2) {
         refill(2 * j, s);
         advance();
-        mbar_wait(&my_full[s], ph);
+        arrived();
         st = my_ring + s * SL::kBytes;
       }
       if (live) {
@@ -575,44 +594,29 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
           // sum_t p'_t per head, from the very operand the V MMAs consume: an all-ones A tile (every output row is the sum)
           mma_full(spa[0], spa[1], spa[2], spa[3], kOnesH2, kOnesH2, kOnesH2, kOnesH2, bp[c][0], bp[c][1]);
         }
-        // ---- O^T += V^T P'^T on biased codes: 2 x 8 MMAs (m-tile = 16 dims) ----
+        // ---- O^T += V^T P'^T on biased codes: 2 x 8 MMAs (m-tile = 16 dims).  The transposing loads bring words of two tokens of one place together: 4 or 2
+        //      dims of tokens q4, 4 + q4 and of 8 + q4, 12 + q4 ----
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const uint8_t* vbase = st + SL::kOffV + (c * kChunk + q4) * kRow;
-          if constexpr (BITS == 4) {
-            const uint2 va = *reinterpret_cast<const uint2*>(vbase + g * 8);
-            const uint2 vb = *reinterpret_cast<const uint2*>(vbase + 4 * kRow + g * 8);
-            const uint2 vcw = *reinterpret_cast<const uint2*>(vbase + 8 * kRow + g * 8);
-            const uint2 vd = *reinterpret_cast<const uint2*>(vbase + 12 * kRow + g * 8);
 #pragma unroll
-            for (int ww = 0; ww < 2; ++ww) {
-              const uint32_t a = ww ? va.y : va.x, bb = ww ? vb.y : vb.x, cc = ww ? vcw.y : vcw.x, dd = ww ? vd.y : vd.x;
+          for (int h = 0; h < kD / (256 / BITS); ++h) {
+            uint32_t w[4];  // of two neighbouring 16-byte words: tokens 0 .. 7, 8 .. 15 each
+            ldmatrix_x4_trans(w, ring + s * SL::kBytes + c * kChunk * SL::kRow + (v_at ^ (h * 32u)));
 #pragma unroll
-              for (int kb = 0; kb < 4; ++kb) {
-                const uint32_t sel = static_cast<uint32_t>(kb) | (static_cast<uint32_t>(kb) << 4) | (static_cast<uint32_t>(4 + kb) << 8) |
-                                     (static_cast<uint32_t>(4 + kb) << 12);  // bytes [a_kb, a_kb, b_kb, b_kb]
-                const uint32_t m01 = __byte_perm(a, bb, sel), m89 = __byte_perm(cc, dd, sel);
-                const int i = 4 * ww + kb;
-                mma_full(o[i][0], o[i][1], o[i][2], o[i][3], lop3_and_or(m01, 0x000f000fu, kMagic), lop3_and_or(m01, 0x00f000f0u, kMagic),
-                         lop3_and_or(m89, 0x000f000fu, kMagic), lop3_and_or(m89, 0x00f000f0u, kMagic), bp[c][0], bp[c][1]);
+            for (int e = 0; e < 2; ++e) {
+              const uint32_t lo = w[2 * e], hi = w[2 * e + 1];
+              if constexpr (BITS == 4) {
+                const int i = 4 * h + 2 * e;  // dims 16 i + 4 g + 0, 1 | 2, 3
+                mma_full(o[i][0], o[i][1], o[i][2], o[i][3], lop3_and_or(lo, 0x000f000fu, kMagic), lop3_and_or(lo, 0x00f000f0u, kMagic),
+                         lop3_and_or(hi, 0x000f000fu, kMagic), lop3_and_or(hi, 0x00f000f0u, kMagic), bp[c][0], bp[c][1]);
+                const uint32_t lo8 = lo >> 8, hi8 = hi >> 8;
+                mma_full(o[i + 1][0], o[i + 1][1], o[i + 1][2], o[i + 1][3], lop3_and_or(lo8, 0x000f000fu, kMagic), lop3_and_or(lo8, 0x00f000f0u, kMagic),
+                         lop3_and_or(hi8, 0x000f000fu, kMagic), lop3_and_or(hi8, 0x00f000f0u, kMagic), bp[c][0], bp[c][1]);
+              } else {
+                const int i = 2 * h + e;  // dims 16 i + 2 g + 0, 1
+                mma_full(o[i][0], o[i][1], o[i][2], o[i][3], __byte_perm(lo, kMagic, 0x7250), __byte_perm(lo, kMagic, 0x7351), __byte_perm(hi, kMagic, 0x7250),
+                         __byte_perm(hi, kMagic, 0x7351), bp[c][0], bp[c][1]);
               }
-            }
-          } else {
-            const uint4 va = *reinterpret_cast<const uint4*>(vbase + g * 16);
-            const uint4 vb = *reinterpret_cast<const uint4*>(vbase + 4 * kRow + g * 16);
-            const uint4 vcw = *reinterpret_cast<const uint4*>(vbase + 8 * kRow + g * 16);
-            const uint4 vd = *reinterpret_cast<const uint4*>(vbase + 12 * kRow + g * 16);
-            const uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
-            const uint32_t wc[4] = {vcw.x, vcw.y, vcw.z, vcw.w}, wd[4] = {vd.x, vd.y, vd.z, vd.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              // dims 16g + 2i (row g) and 16g + 2i + 1 (row g+8): bytes 2i, 2i+1 of the 16-byte row chunk
-              const int w = i >> 1, b0 = 2 * (i & 1), b1 = b0 + 1;
-              const uint32_t sel0 = static_cast<uint32_t>(b0) | (static_cast<uint32_t>(b0) << 4) | (static_cast<uint32_t>(4 + b0) << 8) | (static_cast<uint32_t>(4 + b0) << 12);
-              const uint32_t sel1 = static_cast<uint32_t>(b1) | (static_cast<uint32_t>(b1) << 4) | (static_cast<uint32_t>(4 + b1) << 8) | (static_cast<uint32_t>(4 + b1) << 12);
-              mma_full(o[i][0], o[i][1], o[i][2], o[i][3], lop3_and_or(__byte_perm(wa[w], wb[w], sel0), 0x00ff00ffu, kMagic),
-                       lop3_and_or(__byte_perm(wa[w], wb[w], sel1), 0x00ff00ffu, kMagic), lop3_and_or(__byte_perm(wc[w], wd[w], sel0), 0x00ff00ffu, kMagic),
-                       lop3_and_or(__byte_perm(wc[w], wd[w], sel1), 0x00ff00ffu, kMagic), bp[c][0], bp[c][1]);
             }
           }
         }
@@ -635,10 +639,9 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
       s_l[warp][2 * q4] = l0; s_l[warp][2 * q4 + 1] = l1;
     }
     {
-      // layout [warp][head][(d % 16) * 8 + d / 16] with a head stride of 132 floats: conflict-free for these stores and for the
-      // merge reads below (thread t owns dim 16 (t % 8) + t / 8)
+      // layout [warp][head][(2 i + odd) * 8 + g] with a head stride of 132 floats: conflict-free for these stores and for the merge reads below
       __syncwarp();  // every lane is done with the ring slots this overwrites
-      float* so0 = reinterpret_cast<float*>(my_ring) + (2 * q4) * kOStride + g;  // head 2q4, dims 16g + j at offset 8 j
+      float* so0 = reinterpret_cast<float*>(my_ring) + (2 * q4) * kOStride + g;  // head 2q4
       float* so1 = so0 + kOStride;                                // head 2q4+1
       constexpr float hs = (BITS == 4) ? 0.0625f : 1.f;
       const float b0 = 1024.f * spa[0], b1 = 1024.f * spa[1];
@@ -690,7 +693,8 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
   }
   __syncthreads();
   if (threadIdx.x < kD) {
-    const int d = 16 * (threadIdx.x & 7) + (threadIdx.x >> 3);  // the dim whose partials sit at offset threadIdx.x
+    // the dim whose partials sit at offset threadIdx.x
+    const int t = threadIdx.x, d = BITS == 4 ? 32 * (t >> 5) + 4 * (t & 7) + 2 * ((t >> 4) & 1) + ((t >> 3) & 1) : 16 * (t >> 4) + 2 * (t & 7) + ((t >> 3) & 1);
     float* part = nullptr;
     if (nsplit > 1) part = ws_part + ((static_cast<size_t>(b) * num_heads + h0) * nsplit + split) * (kD + 2);
     const float vd = __half2float(s_v[d]);
