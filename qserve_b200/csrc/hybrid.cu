@@ -1173,7 +1173,7 @@ __global__ void __launch_bounds__(128, TAPS == 4 ? 6 : 0) delta_prepare_walk_ker
                                                                  const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                                                  const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
                                                                  const int* __restrict__ entry_start, const int* __restrict__ entry_slot, int T, int H, int G,
-                                                                 int D, int Dv, int taps, float unit_eps, int run) {
+                                                                 int D, int Dv, int taps, float unit_eps, int run, int shift) {
   const int C = 2 * G * D + H * Dv, P = C + 2 * H;
   const int u = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
@@ -1185,7 +1185,7 @@ __global__ void __launch_bounds__(128, TAPS == 4 ? 6 : 0) delta_prepare_walk_ker
     auto walk = conv_walk<ST, 4, TAPS>(conv_w, nullptr, nullptr, taps, c);
     const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, C, taps};
     const float q_scale = 1.f / sqrtf((float)D);
-    conv_rows<ST, 4>(walk, proj, stride, nullptr, tab, t0, t1, c, false, [&](int t, float(&y)[4]) {
+    conv_rows<ST, 4>(walk, proj, stride, nullptr, tab, t0, t1, c, shift != 0 && in, [&](int t, float(&y)[4]) {
 #pragma unroll
       for (int v = 0; v < 4; ++v) y[v] = silu_f(y[v]);
       float r = 1.f;
@@ -1529,17 +1529,21 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
                  int H, int G, int D, int Dv, int taps, float unit_eps, float eps, cudaStream_t s) {
   const int C = 2 * G * D + H * Dv;
   auto al = [](const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+  // a step of single tokens: a lane of the walk is the only reader of its channels' state and shifts the token's input in (64 sequences, 16 heads of 128: 41.7 us
+  // with a launch of its own for that, 36.9 so; 8 sequences 14.4 and 10.9, 256 127 and 119)
+  bool shift = false;
   if (D % 4 == 0 && D <= 128 && Dv % 4 == 0 && Dv <= 128 && stride % 4 == 0 && (C + 2 * H) % 4 == 0 && al(proj, 4 * sizeof(ST)) && al(prep, 16)) {
     const int run = conv_run(T);
+    shift = T == E && taps > 1;
     auto walk = taps == 4 ? delta_prepare_walk_kernel<ST, 4> : taps == 3 ? delta_prepare_walk_kernel<ST, 3> : taps == 2 ? delta_prepare_walk_kernel<ST, 2>
                                                                                                          : delta_prepare_walk_kernel<ST, 0>;
     walk<<<dim3((T + run - 1) / run, (2 * G + H + 3) / 4), 128, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry, tok_pos,
-                                                                        entry_start, entry_slot, T, H, G, D, Dv, taps, unit_eps, run);
+                                                                        entry_start, entry_slot, T, H, G, D, Dv, taps, unit_eps, run, shift);
   } else {
     delta_prepare_kernel<ST><<<dim3(T, 2 * G + H), kPrepThreads, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry,
                                                                         tok_pos, entry_start, entry_slot, H, G, D, Dv, taps, unit_eps);
   }
-  if (taps > 1)
+  if (taps > 1 && !shift)
     delta_conv_state_kernel<ST><<<dim3((C + 127) / 128, E), 128, 0, s>>>(conv_state, (const ST*)proj, stride, entry_start, entry_len, entry_slot,
                                                                           entry_pos0, C, taps);
   // 16-byte staging needs every q / k / v run of a prepared row on a 16-byte boundary
