@@ -1244,7 +1244,7 @@ int launch_gemm(const GemmArgs& a) {
   cfg.blockDim = dim3(kNumThreads);
   auto resident = [&](int split) {
     // (W8A8's 32-token tiles: two CTAs per SM, whatever the query says, which counts one: 16 tiles 5.6 us by 8 and 6.5 by 4)
-    if (C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return sms / split;
+    if (MODE == kModeW8 && C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return sms / split;
     static std::atomic<int> held[2][kMaxDevices][4] = {};  // per (instantiation, device, split), as the attribute above; 0: not asked yet
     std::atomic<int>& h = held[a.acc_out ? 1 : 0][dev][split == 2 ? 1 : split == 4 ? 2 : 3];
     int n = h.load(std::memory_order_relaxed);
@@ -1418,16 +1418,45 @@ int dispatch_gemm(const GemmArgs& a) {
     // 1796 TOP/s, M = 4096: 2388 vs 2100): a tile's setup, pipeline fill and epilogue hide behind the sibling's main loop
     nt = a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
   }
-  if (nt == 32) return launch_gemm<MODE, 32, (grp || w8 ? 4 : 5), 4>(a);
-  if (nt == 64) return launch_gemm<MODE, 64, (w8 ? 4 : grp ? 3 : 4), (w8 ? 4 : 3)>(a);
+  // Calls that split K (tiles of half the SMs and fewer) run one CTA per SM beside the receive buffer, so their rings may as well have the rest of the shared
+  // memory where stages are bytes rather than latencies.  us, rings as below / as here: W8A8 4096 x 14336 at 16 tokens 15.2 / 12.9, at 64 15.6 / 13.9, at 128 17.2 /
+  // 15.6, 6144 x 4096 9.3 / 8.0, 9.8 / 8.6, 11.6 / 10.7; decoder layers with attention and the row kernels 82.8 / 76.3, 94.2 / 89.8, 125.5 / 123.9.  W4A8 at 128 tokens 4096 x
+  // 14336 per channel 14.2 / 12.3, group scales 16.7 / 15.0; layers of 100 tokens 104.9 / 101.4 and 112.2 / 109.2.  W4A8 up to 64 tokens keeps its small rings: more
+  // weights on their way 4096 x 14336 10.24 / 10.66, a fourth activation stage 6144 x 4096 6.97 / 6.86, but beside 160 KB one CTA of the attention after it fits an SM
+  // early instead of two: a layer of 64 tokens 78.6 / 79.7.
+  const int sms = num_sms(), split_tiles = (a.N / kBM) * ((a.M + nt - 1) / nt);
+  const bool alone = a.force_split != 1 && 2 * split_tiles <= sms;
+  if (nt == 32) {
+    if constexpr (w8) {
+      // (16 to 18 tiles are more clusters of 8 than the device holds where one CTA takes an SM; by 8 beside one another, long K is faster: x 8192 6.8 and 7.2)
+      const bool eighths = split_tiles > 15 && 8 * split_tiles <= sms && a.K >= 6144;
+      if (alone && !eighths) return launch_gemm<MODE, 32, 8, 6>(a);
+    }
+    if constexpr (!grp && !w8) {
+      // a split by four (what choose_split takes for these tiles: 33 clusters of 4 are resident) of up to 16 stages: four hold a CTA's share, and the next call's
+      // CTAs fit beside these: 4096 x 4096 at 16 tokens 5.7 / 5.2
+      const bool quarters = 4 * split_tiles >= 2 * sms / 3 && 4 * split_tiles <= 132;
+      if (quarters && a.force_split == 0 && a.K > 8 * kSub * kBK && a.K <= 16 * kSub * kBK) return launch_gemm<MODE, 32, 4, 4>(a);
+    }
+    return launch_gemm<MODE, 32, (grp || w8 ? 4 : 5), 4>(a);
+  }
+  if (nt == 64) {
+    if constexpr (w8) {
+      if (alone) return launch_gemm<MODE, 64, 8, 6>(a);
+    }
+    return launch_gemm<MODE, 64, (w8 ? 4 : grp ? 3 : 4), (w8 ? 4 : 3)>(a);
+  }
+  if constexpr (!w8) {
+    if (alone) return launch_gemm<MODE, 128, 4, (grp ? 2 : 3)>(a);
+  }
   if constexpr (w8) {
     // W8A8 at 65..128 tokens: layers that want a split run one CTA per SM beside the receive buffer and take a deeper activation ring
     const int tiles = (a.N / kBM) * ((a.M + 127) / 128);
-    if (a.force_split != 1 && tiles * 2 <= num_sms()) return launch_gemm<MODE, 128, 4, 4>(a);
+    if (a.force_split != 1 && tiles * 2 <= num_sms()) return launch_gemm<MODE, 128, 6, 4>(a);
     // One CTA per SM at most: it may as well have all of the shared memory.  With long K also where two per SM leave the second half of a last round empty (an odd
     // number of 128-channel tiles, which pairs do not take; us, two per SM / one): 22144 x 8576 at 162 tokens, 346 tiles, 74.0 / 69.6, 12416 x 8576 at 500 77.1 /
     // 69.9; at 4096 K the second CTA's set-up under the first one's products is worth more, 22144 at 162 37.5 / 39.5
-    const int sms = num_sms(), one = (tiles + sms - 1) / sms, two = (tiles + 2 * sms - 1) / (2 * sms);
+    const int one = (tiles + sms - 1) / sms, two = (tiles + 2 * sms - 1) / (2 * sms);
     if (tiles <= sms || (a.K >= 6144 && one < 2 * two)) return launch_gemm<MODE, 128, 8, 4>(a);
   }
   return launch_gemm<MODE, 128, (w8 ? 4 : 2), 2>(a);
