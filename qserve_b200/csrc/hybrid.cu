@@ -886,11 +886,12 @@ __global__ void __launch_bounds__(128) group_attention_kernel(
 // tile; map m's scores are taken from the products with its own keys).  A warp has its 16 keys of every 64-key tile to itself: a buffer for their keys and
 // one for their values, each refilled as soon as the warp is done with it and waited for when it is needed, without a block barrier.  The output's products have
 // the values as their first operand and the weights' rows as columns of the second (they lie in registers as they should): no half of a tile is empty, half the
-// products and accumulators, and four blocks per SM instead of three.
+// products and accumulators.  BLOCKS per SM: three have all of their registers; four spill some, and are for calls that they hold at once or nearly so: 64 tokens of 512
+// to 1024 positions, two maps of 4 heads, 512 blocks: 47.9 and 45.9 us; 200 tokens of up to 700 70.0 and 76.9.
 // Per head the arithmetic and its order are those of the kernel above: the same bits.
-// 64 tokens of 512 to 1024 positions, 4 kv heads, 2 maps (151 MB, 23 us): 75 us, now 44.
-template <int MAPS>
-__global__ void __launch_bounds__(128, 4) ring_attention_kernel(
+// 64 tokens of 512 to 1024 positions, 4 kv heads, 2 maps (151 MB, 23 us), with the merge: 50 us with the weights as first operand, now 46.
+template <int MAPS, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) ring_attention_kernel(
     float* __restrict__ part, const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ kpool,
     const __nv_bfloat16* __restrict__ vpool, const int* __restrict__ tok_list, const int* __restrict__ tok_slot, const int* __restrict__ tok_pos,
     const int* __restrict__ block_table, int max_blocks, int H, int G, float scale, int page, int shares, int chunk, int window, int keep,
@@ -1534,11 +1535,13 @@ int launch_group(void* out, long long out_stride, float* part, const void* q, lo
     ring = D == 128 && maps * (H / G) <= 8 && page % 16 == 0 && (maps == 1 || ex.softcap == 0.f);
     if (ring) {
       const size_t smem = (size_t)4 * (maps + 1) * 16 * (128 + kPad) * sizeof(__nv_bfloat16);
-      auto kern = maps == 2 ? ring_attention_kernel<2> : ring_attention_kernel<1>;
-      static bool attr_set[2][kMaxDevices] = {};
-      if (smem > 48 * 1024 && !attr_set[maps - 1][device_ordinal()]) {
+      const int sms = num_sms(), blocks = n_list * G * shares;
+      const bool four = blocks > 3 * sms && 2 * blocks <= 9 * sms;
+      auto kern = maps == 2 ? (four ? ring_attention_kernel<2, 4> : ring_attention_kernel<2, 3>) : four ? ring_attention_kernel<1, 4> : ring_attention_kernel<1, 3>;
+      static bool attr_set[2][2][kMaxDevices] = {};
+      if (smem > 48 * 1024 && !attr_set[four ? 1 : 0][maps - 1][device_ordinal()]) {
         if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "ring attention smem")) return rc;
-        attr_set[maps - 1][device_ordinal()] = true;
+        attr_set[four ? 1 : 0][maps - 1][device_ordinal()] = true;
       }
       kern<<<dim3(n_list, G, shares), 128, smem, s>>>(part, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kpool, (const __nv_bfloat16*)vpool, tok_list,
                                                       tok_slot, tok_pos, block_table, max_blocks, H, G, scale, page, shares, chunk, window, ex.keep_first,
