@@ -27,6 +27,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "../../include/qserve_b200.h"
 #include "common.cuh"
@@ -43,7 +44,12 @@ constexpr int kVec = kParts * kSeg;                      // floats of a staged r
 constexpr int kThreads = 128, kSms = 148;  // (the device deals the units by kSms as well: a B200's)
 
 constexpr int scan_vectors(int mode) { return mode == kScanChannelDecay ? 3 : 2; }
-constexpr int scan_chunk(int mode) { return mode == kScanChannelDecay ? 8 : 12; }  // tokens of a staged chunk: two chunks stay below 40 KB
+// Tokens of a staged chunk, two of which are in shared memory.  A chunk costs its barrier, the wait for its copies and the first token's reads: 6 % of the time where
+// two blocks share an SM, 20 % where a block is alone.  us of the layer with 12 / 16 / 24 tokens: state space, 4 x 2048 tokens, 64 heads (4 columns a thread) 691 / 681 /
+// 690, 32 heads (2) 417 / 403 / 409, 1 x 2048, 64 heads (1) 341 / 347 / 337; delta rule, 8 heads (1) 393 / 391 / 385, 16 heads (2) 559 / 562 / 577, retention (2) 438 / 447 / 463.
+constexpr int scan_chunk(int mode, int cpt) {
+  return mode == kScanChannelDecay ? 8 : mode == kScanTokenDecay ? (cpt == 1 ? 24 : 16) : mode == kScanDelta && cpt == 1 ? 24 : 12;
+}
 constexpr bool scan_numbers(int mode) { return mode == kScanTokenDecay || mode == kScanDelta; }
 constexpr int scan_token_floats(int mode, int cpt) { return scan_vectors(mode) * kVec + 16 * cpt + 4; }
 
@@ -117,7 +123,7 @@ __device__ __forceinline__ void scan_unit(const ScanArgs& p, int lane, int cols,
 // cp.async into a double buffer: q | g [| a] in padded segments, v of the block's columns, the head's two numbers.
 template <int MODE, int CPT>
 __global__ void __launch_bounds__(kThreads, CPT == 1 ? 2 : 0) column_scan_kernel(const ScanArgs p) {
-  constexpr int NV = scan_vectors(MODE), CH = scan_chunk(MODE), COLS = 16 * CPT, ROW = scan_token_floats(MODE, CPT), VAL = NV * kVec, NUM = VAL + COLS;
+  constexpr int NV = scan_vectors(MODE), CH = scan_chunk(MODE, CPT), COLS = 16 * CPT, ROW = scan_token_floats(MODE, CPT), VAL = NV * kVec, NUM = VAL + COLS;
   constexpr bool DELTA = MODE == kScanDelta, TOKEN = MODE == kScanTokenDecay;
   extern __shared__ __align__(16) float sm[];  // [2][CH][ROW]
   const int tid = threadIdx.x, lane = tid & 31, part = lane >> 2;
@@ -410,8 +416,16 @@ __global__ void __launch_bounds__(kThreads, CPT == 1 ? 2 : 0) column_scan_kernel
 
 template <int MODE, int CPT>
 int launch(const ScanArgs& p, cudaStream_t s) {
-  constexpr size_t smem = (size_t)2 * scan_chunk(MODE) * scan_token_floats(MODE, CPT) * sizeof(float);
-  static_assert(smem <= 48 * 1024, "staging fits the default limit");
+  constexpr size_t smem = (size_t)2 * scan_chunk(MODE, CPT) * scan_token_floats(MODE, CPT) * sizeof(float);
+  static_assert(smem <= 68 * 1024, "three blocks per SM");
+  if constexpr (smem > 48 * 1024) {
+    static std::atomic<bool> done[kMaxDevices] = {};  // the attribute is a device's own
+    std::atomic<bool>& d = done[device_ordinal()];
+    if (!d.load(std::memory_order_relaxed)) {
+      if (int rc = check_cuda(cudaFuncSetAttribute(column_scan_kernel<MODE, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "column scan smem")) return rc;
+      d.store(true, std::memory_order_relaxed);
+    }
+  }
   column_scan_kernel<MODE, CPT><<<p.E * p.H * ((p.Dv + 16 * CPT - 1) / (16 * CPT)), kThreads, smem, s>>>(p);
   return check_cuda(cudaGetLastError(), "hyb column scan");
 }
@@ -420,7 +434,7 @@ template <int MODE>
 int launch_mode(const ScanArgs& p, cudaStream_t s) {
   auto blocks = [&](int cpt) { return (long long)p.E * p.H * ((p.Dv + 16 * cpt - 1) / (16 * cpt)); };
   // The narrowest blocks of which each SM holds two.  A step costs a warp about 140 cycles and 110 more per column of a thread: few units want short
-  // steps, many want few instructions per element.  us of the whole layer with 1 / 2 / 4 columns, width 2048 unless said: delta rule, 1 x 2048 tokens of
+  // steps, many want few instructions per element.  us of the whole layer with 1 / 2 / 4 columns (chunks of 12 tokens), width 2048 unless said: delta rule, 1 x 2048 tokens of
   // width 1024: 355 / 439 / 648, 2 x 1000: 280 / 292 / 396, 4 x 2048: 869 / 771 / 878, 8 x 1000: 838 / 703 / 654; state space, 1 x 2048 of width 1024:
   // 290 / 339 / 502, 2 x 1000: 372 / 312 / 357, 4 x 2048: 1180 / 1105 / 1035.  The delta rule's single tokens take the same rule; the kernel before this one
   // and this one, 16 heads of 128 x 128: 8 tokens 17.1 / 13.7, 64 61.8 / 42.0, 256 210 / 126 (no other width has been measured for them).
