@@ -1432,12 +1432,6 @@ int dispatch_gemm(const GemmArgs& a) {
       const bool eighths = split_tiles > 15 && 8 * split_tiles <= sms && a.K >= 6144;
       if (alone && !eighths) return launch_gemm<MODE, 32, 8, 6>(a);
     }
-    if constexpr (!grp && !w8) {
-      // a split by four (what choose_split takes for these tiles: 33 clusters of 4 are resident) of up to 16 stages: four hold a CTA's share, and the next call's
-      // CTAs fit beside these: 4096 x 4096 at 16 tokens 5.7 / 5.2
-      const bool quarters = 4 * split_tiles >= 2 * sms / 3 && 4 * split_tiles <= 132;
-      if (quarters && a.force_split == 0 && a.K > 8 * kSub * kBK && a.K <= 16 * kSub * kBK) return launch_gemm<MODE, 32, 4, 4>(a);
-    }
     return launch_gemm<MODE, 32, (grp || w8 ? 4 : 5), 4>(a);
   }
   if (nt == 64) {
