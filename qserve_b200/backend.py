@@ -122,7 +122,7 @@ def apply_bias_rope_update_kv_cache(qkv, seq_lens, padding_offset, kv_pointers: 
     if kv_pointers is not None:
         _require(kv_pointers.is_contiguous() and kv_pointers.dtype == torch.int64, "kv_pointers must be contiguous int64")
         kvp, max_blocks = kv_pointers.data_ptr(), kv_pointers.size(-1)
-    _call(qkv, lib.qs_apply_bias_rope_update_kv_cache, qkv.data_ptr(), seq_lens.data_ptr(), padding_offset.data_ptr(), kvp, seq_lens.size(0), qkv.size(0),
+    _call(qkv, _bind.qs_apply_bias_rope_update_kv_cache, qkv.data_ptr(), seq_lens.data_ptr(), padding_offset.data_ptr(), kvp, seq_lens.size(0), qkv.size(0),
                                                  max_blocks, int(head_num), int(kv_head_num), head_dim, int(seq_len), int(tokens_per_block),
                                                  int(size_per_token), int(rotary_embedding_dim), float(rotary_embedding_base),
                                                  int(rotary_embedding_max_positions), int(bool(neox_rotary_style)), int(bool(int4_kv_cache)),
@@ -134,7 +134,7 @@ def compute_padding_offsets(cu_seqlens, max_seqlen: int, tot_num_tokens: int) ->
     _cuda(cu_seqlens, "cu_seqlens")
     _require(cu_seqlens.dtype == torch.int32, "cu_seqlens must be int32")
     out = torch.empty((tot_num_tokens,), dtype=torch.int32, device=cu_seqlens.device)
-    _call(cu_seqlens, lib.qs_compute_padding_offsets, out.data_ptr(), cu_seqlens.data_ptr(), cu_seqlens.size(0) - 1, int(max_seqlen))
+    _call(cu_seqlens, _bind.qs_compute_padding_offsets, out.data_ptr(), cu_seqlens.data_ptr(), cu_seqlens.size(0) - 1, int(max_seqlen))
     return out
 
 
@@ -160,7 +160,7 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: in
     if T == 0:
         return out
     scale = float(softmax_scale) if softmax_scale is not None else 128 ** -0.5
-    _call(q, lib.qs_prefill_attention, q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), out.data_ptr(), out.stride(0),
+    _call(q, _bind.qs_prefill_attention, q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), out.data_ptr(), out.stride(0),
           cu_seqlens_q.data_ptr(), cu_seqlens_q.size(0) - 1, T, int(max_seqlen_q), hq, hkv, 128, scale)
     return out
 

@@ -18,6 +18,8 @@
 
 #include <stdexcept>
 #include <string>
+#include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/qserve_b200.h"
@@ -346,6 +348,52 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   return nullptr;
 }
+
+// ---- functions of the C ABI as they are declared: conversions in the order and of the types of the declaration (pointers: an address or None; numbers as
+//      ctypes takes them), then the call without the interpreter lock; returns its status.  The attention and state functions of the hybrid decoders have
+//      25 to 40 arguments, a layer of short prompts five such calls: 79 us through ctypes, 69 here; a prompt's attention block 56 and 50 ----
+template <typename T>
+T converted(PyObject* o) {
+  if constexpr (std::is_pointer_v<T>) {
+    if (o == Py_None) return nullptr;
+    if (PyLong_Check(o)) {
+      void* const p = PyLong_AsVoidPtr(o);
+      if (p == nullptr && PyErr_Occurred()) throw python_error();
+      return static_cast<T>(p);
+    }
+  } else if constexpr (std::is_floating_point_v<T>) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    return static_cast<T>(v);
+  } else {
+    static_assert(std::is_integral_v<T>);
+    if (PyLong_Check(o)) return static_cast<T>(PyLong_AsUnsignedLongLongMask(o));
+  }
+  PyErr_Format(PyExc_TypeError, "%s expected, not %s", std::is_pointer_v<T> ? "an address or None" : "an integer", Py_TYPE(o)->tp_name);
+  throw python_error();
+}
+template <auto Fn>
+struct Abi;
+template <typename... A, int (*Fn)(A...)>
+struct Abi<Fn> {
+  static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != static_cast<Py_ssize_t>(sizeof...(A))) {
+      PyErr_Format(PyExc_TypeError, "expected %zu arguments, got %zd", sizeof...(A), n);
+      return nullptr;
+    }
+    try {
+      Py_ssize_t i = 0;
+      const std::tuple<A...> a{converted<A>(args[i++])...};  // in order: a braced list
+      int rc;
+      Py_BEGIN_ALLOW_THREADS rc = std::apply(Fn, a);
+      Py_END_ALLOW_THREADS return PyLong_FromLong(rc);
+    } catch (...) {
+      torch::translate_exception_to_python(std::current_exception());
+    }
+    return nullptr;
+  }
+};
+#define QS_ABI(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&Abi<&name>::call)), METH_FASTCALL, nullptr}
 #define QS_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {QS_ENTRY(w4a8_per_chn, 8),
                          QS_ENTRY(w4a8_per_group, 8),
@@ -361,6 +409,43 @@ PyMethodDef methods[] = {QS_ENTRY(w4a8_per_chn, 8),
                          QS_ENTRY(add_rms_norm_general, 8),
                          QS_ENTRY(gemm_workspace, 1),
                          QS_ENTRY(attention_workspace, 4),
+                         QS_ABI(qs_apply_bias_rope_update_kv_cache),
+                         QS_ABI(qs_compute_padding_offsets),
+                         QS_ABI(qs_prefill_attention),
+                         QS_ABI(qs_hyb_attention),
+                         QS_ABI(qs_hyb_attention_fast),
+                         QS_ABI(qs_hyb_bias_gated_act),
+                         QS_ABI(qs_hyb_bias_gelu_tanh),
+                         QS_ABI(qs_hyb_branch_norm_mean),
+                         QS_ABI(qs_hyb_cast_rows),
+                         QS_ABI(qs_hyb_embed),
+                         QS_ABI(qs_hyb_gate_recurrence),
+                         QS_ABI(qs_hyb_gated_delta),
+                         QS_ABI(qs_hyb_gated_linear),
+                         QS_ABI(qs_hyb_gated_norm_update),
+                         QS_ABI(qs_hyb_gelu_tanh_mul),
+                         QS_ABI(qs_hyb_latent_attention),
+                         QS_ABI(qs_hyb_latent_attention_fast),
+                         QS_ABI(qs_hyb_latent_gate_out),
+                         QS_ABI(qs_hyb_latent_prepare),
+                         QS_ABI(qs_hyb_latent_query),
+                         QS_ABI(qs_hyb_lru_conv),
+                         QS_ABI(qs_hyb_lru_scan),
+                         QS_ABI(qs_hyb_moe_act),
+                         QS_ABI(qs_hyb_moe_combine),
+                         QS_ABI(qs_hyb_moe_gather),
+                         QS_ABI(qs_hyb_moe_plan),
+                         QS_ABI(qs_hyb_moe_router),
+                         QS_ABI(qs_hyb_post_norm_update),
+                         QS_ABI(qs_hyb_qk_prepare_append),
+                         QS_ABI(qs_hyb_qk_row_norm_append),
+                         QS_ABI(qs_hyb_retention),
+                         QS_ABI(qs_hyb_rms_norm),
+                         QS_ABI(qs_hyb_rope_append),
+                         QS_ABI(qs_hyb_softcap),
+                         QS_ABI(qs_hyb_state_space),
+                         QS_ABI(qs_hyb_stream_norm),
+                         QS_ABI(qs_hyb_stream_update_norm),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_bind", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

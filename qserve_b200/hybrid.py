@@ -24,6 +24,7 @@ import torch
 import ctypes
 
 from ._lib import AttnExtra, check, lib
+from . import _bind  # after the library it links against
 from .cache import HybridCache
 from .modelcfg import (AttentionMixerConfig, DeltaMixerConfig, GatedLinearMixerConfig, GatedUnitMixerConfig, GateRecurrenceMixerConfig,
                        HybridConfig, LatentAttentionMixerConfig, MlpConfig, MoeConfig, ParallelMixerConfig, RetentionMixerConfig,
@@ -303,36 +304,37 @@ class MultiMapAttentionMixer(_Mixer):
         extra = None
         if self.extra:
             gate = proj.data_ptr() + self.col_g * proj.element_size() if self.gated else None
-            extra = ctypes.byref(AttnExtra(m.keep_first, _p(self.slopes), gate, proj.stride(0), 1 if m.gate_wide else 0, m.softcap))
+            options = AttnExtra(m.keep_first, _p(self.slopes), gate, proj.stride(0), 1 if m.gate_wide else 0, m.softcap)  # lives until the call returns
+            extra = ctypes.addressof(options)
         if m.row_norm:
-            check(lib.qs_hyb_qk_row_norm_append(proj.data_ptr(), proj.stride(0), _p(self.bias), self.q_gain.data_ptr(), self.k_gain.data_ptr(), m.temp_coef,
-                                                m.temp_every, _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
-                                                run_cache["k"].data_ptr(), run_cache["v"].data_ptr(), self.eps, b.n_tokens, m.heads * m.dim,
-                                                m.kv_heads * m.dim, m.kv_heads * m.vdim, page_size, dt, stream))
+            check(_bind.qs_hyb_qk_row_norm_append(proj.data_ptr(), proj.stride(0), _p(self.bias), self.q_gain.data_ptr(), self.k_gain.data_ptr(), m.temp_coef,
+                                                  m.temp_every, _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
+                                                  run_cache["k"].data_ptr(), run_cache["v"].data_ptr(), self.eps, b.n_tokens, m.heads * m.dim,
+                                                  m.kv_heads * m.dim, m.kv_heads * m.vdim, page_size, dt, stream))
         elif self.general:
-            check(lib.qs_hyb_qk_prepare_append(proj.data_ptr(), proj.stride(0), _p(self.bias), _p(self.temp), _p(b.tok_slot), _p(b.tok_pos),
-                                               _p(b.block_table), b.block_table.shape[1], run_cache["k"].data_ptr(), run_cache["v"].data_ptr(),
-                                               _p(self.inv_freq), 1 if m.rot is not None and m.rot.layout == "half" else 0,
-                                               m.rot.dims if m.rot is not None else 0, 1 if m.qk_norm else 0, self.eps, b.n_tokens, m.heads,
-                                               m.kv_heads, m.dim, m.vdim, page_size, _p(self.q_gain), _p(self.k_gain), 1 if m.tied_values else 0,
-                                               1 if m.value_norm else 0, dt, stream))
+            check(_bind.qs_hyb_qk_prepare_append(proj.data_ptr(), proj.stride(0), _p(self.bias), _p(self.temp), _p(b.tok_slot), _p(b.tok_pos),
+                                                 _p(b.block_table), b.block_table.shape[1], run_cache["k"].data_ptr(), run_cache["v"].data_ptr(),
+                                                 _p(self.inv_freq), 1 if m.rot is not None and m.rot.layout == "half" else 0,
+                                                 m.rot.dims if m.rot is not None else 0, 1 if m.qk_norm else 0, self.eps, b.n_tokens, m.heads,
+                                                 m.kv_heads, m.dim, m.vdim, page_size, _p(self.q_gain), _p(self.k_gain), 1 if m.tied_values else 0,
+                                                 1 if m.value_norm else 0, dt, stream))
         else:
-            check(lib.qs_hyb_rope_append(proj.data_ptr(), proj.stride(0), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
-                                         run_cache["k"].data_ptr(), run_cache["v"].data_ptr(), self.inv_freq.data_ptr(), self.amp, b.n_tokens,
-                                         m.heads, m.kv_heads, m.maps, m.dim, m.vdim, m.rot.dims, page_size, dt, stream))
+            check(_bind.qs_hyb_rope_append(proj.data_ptr(), proj.stride(0), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
+                                           run_cache["k"].data_ptr(), run_cache["v"].data_ptr(), self.inv_freq.data_ptr(), self.amp, b.n_tokens,
+                                           m.heads, m.kv_heads, m.maps, m.dim, m.vdim, m.rot.dims, page_size, dt, stream))
         if fast:
             # prompt portions as 64-row tiles on the tensor cores, single tokens and short portions with a head group as the tile's rows
-            check(lib.qs_hyb_attention_fast(out.data_ptr(), out.stride(0), proj.data_ptr(), proj.stride(0), run_cache["k"].data_ptr(),
-                                            run_cache["v"].data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
-                                            _p(b.seen_entry), _p(b.seen_row0), b.n_tiles, _p(b.long_tokens), b.n_long, _p(b.short_tokens), b.n_short,
-                                            _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), scratch.data_ptr(), m.heads,
-                                            m.kv_heads, m.maps, m.dim, m.vdim, m.scale, self.lam, self.out_scale, self.eps,
-                                            1 if m.head_norm else 0, page_size, m.chunk, m.window, _p(self.sinks), extra, dt, stream))
+            check(_bind.qs_hyb_attention_fast(out.data_ptr(), out.stride(0), proj.data_ptr(), proj.stride(0), run_cache["k"].data_ptr(),
+                                              run_cache["v"].data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
+                                              _p(b.seen_entry), _p(b.seen_row0), b.n_tiles, _p(b.long_tokens), b.n_long, _p(b.short_tokens), b.n_short,
+                                              _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), scratch.data_ptr(), m.heads,
+                                              m.kv_heads, m.maps, m.dim, m.vdim, m.scale, self.lam, self.out_scale, self.eps,
+                                              1 if m.head_norm else 0, page_size, m.chunk, m.window, _p(self.sinks), extra, dt, stream))
             return
-        check(lib.qs_hyb_attention(out.data_ptr(), out.stride(0), proj.data_ptr(), proj.stride(0), run_cache["k"].data_ptr(),
-                                   run_cache["v"].data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
-                                   b.n_tokens, m.heads, m.kv_heads, m.maps, m.dim, m.vdim, m.scale, self.lam, self.out_scale, self.eps,
-                                   1 if m.head_norm else 0, page_size, m.chunk, m.window, _p(self.sinks), extra, dt, stream))
+        check(_bind.qs_hyb_attention(out.data_ptr(), out.stride(0), proj.data_ptr(), proj.stride(0), run_cache["k"].data_ptr(),
+                                     run_cache["v"].data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table), b.block_table.shape[1],
+                                     b.n_tokens, m.heads, m.kv_heads, m.maps, m.dim, m.vdim, m.scale, self.lam, self.out_scale, self.eps,
+                                     1 if m.head_norm else 0, page_size, m.chunk, m.window, _p(self.sinks), extra, dt, stream))
 
 
 ATTENTION_IMPL = None  # tests: "plain" keeps the attention on the CUDA-core kernel
@@ -366,11 +368,11 @@ class GatedDeltaMixer(_Mixer):
         m, T = self.m, b.n_tokens
         prep = scratch[: T * self.prep_width]
         o_raw = scratch[T * self.prep_width: T * (self.prep_width + self.out_features)]
-        check(lib.qs_hyb_gated_delta(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
-                                     self.conv_w.data_ptr(), run_cache["conv"].data_ptr(), run_cache["state"].data_ptr(), self.a_log.data_ptr(),
-                                     self.dt_bias.data_ptr(), self.norm_w.data_ptr(), _p(b.tok_entry), _p(b.tok_pos), _p(b.entry_start),
-                                     _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.kv_heads, m.dim, m.vdim,
-                                     m.conv, m.unit_eps, self.eps, dt, stream))
+        check(_bind.qs_hyb_gated_delta(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
+                                       self.conv_w.data_ptr(), run_cache["conv"].data_ptr(), run_cache["state"].data_ptr(), self.a_log.data_ptr(),
+                                       self.dt_bias.data_ptr(), self.norm_w.data_ptr(), _p(b.tok_entry), _p(b.tok_pos), _p(b.entry_start),
+                                       _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.kv_heads, m.dim, m.vdim,
+                                       m.conv, m.unit_eps, self.eps, dt, stream))
 
 
 class GateRecurrenceMixer(_Mixer):
@@ -398,10 +400,10 @@ class GateRecurrenceMixer(_Mixer):
         m, T = self.m, b.n_tokens
         prep = scratch[: T * self.in_features]
         o_raw = scratch[T * self.in_features: T * (self.in_features + self.out_features)]
-        check(lib.qs_hyb_gate_recurrence(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
-                                         self.f_bias.data_ptr(), self.lower.data_ptr(), self.norm_w.data_ptr(), run_cache["state"].data_ptr(),
-                                         _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim,
-                                         m.vdim, self.eps, dt, stream))
+        check(_bind.qs_hyb_gate_recurrence(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
+                                           self.f_bias.data_ptr(), self.lower.data_ptr(), self.norm_w.data_ptr(), run_cache["state"].data_ptr(),
+                                           _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim,
+                                           m.vdim, self.eps, dt, stream))
 
 
 class RetentionMixer(_Mixer):
@@ -431,10 +433,10 @@ class RetentionMixer(_Mixer):
         m, T = self.m, b.n_tokens
         prep = scratch[: T * self.prep_width]
         o_raw = scratch[T * self.prep_width: T * (self.prep_width + self.out_features)]
-        check(lib.qs_hyb_retention(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
-                                   self.decay.data_ptr(), _p(self.inv_freq), m.rot.dims if m.rot is not None else 0, float(m.dim) ** -0.5,
-                                   1 if m.gated else 0, run_cache["state"].data_ptr(), _p(b.tok_pos), _p(b.entry_start), _p(b.entry_len),
-                                   _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim, m.vdim, self.eps, dt, stream))
+        check(_bind.qs_hyb_retention(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
+                                     self.decay.data_ptr(), _p(self.inv_freq), m.rot.dims if m.rot is not None else 0, float(m.dim) ** -0.5,
+                                     1 if m.gated else 0, run_cache["state"].data_ptr(), _p(b.tok_pos), _p(b.entry_start), _p(b.entry_len),
+                                     _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim, m.vdim, self.eps, dt, stream))
 
 
 class GatedLinearMixer(_Mixer):
@@ -471,9 +473,9 @@ class GatedLinearMixer(_Mixer):
         prep = scratch[: T * self.prep_width]
         o_raw = scratch[T * self.prep_width: T * (self.prep_width + self.out_features)]
         z = _mm_f32(proj[:, self.col_a:], self.w_a2.t())  # decay logits [T, heads * dim], fp32 from here on
-        check(lib.qs_hyb_gated_linear(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0), z.data_ptr(),
-                                      self.a_bias.data_ptr(), m.tau, self.norm_w.data_ptr(), run_cache["state"].data_ptr(), _p(b.entry_start),
-                                      _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim, m.vdim, self.eps, dt, stream))
+        check(_bind.qs_hyb_gated_linear(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0), z.data_ptr(),
+                                        self.a_bias.data_ptr(), m.tau, self.norm_w.data_ptr(), run_cache["state"].data_ptr(), _p(b.entry_start),
+                                        _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0), T, b.n_entries, m.heads, m.dim, m.vdim, self.eps, dt, stream))
 
 
 class LatentAttentionMixer(_Mixer):
@@ -534,9 +536,9 @@ class LatentAttentionMixer(_Mixer):
         H, D, R, Dv, K, Q = m.heads, m.dim, m.rot_dim, m.vdim, m.kv_rank, m.q_rank
         pool = run_cache["c"]
         cq = torch.empty((T, Q), dtype=proj.dtype, device=dev) if Q else None
-        check(lib.qs_hyb_latent_prepare(_p(cq), proj.data_ptr(), proj.stride(0), self.col_q, self.col_kv, _p(self.gain_q),
-                                        self.gain_kv.data_ptr(), _p(self.inv_freq), self.rot_dims, _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
-                                        b.block_table.shape[1], pool.data_ptr(), T, Q, K, R, page_size, self.eps, self.rot_layout, self.amp, dt, stream))
+        check(_bind.qs_hyb_latent_prepare(_p(cq), proj.data_ptr(), proj.stride(0), self.col_q, self.col_kv, _p(self.gain_q),
+                                          self.gain_kv.data_ptr(), _p(self.inv_freq), self.rot_dims, _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
+                                          b.block_table.shape[1], pool.data_ptr(), T, Q, K, R, page_size, self.eps, self.rot_layout, self.amp, dt, stream))
         q = torch.mm(cq, self.w_uq.t()) if Q else proj[:, :H * (D + R)]          # [T, H (D + R)]
         fast = scratch is not None and LATENT_IMPL != "plain" and lib.qs_hyb_latent_attention_fast_supported(dt, H, K, R) == 1
         # portions of at least StepBatch.TILE_MIN tokens: per-head keys and values (less arithmetic per score than the K + R numbers of a cell);
@@ -548,8 +550,8 @@ class LatentAttentionMixer(_Mixer):
         if latent:
             qlat = torch.bmm(q.unflatten(1, (H, D + R))[:, :, :D].transpose(0, 1), self.w_uk)  # [H, T, K]
             qa = torch.empty((T, H, K + R), dtype=proj.dtype, device=dev)
-        check(lib.qs_hyb_latent_query(_p(qa), qlat.data_ptr() if latent else None, q.data_ptr(), q.stride(0), _p(self.inv_freq), self.rot_dims,
-                                      _p(b.tok_pos), T, H, D, K, R, 1 if per_head else 0, self.rot_layout, self.amp, dt, stream))
+        check(_bind.qs_hyb_latent_query(_p(qa), qlat.data_ptr() if latent else None, q.data_ptr(), q.stride(0), _p(self.inv_freq), self.rot_dims,
+                                        _p(b.tok_pos), T, H, D, K, R, 1 if per_head else 0, self.rot_layout, self.amp, dt, stream))
         if per_head:
             ctx_src, ctx_table = ctx
             cells = pool.index_select(0, ctx_src).view(-1, K + R)
@@ -557,28 +559,28 @@ class LatentAttentionMixer(_Mixer):
             # without single tokens and gates the heads' outputs are already what the output projection reads
             direct = not latent and not m.gate
             otok = out if direct else torch.empty((T, H * Dv), dtype=proj.dtype, device=dev)
-            check(lib.qs_hyb_attention_fast(otok.data_ptr(), otok.stride(0), q.data_ptr(), q.stride(0), keys.data_ptr(), values.data_ptr(), _p(b.tok_slot),
-                                            _p(b.tok_pos), ctx_table.data_ptr(), ctx_table.shape[1], _p(b.seen_entry), _p(b.seen_row0), b.n_tiles,
-                                            _p(b.long_tokens), b.n_long, None, 0, _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0),
-                                            scratch.data_ptr(), H, H, 1, D + R, Dv, m.scale, 0.0, 1.0, self.eps, 0, page_size, m.chunk, m.window,
-                                            _p(self.sinks), None, dt, stream))
+            check(_bind.qs_hyb_attention_fast(otok.data_ptr(), otok.stride(0), q.data_ptr(), q.stride(0), keys.data_ptr(), values.data_ptr(), _p(b.tok_slot),
+                                              _p(b.tok_pos), ctx_table.data_ptr(), ctx_table.shape[1], _p(b.seen_entry), _p(b.seen_row0), b.n_tiles,
+                                              _p(b.long_tokens), b.n_long, None, 0, _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0),
+                                              scratch.data_ptr(), H, H, 1, D + R, Dv, m.scale, 0.0, 1.0, self.eps, 0, page_size, m.chunk, m.window,
+                                              _p(self.sinks), None, dt, stream))
             if direct:
                 return
         if latent:
             olat = torch.empty((H, T, K), dtype=proj.dtype, device=dev)
             if fast:
-                check(lib.qs_hyb_latent_attention_fast(olat.data_ptr(), qa.data_ptr(), pool.data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
-                                                       b.block_table.shape[1], _p(b.tile_entry), _p(b.tile_row0), 0 if per_head else b.n_tiles,
-                                                       _p(b.short_tokens), b.n_short, _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot),
-                                                       _p(b.entry_pos0), T, scratch.data_ptr(), H, K, R, m.scale, page_size, m.chunk, m.window,
-                                                       _p(self.sinks), dt, stream))
+                check(_bind.qs_hyb_latent_attention_fast(olat.data_ptr(), qa.data_ptr(), pool.data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
+                                                         b.block_table.shape[1], _p(b.tile_entry), _p(b.tile_row0), 0 if per_head else b.n_tiles,
+                                                         _p(b.short_tokens), b.n_short, _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot),
+                                                         _p(b.entry_pos0), T, scratch.data_ptr(), H, K, R, m.scale, page_size, m.chunk, m.window,
+                                                         _p(self.sinks), dt, stream))
             else:
-                check(lib.qs_hyb_latent_attention(olat.data_ptr(), qa.data_ptr(), pool.data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
-                                                  b.block_table.shape[1], T, H, K, R, m.scale, page_size, m.chunk, m.window, _p(self.sinks), dt, stream))
+                check(_bind.qs_hyb_latent_attention(olat.data_ptr(), qa.data_ptr(), pool.data_ptr(), _p(b.tok_slot), _p(b.tok_pos), _p(b.block_table),
+                                                    b.block_table.shape[1], T, H, K, R, m.scale, page_size, m.chunk, m.window, _p(self.sinks), dt, stream))
             ov = torch.bmm(olat, self.w_uv)                                      # [H, T, Dv]
-        check(lib.qs_hyb_latent_gate_out(out.data_ptr(), out.stride(0), _p(ov), _p(otok), otok.stride(0) if per_head else 0, _p(b.tok_entry),
-                                         _p(b.entry_len), StepBatch.TILE_MIN if latent else 1, proj.data_ptr() if m.gate else None, proj.stride(0),
-                                         self.col_g, T, H, Dv, 1 if m.gate_wide else 0, dt, stream))
+        check(_bind.qs_hyb_latent_gate_out(out.data_ptr(), out.stride(0), _p(ov), _p(otok), otok.stride(0) if per_head else 0, _p(b.tok_entry),
+                                           _p(b.entry_len), StepBatch.TILE_MIN if latent else 1, proj.data_ptr() if m.gate else None, proj.stride(0),
+                                           self.col_g, T, H, Dv, 1 if m.gate_wide else 0, dt, stream))
 
 
 LATENT_IMPL = None  # tests: "plain" keeps the latent attention on the CUDA-core kernel, "latent" keeps prompt portions on the latent-space tiles
@@ -614,11 +616,11 @@ class StateSpaceMixer(_Mixer):
         m, T = self.m, b.n_tokens
         prep = scratch[: T * self.prep_width]
         o_raw = scratch[T * self.prep_width: T * (self.prep_width + self.out_features)]
-        check(lib.qs_hyb_state_space(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
-                                     self.conv_w.data_ptr(), self.conv_b.data_ptr(), run_cache["conv"].data_ptr(), run_cache["state"].data_ptr(),
-                                     self.a_log.data_ptr(), self.dt_bias.data_ptr(), self.skip.data_ptr(), self.norm_w.data_ptr(), m.norm_groups,
-                                     self.out_scale, _p(b.tok_entry), _p(b.tok_pos), _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot),
-                                     _p(b.entry_pos0), T, b.n_entries, m.heads, m.groups, m.state, m.vdim, m.conv, self.eps, dt, stream))
+        check(_bind.qs_hyb_state_space(out.data_ptr(), out.stride(0), prep.data_ptr(), o_raw.data_ptr(), proj.data_ptr(), proj.stride(0),
+                                       self.conv_w.data_ptr(), self.conv_b.data_ptr(), run_cache["conv"].data_ptr(), run_cache["state"].data_ptr(),
+                                       self.a_log.data_ptr(), self.dt_bias.data_ptr(), self.skip.data_ptr(), self.norm_w.data_ptr(), m.norm_groups,
+                                       self.out_scale, _p(b.tok_entry), _p(b.tok_pos), _p(b.entry_start), _p(b.entry_len), _p(b.entry_slot),
+                                       _p(b.entry_pos0), T, b.n_entries, m.heads, m.groups, m.state, m.vdim, m.conv, self.eps, dt, stream))
 
 
 class GatedUnitMixer(_Mixer):
@@ -653,13 +655,13 @@ class GatedUnitMixer(_Mixer):
         m, T = self.m, b.n_tokens
         u = torch.empty((T, m.width), dtype=proj.dtype, device=proj.device)
         tables = (_p(b.entry_start), _p(b.entry_len), _p(b.entry_slot), _p(b.entry_pos0))
-        check(lib.qs_hyb_lru_conv(u.data_ptr(), proj.data_ptr(), proj.stride(0), self.x_bias.data_ptr(), self.conv_w.data_ptr(), self.conv_b.data_ptr(),
-                                  run_cache["conv"].data_ptr(), _p(b.tok_entry), _p(b.tok_pos), *tables, T, b.n_entries, m.width, m.conv, dt, stream))
+        check(_bind.qs_hyb_lru_conv(u.data_ptr(), proj.data_ptr(), proj.stride(0), self.x_bias.data_ptr(), self.conv_w.data_ptr(), self.conv_b.data_ptr(),
+                                    run_cache["conv"].data_ptr(), _p(b.tok_entry), _p(b.tok_pos), *tables, T, b.n_entries, m.width, m.conv, dt, stream))
         z = _bmm_f32(u.view(T, m.blocks, -1).transpose(0, 1), self.w_gates.transpose(1, 2))  # [blocks, T, 2 W / blocks]
-        check(lib.qs_hyb_lru_scan(out.data_ptr(), out.stride(0), run_cache["state"].data_ptr(), scratch.data_ptr(), u.data_ptr(), z.data_ptr(),
-                                  proj.data_ptr(), proj.stride(0), self.y_bias.data_ptr(), self.r_bias.data_ptr(), self.i_bias.data_ptr(),
-                                  self.rate.data_ptr(), _p(b.tile_entry), _p(b.tile_row0), b.n_tiles, b.n_short, *tables, T, b.n_entries, m.width, m.blocks,
-                                  StepBatch.TILE_ROWS, StepBatch.TILE_MIN, dt, stream))
+        check(_bind.qs_hyb_lru_scan(out.data_ptr(), out.stride(0), run_cache["state"].data_ptr(), scratch.data_ptr(), u.data_ptr(), z.data_ptr(),
+                                    proj.data_ptr(), proj.stride(0), self.y_bias.data_ptr(), self.r_bias.data_ptr(), self.i_bias.data_ptr(),
+                                    self.rate.data_ptr(), _p(b.tile_entry), _p(b.tile_row0), b.n_tiles, b.n_short, *tables, T, b.n_entries, m.width, m.blocks,
+                                    StepBatch.TILE_ROWS, StepBatch.TILE_MIN, dt, stream))
 
 
 class ParallelMixer(_Mixer):
@@ -714,8 +716,8 @@ class ParallelMixer(_Mixer):
             raise NotImplementedError("side-by-side mixers whose own outputs are fp32 rows or have biases")
         T, W = yl.shape
         y = torch.empty((T, W), dtype=torch.float32, device=cat.device)
-        check(lib.qs_hyb_branch_norm_mean(y.data_ptr(), yl.data_ptr(), yr.data_ptr(), self.gain_left.data_ptr(), self.gain_right.data_ptr(),
-                                          self.m.scale, self.eps, T, W, dt, stream))
+        check(_bind.qs_hyb_branch_norm_mean(y.data_ptr(), yl.data_ptr(), yr.data_ptr(), self.gain_left.data_ptr(), self.gain_right.data_ptr(),
+                                            self.m.scale, self.eps, T, W, dt, stream))
         return y, True
 
 
@@ -782,34 +784,34 @@ class MoeFeedForward:
         route = torch.empty((T, c.experts), dtype=torch.float32, device=dev)
         top_idx = torch.empty((T, c.top), dtype=torch.int32, device=dev)
         top_w = torch.empty((T, c.top), dtype=torch.float32, device=dev)
-        check(lib.qs_hyb_moe_router(route.data_ptr(), top_idx.data_ptr(), top_w.data_ptr(), h.data_ptr(), self.w_router.data_ptr(), T, W, c.experts,
-                                    c.top, _ROUTER_MODE[c.router], _p(self.correction), c.groups, c.keep, 1 if c.renormalize else 0, c.weight_scale, dt, stream))
+        check(_bind.qs_hyb_moe_router(route.data_ptr(), top_idx.data_ptr(), top_w.data_ptr(), h.data_ptr(), self.w_router.data_ptr(), T, W, c.experts,
+                                      c.top, _ROUTER_MODE[c.router], _p(self.correction), c.groups, c.keep, 1 if c.renormalize else 0, c.weight_scale, dt, stream))
         if self.impl == "dense":
             gu = torch.mm(h, self.w_in.t())
             act = torch.empty((T, self.F), dtype=h.dtype, device=dev)
-            check(lib.qs_hyb_moe_act(act.data_ptr(), gu.data_ptr(), route.data_ptr(), T, c.experts, c.ff, c.limit, c.shared_ff, c.shared_limit, c.alpha,
-                                     c.up_shift, dt, stream))
+            check(_bind.qs_hyb_moe_act(act.data_ptr(), gu.data_ptr(), route.data_ptr(), T, c.experts, c.ff, c.limit, c.shared_ff, c.shared_limit, c.alpha,
+                                       c.up_shift, dt, stream))
             return torch.mm(act, self.w_down.t()), False
         n = T * c.top
         ends = torch.empty(c.experts, dtype=torch.int32, device=dev)
         row_of = torch.empty(n, dtype=torch.int32, device=dev)
         src = torch.empty(n, dtype=torch.int32, device=dev)
-        check(lib.qs_hyb_moe_plan(ends.data_ptr(), row_of.data_ptr(), src.data_ptr(), self.work.data_ptr(), top_idx.data_ptr(), T, c.experts, c.top,
-                                  stream))
+        check(_bind.qs_hyb_moe_plan(ends.data_ptr(), row_of.data_ptr(), src.data_ptr(), self.work.data_ptr(), top_idx.data_ptr(), T, c.experts, c.top,
+                                    stream))
         xs = torch.empty((n, W), dtype=h.dtype, device=dev)
-        check(lib.qs_hyb_moe_gather(xs.data_ptr(), h.data_ptr(), src.data_ptr(), n, W, dt, stream))
+        check(_bind.qs_hyb_moe_gather(xs.data_ptr(), h.data_ptr(), src.data_ptr(), n, W, dt, stream))
         gu = torch.nn.functional.grouped_mm(xs, self.w_gu.transpose(-2, -1), offs=ends)
         act = torch.empty((n, c.ff), dtype=h.dtype, device=dev)
-        check(lib.qs_hyb_moe_act(act.data_ptr(), gu.data_ptr(), None, n, 0, 0, 0.0, c.ff, c.limit, c.alpha, c.up_shift, dt, stream))
+        check(_bind.qs_hyb_moe_act(act.data_ptr(), gu.data_ptr(), None, n, 0, 0, 0.0, c.ff, c.limit, c.alpha, c.up_shift, dt, stream))
         rows = torch.nn.functional.grouped_mm(act, self.w_dn.transpose(-2, -1), offs=ends)
         shared = None
         if c.shared_ff:
             gs = torch.mm(h, self.w_sh_in.t())
             sa = torch.empty((T, c.shared_ff), dtype=h.dtype, device=dev)
-            check(lib.qs_hyb_moe_act(sa.data_ptr(), gs.data_ptr(), None, T, 0, 0, 0.0, c.shared_ff, c.shared_limit, c.alpha, c.up_shift, dt, stream))
+            check(_bind.qs_hyb_moe_act(sa.data_ptr(), gs.data_ptr(), None, T, 0, 0, 0.0, c.shared_ff, c.shared_limit, c.alpha, c.up_shift, dt, stream))
             shared = torch.mm(sa, self.w_sh_dn.t())
         y = torch.empty((T, W), dtype=torch.float32, device=dev)
-        check(lib.qs_hyb_moe_combine(y.data_ptr(), rows.data_ptr(), _p(shared), row_of.data_ptr(), top_w.data_ptr(), T, c.top, W, dt, stream))
+        check(_bind.qs_hyb_moe_combine(y.data_ptr(), rows.data_ptr(), _p(shared), row_of.data_ptr(), top_w.data_ptr(), T, c.top, W, dt, stream))
         return y, True
 
 
@@ -844,10 +846,10 @@ class DenseFeedForward:
             kernel = lib.qs_hyb_bias_relu_squared if self.act == "relu2" else lib.qs_hyb_bias_gelu_tanh
             check(kernel(act.data_ptr(), act.stride(0), gu.data_ptr(), gu.stride(0), _p(self.in_bias), gu.shape[0], self.ff, dt, stream))
         elif self.in_bias is None and self.act == 0 and gu.stride(0) == 2 * self.ff:
-            check(lib.qs_hyb_gelu_tanh_mul(act.data_ptr(), act.stride(0), gu.data_ptr(), gu.shape[0], self.ff, dt, stream))
+            check(_bind.qs_hyb_gelu_tanh_mul(act.data_ptr(), act.stride(0), gu.data_ptr(), gu.shape[0], self.ff, dt, stream))
         else:
-            check(lib.qs_hyb_bias_gated_act(act.data_ptr(), act.stride(0), gu.data_ptr(), gu.stride(0), _p(self.in_bias), gu.shape[0], self.ff, self.act, dt,
-                                            stream))
+            check(_bind.qs_hyb_bias_gated_act(act.data_ptr(), act.stride(0), gu.data_ptr(), gu.stride(0), _p(self.in_bias), gu.shape[0], self.ff, self.act, dt,
+                                              stream))
         return _mm_f32(act, self.w_down.t()), True
 
 
@@ -1085,8 +1087,8 @@ class HybridDecoder:
         cfg, dev, dt, T, W = self.cfg, self.device, self.dt, b.n_tokens, self.cfg.width
         s = _stream(dev)
         x = torch.empty((T, self.n_streams, W) if cfg.block == "sequential" else (T, W), dtype=torch.float32, device=dev)
-        check(lib.qs_hyb_embed(x.data_ptr(), _p(b.tokens), _p(b.prev), self.embed.data_ptr(), _p(self.pair), T, W, cfg.pair_buckets,
-                               cfg.pair_mul_prev, cfg.pair_mul_cur, cfg.embed_scale, self.n_streams, dt, s))
+        check(_bind.qs_hyb_embed(x.data_ptr(), _p(b.tokens), _p(b.prev), self.embed.data_ptr(), _p(self.pair), T, W, cfg.pair_buckets,
+                                 cfg.pair_mul_prev, cfg.pair_mul_cur, cfg.embed_scale, self.n_streams, dt, s))
         if scratch is None:
             need = self.scratch_floats(T)
             if need and (self._scratch is None or self._scratch.numel() < need):
@@ -1106,9 +1108,9 @@ class HybridDecoder:
         """x <- x + the pending sublayer outputs (rows, rows are fp32, second rows, they are fp32, a bias row); then the norm of x into out_h and /
         or [x | x0] into cat_out."""
         a1, f1, a2, f2, ab = pending if pending is not None else (None, False, None, False, None)
-        check(lib.qs_hyb_stream_update_norm(_p(out_h), _p(cat_out), x.data_ptr(), _p(x0), _p(a1), 1 if f1 else 0, _p(a2), 1 if f2 else 0, _p(ab), _p(w),
-                                            _p(bias), _NORM_KIND[self.cfg.norm_kind] if out_h is not None else 0, self.cfg.eps, x.shape[0],
-                                            self.cfg.width, self.dt, s))
+        check(_bind.qs_hyb_stream_update_norm(_p(out_h), _p(cat_out), x.data_ptr(), _p(x0), _p(a1), 1 if f1 else 0, _p(a2), 1 if f2 else 0, _p(ab), _p(w),
+                                              _p(bias), _NORM_KIND[self.cfg.norm_kind] if out_h is not None else 0, self.cfg.eps, x.shape[0],
+                                              self.cfg.width, self.dt, s))
 
     def _forward_parallel(self, x, b: StepBatch, cache: HybridCache, tap, scratch, s) -> torch.Tensor:
         cfg, dev, dt, T, W = self.cfg, self.device, self.dt, b.n_tokens, self.cfg.width
@@ -1128,8 +1130,8 @@ class HybridDecoder:
             has_ff = ly.ff > 0 or ly.side_ff is not None
             plain = pending is None or (pending[2] is None and pending[4] is None and not pending[1])
             if cfg.norm_kind == "rms" and not cfg.shared_norm and plain:
-                check(lib.qs_hyb_rms_norm(h1.data_ptr(), _p(h2) if has_ff else None, x.data_ptr(), _p(pending[0]) if pending else None,
-                                          ly.norm1.data_ptr(), _p(ly.norm2), cfg.norm_offset, cfg.eps, T, W, dt, s))
+                check(_bind.qs_hyb_rms_norm(h1.data_ptr(), _p(h2) if has_ff else None, x.data_ptr(), _p(pending[0]) if pending else None,
+                                            ly.norm1.data_ptr(), _p(ly.norm2), cfg.norm_offset, cfg.eps, T, W, dt, s))
             else:
                 self._land(x, pending, s, out_h=h1, w=ly.norm1, bias=ly.norm1_b)
                 if has_ff and not cfg.shared_norm:
@@ -1146,9 +1148,9 @@ class HybridDecoder:
             if ly.ff:
                 act = cat.data_ptr() + ly.mixer.out_features * cat.element_size()
                 if ly.gated:
-                    check(lib.qs_hyb_gelu_tanh_mul(act, cat.stride(0), gu.data_ptr(), T, ly.ff, dt, s))
+                    check(_bind.qs_hyb_gelu_tanh_mul(act, cat.stride(0), gu.data_ptr(), T, ly.ff, dt, s))
                 else:
-                    check(lib.qs_hyb_bias_gelu_tanh(act, cat.stride(0), gu.data_ptr(), gu.stride(0), _p(ly.mlp_in_bias), T, ly.ff, dt, s))
+                    check(_bind.qs_hyb_bias_gelu_tanh(act, cat.stride(0), gu.data_ptr(), gu.stride(0), _p(ly.mlp_in_bias), T, ly.ff, dt, s))
             upd = torch.mm(cat, ly.w_out.t())
             side, side32 = ly.side_ff.run(h2, dt, s) if ly.side_ff is not None else (None, False)
             pending = (upd, False, side, side32, ly.out_bias)
@@ -1165,9 +1167,9 @@ class HybridDecoder:
         into out_h and / or that sum itself (cin None: the plain sum) into out_sum."""
         cfg = self.cfg
         y, y32, hc = pending if pending is not None else (None, False, None)
-        check(lib.qs_hyb_stream_norm(_p(out_h), _p(out_sum), x.data_ptr(), self.n_streams, _p(y), 1 if y32 else 0, _p(hc.mix) if hc else None,
-                                     _p(hc.cout) if hc else None, _p(cin), _p(w), cfg.norm_groups, cfg.norm_offset, cfg.eps, x.shape[0], cfg.width,
-                                     self.dt, s))
+        check(_bind.qs_hyb_stream_norm(_p(out_h), _p(out_sum), x.data_ptr(), self.n_streams, _p(y), 1 if y32 else 0, _p(hc.mix) if hc else None,
+                                       _p(hc.cout) if hc else None, _p(cin), _p(w), cfg.norm_groups, cfg.norm_offset, cfg.eps, x.shape[0], cfg.width,
+                                       self.dt, s))
 
     def _forward_sequential(self, x, b: StepBatch, cache: HybridCache, tap, scratch, s) -> torch.Tensor:
         dev, dt, T, W = self.device, self.dt, b.n_tokens, self.cfg.width
@@ -1230,18 +1232,18 @@ class HybridDecoder:
         else:
             h = torch.empty((T, W), dtype=self.dtype, device=dev)
             h_ptr = h.data_ptr()
-            check(lib.qs_hyb_cast_rows(h_ptr, x.data_ptr(), T * W, dt, s))
+            check(_bind.qs_hyb_cast_rows(h_ptr, x.data_ptr(), T * W, dt, s))
         for run, li in enumerate(self.schedule):
             ly = self.layers[li]
             proj = torch.mm(h, ly.mixer.w_in.t())
             cat = torch.empty((T, ly.mixer.out_features), dtype=self.dtype, device=dev)
             ly.mixer.run(proj, cat, b, cache.runs[run], cache.page_size, scratch, dt, s)
             y = _mm_f32(cat, ly.mixer.w_out.t())
-            check(lib.qs_hyb_post_norm_update(h_ptr, x.data_ptr(), y.data_ptr(), 1, _p(ly.mixer.out_bias), ly.norm1.data_ptr(), _p(ly.ls1), cfg.norm_offset, cfg.eps, T, W, dt, s))
+            check(_bind.qs_hyb_post_norm_update(h_ptr, x.data_ptr(), y.data_ptr(), 1, _p(ly.mixer.out_bias), ly.norm1.data_ptr(), _p(ly.ls1), cfg.norm_offset, cfg.eps, T, W, dt, s))
             if ly.ff is not None:
                 y, y32 = ly.ff.run(h, dt, s)
-                check(lib.qs_hyb_post_norm_update(h_ptr, x.data_ptr(), y.data_ptr(), 1 if y32 else 0, _p(getattr(ly.ff, "out_bias", None)),
-                                                  ly.norm2.data_ptr(), _p(ly.ls2), cfg.norm_offset, cfg.eps, T, W, dt, s))
+                check(_bind.qs_hyb_post_norm_update(h_ptr, x.data_ptr(), y.data_ptr(), 1 if y32 else 0, _p(getattr(ly.ff, "out_bias", None)),
+                                                    ly.norm2.data_ptr(), _p(ly.ls2), cfg.norm_offset, cfg.eps, T, W, dt, s))
             if tap is not None:
                 tap(run, x)
         return x
@@ -1249,9 +1251,9 @@ class HybridDecoder:
     def _sandwich_land(self, out_h, x, rows, rows_f32, bias, gate, gate_b, w, mult, w_next, s, fresh: bool = False) -> None:
         """x <- [x +] mult norm(sigmoid(gate + gate_b) * (rows + bias)) w; the norm of x times w_next into out_h (None: not wanted)."""
         cfg = self.cfg
-        check(lib.qs_hyb_gated_norm_update(_p(out_h), x.data_ptr(), 1 if fresh else 0, rows.data_ptr(), 1 if rows_f32 else 0, _p(bias), _p(gate),
-                                           gate.stride(0) if gate is not None else 0, _p(gate_b), w.data_ptr(), mult, _p(w_next), cfg.norm_groups,
-                                           cfg.norm_offset, cfg.eps, x.shape[0], cfg.width, self.dt, s))
+        check(_bind.qs_hyb_gated_norm_update(_p(out_h), x.data_ptr(), 1 if fresh else 0, rows.data_ptr(), 1 if rows_f32 else 0, _p(bias), _p(gate),
+                                             gate.stride(0) if gate is not None else 0, _p(gate_b), w.data_ptr(), mult, _p(w_next), cfg.norm_groups,
+                                             cfg.norm_offset, cfg.eps, x.shape[0], cfg.width, self.dt, s))
 
     def _forward_sandwich(self, x, b: StepBatch, cache: HybridCache, tap, scratch, s) -> torch.Tensor:
         cfg, dev, dt, T, W = self.cfg, self.device, self.dt, b.n_tokens, self.cfg.width
@@ -1262,8 +1264,8 @@ class HybridDecoder:
             e, x = x, torch.empty_like(x)
             self._sandwich_land(h if layers else None, x, e, True, None, None, None, self.embed_norm, 1.0, first, s, fresh=True)
         elif layers:
-            check(lib.qs_hyb_stream_norm(h.data_ptr(), None, x.data_ptr(), 1, None, 0, None, None, None, first.data_ptr(), cfg.norm_groups, cfg.norm_offset,
-                                         cfg.eps, T, W, dt, s))
+            check(_bind.qs_hyb_stream_norm(h.data_ptr(), None, x.data_ptr(), 1, None, 0, None, None, None, first.data_ptr(), cfg.norm_groups, cfg.norm_offset,
+                                           cfg.eps, T, W, dt, s))
         for run, ly in enumerate(layers):
             after = layers[run + 1].norm1 if run + 1 < len(layers) else None  # gain of the norm the next layer reads; none after the last
             rows = torch.mm(h, ly.w_mix_in.t())
@@ -1289,16 +1291,16 @@ class HybridDecoder:
         h = torch.empty((n, W), dtype=self.dtype, device=self.device)
         s = _stream(self.device)
         if self.cfg.block in ("sequential", "sandwich"):
-            check(lib.qs_hyb_stream_norm(h.data_ptr(), None, x_rows.data_ptr(), 1, None, 0, None, None, None, self.final_norm.data_ptr(),
-                                         self.cfg.norm_groups, self.cfg.norm_offset, self.cfg.eps, n, W, self.dt, s))
+            check(_bind.qs_hyb_stream_norm(h.data_ptr(), None, x_rows.data_ptr(), 1, None, 0, None, None, None, self.final_norm.data_ptr(),
+                                           self.cfg.norm_groups, self.cfg.norm_offset, self.cfg.eps, n, W, self.dt, s))
         elif self.cfg.norm_kind == "rms":
-            check(lib.qs_hyb_rms_norm(h.data_ptr(), None, x_rows.data_ptr(), None, self.final_norm.data_ptr(), None, self.cfg.norm_offset, self.cfg.eps, n,
-                                      W, self.dt, s))
+            check(_bind.qs_hyb_rms_norm(h.data_ptr(), None, x_rows.data_ptr(), None, self.final_norm.data_ptr(), None, self.cfg.norm_offset, self.cfg.eps, n,
+                                        W, self.dt, s))
         else:
             self._land(x_rows, None, s, out_h=h, w=self.final_norm, bias=self.final_norm_b)
         out = _mm_f32(h, self.head.t()) if self.cfg.logit_softcap > 0.0 or self.cfg.block in ("post", "sandwich") or self.one_stream else torch.mm(h, self.head.t()).float()
         if self.cfg.logit_softcap > 0.0:
-            check(lib.qs_hyb_softcap(out.data_ptr(), out.numel(), self.cfg.logit_softcap, s))
+            check(_bind.qs_hyb_softcap(out.data_ptr(), out.numel(), self.cfg.logit_softcap, s))
         return out
 
 
