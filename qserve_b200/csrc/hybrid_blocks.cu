@@ -5,6 +5,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "../../include/qserve_b200.h"
@@ -743,6 +744,24 @@ __global__ void stream_update_norm_kernel(ST* __restrict__ out_h, ST* __restrict
   }
 }
 
+// The additions alone, no norm behind them: bound by memory, so a word a thread, all of an SM's threads resident, parts of a row in blocks of their own.  (An
+// attention layer over 4 prompts of up to 2048 tokens, 6758 rows of 2048, against one block per row and a short loop, runs in turn: 467.4 / 469.2 us; the kernel
+// below, whose registers are a norm's, 482.5 / 480.3.)
+template <typename ST>
+__global__ void __launch_bounds__(256) stream_update_vec_kernel(float* __restrict__ x, const void* __restrict__ add1, int add1_f32, const void* __restrict__ add2,
+                                                                int add2_f32, const float* __restrict__ add_bias, int W, int parts) {
+  const int row = blockIdx.x / parts, i = ((blockIdx.x - row * parts) * blockDim.x + threadIdx.x) * 4;
+  if (i >= W) return;
+  const size_t at = (size_t)row * W + i;
+  auto rows4 = [&](const void* p, int f32) { return f32 ? ld4(static_cast<const float*>(p) + at) : ld4(static_cast<const ST*>(p) + at); };
+  float4 v = ld4(x + at), u = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (add1 != nullptr) { const float4 a = rows4(add1, add1_f32); u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w; }
+  if (add2 != nullptr) { const float4 a = rows4(add2, add2_f32); u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w; }
+  if (add_bias != nullptr) { const float4 a = ld4(add_bias + i); u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w; }
+  v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  st4(x + at, v);
+}
+
 // the same for widths that are multiples of 4 and 16-byte aligned rows: four elements per access.  A thread holds its V words of the row (0: any number, read
 // again); all of a row's loads and the gains are on their way together (6758 rows of 2048, norm alone: 19.8 us where the row was read again, 18.4 so; 64 rows 4.4 and 3.7)
 template <typename ST, int V>
@@ -1327,17 +1346,21 @@ int qs_hyb_stream_update_norm(void* out_h, void* cat_out, float* x, const float*
   const int threads = width >= 1024 ? 256 : 128;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (width % 4 == 0 && al16(out_h) && al16(cat_out) && al16(x) && al16(x0) && al16(add1) && al16(add2) && al16(add_bias) && al16(w) && al16(b)) {
+    const int parts = (width / 4 + threads - 1) / threads;
+    if (out_h == nullptr && cat_out == nullptr && (add1 != nullptr || add2 != nullptr || add_bias != nullptr) && (long long)tokens_n * parts <= INT_MAX) {
+      QS_DT(dtype, (stream_update_vec_kernel<__nv_bfloat16><<<tokens_n * parts, threads, 0, s>>>(x, add1, add1_f32, add2, add2_f32, add_bias, width, parts)),
+            (stream_update_vec_kernel<float><<<tokens_n * parts, threads, 0, s>>>(x, add1, add1_f32, add2, add2_f32, add_bias, width, parts)));
+      return check_cuda(cudaGetLastError(), "hyb_stream_update_norm");
+    }
     auto go = [&](auto st, auto v) {
       using ST = decltype(st);
       stream_update_norm_vec_kernel<ST, decltype(v)::value><<<tokens_n, threads, 0, s>>>((ST*)out_h, (ST*)cat_out, x, x0, add1, add1_f32, add2, add2_f32, add_bias, w,
                                                                                          b, kind, eps, width);
     };
     auto words = [&](auto st) {
-      // (a prompt's rows without a norm: nothing is read again, 6758 rows 17.6 us word by word and 19.3 with all of a row's words ahead)
-      const int n = out_h == nullptr && tokens_n > 8 * num_sms() ? 5 : (width / 4 + threads - 1) / threads;
-      if (n <= 1) go(st, std::integral_constant<int, 1>{});
-      else if (n <= 2) go(st, std::integral_constant<int, 2>{});
-      else if (n <= 4) go(st, std::integral_constant<int, 4>{});
+      if (parts <= 1) go(st, std::integral_constant<int, 1>{});
+      else if (parts <= 2) go(st, std::integral_constant<int, 2>{});
+      else if (parts <= 4) go(st, std::integral_constant<int, 4>{});
       else go(st, std::integral_constant<int, 0>{});
     };
     QS_DT(dtype, words(__nv_bfloat16{}), words(float{}));
