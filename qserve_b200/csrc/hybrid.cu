@@ -1209,13 +1209,14 @@ __global__ void __launch_bounds__(kPrepThreads) delta_prepare_kernel(
 // The same for heads of up to 128 channels, four channels per lane: a warp owns one unit and walks a run of neighbouring tokens with the unit's taps
 // and the window of inputs in registers, the unit length is a warp sum, and nothing is loaded twice.  (One block per (token, unit) read every
 // input `taps` times with 2-byte accesses and met in shared memory for every unit: 6758 tokens, 24 units of 128, 253 us; now 56, floor 22.)
-template <typename ST, int TAPS>
+// SHIFT: a step of single tokens, whose lanes shift the state that they read (prompts have an instance without that: the layer of 2 x 150 tokens 83.9 us with the choice in the kernel, 82.2 so).
+template <typename ST, int TAPS, bool SHIFT>
 __global__ void __launch_bounds__(128, TAPS == 4 ? 6 : 0) delta_prepare_walk_kernel(float* __restrict__ prep, const ST* __restrict__ proj, long long stride,
                                                                  const float* __restrict__ conv_w, float* __restrict__ conv_state,
                                                                  const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                                                  const int* __restrict__ tok_entry, const int* __restrict__ tok_pos,
                                                                  const int* __restrict__ entry_start, const int* __restrict__ entry_slot, int T, int H, int G,
-                                                                 int D, int Dv, int taps, float unit_eps, int run, int shift) {
+                                                                 int D, int Dv, int taps, float unit_eps, int run) {
   const int C = 2 * G * D + H * Dv, P = C + 2 * H;
   const int u = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * run, t1 = min(T, t0 + run);
@@ -1227,7 +1228,7 @@ __global__ void __launch_bounds__(128, TAPS == 4 ? 6 : 0) delta_prepare_walk_ker
     auto walk = conv_walk<ST, 4, TAPS>(conv_w, nullptr, nullptr, taps, c);
     const ConvTables tab{conv_state, tok_entry, tok_pos, entry_start, entry_slot, C, taps};
     const float q_scale = 1.f / sqrtf((float)D);
-    conv_rows<ST, 4>(walk, proj, stride, nullptr, tab, t0, t1, c, shift != 0 && in, [&](int t, float(&y)[4]) {
+    conv_rows<ST, 4>(walk, proj, stride, nullptr, tab, t0, t1, c, SHIFT && in, [&](int t, float(&y)[4]) {
 #pragma unroll
       for (int v = 0; v < 4; ++v) y[v] = silu_f(y[v]);
       float r = 1.f;
@@ -1579,10 +1580,16 @@ int launch_delta(void* out, long long out_stride, float* prep, float* o_raw, con
   if (D % 4 == 0 && D <= 128 && Dv % 4 == 0 && Dv <= 128 && stride % 4 == 0 && (C + 2 * H) % 4 == 0 && al(proj, 4 * sizeof(ST)) && al(prep, 16)) {
     const int run = conv_run(T);
     shift = T == E && taps > 1;
-    auto walk = taps == 4 ? delta_prepare_walk_kernel<ST, 4> : taps == 3 ? delta_prepare_walk_kernel<ST, 3> : taps == 2 ? delta_prepare_walk_kernel<ST, 2>
-                                                                                                         : delta_prepare_walk_kernel<ST, 0>;
+    auto pick = [&](auto sh) {
+      constexpr bool kShift = decltype(sh)::value;
+      return taps == 4   ? delta_prepare_walk_kernel<ST, 4, kShift>
+             : taps == 3 ? delta_prepare_walk_kernel<ST, 3, kShift>
+             : taps == 2 ? delta_prepare_walk_kernel<ST, 2, kShift>
+                         : delta_prepare_walk_kernel<ST, 0, kShift>;
+    };
+    auto walk = shift ? pick(std::true_type{}) : pick(std::false_type{});
     walk<<<dim3((T + run - 1) / run, (2 * G + H + 3) / 4), 128, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry, tok_pos,
-                                                                        entry_start, entry_slot, T, H, G, D, Dv, taps, unit_eps, run, shift);
+                                                                        entry_start, entry_slot, T, H, G, D, Dv, taps, unit_eps, run);
   } else {
     delta_prepare_kernel<ST><<<dim3(T, 2 * G + H), kPrepThreads, 0, s>>>(prep, (const ST*)proj, stride, conv_w, conv_state, a_log, dt_bias, tok_entry,
                                                                         tok_pos, entry_start, entry_slot, H, G, D, Dv, taps, unit_eps);
