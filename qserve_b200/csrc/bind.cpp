@@ -349,9 +349,10 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return nullptr;
 }
 
-// ---- functions of the C ABI as they are declared: conversions in the order and of the types of the declaration (pointers: an address or None; numbers as
-//      ctypes takes them), then the call without the interpreter lock; returns its status.  The attention and state functions of the hybrid decoders have
-//      25 to 40 arguments, a layer of short prompts five such calls: 79 us through ctypes, 69 here; a prompt's attention block 56 and 50 ----
+// ---- functions of the C ABI as they are declared: conversions in the order and of the types of the declaration (pointers: an address or None;
+//      integers: whatever has an __index__, as ctypes takes them), then the call without the interpreter lock; returns its status.  The attention and state
+//      functions of the hybrid decoders have 25 to 40 arguments, a layer of short prompts five such calls: 79 us through ctypes, 69 here; a prompt's attention
+//      block 56 and 50 ----
 template <typename T>
 T converted(PyObject* o) {
   if constexpr (std::is_pointer_v<T>) {
@@ -368,6 +369,13 @@ T converted(PyObject* o) {
   } else {
     static_assert(std::is_integral_v<T>);
     if (PyLong_Check(o)) return static_cast<T>(PyLong_AsUnsignedLongLongMask(o));
+    if (PyIndex_Check(o)) {  // numbers of numpy, tensors of one integer: sizes that a program read out of an array
+      PyObject* const i = PyNumber_Index(o);
+      if (i == nullptr) throw python_error();
+      const T v = static_cast<T>(PyLong_AsUnsignedLongLongMask(i));
+      Py_DECREF(i);
+      return v;
+    }
   }
   PyErr_Format(PyExc_TypeError, "%s expected, not %s", std::is_pointer_v<T> ? "an address or None" : "an integer", Py_TYPE(o)->tp_name);
   throw python_error();

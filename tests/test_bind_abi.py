@@ -2,8 +2,9 @@
 no number refused with TypeError."""
 import re
 
+import numpy
 import pytest
-import torch  # noqa: F401 -- the binding is linked against it
+import torch
 
 from qserve_b200 import _bind
 from qserve_b200._lib import SIGNATURES, lib
@@ -32,7 +33,30 @@ def test_numbers_as_ctypes_hands_them_on(change):
     assert got[0] == got[1] and got[0][0] != 0
 
 
-@pytest.mark.parametrize("at,value", [(0, "x"), (0, 1.5), (3, 1.5), (3, None), (9, "1"), (15, "0.5"), (15, None), (16, b"")])
+class _Index:
+    def __init__(self, v):
+        self.v = v
+
+    def __index__(self):
+        return self.v
+
+
+@pytest.mark.parametrize("kind", [numpy.int32, numpy.int64, numpy.uint8, torch.tensor, _Index], ids=lambda k: k.__name__)
+@pytest.mark.parametrize("at", [3, 9, 12, 14])
+def test_whatever_has_an_index_is_an_integer(kind, at):  # sizes that a program read out of an array
+    args = [16, 16, 16, 384, 384, 384, 16, 128, 16, 1, 4, 4, 3, 2, 96, 0.5, None]
+    args[at] = kind(args[at] % 256)
+    got = [_refused(f, args) for f in (_bind.qs_prefill_attention, lib.qs_prefill_attention)]
+    assert got[0] == got[1] and got[0][0] != 0
+
+
+def test_an_index_that_raises():
+    args = [16, 16, 16, 384, 384, 384, 16, 128, 16, 1, 4, 4, 3, 2, torch.tensor([96, 96]), 0.5, None]
+    with pytest.raises(TypeError, match="index"):  # (torch's own words)
+        _bind.qs_prefill_attention(*args)
+
+
+@pytest.mark.parametrize("at,value", [(0, numpy.int64(16)), (0, torch.tensor(16)), (9, numpy.float32(1)), (9, torch.tensor(1.5)), (0, "x"), (0, 1.5), (3, 1.5), (3, None), (9, "1"), (15, "0.5"), (15, None), (16, b"")])
 def test_what_is_no_number_is_refused(at, value):
     args = [16, 16, 16, 384, 384, 384, 16, 128, 16, 1, 4, 4, 3, 2, 96, 0.5, None]
     args[at] = value
