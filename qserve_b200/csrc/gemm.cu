@@ -55,7 +55,7 @@ constexpr bool kPairCvt = QS_PAIR_CVT != 0;
 #define QS_DECODE_CVT 1
 #endif
 constexpr bool kDecodeCvt = QS_DECODE_CVT != 0;  // the same choice for the epilogue of gemm_kernel
-constexpr int kPairThreads = 384, kPairRoundsThreads = 640;  // CTAs of the pair kernels; with warps of their own for the epilogue (W4A8, tiles in several rounds)
+constexpr int kPairThreads = 384;  // CTAs of the pair kernels; kPairRoundsThreads with warps of their own for the epilogue (W4A8, tiles in several rounds)
 // warp roles: 0 weight producer | 1 TMEM owner + MMA issuer (even stages) | 2..5 unpack + TMEM epilogue | 6 activation producer |
 // 7 MMA issuer (odd stages).
 // All eight warps take part in the final reduce / scale / store phase.
@@ -747,8 +747,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
   auto tile_m = [&](int lt) { return (pair + lt * n_pairs) % p.m_tiles; };
   auto tile_n = [&](int lt) { return 2 * ((pair + lt * n_pairs) / p.m_tiles) + static_cast<int>(rank); };
 
-  // 4 x 48 + 8 x 64 + 8 x 152 registers of 32 lanes: the 61440 that 640 threads are launched with
-  if (ROUNDS && warp < 4) set_max_regs<false, 48>();
+  // 4 x 48 + 8 x 64 + 8 x 152 registers of 32 lanes: the 61440 that 640 threads are launched with (the host makes sure of that: pair_registers_suffice)
+  if (ROUNDS && warp < 4) set_max_regs<false, kPairLoadRegs>();
   if (warp == 0) {
     // ===================================== weight producer (static data: never waits for the previous kernel) =====================================
     if (lane == 0) {
@@ -921,12 +921,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_cons
     };
     if constexpr (ROUNDS) {
       if (unpacks) {
-        set_max_regs<false, 64>();
+        set_max_regs<false, kPairUnpackRegs>();
         unpack(my_tiles * n_kb);
         pdl_wait();
       } else {
         zero_fill();
-        set_max_regs<true, 152>();
+        set_max_regs<true, kPairEpilogueRegs>();
         pdl_wait();
         for (int lt = 0; lt < my_tiles; ++lt) finish(lt);
       }
@@ -1377,6 +1377,12 @@ int launch_gemm_pair(const GemmArgs& a) {
   if (!done) {
     rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes), "cudaFuncSetAttribute(gemm pair smem)");
     if (rc) return rc;
+    if (!w8 && rounds) {
+      cudaFuncAttributes built;
+      rc = check_cuda(cudaFuncGetAttributes(&built, kern), "cudaFuncGetAttributes(gemm pair)");
+      if (rc) return rc;
+      QS_REQUIRE(pair_registers_suffice(built.numRegs), "gemm: the pair kernel was built with %d registers per thread, fewer than its warps share out", built.numRegs);
+    }
     done = true;
   }
   cudaLaunchConfig_t cfg{};

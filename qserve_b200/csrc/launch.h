@@ -12,6 +12,14 @@ int device_ordinal();
 int num_sms();
 int num_sms(int dev);  // dev: what device_ordinal() said
 
+// Registers per thread that the warpgroups of a pair kernel with warps of its own for the epilogue (gemm.cu) trade for the launch's: one of loads and issue, two of
+// unpacking, two of the epilogue.  The epilogue's increase waits until its share is free, for good where the launch brought fewer than all shares together.
+// The compiler may not give a kernel more than its launch bounds allow, 96 here, but nothing makes it give as many: the host asks before the first launch.
+constexpr int kPairRoundsThreads = 640, kPairLoadRegs = 48, kPairUnpackRegs = 64, kPairEpilogueRegs = 152;
+constexpr bool pair_registers_suffice(int per_thread) {
+  return kPairRoundsThreads * per_thread >= 128 * (kPairLoadRegs + 2 * kPairUnpackRegs + 2 * kPairEpilogueRegs);
+}
+
 struct GemmArgs {
   const void* act = nullptr;        // int8 [M, K]
   const void* weight = nullptr;     // W4: packed int4 [N, K/2] (reference layout); W8: int8 [N, K]
