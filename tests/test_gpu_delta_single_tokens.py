@@ -29,3 +29,22 @@ def test_bits_of_a_step_with_a_run(dtype, taps, H, G, D, Dv):
         assert torch.isfinite(prep[:n]).all()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [511, 512, 515, 700, 2049])
+def test_bits_of_walks_over_several_sequences(n):
+    """From 512 tokens on a lane walks several of them, from 2048 on 16: tokens of different sequences, each of which shifts a state of its own."""
+    got = []
+    for more in (0, 1):
+        layer = GatedDelta(6, BF, n + 1, 2, 1, 32, 40)
+        layer.conv = layer.rand(n + 1, 3, layer.C)
+        slots, pos = list(range(n + 1))[::-1], [(7 * i) % 11 for i in range(n)]
+        for slot, a in zip(slots, pos):
+            layer.conv[slot, :max(0, 3 - a)] = 0.0  # ahead of the sequence
+        proj = layer.rand(n + 2, layer.W).to(BF)
+        prep, _, out = layer.step(proj[:n + 2 * more], [1] * n + [2] * more, pos + [5] * more, slots[:n + more])
+        used = slots[:n]
+        got.append((prep[:n], out[:n], layer.state[used], layer.conv[used]))
+        assert torch.isfinite(prep[:n]).all()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

@@ -43,3 +43,10 @@ def test_ranges(dev, kind, M, N, K):
     op.gemm_forward_cuda(*(to_dev(t, dev) for t in (aq, qw, z, s, s1, sa)), out, _acc_out=acc)
     assert np.array_equal(np_of(acc), acc_o)
     assert np.array_equal(np_of(out).view(np.uint16), out_o.view(np.uint16))
+
+
+@pytest.mark.parametrize("kind", ["edge", "past", "one_past"])
+@pytest.mark.parametrize("M,N,K", [(393, 9728, 512), (192, 19200, 512)])
+def test_ranges_over_rounds(dev, kind, M, N, K):
+    """76 and 75 tiles of 256 tokens on 74 pairs: the kernel with warps of its own for the epilogue, which unpacks while they store."""
+    test_ranges(dev, kind, M, N, K)
