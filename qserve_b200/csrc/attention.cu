@@ -465,12 +465,13 @@ decode_attention_kernel(const __half* __restrict__ q_in, const __half* __restric
     float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, l0 = 0.f, l1 = 0.f, cr0 = 0.f, cr1 = 0.f;
     float spa[4] = {0.f, 0.f, 0.f, 0.f};  // [0], [1]: sum p' of heads 2q4, 2q4+1 over ALL tokens this warp has seen
 
-    // S^T = K Q^T: A rows g / g+8 <-> chunk tokens tokA / 8+tokA (the permutation keeps the V row reads at a 2-way conflict)
+    // S^T = K Q^T: A rows g / g+8 <-> chunk tokens tokA / 8+tokA.  The rows' order is that of v_at's: row 2 i + e is token i + 4 e in both, so the pairs of tokens
+    // in which a lane has the weights (q4, 4 + q4, and 8 further on) are those of the V words that its transposing loads bring.
     const int tokA = (g & 1) * 4 + (g >> 1);
     const uint32_t k_at = SL::place(tokA, BITS == 4 ? q4 : 2 * q4);                                                // + 512 or 1024 bytes: tokens 8 on
     const uint32_t v_at = SL::place((lane & 1) * 4 + ((lane >> 1) & 3) + (lane & 8), lane >> 4) + SL::kOffV;  // matrices: tokens 0 .. 7, 8 .. 15, next word
     // warp w consumes tokens [32 (w & 1), +32) of the pages whose index has parity (w >> 1): two 16-token MMA chunks per
-    // iteration share one barrier wait, one max reduction and one set of address computations
+    // iteration share one wait for a copy group, one max reduction and one set of address computations
     const int hbase = hslice * kSliceTokens;
     int s = 0;  // the slot at hand
     auto advance = [&]() { if (++s == R) s = 0; };

@@ -159,7 +159,7 @@ __device__ __forceinline__ void st_dsmem_u32(uint32_t addr, uint32_t v) {
 // INT32 -> FP32, round to nearest even, without the conversion instruction:  v = hi * 65536 + lo, both halves are converted exactly by the
 // 1.5 * 2^23 magic-number add, and the single rounding of the fused multiply-add equals cvt.rn.f32.s32(v).  The conversion instruction
 // is faster (2.5 cycles per warp instruction measured, against 5 x ~2 for this sequence; decode step 2.797 -> 2.771 ms, prefill tiles +2 %), so the
-// kernels convert with it; this stays as the -DQS_DECODE_CVT=0 / -DQS_PAIR_CVT=0 variant.
+// kernels convert with it; this stays as the -DQS_DECODE_CVT=0 / -DQS_PAIR_CVT=0 variant (of whole chunks of group scales in pairs there is none: pair_finish).
 __device__ __forceinline__ float int2float_rn_noxu(int32_t v) {
   const int32_t hi = v >> 16, lo = v & 0xFFFF;
   const float fhi = __fsub_rn(__int_as_float(0x4B400000 + hi), 12582912.f);
@@ -1244,7 +1244,7 @@ int launch_gemm(const GemmArgs& a) {
   cfg.blockDim = dim3(kNumThreads);
   auto resident = [&](int split) {
     // (W8A8's 32-token tiles: two CTAs per SM, whatever the query says, which counts one: 16 tiles 5.6 us by 8 and 6.5 by 4)
-    if (MODE == kModeW8 && C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return sms / split;
+    if (C::kSmemBytesSplit <= 113 * 1024 && C::kTmemCols <= 256) return sms / split;
     static std::atomic<int> held[2][kMaxDevices][4] = {};  // per (instantiation, device, split), as the attribute above; 0: not asked yet
     std::atomic<int>& h = held[a.acc_out ? 1 : 0][dev][split == 2 ? 1 : split == 4 ? 2 : 3];
     int n = h.load(std::memory_order_relaxed);
@@ -1308,17 +1308,18 @@ int pair_tokens(int M, int N, int K, int mode) {
 }
 
 // Whether CTA pairs are faster than the 128-token tiles of gemm_kernel.  A pair stages half of its tokens per SM and walks its tiles in one ring, so it wins
-// wherever the other kernel has one CTA per SM and no split over K (us, other kernel / pairs): per channel 12288 x 4096 at 65 to 128 tokens 17 / 13,
-// 4096 x 14336 at 257 41 / 28, 6144 x 4096 at 200 16.9 / 12.4; group scales 22 / 15, 60 / 40, 22.3 / 14.9; W8A8 at 128 16.5 / 15.3, at 257 37.7 / 32.2.
-// It does not
-//  - where gemm_kernel can split K over clusters, unless K is too short for that: below 512 tokens 4096 x 1024 at 140 7.2 / 6.6, 4096 x 2048 8.5 / 8.3,
-//    1024 x 1024 at 257 (split 4) 6.2 / 6.3; from 512 tokens on the pairs' tiles are full: 2048 x 4096 at 512 11.0 / 10.9, x 8192 15.8 / 17.1, 1024 x 1024
-//    at 512 (split 4) 6.6 / 5.9, x 2048 7.1 / 7.8 (W8A8 x 4096 at 600 11.7 / 12.7);
-//  - W4A8 with two CTAs per SM (at most 2 x SMs tiles) where the pairs take a second round: 12288 x 4096 at 300 19.2 / 21.1, 4096 x 4096 at 1100 18.2 / 20.2
-//    (at 400, 384 tiles, 33.4 / 22.5).  W8A8's tiles run one per SM there: 24.3 / 22.0;
-//  - calls of a few us, whose set-up counts: group scales with 512 K 12288 at 140 7.6 / 7.8, with 1024 K at 80 7.8 / 8.2, per channel with 512 K 18688 at 200
-//    8.3 / 9.3, W8A8 with 1024 K 6144 at 200 7.1 / 7.2, 9728 at 65 with 2048 K 10.1 / 10.2.  An even number of 128-token tiles on two CTAs per SM and more is no
-//    such call: per channel 512 K 28672 at 256 14.0 / 11.2, 1024 K 12288 at 448 14.9 / 11.7, group scales 640 K 9728 at 448 13.9 / 11.0.
+// wherever the other kernel has one CTA per SM and no split over K (us a call, back to back in a graph, other kernel / pairs): per channel 12288 x 4096 at 65 to
+// 128 tokens 15 / 11, 4096 x 14336 at 257 37 / 26, 6144 x 4096 at 200 15.1 / 10.8; group scales 17.5 / 12.5, 48 / 34, 17.4 / 12.2; W8A8 at 128 13.7 / 13.9, at 257
+// 34.7 / 30.7.  It does not
+//  - where gemm_kernel can split K over clusters, unless K is too short for that: below 512 tokens 4096 x 1024 at 140 6.7 / 5.3, 4096 x 2048 7.7 / 6.8,
+//    1024 x 1024 at 257 (split 4) 5.8 / 5.2; from 512 tokens on the pairs' tiles are full: 2048 x 4096 at 512 9.5 / 9.9, x 8192 12.5 / 15.8, 1024 x 1024
+//    at 512 (split 4) 6.3 / 5.3, x 2048 6.7 / 6.8 (W8A8 x 4096 at 600 9.3 / 10.6);
+//  - W4A8 with two CTAs per SM (at most 2 x SMs tiles) where the pairs take a second round: 12288 x 4096 at 300 17.6 / 19.4, 4096 x 4096 at 1100 19.0 / 20.6, group
+//    scales 21.6 / 25.3 and 21.3 / 24.5 (at 400, 384 tiles, 32.2 / 21.8).  W8A8's tiles run one per SM there: 21.7 / 22.0 and 22.5 / 21.7;
+//  - calls of a few us, whose set-up counts: per channel with 512 K 18688 at 200 7.5 / 8.0, W8A8 with 1024 K 6144 at 200 6.1 / 6.3, 9728 at 65 with 2048 K 8.7 / 8.9;
+//    group scales keep to the line too, though pairs have become the faster there (512 K 12288 at 140 7.6 / 6.8, 1024 K at 80 7.3 / 6.6).  An even number of 128-token
+//    tiles on two CTAs per SM and more is no such call: per channel 512 K 28672 at 256 13.8 / 10.7, 1024 K 12288 at 448 14.8 / 11.6, group scales 640 K 9728 at 448
+//    13.5 / 9.4.
 bool pairs_pay(int M, int N, int K, int mode) {
   if (M <= 64 || (N / kBM) % 2 != 0 || K < 512) return false;
   const bool w8 = mode == kModeW8;
