@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Capture golden vectors from the UNMODIFIED reference CUDA kernels (oracle/_ref, built by oracle/build_ref.py for
-sm_100a) on a B200:  python tests/golden/make_golden_ref_gpu.py
+sm_100a) on a B200:  python tests/golden/make_golden_ref_gpu.py [folder]
 The files it writes are then committed under tests/golden/ref_*.npz and pin the CPU oracle
 (tests/test_oracle_vs_reference_golden.py).  Inputs are seeded; every output of the reference kernels is stored."""
 import os
@@ -14,7 +14,7 @@ sys.path.insert(0, ROOT)
 from oracle import kv, ops, w4a8  # noqa: E402
 from tests import refmods  # noqa: E402
 
-OUT = os.path.join(ROOT, "gpurun_out", "golden_ref")
+OUT = sys.argv[1] if len(sys.argv) > 1 else os.path.join(ROOT, "build", "golden_ref")
 os.makedirs(OUT, exist_ok=True)
 dev = torch.device("cuda:0")
 t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)

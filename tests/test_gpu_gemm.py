@@ -11,7 +11,7 @@ from oracle import ops, w4a8
 from tests.util import bits16, np_of, to_dev, ulp16_diff
 
 pytestmark = pytest.mark.gpu
-OUT = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out")
+OUT = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "build", "diag")  # (ignored by git)
 
 
 def _acts(rng, M, K):
