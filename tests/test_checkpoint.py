@@ -121,7 +121,7 @@ def test_convert_and_fuse_tensor_parallel_shards_reassemble(group):
 
 
 def test_w4a8_loader_skips_norm_tensors_w8a8_loads_them():
-    """a W4A8 checkpoint with NON-unit norm tensors must not get gamma applied twice -- the reference's W4A8 loader
+    """A W4A8 checkpoint with NON-unit norm tensors must not get gamma applied twice -- the reference's W4A8 loader
     skips every tensor whose name contains 'norm' (gamma stays 1, LMQuant folded it into the next linear); the W8A8 loader keeps them."""
     H = 128
     sd = {"model.layers.0.input_layernorm.weight": torch.full((H,), 3.0), "model.layers.0.post_attention_layernorm.weight": torch.full((H,), 5.0),

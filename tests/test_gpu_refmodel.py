@@ -1,5 +1,5 @@
-"""The reference's UNMODIFIED Python model code running over this repo's `qserve_backend` (VERDICT r1 row b2,
-north_star: "so qserve/modeling ... drop in unchanged").
+"""The reference's UNMODIFIED Python model code running over this repo's `qserve_backend`, into which it drops
+unchanged.
 
 `qserve_b200.refmodel.RefModel` imports `qserve.modeling.models.llama_w4a8_unpad.LlamaForCausalLM` (and with it the
 reference's W4A8 linear / RMSNormGeneral / SiluAndMulQuant / InputMetadata / ActivationBuffer classes) from the

@@ -1,13 +1,12 @@
-"""DIRECT comparison of this repo's CUDA kernels with the reference's kernels (the r1 chain was only
-CUDA == oracle and oracle ~ reference).
+"""DIRECT comparison of this repo's CUDA kernels with the reference's kernels (elsewhere the chain is CUDA == oracle
+and oracle ~ reference).
 
-Part 1 (always runs on the GPU box): the committed golden vectors `tests/golden/ref_*.npz` hold inputs AND outputs of the
+Part 1 (runs wherever there is a GPU): the committed golden vectors `tests/golden/ref_*.npz` hold inputs AND outputs of the
 UNMODIFIED reference CUDA kernels run on a B200; our kernels are fed the same inputs through the C ABI and must reproduce the
 outputs within the bars of tests/test_oracle_vs_reference_golden.py (the reference is built with --use_fast_math: approximate
 division / sin / cos and FMA contraction move a result by at most one rounding step).
 
-Part 2 (runs when oracle/_ref/*.so are present: they are built from /root/reference by oracle/build_ref.py and travel to the
-GPU box): the reference extensions are loaded LIVE next to ours and both run on the same seeded inputs at the BASELINE config
+Part 2 (runs when oracle/_ref/*.so are present: oracle/build_ref.py builds them from the reference's sources): the reference extensions are loaded LIVE next to ours and both run on the same seeded inputs at the BASELINE config
 shapes (config 2: Llama-3-8B M=64 per-channel; config 3: g128; config 4: W8A8 M=128; config-2 attention B=64 ctx=1024).
 """
 import os
@@ -289,7 +288,7 @@ def test_live_norm_quant_silu_at_model_width(dev):
 
 
 def test_lengths_none_matches_reference_semantics(dev):
-    """with length_per_sample = None the reference uses tlength = timestep (Template.hpp:901), i.e. the cache holds
+    """With length_per_sample = None the reference uses tlength = timestep (Template.hpp:901), i.e. the cache holds
     `timestep` tokens and the new token lands in slot `timestep`.  Must equal the call with lengths = timestep + 1."""
     qb = _qb()
     from qserve_b200.decode import DecodeRunner
