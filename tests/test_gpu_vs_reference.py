@@ -6,8 +6,9 @@ UNMODIFIED reference CUDA kernels run on a B200; our kernels are fed the same in
 outputs within the bars of tests/test_oracle_vs_reference_golden.py (the reference is built with --use_fast_math: approximate
 division / sin / cos and FMA contraction move a result by at most one rounding step).
 
-Part 2 (runs when oracle/_ref/*.so are present: oracle/build_ref.py builds them from the reference's sources): the reference extensions are loaded LIVE next to ours and both run on the same seeded inputs at the BASELINE config
-shapes (config 2: Llama-3-8B M=64 per-channel; config 3: g128; config 4: W8A8 M=128; config-2 attention B=64 ctx=1024).
+Part 2 (runs when oracle/_ref/*.so are present: oracle/build_ref.py builds them from the reference's sources): the reference
+extensions are loaded LIVE next to ours and both run on the same seeded inputs at the BASELINE config shapes (config 2:
+Llama-3-8B M=64 per-channel; config 3: g128; config 4: W8A8 M=128; config-2 attention B=64 ctx=1024).
 """
 import os
 
